@@ -1090,64 +1090,107 @@ __global__ void __launch_bounds__(256) k_diag_final(const double* part, int nblo
 // ---------------------------------------------------------------------------
 // scalar transport, buoyancy and momentum forcing
 
-// Plane means (FP64, Neumaier) of up to six fields on levels k0..k0 +
-// gridDim.x - 1: one block per level, out[f * L + k].  Fixed reduction order
-// (per thread, then threads in order), so repeated runs give the same bits.
+// Compensated FP64 sums of up to six fields over each level: the reduction of
+// the plane means, the dynamic Prandtl coefficient and the plane-averaged
+// dynamic Smagorinsky coefficient.  grid (nch, levels, fields): a block sums
+// one of the nch chunks of a level (256 threads, four consecutive points per
+// iteration where the plane allows) and writes the pair (sum, compensation)
+// to part[((f levels + level) nch + chunk) 2].  Every addition is compensated
+// and every combination runs in a fixed order (thread, shuffle tree, warps,
+// then chunks in k_sums_*), so repeated runs give the same bits.
+// Bound by HBM once the chip is full: with one block per level (nch = 1) the
+// 96 levels of a 512 x 512 grid left 52 of 148 SMs without work and ran at
+// 400 GB/s (three fields: 753 us); chunks that give ~8 blocks per SM run at
+// 4.1 TB/s (73 us).
 template <typename T>
-__global__ void k_plane_means(const T* f0, const T* f1, const T* f2, const T* f3, int nf, double* out, long plane,
-                              int k0, int L, const T* f4 = nullptr, const T* f5 = nullptr) {
-  const int k = k0 + blockIdx.x;
-  const T* fs[6] = {f0, f1, f2, f3, f4, f5};
-  __shared__ double sh[6][2][256];
-  for (int f = 0; f < nf; ++f) {
-    Neu a;
-    const T* x = fs[f] + (long)k * plane;
-    for (long p = threadIdx.x; p < plane; p += blockDim.x) a.add(double(x[p]));
-    sh[f][0][threadIdx.x] = a.s;
-    sh[f][1][threadIdx.x] = a.c;
-  }
-  __syncthreads();
-  if (threadIdx.x < nf) {
-    const int f = threadIdx.x;
-    Neu t;
-    for (int i = 0; i < blockDim.x; ++i) {
-      t.add(sh[f][0][i]);
-      t.add(sh[f][1][i]);
+struct PlaneSumIn {
+  const T* f[6];
+};
+template <typename T>
+__global__ void __launch_bounds__(256) k_plane_sums(const PlaneSumIn<T> in, double* part, long plane, int k0,
+                                                    long chunk) {
+  const int k = k0 + blockIdx.y;
+  const T* x = in.f[blockIdx.z] + (long)k * plane;
+  const long q0 = blockIdx.x * chunk, q1 = min(plane, q0 + chunk);
+  Neu a;
+  if (plane % 4 == 0) {  // chunks are multiples of four points
+    for (long q = q0 + 4 * threadIdx.x; q < q1; q += 4 * 256) {
+      T v[4];
+      ld4(x + q, v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a.add(double(v[i]));
     }
-    out[f * L + k] = t.val() / double(plane);
+  } else {
+    for (long q = q0 + threadIdx.x; q < q1; q += 256) a.add(double(x[q]));
   }
-}
-
-// Plane-averaged least-squares coefficient per level k = 1..nz+1 (one block
-// per level): kapd[k] = max(0, <KX> / <XX>) * scale (FP64 Neumaier sums; 0
-// where <XX> = 0), the reduction of compute_DynSmag.f90:61-245 written to a
-// per-level array.
-template <typename T>
-__global__ void k_level_ratio(const T* KX, const T* XX, double* kapd, long plane, double scale) {
-  const int k = blockIdx.x + 1;
-  __shared__ double sh[4][256];
-  Neu a, b;
-  for (long p = threadIdx.x; p < plane; p += blockDim.x) {
-    a.add(double(KX[(long)k * plane + p]));
-    b.add(double(XX[(long)k * plane + p]));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    Neu o;
+    o.s = __shfl_down_sync(0xffffffffu, a.s, off);
+    o.c = __shfl_down_sync(0xffffffffu, a.c, off);
+    a.merge(o);
   }
-  sh[0][threadIdx.x] = a.s;
-  sh[1][threadIdx.x] = a.c;
-  sh[2][threadIdx.x] = b.s;
-  sh[3][threadIdx.x] = b.c;
+  __shared__ double sh[8][2];
+  if ((threadIdx.x & 31) == 0) {
+    sh[threadIdx.x >> 5][0] = a.s;
+    sh[threadIdx.x >> 5][1] = a.c;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    Neu x, y;
-    for (int i = 0; i < blockDim.x; ++i) {
-      x.add(sh[0][i]);
-      x.add(sh[1][i]);
-      y.add(sh[2][i]);
-      y.add(sh[3][i]);
+    for (int w = 1; w < 8; ++w) {
+      Neu o;
+      o.s = sh[w][0];
+      o.c = sh[w][1];
+      a.merge(o);
     }
-    const double num = x.val() / double(plane), den = y.val() / double(plane);
-    const double c = (den != 0.0) ? num / den : 0.0;
-    kapd[k] = fmax(0.0, c) * scale;
+    double* r = part + (((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 2;
+    r[0] = a.s;
+    r[1] = a.c;
   }
+}
+// the nch chunks of field f, level index i, in order
+__device__ __forceinline__ double plane_sum_of(const double* part, int f, int i, int nlev, int nch) {
+  Neu t;
+  const double* r = part + ((long)f * nlev + i) * nch * 2;
+  for (int c = 0; c < nch; ++c) {
+    Neu o;
+    o.s = r[2 * c];
+    o.c = r[2 * c + 1];
+    t.merge(o);
+  }
+  return t.val();
+}
+// plane means out[f L + k], k = k0 .. k0 + nlev - 1
+__global__ void k_sums_mean(const double* part, double* out, int nf, int nlev, int nch, long plane, int k0, int L) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < nf * nlev) out[(q / nlev) * L + k0 + q % nlev] = plane_sum_of(part, q / nlev, q % nlev, nlev, nch) / double(plane);
+}
+// <f0> / <f1> of a level, not below zero; 0 where <f1> = 0
+__device__ __forceinline__ double level_ratio(const double* part, int i, int nlev, int nch, long plane) {
+  const double num = plane_sum_of(part, 0, i, nlev, nch) / double(plane);
+  const double den = plane_sum_of(part, 1, i, nlev, nch) / double(plane);
+  return fmax(0.0, (den != 0.0) ? num / den : 0.0);
+}
+// Plane-averaged least-squares coefficient per level k = 1..nlev: kapd[k] =
+// max(0, <KX> / <XX>) * scale, the reduction of compute_DynSmag.f90:61-245
+// written to a per-level array.
+__global__ void k_sums_ratio(const double* part, double* kapd, int nlev, int nch, long plane, double scale) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nlev) kapd[1 + i] = level_ratio(part, i, nlev, nch, plane) * scale;
+}
+// the same spread over the level's points (plane-averaged dynamic
+// Smagorinsky): grid (blocks per level, nlev)
+template <typename T>
+__global__ void k_sums_spread(const double* part, T* cs, int nlev, int nch, long plane, double cs_max) {
+  __shared__ double res;
+  if (threadIdx.x == 0) {
+    res = level_ratio(part, blockIdx.y, nlev, nch, plane);
+    if (cs_max > 0.0) res = fmin(res, cs_max);  // optional upper clip (off: the reference)
+  }
+  __syncthreads();
+  const T v = T(res);
+  T* c = cs + (long)(1 + blockIdx.y) * plane;
+  for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) c[p] = v;
 }
 
 // Wall value of d theta/dz (level 1): the log law of the prescribed surface

@@ -14,6 +14,7 @@
 #include "stats.cuh"
 #include "mlp.cuh"
 #include <algorithm>
+#include <initializer_list>
 #include <random>
 #include "launch.cuh"
 #include "solver.cuh"
@@ -295,6 +296,30 @@ class Solver final : public SolverBase {
   }
   void fill_plane(T* f, T v) {
     KL("k_fill", double(g.plane()) * sizeof(T), k_fill<T><<<grid_for(g.plane()), 256, 0, st>>>(f, g.plane(), v));
+  }
+
+  // Compensated FP64 sums of each of levels k0 .. k0 + nlev - 1 of up to six
+  // fields, in nch chunks per level (returned) into psum.  Chunks: ~8 blocks
+  // per SM over the whole launch, none below 2048 points (eight points per
+  // thread, under which a block is all reduction).
+  double* psum = nullptr;
+  static constexpr int PSUM_CHUNKS = 128;
+  int plane_sums(std::initializer_list<const T*> f, int k0, int nlev) {
+    if (!psum) psum = track(dalloc<double>((long)6 * g.L * PSUM_CHUNKS * 2));
+    PlaneSumIn<T> in{};
+    int nf = 0;
+    for (const T* x : f) in.f[nf++] = x;
+    const long want = ceil_div(148L * 8, (long)nf * nlev);
+    const int nch = int(std::max(1L, std::min({want, g.plane() / 2048, (long)PSUM_CHUNKS})));
+    const long chunk = (long)ceil_div(ceil_div(g.plane(), nch), 4) * 4;
+    KL("k_plane_sums", double(nf) * nlev * g.plane() * sizeof(T),
+       k_plane_sums<T><<<dim3(unsigned(nch), unsigned(nlev), unsigned(nf)), 256, 0, st>>>(in, psum, g.plane(), k0, chunk));
+    return nch;
+  }
+  void plane_means(std::initializer_list<const T*> f, int k0, int nlev, double* out) {
+    const int nch = plane_sums(f, k0, nlev), nf = int(f.size());
+    KL("k_sums_mean", 16.0 * nf * nlev * nch,
+       k_sums_mean<<<ceil_div((long)nf * nlev, 64), 64, 0, st>>>(psum, out, nf, nlev, nch, g.plane(), k0, g.L));
   }
 
   // row pitch of the spectral buffers: whole 8-value groups (64 B in FP32),
@@ -1629,9 +1654,7 @@ class Solver final : public SolverBase {
     // rhs_z carries the mean vertical pressure gradient (thousands at the
     // wall), which an FP32 transform would round
     if (!means) means = track(dalloc<double>(6 * g.L));
-    KL("k_plane_means", 5.0 * nz * g.plane() * sizeof(T),
-       k_plane_means<T><<<nz, 256, 0, st>>>(F[LES_RHSZ], F[LES_RHSZ_F], F[LES_DUDX], F[LES_DVDY], 5, means, g.plane(), 1,
-                                            g.L, F[LES_DWDZ]));
+    plane_means({F[LES_RHSZ], F[LES_RHSZ_F], F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ]}, 1, nz, means);
     dim3 tg(ceil_div(g.lhx, 64), g.ny);
     KL("k_tridiag", (4.0 * 2 * sizeof(T) + 2 * sizeof(T) + 24.0) * double(g.L) * g.ny * g.lhx,
        k_tridiag<T, T, true><<<tg, 64, 0, st>>>(spec[2], spec[3], spec[4], spec[5], bot, top, kkxd, kkyd, spec[0], xs, gam,
@@ -1991,8 +2014,9 @@ class Solver final : public SolverBase {
     z.out[0] = sc[7];
     z.out[1] = sc[8];
     launch_xinv<T>(g.nx, z, st);
-    KL("k_level_ratio", 2.0 * n1 * sizeof(T),
-       k_level_ratio<T><<<nlev, 256, 0, st>>>(sc[7], sc[8], kapd, g.plane(), delta * delta));
+    const int nch = plane_sums({sc[7], sc[8]}, 1, nlev);
+    KL("k_sums_ratio", 32.0 * nlev * nch, k_sums_ratio<<<ceil_div(nlev, 64), 64, 0, st>>>(psum, kapd, nlev, nch, g.plane(),
+                                                                                   delta * delta));
   }
 
   // scalar convective term into rhs_t (levels 1..nz); the padded -u, -v, -w
@@ -2067,8 +2091,7 @@ class Solver final : public SolverBase {
     if (coriol != 0.0 || sponge_frac > 0.0) {
       Tag tag_(this, "forcing");
       if (sponge_frac > 0.0)
-        KL("k_plane_means", 3.0 * g.nz * g.plane() * sizeof(T),
-           k_plane_means<T><<<g.nz, 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], nullptr, 3, means, g.plane(), 1, L));
+        plane_means({F[LES_U], F[LES_V], F[LES_W]}, 1, g.nz, means);
       KL("k_forcing", 7.0 * g.nz * g.plane() * sizeof(T),
          k_forcing<T><<<grid_for((long)g.nz * g.plane()), 256, 0, st>>>(
              F[LES_RHSX], F[LES_RHSY], F[LES_RHSZ], F[LES_U], F[LES_V], F[LES_W], means,
@@ -2089,8 +2112,7 @@ class Solver final : public SolverBase {
     }
     if (SP.buoyancy != 0.0) {
       Tag tag_(this, "scalar");
-      KL("k_plane_means", double(L) * g.plane() * sizeof(T),
-         k_plane_means<T><<<L, 256, 0, st>>>(F[LES_THETA], nullptr, nullptr, nullptr, 1, means + 3 * L, g.plane(), 0, L));
+      plane_means({F[LES_THETA]}, 0, L, means + 3 * L);
       KL("k_buoyancy", 3.0 * (g.nz - 1) * g.plane() * sizeof(T),
          k_buoyancy<T><<<grid_for((long)(g.nz - 1) * g.plane()), 256, 0, st>>>(F[LES_RHSZ], F[LES_THETA], means + 3 * L,
                                                                                g.plane(), g.nz, T(SP.buoyancy)));
@@ -2325,39 +2347,6 @@ void Solver<T>::wall_plain() {
 
 // plane-averaged dynamic Smagorinsky (compute_DynSmag.f90:61-245)
 template <typename T>
-__global__ void k_plane_ratio(const T* LM, const T* MM, T* cs, long plane, int nz, double cs_max) {
-  // one block per level k = 1..nz+1; Neumaier sums in FP64
-  const int k = blockIdx.x + 1;
-  __shared__ double s[4][256];
-  Neu a, b;
-  for (long p = threadIdx.x; p < plane; p += blockDim.x) {
-    a.add(double(LM[(long)k * plane + p]));
-    b.add(double(MM[(long)k * plane + p]));
-  }
-  s[0][threadIdx.x] = a.s;
-  s[1][threadIdx.x] = a.c;
-  s[2][threadIdx.x] = b.s;
-  s[3][threadIdx.x] = b.c;
-  __syncthreads();
-  __shared__ double res;
-  if (threadIdx.x == 0) {
-    Neu x, y;
-    for (int i = 0; i < blockDim.x; ++i) {
-      x.add(s[0][i]);
-      x.add(s[1][i]);
-      y.add(s[2][i]);
-      y.add(s[3][i]);
-    }
-    const double num = x.val() / double(plane), den = y.val() / double(plane);
-    double c = (den != 0.0) ? num / den : 0.0;
-    res = fmax(0.0, c);
-    if (cs_max > 0.0) res = fmin(res, cs_max);  // optional upper clip (off: the reference)
-  }
-  __syncthreads();
-  for (long p = threadIdx.x; p < plane; p += blockDim.x) cs[(long)k * plane + p] = T(res);
-}
-
-template <typename T>
 void Solver<T>::dynsmag(SgsArgs<T>& a, int jt, int jtt) {
   if (jtt < P.dyn_init) {
     fill(F[LES_CS_OPT2], 1, g.nz + 1, T(0.03));
@@ -2365,7 +2354,10 @@ void Solver<T>::dynsmag(SgsArgs<T>& a, int jt, int jtt) {
   }
   if (jt % P.cs_count != 0) return;
   dynamic_mum(a, false);
-  KL("k_plane_ratio", 3.0 * (g.nz + 1) * g.plane() * sizeof(T), k_plane_ratio<T><<<g.nz + 1, 256, 0, st>>>(sc[7], sc[8], F[LES_CS_OPT2], g.plane(), g.nz, cs2_max));
+  const int nlev = g.nz + 1, nch = plane_sums({sc[7], sc[8]}, 1, nlev);
+  KL("k_sums_spread", double(nlev) * g.plane() * sizeof(T),
+     k_sums_spread<T><<<dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256), 32)), unsigned(nlev)), 256, 0, st>>>(
+         psum, F[LES_CS_OPT2], nlev, nch, g.plane(), cs2_max));
 }
 
 std::string SolverBase::profile_report() {
