@@ -1472,6 +1472,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       }
       continue;
     }
+    if (a.op == XI_WALL) continue;  // below, one point per thread
 #pragma unroll 1
     for (int q4 = 0; q4 < 4; ++q4) {
     const int i = i0 + q4;
@@ -1530,33 +1531,40 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         a.out[1][off] = x1 * x1 + x2 * x2 + x3 * x3;
         break;
       }
-      case XI_WALL: {
-        // compute_wall_law.f90:143-183, 247-251 on the filtered first level.
-        // c0 = dz, c1 = 1/log-free constant unused; aux[0] = z0 plane.
-        // out: u_star_avg, lbc_u, lbc_v, txz(1), tyz(1), dudz(1), dvdz(1)
-        const long p2 = (long)j * NX + i;
-        const double u1 = double(x[0]), v1 = double(x[XS]);
-        const double uavg = sqrt(u1 * u1 + v1 * v1);
-        const double dz = a.c0;
-        const double ustar = KVONK * uavg / log((0.5 * dz) / double(a.aux[0][p2]));
-        double bu = 0.0, bv = 0.0, tx = 0.0, ty = 0.0;
-        if (uavg != 0.0) {
-          bu = ustar / (0.5 * dz * KVONK) * u1 / uavg;
-          bv = ustar / (0.5 * dz * KVONK) * v1 / uavg;
-          tx = (ustar * ustar) * u1 / uavg;
-          ty = (ustar * ustar) * v1 / uavg;
-        }
-        a.out[0][p2] = T(ustar);
-        a.out[1][p2] = T(bu);
-        a.out[2][p2] = T(bv);
-        const long o1 = a.out_pstride + p2;  // level 1 of a field
-        a.out[3][o1] = T(tx);
-        a.out[4][o1] = T(ty);
-        a.out[5][o1] = T(bu);
-        a.out[6][o1] = T(bv);
-        break;
-      }
     }
+    }
+  }
+  if (a.op == XI_WALL) {
+    // compute_wall_law.f90:143-183, 247-251 on the filtered first level, one
+    // point per thread (a plane is few rows, and the FP64 logarithm and
+    // divisions of a point are a long dependent chain): c0 = dz, aux[0] = z0
+    // plane; out: u_star_avg, lbc_u, lbc_v, txz(1), tyz(1), dudz(1), dvdz(1)
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < a.R * NX; idx += blockDim.x) {
+      const int r = idx / NX;
+      const int i = idx - r * NX;
+      if (rowl[r] < 0) continue;
+      const long p2 = (long)rowj[r] * NX + i;
+      const T* x = xs + (long)(r * a.nin) * XS + i;
+      const double u1 = double(x[0]), v1 = double(x[XS]);
+      const double uavg = sqrt(u1 * u1 + v1 * v1);
+      const double dz = a.c0;
+      const double ustar = KVONK * uavg / log((0.5 * dz) / double(a.aux[0][p2]));
+      double bu = 0.0, bv = 0.0, tx = 0.0, ty = 0.0;
+      if (uavg != 0.0) {
+        bu = ustar / (0.5 * dz * KVONK) * u1 / uavg;
+        bv = ustar / (0.5 * dz * KVONK) * v1 / uavg;
+        tx = (ustar * ustar) * u1 / uavg;
+        ty = (ustar * ustar) * v1 / uavg;
+      }
+      a.out[0][p2] = T(ustar);
+      a.out[1][p2] = T(bu);
+      a.out[2][p2] = T(bv);
+      const long o1 = a.out_pstride + p2;  // level 1 of a field
+      a.out[3][o1] = T(tx);
+      a.out[4][o1] = T(ty);
+      a.out[5][o1] = T(bu);
+      a.out[6][o1] = T(bv);
     }
   }
   }  // the combining ops

@@ -3,6 +3,7 @@
 // attributes of their kernels.  The kernels are instantiated and launched
 // in spectral_xfwd.cu, spectral_xinv.cu and spectral_ypass.cu.
 #include "spectral_launch.cuh"
+#include <atomic>
 #include <mutex>
 
 #include "launch.cuh"
@@ -10,6 +11,21 @@
 namespace les {
 
 thread_local LaunchHook* g_hook = nullptr;
+
+// SMs of the current device
+int sm_count() {
+  static std::atomic<int> count[256] = {};
+  int dev = 0;
+  LES_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 256) throw CudaError(1, "device ordinal out of range");
+  int n = count[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    LES_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    n = std::max(1, n);
+    count[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 
 // CTAs of `kern` resident on the current device at once; cached in a fixed
 // table (no heap allocation: the allocation-free entry point launches these
@@ -32,10 +48,9 @@ int resident_ctas(const void* kern, int threads, size_t smem) {
     const ResidentEntry& e = table[i];
     if (e.dev == dev && e.kern == kern && e.threads == threads && e.smem == smem) return e.n;
   }
-  int per_sm = 0, sms = 0;
+  int per_sm = 0;
   LES_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-  LES_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int n = std::max(1, per_sm) * std::max(1, sms);
+  const int n = std::max(1, per_sm) * sm_count();
   if (used < 256) table[used++] = ResidentEntry{dev, kern, threads, smem, n};
   return n;
 }

@@ -26,20 +26,32 @@ int pad_seqs(int nseq, int M);
 inline constexpr int SMEM_CAP = 200 * 1024;
 inline constexpr size_t SM_SMEM = 228 * 1024;  // shared memory per SM (1 KB of it reserved per CTA)
 
-// Rows per work item of an x pass (256-thread CTAs, TL lanes per sequence,
-// seq_per_row sequences per grid row): the count that keeps the most sequence
-// slots of an SM busy -- resident CTAs (shared memory, registers) times the
-// fraction of the 256 / TL slots of each pass that hold a sequence; on a tie
-// the larger count (fewer items).
+int sm_count();  // of the current device (cached)
+
+// Rows per work item of an x pass (TL lanes per sequence, seq_per_row
+// sequences per grid row, nrows rows in the launch): the count that keeps the
+// most sequence slots of an SM busy -- resident CTAs (shared memory,
+// registers) times the fraction of the slots of each pass that hold a
+// sequence; on a tie the larger count (fewer items).
+// A launch whose items at that count fill less than two rounds of resident
+// CTAs (a plane of the wall law, a small grid) is bound by the time of one
+// item, not by throughput: it takes the count with the fewest rounds of
+// passes, on a tie the fewest rows, so that its items spread over the chip
+// (the wall law's x inverse of a 256 x 256 plane in FP32: 32 CTAs became 256,
+// 35.5 -> 14.5 us; of 64 x 64: 20.8 -> 11.3 us).
 template <typename SmemFn>
-inline int best_rows(const void* kern, int seq_per_row, int TL, SmemFn smem_for, int rmax = 32, double* best_score = nullptr,
+inline int best_rows(const void* kern, int seq_per_row, int TL, SmemFn smem_for, long nrows, double* best_score = nullptr,
               int threads = 256) {
+  const int rmax = 32;
   const int regs = kernel_regs(kern);
   const int warp_regs = ((regs * 32 + 255) / 256) * 256;
   const int by_regs = std::max(1, 65536 / (warp_regs * (threads / 32)));
   const int S = threads / TL;
+  const long sms = sm_count();
   double best = -1.0;
-  int best_r = 1;
+  int best_r = 1, best_ctas = 1;
+  long few = -1;  // rounds of passes of the launch at few_r
+  int few_r = 1;
   for (int R = 1; R <= rmax; ++R) {
     const size_t sm = smem_for(R);
     if (sm > SMEM_CAP) break;
@@ -51,10 +63,17 @@ inline int best_rows(const void* kern, int seq_per_row, int TL, SmemFn smem_for,
     if (score >= best - 1e-9) {
       best = score;
       best_r = R;
+      best_ctas = ctas;
+    }
+    const long items = (nrows + R - 1) / R;
+    const long rounds = ((items + sms * ctas - 1) / (sms * ctas)) * passes;
+    if (few < 0 || rounds < few) {
+      few = rounds;
+      few_r = R;
     }
   }
   if (best_score) *best_score = best;
-  return best_r;
+  return (nrows + best_r - 1) / best_r < 2 * sms * best_ctas ? few_r : best_r;
 }
 
 

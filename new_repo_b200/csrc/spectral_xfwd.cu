@@ -44,7 +44,7 @@ static void launch_xfwd_st(int NX, XFArgs<T>& a, cudaStream_t st) {
     default:
       throw CudaError(1, "xfwd: unsupported transform length " + std::to_string(NX));
   }
-  a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for);
+  a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, a.nrows);
   const size_t smem = smem_for(a.R);
   if (smem > SMEM_CAP) throw CudaError(1, "xfwd: shared memory request too large");
   const long nitems = ceil_div(a.nrows, a.R);
@@ -98,7 +98,7 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   // the other ops keep 256 threads (the stress divergence measured slower
   // with 128: 0.236 -> 0.256 ms)
   const int XF_THREADS = (a.op == XF_CONV_IN || a.op == XF_PROD || a.op == XF_PROD_SC) ? 128 : 256;
-  a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, 32, nullptr, XF_THREADS);
+  a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, a.nrows, nullptr, XF_THREADS);
   const size_t smem = smem_for(a.R);
   if (smem > SMEM_CAP) throw CudaError(1, "xfwd: shared memory request too large");
   const int grid = ceil_div(a.nrows, a.R);

@@ -61,8 +61,8 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   // (more resident CTAs where shared memory limits them)
   {
     double s2 = -1.0, s1 = -1.0;
-    const int r2 = best_rows((const void*)kern, a.nin, lanes(M), [&](int R) { return smem_nb(R, 2); }, 32, &s2);
-    const int r1 = best_rows((const void*)kern, a.nin, lanes(M), [&](int R) { return smem_nb(R, 1); }, 32, &s1);
+    const int r2 = best_rows((const void*)kern, a.nin, lanes(M), [&](int R) { return smem_nb(R, 2); }, a.nrows, &s2);
+    const int r1 = best_rows((const void*)kern, a.nin, lanes(M), [&](int R) { return smem_nb(R, 1); }, a.nrows, &s1);
     a.nbuf = (s1 > s2 + 1e-9) ? 1 : 2;
     a.R = (a.nbuf == 1) ? r1 : r2;
   }

@@ -82,6 +82,13 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
           best_ns = ns;
         }
       }
+    // a launch of few columns (a plane of the wall law, a small grid): narrower
+    // items while they do not fill the chip, down to 32-byte row pieces (whole
+    // sectors) -- the time of an item hardly depends on its columns
+    const auto items = [&](int lc) { return (long)ceil_div(a.ncols, 1 << lc) * nplanes * ngroups; };
+    while (best_lc > 0 && items(best_lc) < sm_count() && (TL << (best_lc - 1)) >= 32 &&
+           (sizeof(cplx<T>) << (best_lc - 1)) >= 32)
+      --best_lc;
     a.lc = best_lc;
     a.nstage = best_ns;
   }
