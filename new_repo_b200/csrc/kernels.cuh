@@ -754,17 +754,143 @@ __global__ void k_p_finish(T* p, const double* pmean, long plane, int nz) {
 // ---------------------------------------------------------------------------
 // pressure: one Thomas solve per (kx, ky) (compute_pressure.f90:256-305,
 // 448-493, matrix of build_matrix :544-619), always in FP64.
-// O: type of the pressure spectrum written (FP32 in mixed precision, whose
-// inverse transforms run in FP32); its rows are opitch values apart
-// G (optional): a fourth spectrum added to the right-hand side of every
-// interior row (the divergence of u^n over dt tadv1 when Hx, Hy, Hz hold the
-// AB2 increment only; compiled in with INC).  pm (with G): FP64 plane means per level
-// (pm[f * pm_L + k]: f = 0 rz, 1 rfz, 2 dudx, 3 dvdy, 4 dwdz) from which
-// the kx = ky = 0 column forms its right-hand side,
+// The matrix depends on the grid alone, so its elimination runs once per
+// state: piv[k] = 1 / bet_k per level and column (ny x lhx, unpadded rows),
+// from which the sweep's factors follow as gam_{k+1} = c_k piv_k.  A zero
+// pivot leaves an infinite entry, which every solve checks
+// (compute_pressure.f90:411-418).  Multiplying by 1/bet and 1/dz where the
+// reference divides differs by rounding only (an ulp per operation).
+__global__ void k_tridiag_factor(double* __restrict__ piv, const double* __restrict__ kkx,
+                                 const double* __restrict__ kky, int lhx, int ny, int nz, double dz) {
+  const long sp = (long)ny * lhx;
+  const long col = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (col >= sp) return;
+  const bool mean = col == 0;
+  const double a_in = 1.0 / (dz * dz);
+  const double kxv = kkx[col], kyv = kky[col];
+  const double b_in = -((kxv * kxv + kyv * kyv) + 2.0 / (dz * dz));
+  double ib = mean ? 1.0 : -1.0;  // row 0: p1 - p0 = dz * bottom layer, or p0 = 0
+  double cprev = mean ? 0.0 : 1.0;
+  piv[col] = ib;
+  for (int k = 1; k <= nz; ++k) {
+    ib = 1.0 / (b_in - a_in * (cprev * ib));
+    piv[(long)k * sp + col] = ib;
+    cprev = a_in;
+  }
+  piv[(long)(nz + 1) * sp + col] = 1.0 / (1.0 - (-1.0) * (cprev * ib));  // row nz+1: p(nz+1) - p(nz)
+}
+
+// The solve: r (rows 0..nz+1 of every column: bottom layer, right-hand side,
+// top layer; ny x lhx complex, unpadded) -> p^ as O (FP32 in mixed precision,
+// rows opitch apart), overwriting r with the forward sweep's intermediate.
+// The real and the imaginary part of a column are separate systems of one
+// matrix: one thread each, on consecutive threads (33 K columns at 256^2 are
+// only ~7 warps per SM; two threads per column give ~14, and every access of
+// a warp is contiguous).  The levels are loaded in batches of TB, the next
+// batch's loads issued before the recurrence runs through the current one.
+// Bytes per complex value: 16 read + 16 written + 8 (pivots) down, 24 read
+// and p^ written up.
+template <typename O>
+__global__ void __launch_bounds__(128) k_tridiag(double* r, const double* __restrict__ piv, O* __restrict__ phat,
+                                                 double* pmean, unsigned* status, int lhx, int ny, int nz, double dz,
+                                                 int drop_mean, int opitch) {
+  const long sp = (long)ny * lhx;
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t >= 2 * sp) return;
+  const long col = t >> 1;
+  const int ky = udiv32(col, lhx), kx = int(col - (long)ky * lhx);
+  const long osp = 2L * ny * opitch;
+  O* out = phat + 2 * ((long)ky * opitch + kx) + (t & 1);
+  if (kx == lhx - 1 || ky == ny / 2) {
+    for (int l = 0; l <= nz + 1; ++l) out[l * osp] = O(0);
+    return;
+  }
+  const bool mean = col == 0;
+  const double a_in = 1.0 / (dz * dz);
+  double* rc = r + t;
+  const double* pc = piv + col;
+  const long rs = 2 * sp;
+  constexpr int TB = 8;
+  double x = mean ? 0.0 : rc[0] * dz * pc[0];
+  rc[0] = x;
+  bool bad = false;
+  double cr[TB], cp[TB];
+  auto load_fwd = [&](int k0, double* ar, double* ap) {
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      const int k = min(k0 + j, nz);
+      ar[j] = rc[k * rs];
+      ap[j] = pc[k * sp];
+    }
+  };
+  load_fwd(1, cr, cp);
+  for (int k0 = 1; k0 <= nz; k0 += TB) {
+    double nr[TB], np[TB];
+    load_fwd(k0 + TB, nr, np);
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      const int k = k0 + j;
+      if (k <= nz) {
+        x = (cr[j] - a_in * x) * cp[j];
+        bad |= isinf(cp[j]);
+        rc[k * rs] = x;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      cr[j] = nr[j];
+      cp[j] = np[j];
+    }
+  }
+  {  // top row: -p(nz) + p(nz+1) = dz * top layer
+    const double ib = pc[(nz + 1) * sp];
+    x = (rc[(nz + 1) * rs] * dz - (-1.0) * x) * ib;
+    bad |= isinf(ib);
+  }
+  if (bad) atomicOr(status, ST_PIVOT);
+  out[(nz + 1) * osp] = O(0);
+  // backward sweep, levels nz..0: x_k -= c_k piv_k x_{k+1}
+  auto load_bwd = [&](int k0, double* ar, double* ap) {
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      const int k = max(k0 - j, 0);
+      ar[j] = rc[k * rs];
+      ap[j] = pc[k * sp];
+    }
+  };
+  load_bwd(nz, cr, cp);
+  for (int k0 = nz; k0 >= 0; k0 -= TB) {
+    double nr[TB], np[TB];
+    load_bwd(k0 - TB, nr, np);
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      const int k = k0 - j;
+      if (k >= 0) {
+        const double ck = k > 0 ? a_in : (mean ? 0.0 : 1.0);
+        x = cr[j] - (ck * cp[j]) * x;
+        if (mean && pmean && t == 0) pmean[k] = x;
+        out[k * osp] = (mean && drop_mean) ? O(0) : O(x);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < TB; ++j) {
+      cr[j] = nr[j];
+      cp[j] = np[j];
+    }
+  }
+  if (t == 0 && pmean) pmean[nz + 1] = 0.0;
+}
+
+// The increment form of the right-hand side (les_press_from_increment): three
+// spectra and a fourth, G, added to the right-hand side of every interior row
+// (the divergence of u^n over dt tadv1 when Hx, Hy, Hz hold the AB2 increment
+// only); one thread per column, pivots formed in the sweep.  pm: FP64 plane
+// means per level (pm[f * pm_L + k]: f = 0 rz, 1 rfz, 2 dudx, 3 dvdy, 4 dwdz)
+// from which the kx = ky = 0 column forms its right-hand side,
 // (hz(k+1) - hz(k)) / dz + (dudx + dvdy + dwdz) idt with hz = rz + r21 rfz,
 // instead of the FP32 spectra's mean coefficients.
-template <typename T, typename O = T, bool INC = false>
-__global__ void k_tridiag(const cplx<T>* __restrict__ Hx, const cplx<T>* __restrict__ Hy,
+template <typename T, typename O = T>
+__global__ void k_tridiag_inc(const cplx<T>* __restrict__ Hx, const cplx<T>* __restrict__ Hy,
                           const cplx<T>* __restrict__ Hz, const cplx<T>* __restrict__ G,
                           const cplx<T>* __restrict__ bot,
                           const cplx<T>* __restrict__ top, const double* __restrict__ kkx,
@@ -821,7 +947,7 @@ __global__ void k_tridiag(const cplx<T>* __restrict__ Hx, const cplx<T>* __restr
       ax[j] = (k <= nz) ? Hx[o] : cplx<T>{T(0), T(0)};
       ay[j] = (k <= nz) ? Hy[o] : cplx<T>{T(0), T(0)};
       az[j] = (k < nz) ? Hz[o + isp] : cplx<T>{T(0), T(0)};
-      if constexpr (INC) agg[j] = (k <= nz) ? G[o] : cplx<T>{T(0), T(0)};
+      agg[j] = (k <= nz) ? G[o] : cplx<T>{T(0), T(0)};
     }
   };
   load_fwd(1, cx, cy, cz, cg);
@@ -837,11 +963,9 @@ __global__ void k_tridiag(const cplx<T>* __restrict__ Hx, const cplx<T>* __restr
         const double sx = kxv * double(hx.x) + kyv * double(hy.x);
         const double sy = kxv * double(hx.y) + kyv * double(hy.y);
         r = {-sy + (double(hzp.x) - double(hz.x)) * idz, sx + (double(hzp.y) - double(hz.y)) * idz};
-        if constexpr (INC) {
-          r.x += double(cg[j].x);
-          r.y += double(cg[j].y);
-        }
-        if (INC && mean) {
+        r.x += double(cg[j].x);
+        r.y += double(cg[j].y);
+        if (mean) {
           const double hk = pm[k] + pm_r21 * pm[pm_L + k];
           const double hkp = (k < nz) ? pm[k + 1] + pm_r21 * pm[pm_L + k + 1] : 0.0;
           r = {(hkp - hk) / dz + ((pm[2 * pm_L + k] + pm[3 * pm_L + k]) + pm[4 * pm_L + k]) * pm_idt, 0.0};
@@ -862,7 +986,7 @@ __global__ void k_tridiag(const cplx<T>* __restrict__ Hx, const cplx<T>* __restr
       cx[j] = nx_[j];
       cy[j] = ny_[j];
       cz[j] = nz_[j];
-      if constexpr (INC) cg[j] = ng_[j];
+      cg[j] = ng_[j];
     }
   }
   {  // top row: -p(nz) + p(nz+1) = dz * top layer
@@ -1286,39 +1410,32 @@ struct SlabRows {
 
 // row k of a column: coefficients (a, b, c) and the right-hand side
 template <typename T>
-__device__ __forceinline__ void tri_row(int k, int nz, bool mean, double a_in, double b_in, double dz, double kxv,
-                                        double kyv, const cplx<T>* Hx, const cplx<T>* Hy, const cplx<T>* Hz,
-                                        const cplx<T>* bot, const cplx<T>* top, long icol, long isp, double& a,
-                                        double& b, double& c, cplx<double>& r) {
+__device__ __forceinline__ void tri_row(int k, int nz, bool mean, double a_in, double b_in, double dz,
+                                        const cplx<T>* R, long icol, long isp, double& a, double& b, double& c,
+                                        cplx<double>& r) {
+  const cplx<T> v = R[(long)k * isp + icol];
   if (k == 0) {
     a = 0.0;
     b = mean ? 1.0 : -1.0;
     c = mean ? 0.0 : 1.0;
-    r = mean ? cplx<double>{0.0, 0.0} : cplx<double>{double(bot[icol].x) * dz, double(bot[icol].y) * dz};
+    r = mean ? cplx<double>{0.0, 0.0} : cplx<double>{double(v.x) * dz, double(v.y) * dz};
   } else if (k == nz + 1) {
     a = -1.0;
     b = 1.0;
     c = 0.0;
-    r = {double(top[icol].x) * dz, double(top[icol].y) * dz};
+    r = {double(v.x) * dz, double(v.y) * dz};
   } else {
     a = a_in;
     b = b_in;
     c = a_in;
-    const long o = (long)k * isp + icol;
-    const cplx<T> hx = Hx[o], hy = Hy[o], hz = Hz[o];
-    const cplx<T> hzp = (k < nz) ? Hz[o + isp] : cplx<T>{T(0), T(0)};
-    const double sx = kxv * double(hx.x) + kyv * double(hy.x);
-    const double sy = kxv * double(hx.y) + kyv * double(hy.y);
-    r = {-sy + (double(hzp.x) - double(hz.x)) / dz, sx + (double(hzp.y) - double(hz.y)) / dz};
+    r = {double(v.x), double(v.y)};
   }
 }
 
 // grid (ceil(lhx/64), ny, G), 64 threads: one (column, slab) per thread.
 // ys (complex), uu, vv: the slab's solutions at its rows; gam: scratch.
 template <typename T>
-__global__ void k_tri_slab_local(const cplx<T>* __restrict__ Hx, const cplx<T>* __restrict__ Hy,
-                                 const cplx<T>* __restrict__ Hz, const cplx<T>* __restrict__ bot,
-                                 const cplx<T>* __restrict__ top, const double* __restrict__ kkx,
+__global__ void k_tri_slab_local(const cplx<T>* __restrict__ R, const double* __restrict__ kkx,
                                  const double* __restrict__ kky, cplx<double>* __restrict__ ys,
                                  double* __restrict__ uu, double* __restrict__ vv, double* __restrict__ gam,
                                  unsigned* status, int lhx, int ny, int nz, double dz, int ipitch, SlabRows sr) {
@@ -1335,7 +1452,7 @@ __global__ void k_tri_slab_local(const cplx<T>* __restrict__ Hx, const cplx<T>* 
   const int s = sr.start(sb), e = sr.end(sb);
   double a, b, c;
   cplx<double> r;
-  tri_row<T>(s, nz, mean, a_in, b_in, dz, kxv, kyv, Hx, Hy, Hz, bot, top, icol, isp, a, b, c, r);
+  tri_row<T>(s, nz, mean, a_in, b_in, dz, R, icol, isp, a, b, c, r);
   double bet = b;
   bool bad = (bet == 0.0);
   cplx<double> y = {r.x / bet, r.y / bet};
@@ -1346,7 +1463,7 @@ __global__ void k_tri_slab_local(const cplx<T>* __restrict__ Hx, const cplx<T>* 
   uu[(long)s * sp + col] = u;
   vv[(long)s * sp + col] = v;
   for (int k = s + 1; k <= e; ++k) {
-    tri_row<T>(k, nz, mean, a_in, b_in, dz, kxv, kyv, Hx, Hy, Hz, bot, top, icol, isp, a, b, c, r);
+    tri_row<T>(k, nz, mean, a_in, b_in, dz, R, icol, isp, a, b, c, r);
     const double g = cprev / bet;
     bet = b - a * g;
     bad |= (bet == 0.0);

@@ -41,14 +41,6 @@ int grid_for(long n, int bs = 256) {
   return int(g);
 }
 
-template <typename T>
-T* dalloc(size_t n) {
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T) + 256);
-  if (e != cudaSuccess) throw CudaError(3, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  LES_CUDA(cudaMemset(p, 0, n * sizeof(T) + 256));
-  return reinterpret_cast<T*>(p);
-}
 }  // namespace
 
 // file names of the TKE budget profiles, in the order of the avg_var calls
@@ -80,11 +72,10 @@ class Solver final : public SolverBase {
   T* sc[15] = {};  // S, s11..s33, LM, MM, QN, NN, Fn x4
   T* refbuf[MAXIN] = {};  // per-level reference values (mixed precision)
   // FP64 spectral workspace of the pressure path in mixed precision
-  cplx<double>* pspec[8] = {};
+  cplx<double>* pspec[2] = {};
   std::map<int, cplx<double>*> twd;
   double *kkx64 = nullptr, *kky64 = nullptr;
-  cplx<double>* xs = nullptr;
-  double* gam = nullptr;
+  double* piv = nullptr;  // 1 / pivots of the pressure systems (k_tridiag_factor)
   double* pmean = nullptr;
   double* part = nullptr;
   double* dout = nullptr;
@@ -125,8 +116,9 @@ class Solver final : public SolverBase {
     for (auto& f : refbuf) f = track(dalloc<T>(g.L));
     if (mixed())
       for (auto& f : pspec) f = track(dalloc<cplx<double>>((long)g.L * g.ny * g.lhx));
-    xs = track(dalloc<cplx<double>>((long)g.L * g.ny * g.lhx));
-    gam = track(dalloc<double>((long)g.L * g.ny * g.lhx));
+    piv = track(dalloc<double>((long)g.L * g.ny * g.lhx));
+    k_tridiag_factor<<<ceil_div((long)g.ny * g.lhx, 64), 64, 0, st>>>(piv, kkxd, kkyd, g.lhx, g.ny, g.nz, dz());
+    LES_CHECK_LAUNCH();
     pmean = track(dalloc<double>(g.L));
     part = track(dalloc<double>(DIAG_BLOCKS * DIAG_NV));
     dout = track(dalloc<double>(8));
@@ -152,6 +144,16 @@ class Solver final : public SolverBase {
     if (st) cudaStreamDestroy(st);
   }
 
+  // zeroed device memory; the zeroing is ordered on the state's stream, which
+  // runs everything that uses it
+  template <typename U>
+  U* dalloc(size_t n) {
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, n * sizeof(U) + 256);
+    if (e != cudaSuccess) throw CudaError(3, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    LES_CUDA(cudaMemsetAsync(p, 0, n * sizeof(U) + 256, st));
+    return reinterpret_cast<U*>(p);
+  }
   template <typename U>
   U* track(U* q) {
     allocs.push_back(q);
@@ -234,13 +236,15 @@ class Solver final : public SolverBase {
       }
     }
     if (!l2) l2 = track(dalloc<double>(g.L));
-    LES_CUDA(cudaMemcpy(l2, l2h.data(), sizeof(double) * g.L, cudaMemcpyHostToDevice));
+    LES_CUDA(cudaMemcpyAsync(l2, l2h.data(), sizeof(double) * g.L, cudaMemcpyHostToDevice, st));
+    LES_CUDA(cudaStreamSynchronize(st));
   }
 
   template <typename U>
   U* up(const std::vector<U>& h) {
     U* d = track(dalloc<U>(h.size()));
-    LES_CUDA(cudaMemcpy(d, h.data(), sizeof(U) * h.size(), cudaMemcpyHostToDevice));
+    LES_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(U) * h.size(), cudaMemcpyHostToDevice, st));
+    LES_CUDA(cudaStreamSynchronize(st));
     return d;
   }
 
@@ -1411,23 +1415,6 @@ class Solver final : public SolverBase {
     return a;
   }
   template <typename S>
-  XIArgs<S> xi_s(int op, int nin, int plane0, int nplanes) {
-    XIArgs<S> a;
-    std::memset(&a, 0, sizeof(a));
-    a.op = op;
-    a.nin = nin;
-    a.plane0 = plane0;
-    a.rows_pp = g.ny;
-    a.nrows = (long)nplanes * g.ny;
-    a.nk = g.lhx;
-    a.nz = g.nz;
-    a.in_pstride = (long)g.ny * g.lhx;
-    a.out_pstride = (long)g.ny * g.nx;
-    a.tw = twiddles64(g.nx);
-    a.status = dstatus;
-    return a;
-  }
-  template <typename S>
   static void set_in(XFArgs<S>& a, int q, T* f) {
     if constexpr (std::is_same<T, float>::value && std::is_same<S, double>::value) {
       a.inf[q] = f;
@@ -1436,145 +1423,105 @@ class Solver final : public SolverBase {
       a.in[q] = reinterpret_cast<const S*>(f);
     }
   }
-  template <typename S>
-  static void set_out(XIArgs<S>& a, int q, T* f) {
-    if constexpr (std::is_same<T, float>::value && std::is_same<S, double>::value) {
-      a.outf[q] = f;
-      a.out_f32 = 1;
-    } else {
-      a.out[q] = reinterpret_cast<S*>(f);
-    }
-  }
-
   void press_stag_array(double tadv1) override {
     Tag tag_(this, "press");
-    press_tadv1_ = tadv1;
-    if (mixed()) press_impl<double>(pspec);
-    else press_impl<double>(reinterpret_cast<cplx<double>**>(spec));
+    if constexpr (std::is_same<T, float>::value) press_impl(tadv1, pspec[0], pspec[1]);
+    else press_impl(tadv1, spec[0], spec[1]);
   }
 
-  template <typename S>
-  void press_impl(cplx<S>** sp) {
-    const double tadv1 = press_tadv1_;
+  // Right-hand side in two FP64 spectra instead of three, and one after the y
+  // transform: the divergence is linear, so i kx u^ + (dw/dz)^ leaves the x
+  // pass as one spectrum and i ky v^ joins it in the y pass (compute_pressure.
+  // f90:176-190 transforms u, v, w and combines the three).  The two
+  // pressure-BC layers travel as one more plane of the same launches.  At
+  // 256^3 in mixed precision the x and y passes went from 0.296 + 0.327 to
+  // 0.311 + 0.202 ms per step with five launches fewer, and the solve, reading
+  // one spectrum instead of three, from 0.181 to 0.110 (FP64: 0.455 + 0.431 to
+  // 0.325 + 0.278, and 0.190 to 0.119).
+  void press_impl(double tadv1, cplx<double>* s0, cplx<double>* s1) {
+    using S = double;
     const int nz = g.nz;
     const double c = 1.0 / double(g.nx * g.ny);
-    // bottom/top layers (compute_pressure.f90:151-165, 196-203)
-    KL("k_scale", 2.0 * g.plane() * sizeof(T), k_scale<T><<<grid_for(g.plane()), 256, 0, st>>>(PL[LES_BOTTOM_WK_PRESS], g.plane(), T(c)));
-    cplx<S>* bot = sp[0];  // plane 0 of sp[0] / sp[1]
-    cplx<S>* top = sp[1];
-    {
-      auto a = xf_s<S>(XF_SCALE, 1, 0, 1, g.lhx);
-      a.c0 = 1.0;
-      set_in(a, 0, PL[LES_BOTTOM_WK_PRESS]);
-      a.out[0] = bot;
-      launch_xfwd<S>(g.nx, a, st);
-      a.c0 = c;
-      set_in(a, 0, PL[LES_TOP_WK_PRESS]);
-      a.out[0] = top;
-      launch_xfwd<S>(g.nx, a, st);
-      auto b = yp_s<S>(YP_FWDKILL, 1, 1, 0);
-      b.in[0] = bot;
-      b.out[0] = bot;
-      b.in[1] = top;
-      b.out[1] = top;
-      launch_ypass<S>(g.ny, g.ny, b, 1, 2, st);
-    }
-    // H = FFT(u / (dt tadv1 nx ny)), Nyquist killed (levels 1..nz)
-    auto a = xf_s<S>(XF_PRESS, 3, 1, nz, g.lhx);
+    auto a = xf_s<S>(XF_PRESS, 3, 1, nz + 1, g.lhx);
     a.c0 = c / tadv1;
     a.c1 = P.dt;
-    const int uvw[3] = {LES_U, LES_V, LES_W};
-    for (int q = 0; q < 3; ++q) {
-      set_in(a, q, F[uvw[q]]);
-      a.out[q] = sp[2 + q];
-    }
+    a.c2 = c;
+    a.c3 = 1.0 / dz();
+    a.kxr = kkxd;
+    T* const ins[5] = {F[LES_U], F[LES_V], F[LES_W], PL[LES_BOTTOM_WK_PRESS], PL[LES_TOP_WK_PRESS]};
+    for (int q = 0; q < 5; ++q) set_in(a, q, ins[q]);
+    a.out[0] = s0;
+    a.out[1] = s1;
     launch_xfwd<S>(g.nx, a, st);
-    auto b = yp_s<S>(YP_FWDKILL, 1, 1, 1);
-    for (int q = 0; q < 3; ++q) {
-      b.in[q] = sp[2 + q];
-      b.out[q] = sp[2 + q];
-    }
-    launch_ypass<S>(g.ny, g.ny, b, nz, 3, st);
-    // tridiagonal solve per (kx, ky) -> p^ in sp[5], levels 0..nz+1; in
-    // mixed precision the mean mode is kept apart in FP64 (pmean)
-    dim3 tg(ceil_div(g.lhx, 64), g.ny);
-    if constexpr (std::is_same<T, float>::value) {
-      // mixed precision: p^ leaves the FP64 solve as FP32 (its mean mode is
-      // kept apart in FP64); the inverse transforms of p run in FP32 -- only
-      // the forward right-hand side needs FP64, where div u* cancels
-      if (pslabs > 1)
-        slab_solve<S, T>(sp[2], sp[3], sp[4], bot, top, spec[0], pmean, 1, pitch(g.lhx), g.lhx);
-      else
-        KL("k_tridiag", 96.0 * double(g.L) * g.ny * g.lhx,
-           k_tridiag<S, T><<<tg, 64, 0, st>>>(sp[2], sp[3], sp[4], nullptr, bot, top, kkxd, kkyd, spec[0], xs, gam, pmean, dstatus,
-                                              g.lhx, g.ny, nz, dz(), 1, pitch(g.lhx), g.lhx));
-      auto e = yp(YP_PGRAD, 1, 3, g.lhx, g.lhx, g.ny, g.lhx, g.ny, 0);
-      e.in[0] = spec[0];
-      e.out[0] = spec[1];
-      e.out[1] = spec[2];
-      e.out[2] = spec[0];
-      launch_ypass<T>(g.ny, g.ny, e, g.L, 1, st);
-      auto h = xi(XI_STORE, 3, 0, g.L, g.nx, g.ny, g.lhx);
-      h.in[0] = spec[1];
-      h.in[1] = spec[2];
-      h.in[2] = spec[0];
-      h.out[0] = F[LES_DPDX];
-      h.out[1] = F[LES_DPDY];
-      h.out[2] = F[LES_P];
-      h.lo[0] = 1;
-      h.hi[0] = nz;
-      h.lo[1] = 1;
-      h.hi[1] = nz;
-      h.lo[2] = 0;
-      h.hi[2] = nz + 1;
-      launch_xinv<T>(g.nx, h, st);
-      dpdz_only();
-      KL("k_p_finish", 2.0 * g.field() * sizeof(T),
-         k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], pmean, g.plane(), nz));
-      return;
-    }
+    auto b = yp_s<S>(YP_PRESS, 2, 1, 1);
+    b.in[0] = s0;
+    b.in[1] = s1;
+    b.out[0] = s0;  // rows 0..nz+1: bottom layer, right-hand side, top layer
+    launch_ypass<S>(g.ny, g.ny, b, nz + 1, 1, st);
+    // tridiagonal solve per (kx, ky) -> p^, levels 0..nz+1.  In mixed
+    // precision p^ leaves the FP64 solve as FP32 and its mean mode is kept
+    // apart in FP64 (pmean); its inverse transforms run in FP32 -- only the
+    // forward right-hand side needs FP64, where div u* cancels
+    cplx<T>* ph = spec[2];
+    double* pm = mixed() ? pmean : nullptr;
+    const int drop = mixed() ? 1 : 0, pp = pitch(g.lhx);
     if (pslabs > 1)
-      slab_solve<S, S>(sp[2], sp[3], sp[4], bot, top, sp[5], mixed() ? pmean : nullptr, mixed() ? 1 : 0, g.lhx, g.lhx);
+      slab_solve<S, T>(s0, ph, pm, drop, pp, g.lhx);
     else
-      KL("k_tridiag", 112.0 * double(g.L) * g.ny * g.lhx, k_tridiag<S><<<tg, 64, 0, st>>>(sp[2], sp[3], sp[4], nullptr, bot, top, kkxd, kkyd, sp[5], xs, gam,
-                                     mixed() ? pmean : nullptr, dstatus, g.lhx, g.ny, nz, dz(), mixed() ? 1 : 0, g.lhx, g.lhx));
-    // compute_press_grad: i kx p^, i ky p^, p^ -> dpdx, dpdy (1..nz), p (0..nz+1)
-    auto e = yp_s<S>(YP_PGRAD, 1, 3, 0);
-    e.in[0] = sp[5];
-    e.out[0] = sp[6];
-    e.out[1] = sp[7];
-    e.out[2] = sp[5];
-    launch_ypass<S>(g.ny, g.ny, e, g.L, 1, st);
-    auto h = xi_s<S>(XI_STORE, 3, 0, g.L);
-    h.in[0] = sp[6];
-    h.in[1] = sp[7];
-    h.in[2] = sp[5];
-    set_out(h, 0, F[LES_DPDX]);
-    set_out(h, 1, F[LES_DPDY]);
-    set_out(h, 2, F[LES_P]);
-    h.lo[0] = 1;
-    h.hi[0] = nz;
-    h.lo[1] = 1;
-    h.hi[1] = nz;
-    h.lo[2] = 0;
-    h.hi[2] = nz + 1;
-    launch_xinv<S>(g.nx, h, st);
+      KL("k_tridiag", (56.0 + 8.0 + 2.0 * sizeof(T)) * double(g.L) * g.ny * g.lhx,
+         k_tridiag<T><<<ceil_div(2L * g.ny * g.lhx, 128), 128, 0, st>>>(reinterpret_cast<double*>(s0), piv,
+                                                                         reinterpret_cast<T*>(ph), pm, dstatus, g.lhx,
+                                                                         g.ny, nz, dz(), drop, pp));
+    press_grad(ph);
     // dpdz (compute_pressure.f90:359-369), then p(nz+1) = BOGUS (:353-357)
     dpdz_only();
-    KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T), k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], mixed() ? pmean : nullptr, g.plane(), nz));
+    KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
+       k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], pm, g.plane(), nz));
   }
-  double press_tadv1_ = 1.0;
+  // compute_press_grad: p^ (rows pitch(lhx) apart) -> dpdx, dpdy (1..nz), p
+  // (0..nz+1); the y pass forms p and i ky p, the x inverse i kx p from the
+  // staged p row (compute_pressure.f90:320-358)
+  void press_grad(cplx<T>* ph) {
+    auto e = yp(YP_PGRAD, 1, 2, g.lhx, g.lhx, g.ny, g.lhx, g.ny, 0);
+    e.in[0] = ph;
+    e.out[0] = ph;
+    e.out[1] = spec[3];
+    launch_ypass<T>(g.ny, g.ny, e, g.L, 1, st);
+    auto h = xi(XI_STORE, 3, 0, g.L, g.nx, g.ny, g.lhx);
+    h.nstage = 2;
+    h.kxr = kkx;
+    h.in[0] = ph;
+    h.in[1] = spec[3];
+    const int src[3] = {0, 1, 0};
+    T* const out[3] = {F[LES_DPDX], F[LES_DPDY], F[LES_P]};
+    for (int q = 0; q < 3; ++q) {
+      h.src[q] = src[q];
+      h.dx[q] = q == 0;
+      h.out[q] = out[q];
+      h.lo[q] = q < 2 ? 1 : 0;
+      h.hi[q] = q < 2 ? g.nz : g.nz + 1;
+    }
+    launch_xinv<T>(g.nx, h, st);
+  }
   void dpdz_only();
   // z-slab emulation of the pressure solve: the systems solved by the
   // partition method over pslabs row blocks, as pslabs z-slab ranks would
   // (k_tri_slab_*); 1 = the single sweep of k_tridiag
   int pslabs = 1;
   double *slab_u = nullptr, *slab_v = nullptr;
+  cplx<double>* xs = nullptr;  // sweep scratch of the slab and increment forms
+  double* gam = nullptr;
+  void sweep_scratch() {
+    if (xs) return;
+    xs = track(dalloc<cplx<double>>((long)g.L * g.ny * g.lhx));
+    gam = track(dalloc<double>((long)g.L * g.ny * g.lhx));
+  }
   cplx<double>* slab_x = nullptr;
   int slab_x_cap = 1;
   void set_pressure_slabs(int G) override {
     if (G < 1 || G > MAX_SLABS || g.nz % G != 0 || g.nz / G < 2)
       throw CudaError(1, "pressure slabs: 1 <= G <= 64, nz a multiple of G with at least two levels per slab");
+    if (G > 1) sweep_scratch();
     pslabs = G;
     if (G > 1 && !slab_u) {
       const long n = (long)g.L * g.ny * g.lhx;
@@ -1587,13 +1534,12 @@ class Solver final : public SolverBase {
     }
   }
   template <typename S, typename O>
-  void slab_solve(const cplx<S>* Hx, const cplx<S>* Hy, const cplx<S>* Hz, const cplx<S>* bot, const cplx<S>* top,
-                  cplx<O>* phat, double* pm, int drop_mean, int opitch, int ipitch) {
+  void slab_solve(const cplx<S>* R, cplx<O>* phat, double* pm, int drop_mean, int opitch, int ipitch) {
     const SlabRows sr{pslabs, g.nz / pslabs, g.nz};
     const double cols = double(g.ny) * g.lhx;
-    KL("k_tri_slab_local", cols * g.L * (3.0 * 2 * sizeof(S) + 40.0),
+    KL("k_tri_slab_local", cols * g.L * (2.0 * sizeof(S) + 40.0),
        k_tri_slab_local<S><<<dim3(ceil_div(g.lhx, 64), g.ny, pslabs), 64, 0, st>>>(
-           Hx, Hy, Hz, bot, top, kkxd, kkyd, xs, slab_u, slab_v, gam, dstatus, g.lhx, g.ny, g.nz, dz(), ipitch, sr));
+           R, kkxd, kkyd, xs, slab_u, slab_v, gam, dstatus, g.lhx, g.ny, g.nz, dz(), ipitch, sr));
     KL("k_tri_slab_reduced", cols * pslabs * (2 * 32.0 + 32.0),
        k_tri_slab_reduced<<<dim3(ceil_div(g.lhx, 64), g.ny), 64, 0, st>>>(xs, slab_u, slab_v, slab_x, dstatus, g.lhx,
                                                                           g.ny, sr));
@@ -1614,6 +1560,7 @@ class Solver final : public SolverBase {
   // transforms run in the state's precision.  Needs w(nz+1) = 0.
   void press_from_increment(double tadv1, double tadv2) override {
     Tag tag_(this, "press");
+    sweep_scratch();
     const int nz = g.nz;
     const double c = 1.0 / double(g.nx * g.ny);
     KL("k_scale", 2.0 * g.plane() * sizeof(T), k_scale<T><<<grid_for(g.plane()), 256, 0, st>>>(PL[LES_BOTTOM_WK_PRESS], g.plane(), T(c)));
@@ -1657,30 +1604,11 @@ class Solver final : public SolverBase {
     plane_means({F[LES_RHSZ], F[LES_RHSZ_F], F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ]}, 1, nz, means);
     dim3 tg(ceil_div(g.lhx, 64), g.ny);
     KL("k_tridiag", (4.0 * 2 * sizeof(T) + 2 * sizeof(T) + 24.0) * double(g.L) * g.ny * g.lhx,
-       k_tridiag<T, T, true><<<tg, 64, 0, st>>>(spec[2], spec[3], spec[4], spec[5], bot, top, kkxd, kkyd, spec[0], xs, gam,
+       k_tridiag_inc<T><<<tg, 64, 0, st>>>(spec[2], spec[3], spec[4], spec[5], bot, top, kkxd, kkyd, spec[0], xs, gam,
                                           mixed() ? pmean : nullptr, dstatus, g.lhx, g.ny, nz, dz(), mixed() ? 1 : 0,
                                           pitch(g.lhx), pitch(g.lhx), means, tadv2 / tadv1, 1.0 / (P.dt * tadv1),
                                           g.L));
-    auto e = yp(YP_PGRAD, 1, 3, g.lhx, g.lhx, g.ny, g.lhx, g.ny, 0);
-    e.in[0] = spec[0];
-    e.out[0] = spec[1];
-    e.out[1] = spec[2];
-    e.out[2] = spec[0];
-    launch_ypass<T>(g.ny, g.ny, e, g.L, 1, st);
-    auto h = xi(XI_STORE, 3, 0, g.L, g.nx, g.ny, g.lhx);
-    h.in[0] = spec[1];
-    h.in[1] = spec[2];
-    h.in[2] = spec[0];
-    h.out[0] = F[LES_DPDX];
-    h.out[1] = F[LES_DPDY];
-    h.out[2] = F[LES_P];
-    h.lo[0] = 1;
-    h.hi[0] = nz;
-    h.lo[1] = 1;
-    h.hi[1] = nz;
-    h.lo[2] = 0;
-    h.hi[2] = nz + 1;
-    launch_xinv<T>(g.nx, h, st);
+    press_grad(spec[0]);
     dpdz_only();
     KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
        k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], mixed() ? pmean : nullptr, g.plane(), nz));
@@ -1964,7 +1892,8 @@ class Solver final : public SolverBase {
     h[g.nz + 1] = h[g.nz];
     if (!spong) spong = track(dalloc<double>(g.L));
     if (!means) means = track(dalloc<double>(6 * g.L));
-    LES_CUDA(cudaMemcpy(spong, h.data(), sizeof(double) * g.L, cudaMemcpyHostToDevice));
+    LES_CUDA(cudaMemcpyAsync(spong, h.data(), sizeof(double) * g.L, cudaMemcpyHostToDevice, st));
+    LES_CUDA(cudaStreamSynchronize(st));
   }
 
   // gradients of theta (after compute_vel_grad: the wall law's u* is current)

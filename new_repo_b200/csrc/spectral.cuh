@@ -109,7 +109,7 @@ enum XFOp : int {
   XF_CONV_IN = 1, // u,v,w scaled by -c0 and the three vorticity components (c0 scaled)
   XF_PROD = 2,    // fine-grid u x omega products (inputs on the padded grid)
   XF_LASD = 3,    // the 21 test-filter inputs of the dynamic procedure
-  XF_PRESS = 4,   // field f = c0 * (in[f] / c1)   (compute_pressure.f90:138-140)
+  XF_PRESS = 4,   // pressure right-hand side: u*, v*, dw*/dz -> i kx u^ + (dw*/dz)^ and v^
   XF_PROD_SC = 5, // fine-grid scalar advection -(u . grad theta) (inputs on the padded grid)
   XF_SCDYN = 6,   // the 19 test-filter inputs of the dynamic Prandtl model
   XF_PRESS_INC = 7,  // pressure right-hand side from the AB2 increment and div u^n
@@ -131,16 +131,13 @@ struct XFArgs {
   T* refout[MAXIN];
   long in_pstride; // elements per plane of the input grid
   long in_rstride; // elements per row of the input grid (== NX)
-  double c0, c1, c2;
+  double c0, c1, c2, c3;
   const T* in[16];
   const float* inf[16];  // FP32 inputs of an FP64 transform (in_f32 = 1)
   int in_f32;
   cplx<T>* out[MAXIN];
   long out_pstride;  // rows_pp * nk
-  // staged kernel (k_xfwd_st): input rows copied per grid row, source q is
-  // field sf[q] at level offset sdl[q]; scond[q]: only on the wall row (l = 1)
-  int nsrc;
-  int sf[16], sdl[16], scond[16];
+  const T* kxr;      // x wavenumbers (XF_PRESS), Nyquist zero
   const cplx<T>* tw; // exp(-2 pi i m / NX), m < NX
 };
 
@@ -264,10 +261,37 @@ __device__ __forceinline__ void xf_load_op(const XFArgs<T>& a, int l, int j, int
       for (int f = 0; f < a.nf; ++f)
         put(f, T(a.c0) * (a.in_f32 ? vldg<V>(a.inf[f], off) : vldg<V>(a.in[f], off)));
     } else if constexpr (OP == XF_PRESS) {
-      // compute_pressure.f90:138-140
-      for (int f = 0; f < a.nf; ++f) {
-        const V x = a.in_f32 ? vldg<V>(a.inf[f], off) : vldg<V>(a.in[f], off);
-        put(f, T(a.c0) * (x / T(a.c1)));
+      // compute_pressure.f90:138-140, 176-190: u, v and (w(l+1) - w(l)) / dz
+      // over dt tadv1 nx ny (w(nz+1) counts as zero); c0 = 1/(nx ny tadv1),
+      // c1 = dt, c2 = 1/(nx ny).  Level nz+1 carries the two pressure-BC
+      // layers instead (inputs 3, 4): the bottom one, scaled by c2 in place
+      // (compute_pressure.f90:151-165), goes where it reaches output 0 as
+      // itself, the top one to output 1.
+      if constexpr (sizeof(T) == 8) {
+        auto from = [&](auto* const* in) {
+          using S = typename std::remove_const<typename std::remove_pointer<
+              typename std::remove_reference<decltype(in[0])>::type>::type>::type;
+          if (l > a.nz) {
+            const long p2 = (long)j * a.in_rstride + i;
+            S* bot = const_cast<S*>(in[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const S b = S(a.c2) * bot[p2 + q];
+              bot[p2 + q] = b;
+              v[0 * vs + q] = T(0);
+              v[1 * vs + q] = T(a.c2) * T(in[4][p2 + q]);
+              v[2 * vs + q] = T(b);
+            }
+          } else {
+            put(0, T(a.c0) * (vldg<V>(in[0], off) / T(a.c1)));
+            put(1, T(a.c0) * (vldg<V>(in[1], off) / T(a.c1)));
+            const V w0 = vldg<V>(in[2], off);
+            const V w1 = (l < a.nz) ? vldg<V>(in[2], off + a.in_pstride) : vsplat<V>(T(0));
+            put(2, T(a.c0) * (((w1 - w0) * vsplat<V>(T(a.c3))) / T(a.c1)));
+          }
+        };
+        if (a.in_f32) from(a.inf);
+        else from(a.in);
       }
     } else if constexpr (OP == XF_CONV_IN) {
       // compute_convective_padd.f90:133-165
@@ -441,7 +465,6 @@ __device__ __forceinline__ void xf_load(const XFArgs<T>& a, int l, int j, int i,
     case XF_CONV_IN: xf_load_op<T, V, XF_CONV_IN, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_PROD: xf_load_op<T, V, XF_PROD, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_LASD: xf_load_op<T, V, XF_LASD, false>(a, l, j, i, v, vs, nullptr); break;
-    case XF_PRESS: xf_load_op<T, V, XF_PRESS, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_PROD_SC: xf_load_op<T, V, XF_PROD_SC, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_SCDYN: xf_load_op<T, V, XF_SCDYN, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_PRESS_INC: xf_load_op<T, V, XF_PRESS_INC, false>(a, l, j, i, v, vs, nullptr); break;
@@ -551,7 +574,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
 #pragma unroll
       for (int r = 0; r < RO; ++r) seq[lane_t + TL * g + r * (M / RO)] = v[g * RO + r];
     __syncwarp();
-    if (s < nseq) {
+    if (s < nseq && a.op != XF_PRESS) {
       const int r = udiv32(s, a.nf);
       const int f = s - r * a.nf;
       const int l = rowl[r];
@@ -562,63 +585,47 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       }
     }
   }
-}
-
-// Values of the staged ops at level l, columns i..i+3 of row r, from the
-// staged input rows (rows[q] = source q of this grid row).
-template <typename T, typename S>
-__device__ __forceinline__ void xf_load_st(const XFArgs<T>& a, int l, const S* const* rows, int i, T* v, int vs) {
-  using V = V4<T>;
-  auto ld = [&](int q) { return vld<V>(rows[q], (long)i); };
-  switch (a.op) {
-    case XF_SCALE:
-      for (int f = 0; f < a.nf; ++f) vst(v + f * vs, T(a.c0) * ld(f));
-      break;
-    case XF_PRESS:  // compute_pressure.f90:138-140
-      for (int f = 0; f < a.nf; ++f) vst(v + f * vs, T(a.c0) * (ld(f) / T(a.c1)));
-      break;
-    case XF_CONV_IN: {
-      // compute_convective_padd.f90:133-165; sources 0..8 = the inputs at
-      // level l, 9 / 10 = dwdy / dwdx at l + 1 (wall row only)
-      const T c = T(a.c0);
-      vst(v + 0 * vs, -c * ld(0));
-      vst(v + 1 * vs, -c * ld(1));
-      vst(v + 2 * vs, -c * ld(2));
-      if (a.wall && l == 0) {
-        vst(v + 3 * vs, vsplat<V>(T(0)));
-        vst(v + 4 * vs, vsplat<V>(T(0)));
-      } else if (a.wall && l == 1) {
-        vst(v + 3 * vs, c * (T(0.5) * (ld(3) + ld(9)) - ld(4)));
-        vst(v + 4 * vs, c * (ld(5) - T(0.5) * (ld(6) + ld(10))));
-      } else {
-        vst(v + 3 * vs, c * (ld(3) - ld(4)));
-        vst(v + 4 * vs, c * (ld(5) - ld(6)));
+  if constexpr (sizeof(T) == 8) {
+    if (a.op == XF_PRESS) {
+      // two spectra leave for the three transforms of a row: i kx u^ + w'^
+      // and v^ (one warp per row, consecutive modes on consecutive lanes)
+      __syncthreads();
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+      for (int r = warp; r < a.R; r += nwarps) {
+        const int l = rowl[r];
+        if (l < 0) continue;
+        const cplx<T>* zu = buf + (long)(3 * r) * SL;
+        const cplx<T>* zv = zu + SL;
+        const cplx<T>* zw = zv + SL;
+        const long o = (long)l * a.out_pstride + (long)rowj[r] * a.opitch;
+        for (int k = lane; k <= M; k += 32) {
+          const int k0 = k == M ? 0 : k, k1 = k == 0 ? 0 : M - k;  // Z_M is Z_0
+          const cplx<T> h = tw[k];
+          a.out[0][o + k] = c_add(ik_mul(a.kxr[k], r2c_split(zu[k0], zu[k1], h)), r2c_split(zw[k0], zw[k1], h));
+          a.out[1][o + k] = r2c_split(zv[k0], zv[k1], h);
+        }
       }
-      vst(v + 5 * vs, c * (ld(7) - ld(8)));
-      break;
     }
-    default:
-      break;
   }
 }
 
-// start the copies of the staged input rows of batch `item` (one warp per
-// row, 16-byte pieces)
-template <typename T, typename S, int NX>
-__device__ __forceinline__ void xf_issue(const XFArgs<T>& a, long item, S* stage) {
+// start the copies of the input rows of batch `item` (one warp per row,
+// 16-byte pieces)
+template <typename T, int NX>
+__device__ __forceinline__ void xf_issue(const XFArgs<T>& a, long item, T* stage) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  constexpr int PIECES = NX * int(sizeof(S)) / 16;
-  const int nrow = a.R * a.nsrc;
+  constexpr int PIECES = NX * int(sizeof(T)) / 16;
+  const int nrow = a.R * a.nf;
   for (int s = warp; s < nrow; s += nwarps) {
-    const int r = udiv32(s, a.nsrc);
-    const int q = s - r * a.nsrc;
+    const int r = udiv32(s, a.nf);
+    const int q = s - r * a.nf;
     const long g = item * a.R + r;
-    const int l = a.plane0 + udiv32(g, a.rows_pp);
-    const bool valid = g < a.nrows && (!a.scond[q] || (a.wall && l == 1));
-    const S* base = reinterpret_cast<const S*>(std::is_same<S, T>::value ? (const void*)a.in[a.sf[q]]
-                                                                          : (const void*)a.inf[a.sf[q]]);
-    const S* row = valid ? base + (long)(l + a.sdl[q]) * a.in_pstride + long(umod32(g, a.rows_pp)) * a.in_rstride : base;
-    S* dst = stage + (long)s * NX;
+    const bool valid = g < a.nrows;
+    const T* base = a.in[q];
+    const T* row = valid ? base + (long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride +
+                               long(umod32(g, a.rows_pp)) * a.in_rstride
+                         : base;
+    T* dst = stage + (long)s * NX;
     for (int k = lane; k < PIECES; k += 32)
       cp_async<16>(reinterpret_cast<unsigned char*>(dst) + 16 * k,
                    valid ? reinterpret_cast<const unsigned char*>(row) + 16 * k
@@ -627,11 +634,10 @@ __device__ __forceinline__ void xf_issue(const XFArgs<T>& a, long item, S* stage
   }
 }
 
-// The x forward pass for the ops whose inputs are whole rows (scale,
-// pressure input, convective inputs): persistent CTAs over batches of R rows,
-// the input rows of the next batch copied into the other shared stage with
-// cp.async while the current batch is transformed.  S: input element type.
-template <typename T, int NX, typename S>
+// The x forward pass of scalings of a few fields (XF_SCALE): persistent CTAs
+// over batches of R rows, the input rows of the next batch copied into the
+// other shared stage with cp.async while the current batch is transformed.
+template <typename T, int NX>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2) k_xfwd_st(const XFArgs<T> a) {
   constexpr int M = NX / 2;
   constexpr int TL = Geo<M>::T;
@@ -645,9 +651,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   cplx<T>* twm = tw + NX;  // twiddle matrices of the M-point transform
   const int nseq = a.R * a.nf;
   const int npad = seq_pad<M>(nseq);
-  S* stage0 = reinterpret_cast<S*>(twm + Twm<M, false>::len);
-  S* stage1 = stage0 + (long)a.R * a.nsrc * NX;
-  cplx<T>* buf = reinterpret_cast<cplx<T>*>(stage1 + (long)a.R * a.nsrc * NX);
+  T* stage0 = reinterpret_cast<T*>(twm + Twm<M, false>::len);
+  T* stage1 = stage0 + (long)a.R * a.nf * NX;
+  cplx<T>* buf = reinterpret_cast<cplx<T>*>(stage1 + (long)a.R * a.nf * NX);
   T* refs = reinterpret_cast<T*>(buf + (long)npad * SL);
   int* rowl = reinterpret_cast<int*>(refs + a.R * a.nf);
   int* rowj = rowl + a.R;
@@ -655,15 +661,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
   const long nitems = (a.nrows + a.R - 1) / a.R;
   if ((long)blockIdx.x < nitems) {
-    xf_issue<T, S, NX>(a, blockIdx.x, stage0);
+    xf_issue<T, NX>(a, blockIdx.x, stage0);
     cp_async_commit();
   }
   int stg = 0;
   for (long item = blockIdx.x; item < nitems; item += gridDim.x) {
     const long next = item + gridDim.x;
-    const S* stage = stg ? stage1 : stage0;
+    const T* stage = stg ? stage1 : stage0;
     if (next < nitems) {
-      xf_issue<T, S, NX>(a, next, stg ? stage0 : stage1);
+      xf_issue<T, NX>(a, next, stg ? stage0 : stage1);
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -695,9 +701,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       T* dst = xr + (long)(r * a.nf) * XS + i;
       const int l = rowl[r];
       if (l >= 0) {
-        const S* rows[16];
-        for (int q = 0; q < a.nsrc; ++q) rows[q] = stage + (long)(r * a.nsrc + q) * NX;
-        xf_load_st<T, S>(a, l, rows, i, dst, XS);
+        for (int f = 0; f < a.nf; ++f)
+          vst(dst + f * XS, T(a.c0) * vld<V4<T>>(stage + (long)(r * a.nf + f) * NX, (long)i));
         if (a.use_ref)
           for (int f = 0; f < a.nf; ++f) {
             const T rf = refs[r * a.nf + f];
@@ -748,13 +753,15 @@ enum YPOp : int {
   YP_GRAD = 0,     // f -> f, i kx f, i ky f           (Nyquist killed)
   YP_DIV2 = 1,     // (fx, fy) -> i kx fx + i ky fy     (Nyquist killed)
   YP_FWDKILL = 2,  // f -> f, no inverse y transform    (Nyquist killed)
-  YP_PGRAD = 3,    // p^ (already y-spectral) -> i kx p, i ky p, p
+  YP_PGRAD = 3,    // p^ (already y-spectral) -> p, i ky p   (i kx p in the x inverse)
   YP_FILTER2 = 4,  // f -> G0 f, G1 f
   YP_PAD = 5,      // ny -> 3ny/2 zero padding (ky Nyquist dropped)
   YP_TRUNC = 6,    // 3ny/2 -> ny truncation (ky Nyquist zeroed)
   YP_MASK = 7,     // keep |ky| <= tt (2/3-rule truncation)
   YP_FILTER1 = 8,  // f -> G0 f
   YP_GRADY = 9,    // f -> f, i ky f                    (Nyquist killed; i kx f in the x inverse)
+  YP_PRESS = 10,   // (f, v) -> f + i ky v, no inverse y transform (Nyquist killed); the last plane's two
+                   // inputs are the pressure-BC layers: f -> plane 0, v -> its own plane
 };
 
 template <typename T>
@@ -804,11 +811,6 @@ __device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int 
     }
     case YP_FWDKILL:
       return (ky == NY / 2 || kx == a.nxh) ? zero : F0;
-    case YP_PGRAD: {
-      if (q == 0) return ik_mul(a.kkx[ky * a.lhx + kx], F0);
-      if (q == 1) return ik_mul(a.kky[ky * a.lhx + kx], F0);
-      return F0;
-    }
     case YP_FILTER1:
     case YP_FILTER2: {
       const T g = (q == 0 ? a.G0 : a.G1)[ky * a.lhx + kx];
@@ -839,9 +841,8 @@ __device__ __forceinline__ cplx<T> yp_op_c(const YPArgs<T>& a, int q, int kx, in
     if (q == 0) return F0;
     return ik_mul(kyv, F0);
   } else {  // YP_PGRAD: no kill, the Nyquist row / column of the tables are zero
-    if (q == 0) return ik_mul(ky == NY / 2 ? T(0) : kxv, F0);
-    if (q == 1) return ik_mul(kx == a.nxh ? T(0) : kyv, F0);
-    return F0;
+    if (q == 0) return F0;
+    return ik_mul(kx == a.nxh ? T(0) : kyv, F0);
   }
 }
 
@@ -872,8 +873,8 @@ __device__ __forceinline__ void yp_issue(const YPArgs<T>& a, long item, int ncb,
   }
 }
 
-// FWD: forward transform only (YP_FWDKILL), compiled without the inverse so
-// that it keeps fewer registers (more resident warps)
+// FWD: forward transforms only (YP_FWDKILL, YP_PRESS), compiled without the
+// inverse so that it keeps fewer registers (more resident warps)
 template <typename T, int NY, int NYO, bool FWD = false>
 __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
                                   (FWD && sizeof(T) == 8) ? 3 : (sizeof(T) == 4 ? 2 : 1))
@@ -951,7 +952,23 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
 #pragma unroll
         for (int r = 0; r < FI; ++r) f0[g * FI + r] = seq[lt + TL * g + r * (NY / FI)];
       reg_fft<T, NY, false>(f0, seq, lt, twi);
-      if constexpr (SAME) {
+      if constexpr (FWD) {
+        if (a.op == YP_PRESS) {
+          // the first transform rests in its slot (natural order, as the
+          // copy-out wants it) while the registers take the second
+          __syncwarp();
+#pragma unroll
+          for (int g = 0; g < EI / FO; ++g)
+#pragma unroll
+            for (int r = 0; r < FO; ++r) seq[lt + TL * g + r * (NY / FO)] = f0[g * FO + r];
+          cplx<T>* seq1 = bin + (C + c) * SI;
+#pragma unroll
+          for (int g = 0; g < EI / FI; ++g)
+#pragma unroll
+            for (int r = 0; r < FI; ++r) f0[g * FI + r] = seq1[lt + TL * g + r * (NY / FI)];
+          reg_fft<T, NY, false>(f0, seq1, lt, twi);
+        }
+      } else if constexpr (SAME) {
         if (a.op == YP_DIV2) {
           const cplx<T> zero = {T(0), T(0)};
 #pragma unroll
@@ -982,20 +999,31 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
   }
   __syncwarp();  // the column's forward reads are done before its slot is rewritten
   cplx<T>* sout = bin + c * SI;
-  for (int q = 0; q < a.nout; ++q) {
+  const bool layers = FWD && a.op == YP_PRESS && l == a.plane0 + a.nplanes - 1;
+  const int nout = layers ? 2 : a.nout;
+  for (int q = 0; q < nout; ++q) {
     if constexpr (SAME) {
       // forward output layout (groups FO) == inverse input layout; the
       // stress divergence already holds its result in w
       if constexpr (FWD) {
         // YP_FWDKILL: the killed forward output goes straight to the slot in
-        // the forward output layout (groups FO)
+        // the forward output layout (groups FO).  YP_PRESS: the slot holds
+        // the first transform; i ky times the second is added, or, on the
+        // plane of the boundary layers, both leave one after the other.
+        const bool press = a.op == YP_PRESS;
 #pragma unroll
         for (int g = 0; g < EI / FO; ++g)
 #pragma unroll
           for (int r = 0; r < FO; ++r) {
             const int ky = lt + TL * g + r * (NY / FO);
             const bool kill = (ky == NY / 2) || (kx == a.nxh) || (kx >= a.ncols);
-            sout[lt + TL * g + r * (NYO / FO)] = kill ? cplx<T>{T(0), T(0)} : f0[g * FO + r];
+            cplx<T>& slot = sout[lt + TL * g + r * (NYO / FO)];
+            cplx<T> x = f0[g * FO + r];
+            if (press && !(layers && q == 1)) {
+              x = slot;
+              if (!layers) x = c_add(x, ik_mul(kyrow[ky], f0[g * FO + r]));
+            }
+            slot = kill ? cplx<T>{T(0), T(0)} : x;
           }
       } else if (a.op != YP_DIV2) {
         // the derivative ops with the op fixed per loop (no per-element
@@ -1077,7 +1105,8 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
       if (kxx < lim) {
         const int ky0 = threadIdx.x >> a.lc;
         const long opitch = second ? a.opitch1 : a.opitch;
-        cplx<T>* dst = a.out[grp * a.nout + q] + (long)l * (second ? a.out_pstride1 : a.out_pstride) + kxx +
+        const int lo = (layers && q == 0) ? 0 : l;
+        cplx<T>* dst = a.out[layers ? 0 : grp * a.nout + q] + (long)lo * (second ? a.out_pstride1 : a.out_pstride) + kxx +
                        (long)ky0 * opitch;
         const cplx<T>* srow = bin + cc * SI + ky0;
         const long step = (long)TL * opitch;

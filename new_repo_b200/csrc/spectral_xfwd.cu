@@ -6,39 +6,19 @@
 
 namespace les {
 
-// the staged x forward pass (ops whose inputs are whole rows)
-template <typename T, typename S>
+// the staged x forward pass (scalings of few fields)
+template <typename T>
 static void launch_xfwd_st(int NX, XFArgs<T>& a, cudaStream_t st) {
   const int M = NX / 2;
-  a.nsrc = 0;
-  if (a.op == XF_CONV_IN) {
-    for (int f = 0; f < 9; ++f) {
-      a.sf[a.nsrc] = f;
-      a.sdl[a.nsrc] = 0;
-      a.scond[a.nsrc++] = 0;
-    }
-    for (int f : {3, 6}) {  // dwdy, dwdx one level up, read on the wall row only
-      a.sf[a.nsrc] = f;
-      a.sdl[a.nsrc] = 1;
-      a.scond[a.nsrc++] = 1;
-    }
-  } else {
-    for (int f = 0; f < a.nf; ++f) {
-      a.sf[a.nsrc] = f;
-      a.sdl[a.nsrc] = 0;
-      a.scond[a.nsrc++] = 0;
-    }
-  }
   const int SL = slot_stride(M, int(sizeof(cplx<T>)));
   auto smem_for = [&](int R) {
     return sizeof(cplx<T>) * (NX + twm_len(M, false) + (size_t)pad_seqs(R * a.nf, M) * SL) +
-           2 * sizeof(S) * (size_t)R * a.nsrc * NX +
-           sizeof(T) * R * a.nf + 2 * sizeof(int) * R + 16;
+           2 * sizeof(T) * (size_t)R * a.nf * NX + sizeof(T) * R * a.nf + 2 * sizeof(int) * R + 16;
   };
   void (*kern)(XFArgs<T>) = nullptr;
   switch (NX) {
 #define XS_CASE(N) \
-  case N: kern = k_xfwd_st<T, N, S>; break;
+  case N: kern = k_xfwd_st<T, N>; break;
     LES_LENGTHS(XS_CASE)
 #undef XS_CASE
     default:
@@ -58,25 +38,15 @@ template <typename T>
 void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   const int M = NX / 2;
   if (a.opitch == 0) a.opitch = a.nk;
+  a.in_rstride = NX;
   // the staged kernel pays for its two input stages with occupancy: it wins
-  // for the pressure inputs and for scalings of few fields (measured at 256^3)
-  const bool staged = a.op == XF_PRESS || (a.op == XF_SCALE && a.nf <= 3);
-  if (staged) {
-    a.in_rstride = NX;
-    static const int nin_of_op[] = {0, 9, 6, 10, 0, 6, 14, 9};
-    const int nin = (a.op == XF_SCALE || a.op == XF_PRESS) ? a.nf : nin_of_op[a.op];
-    const size_t isz = (a.in_f32 ? sizeof(float) : sizeof(T));
-    hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * a.nf * a.nk * sizeof(cplx<T>));
-    if (a.in_f32) {
-      if constexpr (std::is_same<T, double>::value) launch_xfwd_st<T, float>(NX, a, st);
-      else throw CudaError(1, "xfwd: FP32 inputs are for FP64 transforms");
-    } else {
-      launch_xfwd_st<T, T>(NX, a, st);
-    }
+  // for scalings of few fields (measured at 256^3)
+  if (a.op == XF_SCALE && a.nf <= 3) {
+    hook_before("xfwd", double(a.nrows) * NX * a.nf * sizeof(T) + double(a.nrows) * a.nf * a.nk * sizeof(cplx<T>));
+    launch_xfwd_st<T>(NX, a, st);
     hook_after();
     return;
   }
-  a.in_rstride = NX;
   const int SL = slot_stride(M, int(sizeof(cplx<T>)));
   auto smem_for = [&](int R) {
     return sizeof(cplx<T>) * (NX + twm_len(M, false) + (size_t)pad_seqs(R * a.nf, M) * SL) + sizeof(T) * R * a.nf +
@@ -97,16 +67,17 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   // others at a finer grain (measured at 256^3: 0.667 -> 0.633 ms per step);
   // the other ops keep 256 threads (the stress divergence measured slower
   // with 128: 0.236 -> 0.256 ms)
-  const int XF_THREADS = (a.op == XF_CONV_IN || a.op == XF_PROD || a.op == XF_PROD_SC) ? 128 : 256;
+  const int XF_THREADS = (a.op == XF_CONV_IN || a.op == XF_PROD || a.op == XF_PROD_SC || a.op == XF_PRESS) ? 128 : 256;
   a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, a.nrows, nullptr, XF_THREADS);
   const size_t smem = smem_for(a.R);
   if (smem > SMEM_CAP) throw CudaError(1, "xfwd: shared memory request too large");
   const int grid = ceil_div(a.nrows, a.R);
   if (grid == 0) return;
-  static const int nin_of_op[] = {0, 9, 6, 10, 0, 6, 14, 9};
-  const int nin = (a.op == XF_SCALE || a.op == XF_PRESS) ? a.nf : nin_of_op[a.op];
+  static const int nin_of_op[] = {0, 9, 6, 10, 3, 6, 14, 9};
+  const int nin = a.op == XF_SCALE ? a.nf : nin_of_op[a.op];
+  const int nout = a.op == XF_PRESS ? 2 : a.nf;
   const size_t isz = (a.in_f32 ? sizeof(float) : sizeof(T));
-  hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * a.nf * a.nk * sizeof(cplx<T>));
+  hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * nout * a.nk * sizeof(cplx<T>));
   kern<<<grid, XF_THREADS, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
@@ -117,9 +88,7 @@ template <typename T>
 void set_attrs_xfwd() {
 #define XA(N)                                                                                       \
   LES_CUDA(cudaFuncSetAttribute(k_xfwd<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  LES_CUDA(cudaFuncSetAttribute(k_xfwd_st<T, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  if constexpr (std::is_same<T, double>::value)                                                       \
-    LES_CUDA(cudaFuncSetAttribute(k_xfwd_st<T, N, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
+  LES_CUDA(cudaFuncSetAttribute(k_xfwd_st<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
   LES_LENGTHS(XA)
 #undef XA
 }

@@ -38,7 +38,7 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
            sizeof(T) * ((NY + 3) & ~3);
   };
   const int key = NY * 10000 + NYO;
-  const bool fwd = (a.op == YP_FWDKILL);
+  const bool fwd = (a.op == YP_FWDKILL || a.op == YP_PRESS);
   void (*kern)(YPArgs<T>) = nullptr;
   switch (key) {
 #define YP_CASE(A, B) \
