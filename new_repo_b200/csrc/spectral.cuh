@@ -760,6 +760,8 @@ enum YPOp : int {
   YP_MASK = 7,     // keep |ky| <= tt (2/3-rule truncation)
   YP_FILTER1 = 8,  // f -> G0 f
   YP_GRADY = 9,    // f -> f, i ky f                    (Nyquist killed; i kx f in the x inverse)
+  YP_PADY = 11,    // YP_PAD of f and of i ky f (second output optional)
+  YP_MASKY = 12,   // YP_MASK of f and of i ky f (second output optional)
   YP_PRESS = 10,   // (f, v) -> f + i ky v, no inverse y transform (Nyquist killed); the last plane's two
                    // inputs are the pressure-BC layers: f -> plane 0, v -> its own plane
 };
@@ -817,7 +819,10 @@ __device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int 
       return cplx<T>{F0.x * g, F0.y * g};
     }
     case YP_MASK:
-      return (ky <= a.tt || ky >= NY - a.tt) ? F0 : zero;
+    case YP_MASKY: {
+      if (!(ky <= a.tt || ky >= NY - a.tt)) return zero;
+      return q == 0 ? F0 : ik_mul(a.kky[ky * a.lhx + kx], F0);
+    }
     default:
       return F0;  // YP_PAD / YP_TRUNC: position remap only
   }
@@ -1002,6 +1007,7 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
   const bool layers = FWD && a.op == YP_PRESS && l == a.plane0 + a.nplanes - 1;
   const int nout = layers ? 2 : a.nout;
   for (int q = 0; q < nout; ++q) {
+    if (!layers && !a.out[grp * a.nout + q]) continue;  // an optional output left out (the same for the whole CTA)
     if constexpr (SAME) {
       // forward output layout (groups FO) == inverse input layout; the
       // stress divergence already holds its result in w
@@ -1067,6 +1073,7 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
       constexpr int GI = EI / FO;  // forward output: f0[g FO + r] holds m = g + r GI
       constexpr int GO = EO / II;  // inverse input: w[g II + r] wants m' = g + r GO
       const bool live = kx < a.ncols;
+      auto remap = [&](auto ddy) {  // ddy: the output is i ky f
       static_for<EO>([&](auto mc) {
         constexpr int mo = decltype(mc)::value;
         constexpr int wi = (mo % GO) * II + mo / GO;
@@ -1080,9 +1087,18 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
         } else {
           constexpr int fi = (ms % GI) * FO + ms / GI;
           const bool keep = live && !(drop0 && lt == 0);
-          w[wi] = keep ? f0[fi] : cplx<T>{T(0), T(0)};
+          cplx<T> x = f0[fi];
+          if constexpr (decltype(ddy)::value) x = ik_mul(kyrow[lt + TL * ms], x);
+          w[wi] = keep ? x : cplx<T>{T(0), T(0)};
         }
       });
+      };
+      if constexpr (NYO > NY) {
+        if (a.op == YP_PADY && q == 1) remap(std::true_type{});
+        else remap(std::false_type{});
+      } else {
+        remap(std::false_type{});
+      }
     }
     if constexpr (FWD) {
       // no inverse: stored above
@@ -1129,6 +1145,7 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
 // ---------------------------------------------------------------- xinv ----
 enum XIOp : int {
   XI_STORE = 0,  // out[f](l) = x_f for lo[f] <= l <= hi[f]
+  XI_CONV = 1,   // -u, -v, -w and the vorticity from the spectra of u, v, w and their y derivatives
   XI_DIV = 2,    // rhs += x + dz(tz) + pf ; pressure-BC layers of the w equation
   XI_LASD = 3,   // 21 filtered fields -> L:M and M:M
   XI_WALL = 4,   // filtered u1, v1 -> u*, Neumann ghost value, wall stress
@@ -1167,6 +1184,10 @@ struct XIArgs {
   int src[MAXIN];
   int dx[MAXIN];
   const T* kxr;
+  // XI_CONV: staged rows u, v, w, i ky u, i ky w at level l, then u, v at
+  // l - 1; refin[0..2] the per-plane references of u, v, w; c0 = 1/dz,
+  // c1 the scale of the spectra
+  int wall;
   // set by the launcher: every output (and the plane stride) admits stores of
   // whole (x_2m, x_2m+1) pairs
   int pair_store;
@@ -1175,6 +1196,23 @@ struct XIArgs {
   int bulk;
   unsigned* status;  // device status word (ST_COPY_WAIT), may be null
 };
+
+// Plane of the spectrum that staged row f of level l comes from.  XI_CONV:
+// the values of w on its two boundary levels lie apart (plane 0: level 1,
+// plane nz + 2: level nz + 1), since the planes of those levels keep the w
+// whose derivatives the gradients hold.
+template <typename T>
+__device__ __forceinline__ int xi_plane(const XIArgs<T>& a, int f, int l) {
+  if (a.op != XI_CONV) return l;
+  if (f >= 5) return l - 1;
+  if (f == 2) return l == 1 ? 0 : (l == a.nz + 1 ? l + 1 : l);
+  return l;
+}
+template <typename T>
+__device__ __forceinline__ const cplx<T>* xi_row(const XIArgs<T>& a, int f, long g) {
+  const int l = a.plane0 + udiv32(g, a.rows_pp);
+  return a.in[f] + (long)xi_plane(a, f, l) * a.in_pstride + long(umod32(g, a.rows_pp)) * a.ipitch;
+}
 
 // x inverse pass: start the copies of the spectral rows of batch `item`
 // (R rows x nin fields, nk values each) into the shared stage
@@ -1191,8 +1229,7 @@ __device__ __forceinline__ void xi_issue(const XIArgs<T>& a, long item, cplx<T>*
     const long g = item * a.R + r;
     const bool valid = g < a.nrows;
     const cplx<T>* base = a.in[f];
-    const cplx<T>* row =
-        valid ? base + (long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride + long(umod32(g, a.rows_pp)) * a.ipitch : base;
+    const cplx<T>* row = valid ? xi_row(a, f, g) : base;
     cplx<T>* dst = stage + (long)s * a.nks;
     for (int m = lane; m < a.nk; m += 32) cp_async<int(sizeof(cplx<T>))>(dst + m, valid ? row + m : base, valid);
   }
@@ -1214,9 +1251,7 @@ __device__ __forceinline__ void xi_issue_bulk(const XIArgs<T>& a, long item, cpl
   const unsigned rbulk = rb & ~15u;
   auto aligned = [&](int s) {
     const int r = udiv32(s, ns), f = s - r * ns;
-    const long g = item * a.R + r;
-    const cplx<T>* row = a.in[f] + (long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride +
-                         long(umod32(g, a.rows_pp)) * a.ipitch;
+    const cplx<T>* row = xi_row(a, f, item * a.R + r);
     const cplx<T>* dst = stage + (long)s * a.nks;
     return ((reinterpret_cast<uintptr_t>(row) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
   };
@@ -1232,9 +1267,7 @@ __device__ __forceinline__ void xi_issue_bulk(const XIArgs<T>& a, long item, cpl
   tc::fence_async_smem();  // earlier generic reads of this stage come first
   for (int s = lane; s < nrow; s += 32) {
     const int r = udiv32(s, ns), f = s - r * ns;
-    const long g = item * a.R + r;
-    const cplx<T>* row = a.in[f] + (long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride +
-                         long(umod32(g, a.rows_pp)) * a.ipitch;
+    const cplx<T>* row = xi_row(a, f, item * a.R + r);
     cplx<T>* dst = stage + (long)s * a.nks;
     int m0 = 0;
     if (rbulk && aligned(s)) {
@@ -1331,7 +1364,39 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   }
   // a plain store writes straight from registers; the other ops combine
   // fields per point through shared memory
-  const bool direct = (a.op == XI_STORE);
+  const bool conv = (a.op == XI_CONV);
+  const bool direct = (a.op == XI_STORE) || conv;
+  if (conv) {
+    // the vorticity in the staged rows: o1 over i ky w, o2 over u(l - 1), o3
+    // over i ky u (compute_convective_padd.f90:145-165; the wall rows' means
+    // of w derivatives over levels 1 and 2).  Boundary levels take the w of
+    // the gradients from global memory.
+    cplx<T>* rows = const_cast<cplx<T>*>(stage);
+    const T rdz = T(a.c0);
+    for (int idx = threadIdx.x; idx < a.R * a.nk; idx += blockDim.x) {
+      const int r = udiv32(idx, a.nk);
+      const int m = idx - r * a.nk;
+      const int l = rowl[r];
+      if (l < 0) continue;
+      cplx<T>* q = rows + (long)r * 7 * a.nks + m;
+      const int n = a.nks;
+      cplx<T> wp = q[2 * n], yw = q[4 * n];
+      if (l == 1 || l == a.nz + 1) {
+        const long o = (long)l * a.in_pstride + (long)rowj[r] * a.ipitch + m;
+        wp = a.in[2][o];
+        if (a.wall && l == 1) {
+          wp = c_scl(c_add(wp, a.in[2][o + a.in_pstride]), T(0.5));
+          yw = c_scl(c_add(yw, a.in[4][o + a.in_pstride]), T(0.5));
+        }
+      }
+      const cplx<T> uz = c_scl(c_sub(q[0], q[5 * n]), rdz), vz = c_scl(c_sub(q[n], q[6 * n]), rdz);
+      const T kx = kxs[m];
+      q[3 * n] = c_sub(ik_mul(kx, q[n]), q[3 * n]);
+      q[4 * n] = c_sub(yw, vz);
+      q[5 * n] = c_sub(uz, ik_mul(kx, wp));
+    }
+    __syncthreads();
+  }
   const int lane_t = threadIdx.x % TL;
   for (int base = 0; base < npad; base += blockDim.x / TL) {
     const int s = base + threadIdx.x / TL;
@@ -1344,8 +1409,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       l = rowl[r];
       j = rowj[r];
     }
-    // merged: the staged row of sequence s (staged rows are sequences) is its slot
-    cplx<T>* seq = a.merged ? const_cast<cplx<T>*>(stage) + (long)s * a.nks : buf + (long)s * SL;
+    // merged: the staged row of sequence s is its slot (slots past the last
+    // sequence follow the staged rows)
+    const int srow = conv ? (s < nseq ? r * 7 + a.src[f] : a.R * 7 + (s - nseq)) : s;
+    cplx<T>* seq = a.merged ? const_cast<cplx<T>*>(stage) + (long)srow * a.nks : buf + (long)s * SL;
     // c2r split: Z_m = (X_m + conj X_{M-m}) + i W^{-m} (X_m - conj X_{M-m}),
     // imaginary parts of the DC and Nyquist bins ignored
     cplx<T> v[E];
@@ -1426,8 +1493,21 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     reg_fft<T, M, true>(v, seq, lane_t, twm);
     if (direct) {
       if (valid && l >= a.lo[f] && l <= a.hi[f]) {
-        const T ref = a.refin[f] ? a.refin[f][l] : T(0);
+        T ref = T(0);
+        if (conv) {
+          // -u, -v, -w and their levels' references; the vertical differences'
+          if (f < 3) ref = a.refin[f] ? -a.refin[f][xi_plane(a, f, l)] : T(0);
+          else if (f < 5 && a.refin[0]) {
+            const T* rf = a.refin[f == 3 ? 1 : 0];
+            const double d = (double(rf[l]) - double(rf[l - 1])) * a.c0;
+            ref = T(f == 3 ? -d : d);
+          }
+        } else if (a.refin[f]) {
+          ref = a.refin[f][l];
+        }
         const cplx<T> ref2 = {ref, ref};
+        const T sg = conv ? T(f < 3 ? -a.c1 : a.c1) : T(1);
+        const cplx<T> sg2 = {sg, sg};
         const long off = (long)l * a.out_pstride + (long)j * NX;
         // the store form is chosen once per sequence (outside the unrolled loop)
         auto store = [&](auto form_c) {
@@ -1437,7 +1517,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
 #pragma unroll
             for (int rr = 0; rr < RO; ++rr) {
               const int m = lane_t + TL * gg + rr * (M / RO);
-              const cplx<T> z = c_add(v[gg * RO + rr], ref2);
+              const cplx<T> z = c_fma(v[gg * RO + rr], sg2, ref2);
               if constexpr (FORM == 0) {
                 *reinterpret_cast<float2*>(a.outf[f] + off + 2 * m) = make_float2(float(z.x), float(z.y));
               } else if constexpr (FORM == 1) {

@@ -29,9 +29,12 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   // a plain store with one staged row per sequence transforms each sequence
   // in its own staged row (the exchange slot is the row), which leaves room
   // for more rows per work item
-  a.merged = (a.op == XI_STORE && a.nstage == 0) ? 1 : 0;
+  // (XI_CONV: six of its seven staged rows become sequences)
+  a.merged = ((a.op == XI_STORE && a.nstage == 0) || a.op == XI_CONV) ? 1 : 0;
   if (a.merged) a.nks = std::max(a.nks, SL);
-  auto stage_rows = [&](int R) { return a.merged ? pad_seqs(R * a.nin, M) : R * ns; };
+  auto stage_rows = [&](int R) {
+    return a.merged ? R * (ns - a.nin) + pad_seqs(R * a.nin, M) : R * ns;
+  };
   // bulk staging: one cp.async.bulk per staged row needs 16-byte aligned
   // rows in global memory (pitch and plane stride) and in the stages (stage
   // base and row stride); the kernel checks every row's addresses again and
@@ -81,7 +84,7 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   {
     const size_t osz = (a.out_f32 ? sizeof(float) : sizeof(T));
     int nout = a.nin, rmw = 0;
-    if (a.op == XI_DIV) { nout = a.nin; rmw = 2 * a.nin; }
+    if (a.op == XI_DIV) rmw = 2 * a.nin;
     else if (a.op == XI_LASD || a.op == XI_SCDYN) nout = 2;
     else if (a.op == XI_WALL) nout = 7;
     hook_before("xinv", double(a.nrows) * ns * a.nk * sizeof(cplx<T>) + double(a.nrows) * NX * (nout + rmw) * osz);
