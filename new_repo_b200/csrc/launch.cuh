@@ -33,5 +33,7 @@ template <typename T>
 void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st);
 template <typename T>
 void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaStream_t st);
+template <typename T>
+void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st);
 
 }  // namespace les

@@ -390,6 +390,8 @@ class Solver final : public SolverBase {
     a.in_pstride = (long)rows_pp * a.ipitch;
     a.out_pstride = (long)rows_pp * NX;
     a.tw = twiddles(NX);
+    a.lo_ref = 0;
+    a.hi_ref = g.nz + 1;
     a.status = dstatus;
     return a;
   }
@@ -1384,15 +1386,14 @@ class Solver final : public SolverBase {
     launch_xinv<T>(FNX, c, st);
   }
 
-  // the products of fine[] back to the base grid: cx, cy, cz on levels 1..nz
-  void fine_products(int cx, int cy, int cz) {
-    const int nz = g.nz;
-    const bool padd = this->padd();
-    const int FNX = padd ? g.nx2 : g.nx, FNY = padd ? g.ny2 : g.ny;
-    // 4. products on the fine grid, transformed back (levels 1..nz)
-    const int nkout = padd ? g.nx / 2 : int(std::ceil(double(float(2 * g.lhx)) / 3.0)) - 1;
-    auto d = xf(XF_PROD, 3, 1, nz, FNX, FNY, nkout);
-    d.c0 = padd ? 1.0 / double(g.nx2 * g.ny2) : 1.0 / double(g.nx * g.ny);
+  int nk_back() const { return padd() ? g.nx / 2 : int(std::ceil(double(float(2 * g.lhx)) / 3.0)) - 1; }
+  int back_rows() const { return int(std::ceil(double(float(2 * g.lhy)) / 3.0)) - 2; }
+
+  // x spectra of the products of fine[], levels 1..nz, into spec[0..2]
+  void product_spectra() {
+    const int FNX = padd() ? g.nx2 : g.nx, FNY = padd() ? g.ny2 : g.ny;
+    auto d = xf(XF_PROD, 3, 1, g.nz, FNX, FNY, nk_back());
+    d.c0 = 1.0 / (double(FNX) * FNY);
     for (int q = 0; q < 6; ++q) d.in[q] = fine[q];
     for (int q = 0; q < 3; ++q) d.out[q] = spec[q];
     if (mixed()) {
@@ -1401,22 +1402,19 @@ class Solver final : public SolverBase {
       for (int q = 0; q < 3; ++q) d.refout[q] = refbuf[6 + q];
     }
     launch_xfwd<T>(FNX, d, st);
-    if (padd) {
-      auto e = yp(YP_TRUNC, 1, 1, nkout, nkout, g.ny2, nkout, g.ny, 1);
-      for (int q = 0; q < 3; ++q) {
-        e.in[q] = spec[q];
-        e.out[q] = spec[3 + q];
-      }
-      launch_ypass<T>(g.ny2, g.ny, e, nz, 3, st);
-    } else {
-      auto e = yp(YP_MASK, 1, 1, nkout, nkout, g.ny, nkout, g.ny, 1);
-      e.tt = int(std::ceil(double(float(2 * g.lhy)) / 3.0)) - 2;
-      for (int q = 0; q < 3; ++q) {
-        e.in[q] = spec[q];
-        e.out[q] = spec[3 + q];
-      }
-      launch_ypass<T>(g.ny, g.ny, e, nz, 3, st);
+  }
+
+  // the products of fine[] back to the base grid: cx, cy, cz on levels 1..nz
+  void fine_products(int cx, int cy, int cz) {
+    const int nz = g.nz, nkout = nk_back(), FNY = padd() ? g.ny2 : g.ny;
+    product_spectra();
+    auto e = yp(padd() ? YP_TRUNC : YP_MASK, 1, 1, nkout, nkout, FNY, nkout, g.ny, 1);
+    e.tt = back_rows();
+    for (int q = 0; q < 3; ++q) {
+      e.in[q] = spec[q];
+      e.out[q] = spec[3 + q];
     }
+    launch_ypass<T>(FNY, g.ny, e, nz, 3, st);
     auto h = xi(XI_STORE, 3, 1, nz, g.nx, g.ny, nkout);
     const int outs[3] = {cx, cy, cz};
     for (int q = 0; q < 3; ++q) {
@@ -1427,19 +1425,108 @@ class Solver final : public SolverBase {
       if (mixed()) h.refin[q] = refbuf[6 + q];
     }
     launch_xinv<T>(g.nx, h, st);
-    // ghost levels of the outputs (compute_convective_padd.f90:251-259)
-    if (padd) {
+    convec_ghosts(outs);
+  }
+  // ghost levels of the outputs (compute_convective_padd.f90:251-259)
+  void convec_ghosts(const int* outs) {
+    if (padd()) {
       T* dst[6];
       T val[6];
       for (int q = 0; q < 3; ++q) {
         dst[2 * q] = lev(F[outs[q]], 0);
-        dst[2 * q + 1] = lev(F[outs[q]], nz + 1);
+        dst[2 * q + 1] = lev(F[outs[q]], g.nz + 1);
         val[2 * q] = val[2 * q + 1] = T(BOGUS);
       }
       plane_ops(6, dst, nullptr, val);
     } else {
       trunc_ghosts(outs);
     }
+  }
+
+  // Convective term and stress divergence of a time step in one inverse
+  // transform: the product spectra (spec[0..2]) and the stresses' x spectra
+  // meet in the y pass (k_yrhs), and the x inverse adds the vertical part and
+  // the forcing and writes rhs once.  Apart (fine_products, then div_eqs) the
+  // convective term was inverse transformed in y and x and stored, the
+  // divergence too, and rhs read back and rewritten: at 256^3 in mixed
+  // precision MEASURED.
+  void rhs_from_products() {
+    const int rhs[3] = {LES_RHSX, LES_RHSY, LES_RHSZ};
+    {
+      Tag tag_(this, "convec");
+      product_spectra();
+    }
+    {
+      Tag tag_(this, "divstress");
+      const DivEq e[3] = {{LES_RHSX, LES_TXX, LES_TXY, LES_TXZ, 1, P.pfx},
+                          {LES_RHSY, LES_TXY, LES_TYY, LES_TYZ, 1, P.pfy},
+                          {LES_RHSZ, LES_TXZ, LES_TYZ, LES_TZZ, 0, 0.0}};
+      div_products(e, 3, true);
+    }
+    Tag tag_(this, "convec");
+    convec_ghosts(rhs);
+  }
+  // rhs of neq equations = products (spectra spec[q], references refbuf[6 + q])
+  // + stress divergence + forcing
+  void div_products(const DivEq* e, int neq, bool layers) {
+    const int nz = g.nz, FNY = padd() ? g.ny2 : g.ny, nc = g.nx / 2;
+    int ids[6], nid = 0;
+    auto slot = [&](int fid) {
+      for (int q = 0; q < nid; ++q)
+        if (ids[q] == fid) return q;
+      ids[nid] = fid;
+      return nid++;
+    };
+    YRArgs<T> b;
+    std::memset(&b, 0, sizeof(b));
+    for (int q = 0; q < neq; ++q) {
+      b.p[q] = spec[q];
+      b.sx[q] = spec[11 + slot(e[q].tx)];
+      b.sy[q] = spec[11 + slot(e[q].ty)];
+      b.out[q] = spec[17 + q];
+    }
+    auto a = xf(XF_SCALE, nid, 1, nz + 1, g.nx, g.ny, nc);
+    a.c0 = 1.0 / double(g.nx * g.ny);
+    for (int q = 0; q < nid; ++q) {
+      a.in[q] = F[ids[q]];
+      a.out[q] = spec[11 + q];
+    }
+    use_refs(a, nid);  // derivatives of the per-level constants vanish
+    launch_xfwd<T>(g.nx, a, st);
+    b.ncols = nc;
+    b.nkp = nk_back();
+    b.ppitch = pitch(b.nkp);
+    b.spitch = b.opitch = pitch(nc);
+    b.pstride = (long)FNY * b.ppitch;
+    b.sstride = b.ostride = (long)g.ny * b.spitch;
+    b.plane0 = 1;
+    b.nplanes = nz + 1;
+    b.ngroups = neq;
+    b.lp = nz;
+    b.tt = back_rows();
+    b.nxh = g.nx / 2;
+    b.lhx = g.lhx;
+    b.kkx = kkx;
+    b.kky = kky;
+    b.tw_p = twiddles(FNY);
+    b.tw_s = twiddles(g.ny);
+    launch_yrhs<T>(FNY, g.ny, b, st);
+    auto c = xi(XI_DIV, neq, 1, nz + 1, g.nx, g.ny, nc);
+    c.c0 = 1.0 / dz();
+    c.fresh = 1;
+    for (int q = 0; q < neq; ++q) {
+      c.in[q] = spec[17 + q];
+      c.out[q] = F[e[q].rhs];
+      c.aux[q] = F[e[q].tz];
+      c.lo[q] = e[q].stag;
+      c.pf[q] = e[q].pf;
+      if (mixed()) c.refin[q] = refbuf[6 + q];
+    }
+    c.lo_ref = 1;
+    c.hi_ref = nz;
+    c.out[8] = layers ? PL[LES_BOTTOM_WK_PRESS] : nullptr;
+    c.out[9] = layers ? PL[LES_TOP_WK_PRESS] : nullptr;
+    launch_xinv<T>(g.nx, c, st);
   }
 
   // compute_convective_trunc leaves its vorticity scratch in the ghost levels
@@ -2149,16 +2236,19 @@ class Solver final : public SolverBase {
       plane_ops(6, dst, src, nullptr);
       for (int q = 0; q < 3; ++q) std::swap(F[r[q]], F[rf[q]]);
     }
-    {
-      Tag tag_(this, "convec");
-      if (from_spectra) fine_from_spectra();
-      else fine_from_fields();
-      fine_products(LES_RHSX, LES_RHSY, LES_RHSZ);
+    if (from_spectra) {
+      {
+        Tag tag_(this, "convec");
+        fine_from_spectra();
+      }
+      rhs_from_products();
+    } else {
+      dealias_convec(LES_RHSX, LES_RHSY, LES_RHSZ);
+      DivEq e[3] = {{LES_RHSX, LES_TXX, LES_TXY, LES_TXZ, 1, P.pfx},
+                    {LES_RHSY, LES_TXY, LES_TYY, LES_TYZ, 1, P.pfy},
+                    {LES_RHSZ, LES_TXZ, LES_TYZ, LES_TZZ, 0, 0.0}};
+      div_eqs(e, 3, true);
     }
-    DivEq e[3] = {{LES_RHSX, LES_TXX, LES_TXY, LES_TXZ, 1, P.pfx},
-                  {LES_RHSY, LES_TXY, LES_TYY, LES_TYZ, 1, P.pfy},
-                  {LES_RHSZ, LES_TXZ, LES_TYZ, LES_TZZ, 0, 0.0}};
-    div_eqs(e, 3, true);
     rhs_extras();
   }
 

@@ -1142,6 +1142,186 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
   }
 }
 
+// ------------------------------------------------ right-hand side in y ----
+// One y pass for a whole right-hand side: per column the forward transform of
+// the convective products (NF rows, truncated or masked to N), of the two
+// stresses (i kx t_x + i ky t_y), their sum, and one inverse transform.
+template <typename T>
+struct YRArgs {
+  int C, lc, SI;       // C = 1 << lc columns per CTA, column stride of a shared slot
+  int ncols;           // output columns
+  int nkp;             // columns of the products (the rest are zero)
+  int ppitch, spitch, opitch;  // complex values between rows of products / stresses / output
+  long pstride, sstride, ostride;  // complex values between planes
+  int plane0, nplanes, ngroups, lp;  // products exist on levels up to lp
+  int tt;              // 2/3 rule (NF == N): largest |ky| of the products kept
+  int nxh, lhx;
+  const cplx<T>* p[4];
+  const cplx<T>* sx[4];
+  const cplx<T>* sy[4];
+  cplx<T>* out[4];
+  const T* kkx;
+  const T* kky;
+  const cplx<T>* tw_p;  // length NF table
+  const cplx<T>* tw_s;  // length N table
+};
+
+// start the copy of one input's columns (C columns x NR rows) into a slot
+template <typename T, int NR, int TL>
+__device__ __forceinline__ void yr_copy(const YRArgs<T>& a, const cplx<T>* base, long plane, int pitch, int col0,
+                                        int lim, cplx<T>* slot) {
+  const int c = threadIdx.x & (a.C - 1);
+  const int ky0 = threadIdx.x >> a.lc;
+  const int kx = col0 + c;
+  const bool valid = kx < lim;
+  const cplx<T>* src = valid ? base + plane + kx + (long)ky0 * pitch : base;
+  cplx<T>* dst = slot + c * a.SI + ky0;
+  const long step = (long)TL * pitch;
+#pragma unroll
+  for (int i = 0; i < NR / TL; ++i) cp_async<int(sizeof(cplx<T>))>(dst + TL * i, valid ? src + i * step : base, valid);
+}
+
+// Persistent CTAs over (column block, level, equation).  The three inputs of
+// an item and of the next ones pass through a ring of two shared slots, each
+// refilled with the input after next as soon as its transform has left it, so
+// that a copy runs under every transform; the inverse transform and the
+// copy-out use the slot of the item's last input.  Two slots of the longer
+// length per column keep 16 warps per SM in FP32 (three inputs side by side:
+// 12), the register limit.
+template <typename T, int NF, int N>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRArgs<T> a) {
+  constexpr int TL = Geo<N>::T;
+  static_assert(Geo<NF>::T == TL, "both lengths must share the lanes per sequence");
+  constexpr int EF = Geo<NF>::E, E = Geo<N>::E;
+  constexpr int PI_ = Layout<NF, false>::in, PO = Layout<NF, false>::out;
+  constexpr int FI = Layout<N, false>::in, FO = Layout<N, false>::out;
+  constexpr int II = Layout<N, true>::in, IO = Layout<N, true>::out;
+  static_assert(FO == II, "forward output layout must feed the inverse");
+  constexpr bool SAME = NF == N;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* twp = reinterpret_cast<cplx<T>*>(smem_raw);  // forward NF (shared with forward N where equal)
+  cplx<T>* tws = twp + (SAME ? 0 : Twm<NF, false>::len);
+  cplx<T>* twi = tws + Twm<N, false>::len;
+  T* kyrow = reinterpret_cast<T*>(twi + Twm<N, true>::len);
+  cplx<T>* ring = reinterpret_cast<cplx<T>*>(kyrow + ((N + 3) & ~3));
+  const int C = a.C, SI = a.SI;
+  if constexpr (!SAME) twm_build<T, NF, false>(a.tw_p, twp, threadIdx.x, blockDim.x);
+  twm_build<T, N, false>(a.tw_s, tws, threadIdx.x, blockDim.x);
+  twm_build<T, N, true>(a.tw_s, twi, threadIdx.x, blockDim.x);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) kyrow[i] = a.kky[(long)i * a.lhx];
+  const int ncb = (a.ncols + C - 1) / C;
+  const long nitems = (long)ncb * a.nplanes * a.ngroups;
+  // input `in` (0 products, 1 t_x, 2 t_y) of item `item` into ring slot `sl`
+  auto issue = [&](long item, int in, int sl) {
+    if (item < nitems) {
+      const int col0 = umod32(item, ncb) * C;
+      const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
+      const int grp = udiv32(item, (long)ncb * a.nplanes);
+      cplx<T>* slot = ring + sl * C * SI;
+      if (in == 0)
+        yr_copy<T, NF, TL>(a, a.p[grp], (long)l * a.pstride, a.ppitch, col0, l <= a.lp ? a.nkp : 0, slot);
+      else
+        yr_copy<T, N, TL>(a, in == 1 ? a.sx[grp] : a.sy[grp], (long)l * a.sstride, a.spitch, col0, a.ncols, slot);
+    }
+    cp_async_commit();
+  };
+  issue(blockIdx.x, 0, 0);
+  issue(blockIdx.x, 1, 1);
+  const int c = threadIdx.x / TL;
+  const int lt = threadIdx.x % TL;
+  int sl = 0;  // slot of the current input
+  for (long item = blockIdx.x; item < nitems; item += gridDim.x, sl ^= 1) {
+    const int col0 = umod32(item, ncb) * C;
+    const int kx = col0 + c;
+    const bool live = kx < a.ncols && kx != a.nxh;
+    cplx<T> w[E];  // the sum, forward output layout of N (groups FO)
+    {
+      cp_async_wait<1>();
+      __syncthreads();
+      cplx<T>* seq = ring + (sl * C + c) * SI;
+      cplx<T> f[EF];
+#pragma unroll
+      for (int g = 0; g < EF / PI_; ++g)
+#pragma unroll
+        for (int r = 0; r < PI_; ++r) f[g * PI_ + r] = seq[lt + TL * g + r * (NF / PI_)];
+      reg_fft<T, NF, false>(f, seq, lt, SAME ? tws : twp);
+      if constexpr (SAME) {
+#pragma unroll
+        for (int g = 0; g < E / FO; ++g)
+#pragma unroll
+          for (int r = 0; r < FO; ++r) {
+            const int ky = lt + TL * g + r * (N / FO);
+            const bool keep = ky <= a.tt || ky >= N - a.tt;
+            w[g * FO + r] = keep ? f[g * FO + r] : cplx<T>{T(0), T(0)};
+          }
+      } else {
+        // truncation NF -> N in the lane (as in k_ypass): m' < E/2 from m',
+        // the rest from m' + E/2; lane 0 drops ky = N/2
+        constexpr int GP = EF / PO, GO = E / II;
+        static_for<E>([&](auto mc) {
+          constexpr int mo = decltype(mc)::value;
+          constexpr int ms = mo < E / 2 ? mo : mo + E / 2;
+          constexpr int wi = (mo % GO) * II + mo / GO, fi = (ms % GP) * PO + ms / GP;
+          w[wi] = (mo == E / 2 && lt == 0) ? cplx<T>{T(0), T(0)} : f[fi];
+        });
+      }
+      __syncthreads();
+      issue(item, 2, sl);
+    }
+#pragma unroll 1
+    for (int in = 1; in <= 2; ++in) {
+      sl ^= 1;
+      cp_async_wait<1>();
+      __syncthreads();
+      cplx<T>* seq = ring + (sl * C + c) * SI;
+      cplx<T> f[E];
+#pragma unroll
+      for (int g = 0; g < E / FI; ++g)
+#pragma unroll
+        for (int r = 0; r < FI; ++r) f[g * FI + r] = seq[lt + TL * g + r * (N / FI)];
+      reg_fft<T, N, false>(f, seq, lt, tws);
+      const T kxv = live ? a.kkx[kx] : T(0);
+#pragma unroll
+      for (int g = 0; g < E / FO; ++g)
+#pragma unroll
+        for (int r = 0; r < FO; ++r) {
+          const int ky = lt + TL * g + r * (N / FO);
+          if (live && ky != N / 2)
+            w[g * FO + r] = c_add(w[g * FO + r], ik_mul(in == 1 ? kxv : kyrow[ky], f[g * FO + r]));
+        }
+      if (in == 1) {
+        __syncthreads();
+        issue(item + gridDim.x, 0, sl);
+      }
+    }
+    {
+      cplx<T>* seq = ring + (sl * C + c) * SI;
+      __syncwarp();
+      reg_fft<T, N, true>(w, seq, lt, twi);
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < E / IO; ++g)
+#pragma unroll
+        for (int r = 0; r < IO; ++r) seq[lt + TL * g + r * (N / IO)] = w[g * IO + r];
+      __syncthreads();
+      const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
+      const int grp = udiv32(item, (long)ncb * a.nplanes);
+      const int cc = threadIdx.x & (C - 1);
+      const int kxx = col0 + cc;
+      if (kxx < a.ncols) {
+        const int ky0 = threadIdx.x >> a.lc;
+        cplx<T>* dst = a.out[grp] + (long)l * a.ostride + kxx + (long)ky0 * a.opitch;
+        const cplx<T>* srow = ring + (sl * C + cc) * SI + ky0;
+        const long step = (long)TL * a.opitch;
+#pragma unroll
+        for (int i = 0; i < N / TL; ++i) dst[i * step] = srow[TL * i];
+      }
+      __syncthreads();
+      issue(item + gridDim.x, 1, sl);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- xinv ----
 enum XIOp : int {
   XI_STORE = 0,  // out[f](l) = x_f for lo[f] <= l <= hi[f]
@@ -1172,6 +1352,8 @@ struct XIArgs {
   int lo[MAXIN], hi[MAXIN];
   const cplx<T>* in[MAXIN];
   const T* refin[MAXIN];  // per-level values added back to input field f
+  int lo_ref, hi_ref;     // combining ops: on these levels
+  int fresh;              // XI_DIV: the input is the whole horizontal part, out is not read
   T* out[16];
   float* outf[16];  // FP32 outputs of an FP64 transform (out_f32 = 1, XI_STORE)
   int out_f32;
@@ -1553,7 +1735,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     const int j = rowj[r];
     T* xw0 = const_cast<T*>(xs) + (long)(r * a.nin) * XS + i0;
     for (int f = 0; f < a.nin; ++f)  // this thread alone touches (r, i0..i0+3)
-      if (a.refin[f]) {
+      if (a.refin[f] && l >= a.lo_ref && l <= a.hi_ref) {
         const T rf = a.refin[f][l];
 #pragma unroll
         for (int q = 0; q < 4; ++q) xw0[f * XS + q] += rf;
@@ -1574,7 +1756,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         if (l >= 1 && l <= a.nz) {
           const V dzq = a.lo[q] ? rdz * (vld<V>(tz, off + pl) - vld<V>(tz, off))   // ddz_w
                                 : rdz * (vld<V>(tz, off) - vld<V>(tz, off - pl));  // ddz_uv
-          vst(a.out[q] + off, ((vld<V>(a.out[q], off) + xq) + dzq) + vsplat<V>(T(a.pf[q])));
+          const V base = a.fresh ? xq : vld<V>(a.out[q], off) + xq;
+          vst(a.out[q] + off, (base + dzq) + vsplat<V>(T(a.pf[q])));
           if (!a.lo[q] && l == 1 && a.out[8]) vst(a.out[8] + p2, xq + dzq);
         }
         if (!a.lo[q] && l == a.nz + 1 && a.out[9]) vst(a.out[9] + p2, xq);

@@ -112,7 +112,75 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
 
 
 template <typename T>
+void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
+  const int TL = lanes(N);
+  if (lanes(NF) != TL) throw CudaError(1, "yrhs: length pair with different lane counts");
+  const int W = 128 / int(sizeof(cplx<T>));
+  const int NL = std::max(NF, N);
+  auto stride = [&](int C) {  // as in launch_ypass
+    const int target = (32 / C) % W;
+    const int base = NL + NL / 16;
+    return base + ((target - base % W) % W + W) % W;
+  };
+  auto smem_for = [&](int C) {
+    return sizeof(cplx<T>) * ((NF == N ? 0 : twm_len(NF, false)) + twm_len(N, false) + twm_len(N, true) +
+                              (size_t)2 * C * stride(C)) +
+           sizeof(T) * ((N + 3) & ~3);
+  };
+  void (*kern)(YRArgs<T>) = nullptr;
+  switch (N) {
+#define YR_CASE(B) \
+  case B: kern = NF == B ? k_yrhs<T, B, B> : (NF == 3 * B / 2 ? k_yrhs<T, 3 * B / 2, B> : nullptr); break;
+    YR_CASE(16) YR_CASE(32) YR_CASE(64) YR_CASE(128) YR_CASE(256) YR_CASE(512)
+#undef YR_CASE
+    default: break;
+  }
+  if (!kern) throw CudaError(1, "yrhs: unsupported length pair " + std::to_string(NF) + "->" + std::to_string(N));
+  // columns per CTA: the most busy warps per SM, on a tie the CTA size
+  // nearest 128 threads; narrower where the items do not fill the chip (the
+  // rules of launch_ypass)
+  const KernelLimits lim = kernel_limits((const void*)kern);
+  const int warp_regs = ((lim.regs * 32 + 255) / 256) * 256;
+  double best = -1.0;
+  int lc = 0;
+  auto off128 = [&](int q) { return std::abs(std::log2(double((1 << q) * TL) / 128.0)); };
+  for (int q = 0; (1 << q) * TL <= std::min(256, lim.max_threads); ++q) {
+    const int threads = (1 << q) * TL;
+    const size_t sm = smem_for(1 << q);
+    if (threads < 32) continue;
+    if (sm > SMEM_CAP) break;
+    const int ctas = std::min({int(SM_SMEM / (sm + 1024)), 65536 / (warp_regs * (threads / 32)), 2048 / threads, 32});
+    if (ctas < 1) break;
+    const double busy = ctas * double(threads / 32) * std::min(1.0, double(a.ncols) / (1 << q));
+    if (busy > best + 1e-9 || (busy > best - 1e-9 && off128(q) < off128(lc))) {
+      best = busy;
+      lc = q;
+    }
+  }
+  const auto items = [&](int q) { return (long)ceil_div(a.ncols, 1 << q) * a.nplanes * a.ngroups; };
+  while (lc > 0 && items(lc) < sm_count() && (TL << (lc - 1)) >= 32 && (sizeof(cplx<T>) << (lc - 1)) >= 32) --lc;
+  a.lc = lc;
+  a.C = 1 << lc;
+  a.SI = stride(a.C);
+  const size_t smem = smem_for(a.C);
+  if (smem > SMEM_CAP) throw CudaError(1, "yrhs: shared memory request too large");
+  if (items(lc) == 0) return;
+  const int threads = a.C * TL;
+  const int grid = int(std::min<long>(items(lc), (long)resident_ctas((const void*)kern, threads, smem)));
+  hook_before("yrhs", double(a.nplanes) * a.ngroups * sizeof(cplx<T>) *
+                          (double(a.nkp) * NF + 2.0 * a.ncols * N + double(a.ncols) * N));
+  kern<<<grid, threads, smem, st>>>(a);
+  LES_CHECK_LAUNCH();
+  hook_after();
+}
+
+template <typename T>
 void set_attrs_ypass() {
+#define YR(B)                                                                                                  \
+  LES_CUDA(cudaFuncSetAttribute(k_yrhs<T, B, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
+  LES_CUDA(cudaFuncSetAttribute(k_yrhs<T, 3 * B / 2, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
+  YR(16) YR(32) YR(64) YR(128) YR(256) YR(512)
+#undef YR
 #define YA(A, B) \
   LES_CUDA(cudaFuncSetAttribute(k_ypass<T, A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
 #define YF(A) \
@@ -127,6 +195,8 @@ void set_attrs_ypass() {
 
 template void launch_ypass<float>(int, int, YPArgs<float>, int, int, cudaStream_t);
 template void launch_ypass<double>(int, int, YPArgs<double>, int, int, cudaStream_t);
+template void launch_yrhs<float>(int, int, YRArgs<float>, cudaStream_t);
+template void launch_yrhs<double>(int, int, YRArgs<double>, cudaStream_t);
 template void set_attrs_ypass<float>();
 template void set_attrs_ypass<double>();
 
