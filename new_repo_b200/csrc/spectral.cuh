@@ -879,10 +879,13 @@ __device__ __forceinline__ void yp_issue(const YPArgs<T>& a, long item, int ncb,
 }
 
 // FWD: forward transforms only (YP_FWDKILL, YP_PRESS), compiled without the
-// inverse so that it keeps fewer registers (more resident warps)
+// inverse so that it keeps fewer registers.  FP64: 168 registers (three CTAs
+// of 128 threads) where the compiler would take 255 (two); the passes with
+// several outputs spill ~200 bytes for it and still gain (the 21 test-filtered
+// fields at 256^3: 2965 -> 2286 us, then 1993 without the columns past the
+// narrower filter).
 template <typename T, int NY, int NYO, bool FWD = false>
-__global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
-                                  (FWD && sizeof(T) == 8) ? 3 : (sizeof(T) == 4 ? 2 : 1))
+__global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3 : 2)
     k_ypass(const YPArgs<T> a) {
   constexpr int TL = Geo<NY>::T;
   static_assert(Geo<NYO>::T == TL, "pad/truncate pairs must share the lanes per sequence");
@@ -1008,6 +1011,7 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
   const int nout = layers ? 2 : a.nout;
   for (int q = 0; q < nout; ++q) {
     if (!layers && !a.out[grp * a.nout + q]) continue;  // an optional output left out (the same for the whole CTA)
+    if (a.op == YP_FILTER2 && q == 1 && col0 >= a.ncols1) continue;  // all columns beyond the narrower filter
     if constexpr (SAME) {
       // forward output layout (groups FO) == inverse input layout; the
       // stress divergence already holds its result in w
@@ -1149,6 +1153,7 @@ __global__ void __launch_bounds__((FWD && sizeof(T) == 8) ? 128 : 256,
 template <typename T>
 struct YRArgs {
   int C, lc, SI;       // C = 1 << lc columns per CTA, column stride of a shared slot
+  int nslot;           // shared slots (set by the launcher): 2 = a copy runs under every transform
   int ncols;           // output columns
   int nkp;             // columns of the products (the rest are zero)
   int ppitch, spitch, opitch;  // complex values between rows of products / stresses / output
@@ -1187,9 +1192,13 @@ __device__ __forceinline__ void yr_copy(const YRArgs<T>& a, const cplx<T>* base,
 // that a copy runs under every transform; the inverse transform and the
 // copy-out use the slot of the item's last input.  Two slots of the longer
 // length per column keep 16 warps per SM in FP32 (three inputs side by side:
-// 12), the register limit.
+// 12), the register limit.  Where two slots leave room for fewer warps, one
+// slot refilled between transforms takes their place: FP32 at 512 points 12
+// -> 16 warps (814 -> 651 us, 512 x 512 x 96), FP64 at 512 points 4 -> 8 (400
+// -> 335 us, 512 x 512 x 24), at 256 points 6 -> 12 (198 -> 181 us at 64
+// levels, 741 -> 763 us at 256), at 64 points 22.9 -> 25.1 us.
 template <typename T, int NF, int N>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRArgs<T> a) {
+__global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3 : 2) k_yrhs(const YRArgs<T> a) {
   constexpr int TL = Geo<N>::T;
   static_assert(Geo<NF>::T == TL, "both lengths must share the lanes per sequence");
   constexpr int EF = Geo<NF>::E, E = Geo<N>::E;
@@ -1225,19 +1234,35 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRAr
     }
     cp_async_commit();
   };
-  issue(blockIdx.x, 0, 0);
-  issue(blockIdx.x, 1, 1);
+  // the next input to copy; a slot is free again when its input is transformed
+  const int flip = a.nslot - 1;
+  long aitem = blockIdx.x;
+  int ain = 0, asl = 0;
+  auto issue_next = [&]() {
+    issue(aitem, ain, asl);
+    asl ^= flip;
+    if (++ain == 3) {
+      ain = 0;
+      aitem += gridDim.x;
+    }
+  };
+  auto arrived = [&]() {
+    if (flip) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();
+  };
+  issue_next();
+  if (flip) issue_next();
   const int c = threadIdx.x / TL;
   const int lt = threadIdx.x % TL;
   int sl = 0;  // slot of the current input
-  for (long item = blockIdx.x; item < nitems; item += gridDim.x, sl ^= 1) {
+  for (long item = blockIdx.x; item < nitems; item += gridDim.x, sl ^= flip) {
     const int col0 = umod32(item, ncb) * C;
     const int kx = col0 + c;
     const bool live = kx < a.ncols && kx != a.nxh;
     cplx<T> w[E];  // the sum, forward output layout of N (groups FO)
     {
-      cp_async_wait<1>();
-      __syncthreads();
+      arrived();
       cplx<T>* seq = ring + (sl * C + c) * SI;
       cplx<T> f[EF];
 #pragma unroll
@@ -1266,13 +1291,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRAr
         });
       }
       __syncthreads();
-      issue(item, 2, sl);
+      issue_next();
     }
 #pragma unroll 1
     for (int in = 1; in <= 2; ++in) {
-      sl ^= 1;
-      cp_async_wait<1>();
-      __syncthreads();
+      sl ^= flip;
+      arrived();
       cplx<T>* seq = ring + (sl * C + c) * SI;
       cplx<T> f[E];
 #pragma unroll
@@ -1291,7 +1315,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRAr
         }
       if (in == 1) {
         __syncthreads();
-        issue(item + gridDim.x, 0, sl);
+        issue_next();
       }
     }
     {
@@ -1317,7 +1341,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_yrhs(const YRAr
         for (int i = 0; i < N / TL; ++i) dst[i * step] = srow[TL * i];
       }
       __syncthreads();
-      issue(item + gridDim.x, 1, sl);
+      issue_next();
     }
   }
 }

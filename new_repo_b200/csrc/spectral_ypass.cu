@@ -122,9 +122,9 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
     const int base = NL + NL / 16;
     return base + ((target - base % W) % W + W) % W;
   };
-  auto smem_for = [&](int C) {
+  auto smem_for = [&](int C, int ns) {
     return sizeof(cplx<T>) * ((NF == N ? 0 : twm_len(NF, false)) + twm_len(N, false) + twm_len(N, true) +
-                              (size_t)2 * C * stride(C)) +
+                              (size_t)ns * C * stride(C)) +
            sizeof(T) * ((N + 3) & ~3);
   };
   void (*kern)(YRArgs<T>) = nullptr;
@@ -136,33 +136,36 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
     default: break;
   }
   if (!kern) throw CudaError(1, "yrhs: unsupported length pair " + std::to_string(NF) + "->" + std::to_string(N));
-  // columns per CTA: the most busy warps per SM, on a tie the CTA size
-  // nearest 128 threads; narrower where the items do not fill the chip (the
-  // rules of launch_ypass)
+  // columns per CTA and slots: the most busy warps per SM, on a tie two slots,
+  // then the CTA size nearest 128 threads; narrower where the items do not
+  // fill the chip (the rules of launch_ypass)
   const KernelLimits lim = kernel_limits((const void*)kern);
   const int warp_regs = ((lim.regs * 32 + 255) / 256) * 256;
   double best = -1.0;
-  int lc = 0;
+  int lc = 0, nslot = 2;
   auto off128 = [&](int q) { return std::abs(std::log2(double((1 << q) * TL) / 128.0)); };
-  for (int q = 0; (1 << q) * TL <= std::min(256, lim.max_threads); ++q) {
-    const int threads = (1 << q) * TL;
-    const size_t sm = smem_for(1 << q);
-    if (threads < 32) continue;
-    if (sm > SMEM_CAP) break;
-    const int ctas = std::min({int(SM_SMEM / (sm + 1024)), 65536 / (warp_regs * (threads / 32)), 2048 / threads, 32});
-    if (ctas < 1) break;
-    const double busy = ctas * double(threads / 32) * std::min(1.0, double(a.ncols) / (1 << q));
-    if (busy > best + 1e-9 || (busy > best - 1e-9 && off128(q) < off128(lc))) {
-      best = busy;
-      lc = q;
+  for (int ns = 2; ns >= 1; --ns)
+    for (int q = 0; (1 << q) * TL <= std::min(256, lim.max_threads); ++q) {
+      const int threads = (1 << q) * TL;
+      const size_t sm = smem_for(1 << q, ns);
+      if (threads < 32) continue;
+      if (sm > SMEM_CAP) break;
+      const int ctas = std::min({int(SM_SMEM / (sm + 1024)), 65536 / (warp_regs * (threads / 32)), 2048 / threads, 32});
+      if (ctas < 1) break;
+      const double busy = ctas * double(threads / 32) * std::min(1.0, double(a.ncols) / (1 << q));
+      if (busy > best + 1e-9 || (busy > best - 1e-9 && ns == nslot && off128(q) < off128(lc))) {
+        best = busy;
+        lc = q;
+        nslot = ns;
+      }
     }
-  }
   const auto items = [&](int q) { return (long)ceil_div(a.ncols, 1 << q) * a.nplanes * a.ngroups; };
   while (lc > 0 && items(lc) < sm_count() && (TL << (lc - 1)) >= 32 && (sizeof(cplx<T>) << (lc - 1)) >= 32) --lc;
   a.lc = lc;
   a.C = 1 << lc;
+  a.nslot = nslot;
   a.SI = stride(a.C);
-  const size_t smem = smem_for(a.C);
+  const size_t smem = smem_for(a.C, nslot);
   if (smem > SMEM_CAP) throw CudaError(1, "yrhs: shared memory request too large");
   if (items(lc) == 0) return;
   const int threads = a.C * TL;
