@@ -352,6 +352,7 @@ class Solver final : public SolverBase {
     a.in_pstride = (long)rows_pp * NX;
     a.out_pstride = (long)rows_pp * a.opitch;
     a.tw = twiddles(NX);
+    a.status = dstatus;
     return a;
   }
   YPArgs<T> yp(int op, int nin, int nout, int ncols, int nk_in, int NY, int nk_out, int NYO, int plane0) {
@@ -1555,6 +1556,7 @@ class Solver final : public SolverBase {
     a.in_pstride = (long)g.ny * g.nx;
     a.out_pstride = (long)g.ny * nk;
     a.tw = twiddles64(g.nx);
+    a.status = dstatus;
     return a;
   }
   template <typename S>
@@ -1609,6 +1611,7 @@ class Solver final : public SolverBase {
     auto a = xf_s<S>(XF_PRESS, 3, 1, nz + 1, g.lhx);
     a.c0 = c / tadv1;
     a.c1 = P.dt;
+    a.rc1 = 1.0 / P.dt;
     a.c2 = c;
     a.c3 = 1.0 / dz();
     a.kxr = kkxd;

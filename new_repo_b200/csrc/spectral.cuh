@@ -132,12 +132,15 @@ struct XFArgs {
   long in_pstride; // elements per plane of the input grid
   long in_rstride; // elements per row of the input grid (== NX)
   double c0, c1, c2, c3;
+  double rc1;      // XF_PRESS: 1 / c1
   const T* in[16];
   const float* inf[16];  // FP32 inputs of an FP64 transform (in_f32 = 1)
   int in_f32;
   cplx<T>* out[MAXIN];
   long out_pstride;  // rows_pp * nk
   const T* kxr;      // x wavenumbers (XF_PRESS), Nyquist zero
+  int nsrc, nbuf, stage_rows;  // k_xfwd_row: staged rows per grid row, stages, slots per stage (set by the launcher)
+  unsigned* status;  // device status word (ST_COPY_WAIT), may be null
   const cplx<T>* tw; // exp(-2 pi i m / NX), m < NX
 };
 
@@ -260,39 +263,6 @@ __device__ __forceinline__ void xf_load_op(const XFArgs<T>& a, int l, int j, int
     if constexpr (OP == XF_SCALE) {
       for (int f = 0; f < a.nf; ++f)
         put(f, T(a.c0) * (a.in_f32 ? vldg<V>(a.inf[f], off) : vldg<V>(a.in[f], off)));
-    } else if constexpr (OP == XF_PRESS) {
-      // compute_pressure.f90:138-140, 176-190: u, v and (w(l+1) - w(l)) / dz
-      // over dt tadv1 nx ny (w(nz+1) counts as zero); c0 = 1/(nx ny tadv1),
-      // c1 = dt, c2 = 1/(nx ny).  Level nz+1 carries the two pressure-BC
-      // layers instead (inputs 3, 4): the bottom one, scaled by c2 in place
-      // (compute_pressure.f90:151-165), goes where it reaches output 0 as
-      // itself, the top one to output 1.
-      if constexpr (sizeof(T) == 8) {
-        auto from = [&](auto* const* in) {
-          using S = typename std::remove_const<typename std::remove_pointer<
-              typename std::remove_reference<decltype(in[0])>::type>::type>::type;
-          if (l > a.nz) {
-            const long p2 = (long)j * a.in_rstride + i;
-            S* bot = const_cast<S*>(in[3]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const S b = S(a.c2) * bot[p2 + q];
-              bot[p2 + q] = b;
-              v[0 * vs + q] = T(0);
-              v[1 * vs + q] = T(a.c2) * T(in[4][p2 + q]);
-              v[2 * vs + q] = T(b);
-            }
-          } else {
-            put(0, T(a.c0) * (vldg<V>(in[0], off) / T(a.c1)));
-            put(1, T(a.c0) * (vldg<V>(in[1], off) / T(a.c1)));
-            const V w0 = vldg<V>(in[2], off);
-            const V w1 = (l < a.nz) ? vldg<V>(in[2], off + a.in_pstride) : vsplat<V>(T(0));
-            put(2, T(a.c0) * (((w1 - w0) * vsplat<V>(T(a.c3))) / T(a.c1)));
-          }
-        };
-        if (a.in_f32) from(a.inf);
-        else from(a.in);
-      }
     } else if constexpr (OP == XF_CONV_IN) {
       // compute_convective_padd.f90:133-165
       const T c = T(a.c0);
@@ -548,7 +518,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     case XF_CONV_IN: load_op(std::integral_constant<int, XF_CONV_IN>{}); break;
     case XF_PROD: load_op(std::integral_constant<int, XF_PROD>{}); break;
     case XF_LASD: load_op(std::integral_constant<int, XF_LASD>{}); break;
-    case XF_PRESS: load_op(std::integral_constant<int, XF_PRESS>{}); break;
     case XF_PROD_SC: load_op(std::integral_constant<int, XF_PROD_SC>{}); break;
     case XF_SCDYN: load_op(std::integral_constant<int, XF_SCDYN>{}); break;
     case XF_PRESS_INC: load_op(std::integral_constant<int, XF_PRESS_INC>{}); break;
@@ -574,7 +543,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
 #pragma unroll
       for (int r = 0; r < RO; ++r) seq[lane_t + TL * g + r * (M / RO)] = v[g * RO + r];
     __syncwarp();
-    if (s < nseq && a.op != XF_PRESS) {
+    if (s < nseq) {
       const int r = udiv32(s, a.nf);
       const int f = s - r * a.nf;
       const int l = rowl[r];
@@ -585,166 +554,247 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       }
     }
   }
-  if constexpr (sizeof(T) == 8) {
-    if (a.op == XF_PRESS) {
-      // two spectra leave for the three transforms of a row: i kx u^ + w'^
-      // and v^ (one warp per row, consecutive modes on consecutive lanes)
-      __syncthreads();
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-      for (int r = warp; r < a.R; r += nwarps) {
-        const int l = rowl[r];
-        if (l < 0) continue;
-        const cplx<T>* zu = buf + (long)(3 * r) * SL;
-        const cplx<T>* zv = zu + SL;
-        const cplx<T>* zw = zv + SL;
-        const long o = (long)l * a.out_pstride + (long)rowj[r] * a.opitch;
-        for (int k = lane; k <= M; k += 32) {
-          const int k0 = k == M ? 0 : k, k1 = k == 0 ? 0 : M - k;  // Z_M is Z_0
-          const cplx<T> h = tw[k];
-          a.out[0][o + k] = c_add(ik_mul(a.kxr[k], r2c_split(zu[k0], zu[k1], h)), r2c_split(zw[k0], zw[k1], h));
-          a.out[1][o + k] = r2c_split(zv[k0], zv[k1], h);
-        }
-      }
-    }
-  }
 }
 
-// start the copies of the input rows of batch `item` (one warp per row,
-// 16-byte pieces)
-template <typename T, int NX>
-__device__ __forceinline__ void xf_issue(const XFArgs<T>& a, long item, T* stage) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  constexpr int PIECES = NX * int(sizeof(T)) / 16;
-  const int nrow = a.R * a.nf;
-  for (int s = warp; s < nrow; s += nwarps) {
-    const int r = udiv32(s, a.nf);
-    const int q = s - r * a.nf;
+// ---- x forward pass of whole rows (k_xfwd_row) ----
+// For ops whose inputs are rows as they stand: scalings (XF_SCALE) and the
+// pressure right-hand side (XF_PRESS).  A bulk copy brings each input row
+// straight into the shared slot its transform works in; the scale, the
+// reference and the conversion of FP32 rows are applied as the registers are
+// loaded.  Source row f of level l, row j (nullptr: none).
+template <typename T, typename S>
+__device__ __forceinline__ const S* xr_source(const XFArgs<T>& a, int f, int l, int j) {
+  const S* const* in;
+  if constexpr (std::is_same<S, T>::value) in = a.in;
+  else in = a.inf;
+  const long row = (long)l * a.in_pstride + (long)j * a.in_rstride;
+  if (a.op != XF_PRESS) return in[f] + row;
+  // XF_PRESS: sources u, v, w at l, w at l + 1 (none above level nz: w(nz+1)
+  // counts as zero); the plane past level nz holds the two boundary layers,
+  // the top one in place of v, the bottom one in place of w
+  if (l > a.nz) return f == 1 ? in[4] + (long)j * a.in_rstride : (f == 2 ? in[3] + (long)j * a.in_rstride : nullptr);
+  if (f < 3) return in[f] + row;
+  return l < a.nz ? in[2] + row + a.in_pstride : nullptr;
+}
+
+// warp 0: announce the bytes of batch `item` and start one bulk copy per row
+template <typename T, typename S, int NX, int SL>
+__device__ __forceinline__ void xr_issue(const XFArgs<T>& a, long item, cplx<T>* stage, uint64_t* mbar) {
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  const int ns = a.nsrc;
+  const long left = a.nrows - item * a.R;
+  const int nrow = int(left < a.R ? left : a.R) * ns;
+  constexpr unsigned RB = NX * sizeof(S);
+  auto source = [&](int s) {
+    const int r = udiv32(s, ns), f = s - r * ns;
     const long g = item * a.R + r;
-    const bool valid = g < a.nrows;
-    const T* base = a.in[q];
-    const T* row = valid ? base + (long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride +
-                               long(umod32(g, a.rows_pp)) * a.in_rstride
-                         : base;
-    T* dst = stage + (long)s * NX;
-    for (int k = lane; k < PIECES; k += 32)
-      cp_async<16>(reinterpret_cast<unsigned char*>(dst) + 16 * k,
-                   valid ? reinterpret_cast<const unsigned char*>(row) + 16 * k
-                         : reinterpret_cast<const unsigned char*>(base),
-                   valid);
+    return xr_source<T, S>(a, f, a.plane0 + udiv32(g, a.rows_pp), umod32(g, a.rows_pp));
+  };
+  unsigned mine = 0;
+  for (int s = lane; s < nrow; s += 32)
+    if (source(s)) mine += RB;
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane == 0) mbar_expect_tx(mbar, mine);
+  __syncwarp();
+  tc::fence_async_smem();  // earlier generic accesses of this stage come first
+  for (int s = lane; s < nrow; s += 32) {
+    const S* src = source(s);
+    if (src) bulk_g2s(stage + (long)s * SL, src, RB, mbar);
   }
 }
 
-// The x forward pass of scalings of a few fields (XF_SCALE): persistent CTAs
-// over batches of R rows, the input rows of the next batch copied into the
-// other shared stage with cp.async while the current batch is transformed.
-template <typename T, int NX>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2) k_xfwd_st(const XFArgs<T> a) {
+// x / c for a fixed c with rc = 1/c: Markstein's correction of the product
+// (P. Markstein, IBM J. Res. Dev. 34, 1990), the correctly rounded quotient
+// for a correctly rounded rc.  The pressure inputs are velocities over dt
+// whose divergence cancels; rounded as the reference's division rounds them
+// they cancel as its do (a plain product moved p's gradients by 2e-12).
+__device__ __forceinline__ double quot(double x, double c, double rc) {
+  const double q = x * rc;
+  return fma(fma(-q, c, x), rc, q);
+}
+
+// Persistent CTAs over batches of R rows with one or two stages of slots (two:
+// the next batch is copied while this one is transformed).  Against loading
+// through registers into the slots (k_xfwd) the pass has no load phase: at
+// 256^3 the gradients' pass went from 0.166 to 0.111, the stresses' from 0.213
+// to 0.203, the pressure's from 0.311 to 0.222 ms per step (mixed; FP64 0.298
+// to 0.203, 0.438 to 0.323, 0.326 to 0.228).  The smallest launches pay for
+// the barrier set-up (32^3: 8.9 -> 10.7 us).
+template <typename T, int NX, typename S>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const XFArgs<T> a) {
   constexpr int M = NX / 2;
   constexpr int TL = Geo<M>::T;
   constexpr int E = Geo<M>::E;
   constexpr int RI = Layout<M, false>::in;
   constexpr int RO = Layout<M, false>::out;
   constexpr int SL = slot_stride(M, int(sizeof(cplx<T>)));
-  constexpr int XS = 2 * SL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
   cplx<T>* twm = tw + NX;  // twiddle matrices of the M-point transform
+  const int ns = a.nsrc;   // staged rows per grid row
   const int nseq = a.R * a.nf;
   const int npad = seq_pad<M>(nseq);
-  T* stage0 = reinterpret_cast<T*>(twm + Twm<M, false>::len);
-  T* stage1 = stage0 + (long)a.R * a.nf * NX;
-  cplx<T>* buf = reinterpret_cast<cplx<T>*>(stage1 + (long)a.R * a.nf * NX);
-  T* refs = reinterpret_cast<T*>(buf + (long)npad * SL);
-  int* rowl = reinterpret_cast<int*>(refs + a.R * a.nf);
+  const long stage_len = (long)a.stage_rows * SL;
+  cplx<T>* stage0 = twm + Twm<M, false>::len;
+  cplx<T>* stage1 = stage0 + (a.nbuf > 1 ? stage_len : 0L);  // stage 0 again when single
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stage0 + a.nbuf * stage_len);
+  T* refs = reinterpret_cast<T*>(bars + 2);  // R * nf per-level references
+  int* rowl = reinterpret_cast<int*>(refs + ((nseq + 1) & ~1));
   int* rowj = rowl + a.R;
+  const long nitems = (a.nrows + a.R - 1) / a.R;
+  // the first copies start before the tables are built (warp 0 sets up the
+  // barriers and issues them)
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      tc::mbar_init(&bars[0], 1);
+      tc::mbar_init(&bars[1], 1);
+      tc::fence_mbar_init();
+    }
+    __syncwarp();
+    if ((long)blockIdx.x < nitems) xr_issue<T, S, NX, SL>(a, blockIdx.x, stage0, &bars[0]);
+  }
+  // the reference of row r, field f of a batch (one per thread; R nf <= 256)
+  auto ref_of = [&](long item) -> T {
+    if (!a.use_ref || item >= nitems || threadIdx.x >= nseq) return T(0);
+    const int r = udiv32(threadIdx.x, a.nf), f = threadIdx.x - r * a.nf;
+    const long g = item * a.R + r;
+    if (g >= a.nrows || !a.refout[f]) return T(0);
+    return T(a.c0) * a.in[f][(long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride];
+  };
+  T ref_next = ref_of(blockIdx.x);
   for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = c_scl(a.tw[i], T(0.5));  // W^k / 2 for the split
   twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
-  const long nitems = (a.nrows + a.R - 1) / a.R;
-  if ((long)blockIdx.x < nitems) {
-    xf_issue<T, NX>(a, blockIdx.x, stage0);
-    cp_async_commit();
-  }
+  __syncthreads();
+  unsigned phase = 0;  // bit b: parity of the next completion of bars[b]
   int stg = 0;
   for (long item = blockIdx.x; item < nitems; item += gridDim.x) {
     const long next = item + gridDim.x;
-    const T* stage = stg ? stage1 : stage0;
-    if (next < nitems) {
-      xf_issue<T, NX>(a, next, stg ? stage0 : stage1);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    cplx<T>* stage = stg ? stage1 : stage0;
+    if (a.nbuf > 1 && next < nitems) xr_issue<T, S, NX, SL>(a, next, stg ? stage0 : stage1, &bars[stg ^ 1]);
     const long g0 = item * a.R;
     for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
       const long g = g0 + r;
       rowl[r] = (g < a.nrows) ? a.plane0 + udiv32(g, a.rows_pp) : -1;
       rowj[r] = (g < a.nrows) ? umod32(g, a.rows_pp) : 0;
     }
-    __syncthreads();
-    if (a.use_ref) {  // per-level references: the (0,0) value of each field (from global)
-      for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
-        const int l = rowl[r];
-        if (l < 0) continue;
-        xf_load<T, T>(a, l, 0, 0, refs + r * a.nf, 1);
-        for (int f = 0; f < a.nf; ++f) {
-          if (!a.refout[f]) refs[r * a.nf + f] = T(0);
-          else if (rowj[r] == 0) a.refout[f][l] = T(double(refs[r * a.nf + f]) * a.ref_mul);
-        }
-      }
-      __syncthreads();
+    if (a.use_ref && threadIdx.x < nseq) {
+      const int r = udiv32(threadIdx.x, a.nf), f = threadIdx.x - r * a.nf;
+      const long g = g0 + r;
+      refs[threadIdx.x] = ref_next;
+      if (g < a.nrows && a.refout[f] && umod32(g, a.rows_pp) == 0)
+        a.refout[f][a.plane0 + udiv32(g, a.rows_pp)] = T(double(ref_next) * a.ref_mul);
     }
-    T* xr = reinterpret_cast<T*>(buf);
-    for (int idx = threadIdx.x; idx < a.R * (NX / 4); idx += blockDim.x) {
-      const int r = idx / (NX / 4);
-      const int i = 4 * (idx - r * (NX / 4));
-      T* dst = xr + (long)(r * a.nf) * XS + i;
-      const int l = rowl[r];
-      if (l >= 0) {
-        for (int f = 0; f < a.nf; ++f)
-          vst(dst + f * XS, T(a.c0) * vld<V4<T>>(stage + (long)(r * a.nf + f) * NX, (long)i));
-        if (a.use_ref)
-          for (int f = 0; f < a.nf; ++f) {
-            const T rf = refs[r * a.nf + f];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) dst[f * XS + q] -= rf;
-          }
-      } else {
-        for (int f = 0; f < a.nf; ++f) vst(dst + f * XS, vsplat<V4<T>>(T(0)));
-      }
+    ref_next = ref_of(next);
+    const bool late = !tc::mbar_wait(&bars[stg], (phase >> stg) & 1u);
+    phase ^= 1u << stg;
+    if (__syncthreads_or(late)) {
+      // as in k_xinv: record it, a last bounded wait for the copies in
+      // flight, and every thread of the CTA leaves
+      if (threadIdx.x == 0 && a.status) atomicOr(a.status, unsigned(ST_COPY_WAIT));
+      tc::mbar_wait(&bars[stg], (phase >> stg) & 1u ^ 1u);
+      if (a.nbuf > 1 && next < nitems) tc::mbar_wait(&bars[stg ^ 1], (phase >> (stg ^ 1)) & 1u);
+      return;
     }
-    for (int idx = nseq * SL + threadIdx.x; idx < npad * SL; idx += blockDim.x) buf[idx] = cplx<T>{T(0), T(0)};
-    __syncthreads();
     const int lane_t = threadIdx.x % TL;
     for (int base = 0; base < npad; base += blockDim.x / TL) {
       const int s = base + threadIdx.x / TL;
-      if (base + (threadIdx.x / 32) * (32 / TL) >= npad) break;
-      cplx<T>* seq = buf + (long)s * SL;
+      if (base + (threadIdx.x / 32) * (32 / TL) >= npad) break;  // whole warp beyond the slots
+      const bool valid = s < nseq;
+      const int r = valid ? udiv32(s, a.nf) : 0;
+      const int f = valid ? s - r * a.nf : 0;
+      const int l = valid ? rowl[r] : -1;
+      // slots past the last sequence follow the staged rows
+      cplx<T>* seq = stage + (long)(valid ? r * ns + f : a.R * ns + (s - nseq)) * SL;
       cplx<T> v[E];
+      if (l < 0) {
 #pragma unroll
-      for (int g = 0; g < E / RI; ++g)
+        for (int i = 0; i < E; ++i) v[i] = cplx<T>{T(0), T(0)};
+      } else {
+        // the row as pairs: z_m = x_2m + i x_2m+1
+        const cplx<S>* row = reinterpret_cast<const cplx<S>*>(seq);
+        auto at = [&](const cplx<S>* p, int m) { return cplx<T>{T(p[m].x), T(p[m].y)}; };
+        auto load = [&](auto get) {
 #pragma unroll
-        for (int r = 0; r < RI; ++r) v[g * RI + r] = seq[lane_t + TL * g + r * (M / RI)];
+          for (int g = 0; g < E / RI; ++g)
+#pragma unroll
+            for (int q = 0; q < RI; ++q) v[g * RI + q] = get(lane_t + TL * g + q * (M / RI));
+        };
+        const T c0 = T(a.c0);
+        if (a.op == XF_SCALE) {
+          const T rf = a.use_ref ? -refs[s] : T(0);
+          const cplx<T> cc = {c0, c0}, rr = {rf, rf};
+          load([&](int m) { return c_fma(at(row, m), cc, rr); });
+        } else if constexpr (sizeof(T) == 8) {  // XF_PRESS
+          if (l > a.nz) {
+            // boundary layers: nothing, the top one over nx ny, the bottom
+            // one scaled in place (compute_pressure.f90:151-165)
+            if (f == 0) {
+              load([&](int) { return cplx<T>{T(0), T(0)}; });
+            } else if (f == 1) {
+              load([&](int m) { return c_scl(at(row, m), T(a.c2)); });
+            } else {
+              cplx<S>* plane = reinterpret_cast<cplx<S>*>(const_cast<S*>(xr_source<T, S>(a, 2, l, rowj[r])));
+              const S sc = S(a.c2);
+              load([&](int m) {
+                const cplx<S> b = {sc * row[m].x, sc * row[m].y};
+                plane[m] = b;
+                return cplx<T>{T(b.x), T(b.y)};
+              });
+            }
+          } else {
+            // compute_pressure.f90:138-140: c0 (x / dt)
+            const double dt = a.c1, rdt = a.rc1;
+            auto h = [&](cplx<T> x) { return cplx<T>{c0 * quot(x.x, dt, rdt), c0 * quot(x.y, dt, rdt)}; };
+            if (f < 2) {
+              load([&](int m) { return h(at(row, m)); });
+            } else {
+              // (w(l+1) - w(l)) / dz, w(nz+1) = 0
+              const cplx<S>* up = reinterpret_cast<const cplx<S>*>(seq + SL);
+              const T cz = T(a.c3);
+              if (l < a.nz) load([&](int m) { return h(c_scl(c_sub(at(up, m), at(row, m)), cz)); });
+              else load([&](int m) { return h(c_scl(at(row, m), -cz)); });
+            }
+          }
+        }
+      }
       reg_fft<T, M, false>(v, seq, lane_t, twm);
       __syncwarp();
 #pragma unroll
       for (int g = 0; g < E / RO; ++g)
 #pragma unroll
-        for (int r = 0; r < RO; ++r) seq[lane_t + TL * g + r * (M / RO)] = v[g * RO + r];
+        for (int q = 0; q < RO; ++q) seq[lane_t + TL * g + q * (M / RO)] = v[g * RO + q];
       __syncwarp();
-      if (s < nseq) {
-        const int r = udiv32(s, a.nf);
-        const int f = s - r * a.nf;
-        const int l = rowl[r];
-        if (l >= 0) {
-          const int j = rowj[r];
-          cplx<T>* orow = a.out[f] + (long)l * a.out_pstride + (long)j * a.opitch;
-          xf_split_store<T, M, TL, E>(seq, tw, orow, lane_t, a.nk);
-        }
+      if (l >= 0 && a.op == XF_SCALE) {
+        cplx<T>* orow = a.out[f] + (long)l * a.out_pstride + (long)rowj[r] * a.opitch;
+        xf_split_store<T, M, TL, E>(seq, tw, orow, lane_t, a.nk);
       }
     }
     __syncthreads();
-    stg ^= 1;
+    if constexpr (sizeof(T) == 8) {
+      if (a.op == XF_PRESS) {
+        // two spectra leave for the three transforms of a row: i kx u^ + w'^
+        // and v^ (one warp per row, consecutive modes on consecutive lanes)
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+        for (int r = warp; r < a.R; r += nwarps) {
+          const int l = rowl[r];
+          if (l < 0) continue;
+          const cplx<T>* zu = stage + (long)(r * ns) * SL;
+          const cplx<T>* zv = zu + SL;
+          const cplx<T>* zw = zv + SL;
+          const long o = (long)l * a.out_pstride + (long)rowj[r] * a.opitch;
+          for (int k = lane; k <= M; k += 32) {
+            const int k0 = k == M ? 0 : k, k1 = k == 0 ? 0 : M - k;  // Z_M is Z_0
+            const cplx<T> h = tw[k];
+            a.out[0][o + k] = c_add(ik_mul(a.kxr[k], r2c_split(zu[k0], zu[k1], h)), r2c_split(zw[k0], zw[k1], h));
+            a.out[1][o + k] = r2c_split(zv[k0], zv[k1], h);
+          }
+        }
+        __syncthreads();
+      }
+    }
+    if (a.nbuf > 1) stg ^= 1;
+    else if (next < nitems) xr_issue<T, S, NX, SL>(a, next, stage0, &bars[0]);
   }
 }
 
@@ -1512,31 +1562,32 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   // one mbarrier per input stage (bulk staging)
   uint64_t* bars = reinterpret_cast<uint64_t*>(
       (reinterpret_cast<uintptr_t>(kxs + (a.nstage ? a.nk + 2 : 0)) + 7) & ~uintptr_t(7));
+  // persistent CTAs over batches of R rows; with two stages the spectral
+  // rows of the next batch are copied into the other stage while this one
+  // is transformed, with one stage after this batch's last read of it.  The
+  // first copies start before the tables are built (warp 0 sets up the
+  // barriers and issues them).
+  const long nitems = (a.nrows + a.R - 1) / a.R;
+  if (a.bulk) {
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        tc::mbar_init(&bars[0], 1);
+        tc::mbar_init(&bars[1], 1);
+        tc::fence_mbar_init();
+      }
+      __syncwarp();
+      if ((long)blockIdx.x < nitems) xi_issue_bulk<T>(a, blockIdx.x, stage0, &bars[0]);
+    }
+  } else if ((long)blockIdx.x < nitems) {
+    xi_issue<T>(a, blockIdx.x, stage0);
+    cp_async_commit();
+  }
   for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = a.tw[i];
   twm_build<T, M, true, 2>(a.tw, twm, threadIdx.x, blockDim.x);
   if (a.nstage)
     for (int i = threadIdx.x; i < a.nk; i += blockDim.x) kxs[i] = a.kxr[i];
-  if (a.bulk) {
-    if (threadIdx.x == 0) {
-      tc::mbar_init(&bars[0], 1);
-      tc::mbar_init(&bars[1], 1);
-      tc::fence_mbar_init();
-    }
-    __syncthreads();
-  }
+  __syncthreads();
   unsigned phase = 0;  // bit b: parity of the next completion of bars[b]
-  // persistent CTAs over batches of R rows; with two stages the spectral
-  // rows of the next batch are copied into the other stage while this one
-  // is transformed, with one stage after this batch's last read of it
-  const long nitems = (a.nrows + a.R - 1) / a.R;
-  if ((long)blockIdx.x < nitems) {
-    if (a.bulk) {
-      xi_issue_bulk<T>(a, blockIdx.x, stage0, &bars[0]);
-    } else {
-      xi_issue<T>(a, blockIdx.x, stage0);
-      cp_async_commit();
-    }
-  }
   int stg = 0;
   for (long item = blockIdx.x; item < nitems; item += gridDim.x) {
   const long next = item + gridDim.x;

@@ -6,27 +6,36 @@
 
 namespace les {
 
-// the staged x forward pass (scalings of few fields)
-template <typename T>
-static void launch_xfwd_st(int NX, XFArgs<T>& a, cudaStream_t st) {
+// the x forward pass of whole rows
+template <typename T, typename S>
+static void launch_xfwd_row(int NX, XFArgs<T>& a, cudaStream_t st) {
   const int M = NX / 2;
   const int SL = slot_stride(M, int(sizeof(cplx<T>)));
-  auto smem_for = [&](int R) {
-    return sizeof(cplx<T>) * (NX + twm_len(M, false) + (size_t)pad_seqs(R * a.nf, M) * SL) +
-           2 * sizeof(T) * (size_t)R * a.nf * NX + sizeof(T) * R * a.nf + 2 * sizeof(int) * R + 16;
+  a.nsrc = a.op == XF_PRESS ? 4 : a.nf;
+  auto stage_rows = [&](int R) { return R * (a.nsrc - a.nf) + pad_seqs(R * a.nf, M); };
+  auto smem_nb = [&](int R, int nb) {
+    return sizeof(cplx<T>) * (NX + twm_len(M, false) + (size_t)nb * stage_rows(R) * SL) + 2 * sizeof(uint64_t) +
+           sizeof(T) * ((R * a.nf + 1) & ~1) + 2 * sizeof(int) * R + 16;
   };
   void (*kern)(XFArgs<T>) = nullptr;
   switch (NX) {
-#define XS_CASE(N) \
-  case N: kern = k_xfwd_st<T, N>; break;
-    LES_LENGTHS(XS_CASE)
-#undef XS_CASE
+#define XR_CASE(N) \
+  case N: kern = k_xfwd_row<T, N, S>; break;
+    LES_LENGTHS(XR_CASE)
+#undef XR_CASE
     default:
       throw CudaError(1, "xfwd: unsupported transform length " + std::to_string(NX));
   }
-  a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, a.nrows);
-  const size_t smem = smem_for(a.R);
-  if (smem > SMEM_CAP) throw CudaError(1, "xfwd: shared memory request too large");
+  // two stages unless one keeps strictly more sequence slots busy (as
+  // launch_xinv)
+  double s2 = -1.0, s1 = -1.0;
+  const int r2 = best_rows((const void*)kern, a.nf, lanes(M), [&](int R) { return smem_nb(R, 2); }, a.nrows, &s2);
+  const int r1 = best_rows((const void*)kern, a.nf, lanes(M), [&](int R) { return smem_nb(R, 1); }, a.nrows, &s1);
+  a.nbuf = (s1 > s2 + 1e-9) ? 1 : 2;
+  a.R = (a.nbuf == 1) ? r1 : r2;
+  a.stage_rows = stage_rows(a.R);
+  const size_t smem = smem_nb(a.R, a.nbuf);
+  if (smem > SMEM_CAP || a.R * a.nf > 256) throw CudaError(1, "xfwd: shared memory request too large");
   const long nitems = ceil_div(a.nrows, a.R);
   if (nitems == 0) return;
   const int grid = int(std::min<long>(nitems, (long)resident_ctas((const void*)kern, 256, smem)));
@@ -39,11 +48,27 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   const int M = NX / 2;
   if (a.opitch == 0) a.opitch = a.nk;
   a.in_rstride = NX;
-  // the staged kernel pays for its two input stages with occupancy: it wins
-  // for scalings of few fields (measured at 256^3)
-  if (a.op == XF_SCALE && a.nf <= 3) {
-    hook_before("xfwd", double(a.nrows) * NX * a.nf * sizeof(T) + double(a.nrows) * a.nf * a.nk * sizeof(cplx<T>));
-    launch_xfwd_st<T>(NX, a, st);
+  const bool press = a.op == XF_PRESS;
+  static const int nin_of_op[] = {0, 9, 6, 10, 3, 6, 14, 9};
+  const int nin = a.op == XF_SCALE ? a.nf : nin_of_op[a.op];
+  const size_t isz = (a.in_f32 ? sizeof(float) : sizeof(T));
+  hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * (press ? 2 : a.nf) * a.nk * sizeof(cplx<T>));
+  // whole rows go by bulk copies, which want 16-byte aligned rows; XF_PRESS
+  // runs on the solver's own (aligned) fields only
+  bool rows = press || a.op == XF_SCALE;
+  for (int f = 0; f < (press ? 5 : a.nf) && rows; ++f) {
+    const void* q = a.in_f32 ? (const void*)a.inf[f] : (const void*)a.in[f];
+    rows = reinterpret_cast<uintptr_t>(q) % 16 == 0;
+  }
+  rows = rows && (isz * a.in_pstride) % 16 == 0 && (isz * NX) % 16 == 0;
+  if (press && !rows) throw CudaError(1, "xfwd: pressure inputs not 16-byte aligned");
+  if (rows) {
+    if (a.in_f32) {
+      if constexpr (std::is_same<T, double>::value) launch_xfwd_row<T, float>(NX, a, st);
+      else throw CudaError(1, "xfwd: FP32 inputs are for FP64 transforms");
+    } else {
+      launch_xfwd_row<T, T>(NX, a, st);
+    }
     hook_after();
     return;
   }
@@ -67,17 +92,12 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   // others at a finer grain (measured at 256^3: 0.667 -> 0.633 ms per step);
   // the other ops keep 256 threads (the stress divergence measured slower
   // with 128: 0.236 -> 0.256 ms)
-  const int XF_THREADS = (a.op == XF_CONV_IN || a.op == XF_PROD || a.op == XF_PROD_SC || a.op == XF_PRESS) ? 128 : 256;
+  const int XF_THREADS = (a.op == XF_CONV_IN || a.op == XF_PROD || a.op == XF_PROD_SC) ? 128 : 256;
   a.R = best_rows((const void*)kern, a.nf, lanes(M), smem_for, a.nrows, nullptr, XF_THREADS);
   const size_t smem = smem_for(a.R);
   if (smem > SMEM_CAP) throw CudaError(1, "xfwd: shared memory request too large");
   const int grid = ceil_div(a.nrows, a.R);
   if (grid == 0) return;
-  static const int nin_of_op[] = {0, 9, 6, 10, 3, 6, 14, 9};
-  const int nin = a.op == XF_SCALE ? a.nf : nin_of_op[a.op];
-  const int nout = a.op == XF_PRESS ? 2 : a.nf;
-  const size_t isz = (a.in_f32 ? sizeof(float) : sizeof(T));
-  hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * nout * a.nk * sizeof(cplx<T>));
   kern<<<grid, XF_THREADS, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
@@ -88,7 +108,9 @@ template <typename T>
 void set_attrs_xfwd() {
 #define XA(N)                                                                                       \
   LES_CUDA(cudaFuncSetAttribute(k_xfwd<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  LES_CUDA(cudaFuncSetAttribute(k_xfwd_st<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
+  LES_CUDA(cudaFuncSetAttribute(k_xfwd_row<T, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
+  if constexpr (std::is_same<T, double>::value)                                                       \
+    LES_CUDA(cudaFuncSetAttribute(k_xfwd_row<T, N, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
   LES_LENGTHS(XA)
 #undef XA
 }
