@@ -50,44 +50,116 @@ __device__ __forceinline__ void st4(double* p, const double* v) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
+// set_bc and the vertical differences in one pass over levels 1..nz+1, four
+// consecutive points per thread: the threads of level 1 write the lower ghost
+// values (and w(1)), those of level nz+1 the upper ones, and each uses the new
+// values it needs (w(nz+1) at level nz is recomputed, not read).  With ul the
+// velocity is also added to the Lagrangian accumulators on levels 0..nacc
+// (compute_LagScaleDep.f90:204-215), which would otherwise read the three
+// fields again.  Bound by HBM: 6 fields (12 with the accumulation); apart
+// (k_set_bc, k_ddz_vel, k_lag_accum) 15 fields and two more launches, 0.333
+// ms per step at 256^3 FP64 against 0.252.
 template <typename T>
-__global__ void k_ddz_vel(const T* u, const T* v, const T* w, T* dudz, T* dvdz, T* dwdz, long plane, int nz,
-                          T rdz) {
-  const long n = (long)(nz + 1) * plane;
-  if (plane % 4 == 0) {  // four consecutive points (one level) per thread, vector loads and stores
-    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n / 4; q += (long)gridDim.x * blockDim.x) {
-      const long o = plane + 4 * q;
-      const int k = udiv32(o, plane);
-      T a[4], b[4], r[4];
-      ld4(u + o, a);
-      ld4(u + o - plane, b);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = rdz * (a[i] - b[i]);
-      st4(dudz + o, r);
-      ld4(v + o, a);
-      ld4(v + o - plane, b);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = rdz * (a[i] - b[i]);
-      st4(dvdz + o, r);
-      if (k <= nz) {
-        ld4(w + o + plane, a);
-        ld4(w + o, b);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = rdz * (a[i] - b[i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = T(0);
-      }
-      st4(dwdz + o, r);
-    }
-    return;
-  }
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-    const long o = plane + q;  // levels 1..nz+1
+struct BcArgs {
+  T *u, *v, *w;
+  const T *lu, *lv, *lw, *tu, *tv, *tw;  // boundary planes
+  int lt[3], ut[3];                       // types: 0 none, 1 'drc', 2 'neu'
+  long plane;
+  int nz;
+  T dz;
+};
+// ghost value of a uvp-node field below (above) the value x next to it
+template <typename T>
+__device__ __forceinline__ T ghost_lo(int t, T x, T b, T dz, T old) {
+  return t == 1 ? T(2) * b - x : (t == 2 ? x - b * dz : old);
+}
+template <typename T>
+__device__ __forceinline__ T ghost_hi(int t, T x, T b, T dz, T old) {
+  return t == 1 ? T(2) * b - x : (t == 2 ? x + b * dz : old);
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_bc_ddz(const BcArgs<T> a, T* dudz, T* dvdz, T* dwdz, T rdz, T* ul, T* vl,
+                                                T* wl, int nacc) {
+  const long plane = a.plane, n4 = (long)(a.nz + 1) * plane / 4;
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+    const long o = plane + 4 * q;
     const int k = udiv32(o, plane);
-    dudz[o] = rdz * (u[o] - u[o - plane]);
-    dvdz[o] = rdz * (v[o] - v[o - plane]);
-    dwdz[o] = (k <= nz) ? rdz * (w[o + plane] - w[o]) : T(0);
+    const long p2 = o - (long)k * plane;
+    const bool lo = k == 1, hi = k == a.nz + 1;
+    T x[4], xm[4], r[4], z[4];
+    // u, v: (f(k) - f(k-1)) / dz
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      T* f = c ? a.v : a.u;
+      T* d = c ? dvdz : dudz;
+      T* acc = c ? vl : ul;
+      ld4(f + o, x);
+      ld4(f + o - plane, xm);
+      if (hi && a.ut[c]) {
+        ld4((c ? a.tv : a.tu) + p2, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = ghost_hi(a.ut[c], xm[i], z[i], a.dz, x[i]);
+        st4(f + o, x);
+      }
+      if (lo && a.lt[c]) {
+        ld4((c ? a.lv : a.lu) + p2, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) xm[i] = ghost_lo(a.lt[c], x[i], z[i], a.dz, xm[i]);
+        st4(f + o - plane, xm);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = rdz * (x[i] - xm[i]);
+      st4(d + o, r);
+      if (ul) {
+        if (k <= nacc) {
+          ld4(acc + o, z);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) z[i] = z[i] + x[i];
+          st4(acc + o, z);
+        }
+        if (lo) {
+          ld4(acc + o - plane, z);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) z[i] = z[i] + xm[i];
+          st4(acc + o - plane, z);
+        }
+      }
+    }
+    // w: (w(k+1) - w(k)) / dz, zero on the top level
+    ld4(a.w + o, x);
+    if (lo && a.lt[2] == 1) {
+      ld4(a.lw + p2, x);
+      st4(a.w + o, x);
+    }
+    if (hi && a.ut[2] == 1) {
+      ld4(a.tw + p2, x);
+      st4(a.w + o, x);
+    }
+    if (!hi) {
+      if (k == a.nz && a.ut[2] == 1) ld4(a.tw + p2, z);
+      else ld4(a.w + o + plane, z);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = rdz * (z[i] - x[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = T(0);
+    }
+    st4(dwdz + o, r);
+    if (ul) {
+      if (k <= nacc) {
+        ld4(wl + o, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = z[i] + x[i];
+        st4(wl + o, z);
+      }
+      if (lo) {
+        ld4(a.w + o - plane, x);
+        ld4(wl + o - plane, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = z[i] + x[i];
+        st4(wl + o - plane, z);
+      }
+    }
   }
 }
 
@@ -123,6 +195,25 @@ __global__ void k_plane_ops(const PlaneOps<T> ops, long n) {
   const T v = ops.val[op];
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x)
     d[q] = s ? s[q] : v;
+}
+
+// Ghost levels of the three right-hand sides as their buffers change roles:
+// the old buffer (next rhs_f) takes rhs_f's ghost levels, the new one val.
+// grid (.., 6): blockIdx.y = equation and level.
+template <typename T>
+struct RhsGhosts {
+  T *oldr[3], *newr[3];  // the two buffers of each equation
+  long top;              // offset of level nz + 1
+  T val;
+};
+template <typename T>
+__global__ void k_rhs_ghosts(const RhsGhosts<T> a, long plane) {
+  const int q = blockIdx.y >> 1;
+  const long o = (blockIdx.y & 1) ? a.top : 0;
+  for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
+    a.oldr[q][o + p] = a.newr[q][o + p];
+    a.newr[q][o + p] = a.val;
+  }
 }
 
 template <typename T>
@@ -1114,100 +1205,240 @@ __device__ __forceinline__ void diag_block_reduce(DiagAcc& a) {
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_diag_partial(const T* u, const T* v, const T* w, const T* dudx,
-                                                      const T* dvdy, const T* dwdz, const T* ustar, long plane,
-                                                      int nz, double* part) {
-  DiagAcc a;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < plane; q += (long)gridDim.x * blockDim.x)
-    a.sum[4].add(double(ustar[q]));
-  const long n = (long)nz * plane;
-  int nan = 0;
-  auto point = [&](double uu, double vv, double ww, double wu, double dx, double dy, double dz) {
-    nan |= (uu != uu) | (vv != vv) | (ww != ww);
-    a.mx[0] = fmax(a.mx[0], fabs(uu));
-    a.mx[1] = fmax(a.mx[1], fabs(vv));
-    a.mx[2] = fmax(a.mx[2], fabs(ww));
-    a.sum[0].add(uu);
-    a.sum[1].add(vv);
-    a.sum[2].add(0.5 * (ww + wu));
-    const double dv = dx + dy + dz;
-    a.sum[3].add(dv * dv);
-  };
-  if (plane % 4 == 0) {
-    // four consecutive points per thread and iteration: all 28 loads are
-    // issued (as 16-byte vectors for FP32) before the compensated sums run
-    const long n4 = n / 4;
-    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
-      const long o = plane + 4 * q;
-      T U[4], V[4], W[4], WU[4], DX[4], DY[4], DZ[4];
-      ld4(u + o, U);
-      ld4(v + o, V);
-      ld4(w + o, W);
-      ld4(w + o + plane, WU);
-      ld4(dudx + o, DX);
-      ld4(dvdy + o, DY);
-      ld4(dwdz + o, DZ);
-      // the four points' values summed in plain FP64, then one compensated
-      // addition per sum (the compensated sum is the cost, not the loads)
-      double su = 0.0, sv = 0.0, sw = 0.0, sd = 0.0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double uu = U[i], vv = V[i], ww = W[i];
-        nan |= (uu != uu) | (vv != vv) | (ww != ww);
-        a.mx[0] = fmax(a.mx[0], fabs(uu));
-        a.mx[1] = fmax(a.mx[1], fabs(vv));
-        a.mx[2] = fmax(a.mx[2], fabs(ww));
-        su += uu;
-        sv += vv;
-        sw += 0.5 * (ww + double(WU[i]));
-        const double dv = double(DX[i]) + double(DY[i]) + double(DZ[i]);
-        sd += dv * dv;
-      }
-      a.sum[0].add(su);
-      a.sum[1].add(sv);
-      a.sum[2].add(sw);
-      a.sum[3].add(sd);
-    }
-  } else {
-    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-      const long o = plane + q;
-      point(u[o], v[o], w[o], w[o + plane], dudx[o], dvdy[o], dwdz[o]);
-    }
-  }
-  a.nan = nan;
+// The diagnostics' sums of a block, and, in the last block to arrive (done
+// counts them and returns to zero), their combination in block order:
+// deterministic, and one launch instead of two.
+struct DiagOut {
+  double* part;      // [gridDim.x][DIAG_NV]
+  unsigned* done;    // zero between launches
+  double* out;       // cfl, mke, u*, rms div u
+  unsigned* status;
+  long plane;
+  double dt, dx, dy, dz, npts;
+};
+__device__ __forceinline__ void diag_finish(DiagAcc& a, const DiagOut& d) {
   diag_block_reduce(a);
+  __shared__ bool last;
   if (threadIdx.x == 0) {
-    double* out = part + (long)blockIdx.x * DIAG_NV;
-    for (int i = 0; i < 3; ++i) out[i] = a.mx[i];
-    for (int q = 0; q < 4; ++q) out[3 + q] = a.sum[q].val();
-    out[7] = a.nan;
-    out[8] = a.sum[4].val();
+    double* q = d.part + (long)blockIdx.x * DIAG_NV;
+    for (int i = 0; i < 3; ++i) q[i] = a.mx[i];
+    for (int i = 0; i < 4; ++i) q[3 + i] = a.sum[i].val();
+    q[7] = a.nan;
+    q[8] = a.sum[4].val();
+    __threadfence();
+    last = atomicAdd(d.done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  DiagAcc t;
+  t.mx[0] = t.mx[1] = t.mx[2] = -1e300;
+  for (int b = threadIdx.x; b < int(gridDim.x); b += blockDim.x) {
+    const double* q = d.part + (long)b * DIAG_NV;
+    for (int i = 0; i < 3; ++i) t.mx[i] = fmax(t.mx[i], __ldcg(q + i));
+    for (int i = 0; i < 4; ++i) t.sum[i].add(__ldcg(q + 3 + i));
+    t.sum[4].add(__ldcg(q + 8));
+    t.nan = fmax(t.nan, __ldcg(q + 7));
+  }
+  diag_block_reduce(t);
+  if (threadIdx.x == 0) {
+    *d.done = 0u;
+    d.out[0] = d.dt * (t.mx[0] / d.dx + t.mx[1] / d.dy + t.mx[2] / d.dz);
+    const double um = t.sum[0].val() / d.npts, vm = t.sum[1].val() / d.npts, wm = t.sum[2].val() / d.npts;
+    d.out[1] = 0.5 * (um * um + vm * vm + wm * wm);
+    d.out[2] = t.sum[4].val() / double(d.plane);
+    d.out[3] = sqrt(t.sum[3].val() / d.npts);
+    if (t.nan != 0.0) atomicOr(d.status, ST_NAN);
   }
 }
-
-__global__ void __launch_bounds__(256) k_diag_final(const double* part, int nblocks, long plane, double dt,
-                                                    double dx, double dy, double dz, double npts, double* out,
-                                                    unsigned* status) {
-  // fixed-order combination of the block partials (deterministic)
-  DiagAcc a;
-  a.mx[0] = a.mx[1] = a.mx[2] = -1e300;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    const double* q = part + (long)b * DIAG_NV;
-    for (int i = 0; i < 3; ++i) a.mx[i] = fmax(a.mx[i], q[i]);
-    for (int i = 0; i < 4; ++i) a.sum[i].add(q[3 + i]);
-    a.sum[4].add(q[8]);
-    a.nan = fmax(a.nan, q[7]);
+// four points' velocity and divergence added to the sums: the four values in
+// plain FP64, then one compensated addition per sum (the compensated sum is
+// the cost, not the loads); ww: the four points' share of the w sum
+template <typename T>
+__device__ __forceinline__ void diag_add4(DiagAcc& a, int& nan, const T* U, const T* V, const T* W, double ww,
+                                          const T* DX, const T* DY, const T* DZ) {
+  double su = 0.0, sv = 0.0, sd = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double uu = U[i], vv = V[i], w = W[i];
+    nan |= (uu != uu) | (vv != vv) | (w != w);
+    a.mx[0] = fmax(a.mx[0], fabs(uu));
+    a.mx[1] = fmax(a.mx[1], fabs(vv));
+    a.mx[2] = fmax(a.mx[2], fabs(w));
+    su += uu;
+    sv += vv;
+    const double dv = double(DX[i]) + double(DY[i]) + double(DZ[i]);
+    sd += dv * dv;
   }
-  diag_block_reduce(a);
-  if (threadIdx.x == 0) {
-    const double cfl = dt * (a.mx[0] / dx + a.mx[1] / dy + a.mx[2] / dz);
-    const double um = a.sum[0].val() / npts, vm = a.sum[1].val() / npts, wm = a.sum[2].val() / npts;
-    out[0] = cfl;
-    out[1] = 0.5 * (um * um + vm * vm + wm * wm);
-    out[2] = a.sum[4].val() / double(plane);
-    out[3] = sqrt(a.sum[3].val() / npts);
-    if (a.nan != 0.0) atomicOr(status, ST_NAN);
+  a.sum[0].add(su);
+  a.sum[1].add(sv);
+  a.sum[2].add(ww);
+  a.sum[3].add(sd);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_diag(const T* u, const T* v, const T* w, const T* dudx, const T* dvdy,
+                                              const T* dwdz, const T* ustar, int nz, const DiagOut d) {
+  DiagAcc a;
+  const long plane = d.plane;
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < plane; q += (long)gridDim.x * blockDim.x)
+    a.sum[4].add(double(ustar[q]));
+  int nan = 0;
+  // four consecutive points per thread and iteration: all 28 loads are
+  // issued (as 16-byte vectors for FP32) before the compensated sums run
+  const long n4 = (long)nz * plane / 4;
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+    const long o = plane + 4 * q;
+    T U[4], V[4], W[4], WU[4], DX[4], DY[4], DZ[4];
+    ld4(u + o, U);
+    ld4(v + o, V);
+    ld4(w + o, W);
+    ld4(w + o + plane, WU);
+    ld4(dudx + o, DX);
+    ld4(dvdy + o, DY);
+    ld4(dwdz + o, DZ);
+    double ww = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ww += 0.5 * (double(W[i]) + double(WU[i]));
+    diag_add4(a, nan, U, V, W, ww, DX, DY, DZ);
+  }
+  a.nan = nan;
+  diag_finish(a, d);
+}
+
+// ---------------------------------------------------------------------------
+// The end of a time step in one pass (four consecutive points per thread):
+// dp/dz, the pressure with its mean mode (mixed precision), the projection of
+// u, v, w and of the right-hand sides (as k_dpdz, k_p_finish, k_projection),
+// the boundary conditions (k_set_bc) and, with DIAG, the running diagnostics.
+// pf: the pressure without its mean (mixed; p itself otherwise): each level is
+// read once as its own and once as the lower neighbour (L2).  The w sum of
+// the diagnostics, sum_k (w(k) + w(k+1)) / 2 over levels 1..nz, takes each
+// level once, its ends by half, so that no thread reads a neighbour's new w.
+// Bound by HBM: 20 fields (DIAG), 29 and six launches apart; at 256^3 FP64
+// 0.52 -> 0.46 ms per step, mixed (diagnostics apart) 0.33 -> 0.29, 128 x 64 x
+// 41 and smaller six launches of ~7 us -> one of 17-23.
+template <typename T, bool DIAG>
+__global__ void __launch_bounds__(256) k_step_finish(const BcArgs<T> a, const T* pf, T* p, const double* pmean,
+                                                     const T* dpdx, const T* dpdy, T* dpdz, T* rx, T* ry, T* rz,
+                                                     T rdz, double dtt_d, const T* dudx, const T* dvdy,
+                                                     const T* dwdz, const T* ustar, const DiagOut dg) {
+  const long plane = a.plane;
+  const int nz = a.nz;
+  const T dtt = T(dtt_d);
+  const long t0 = blockIdx.x * (long)blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
+  DiagAcc acc;
+  int nan = 0;
+  if constexpr (DIAG)
+    for (long q = t0; q < plane; q += ts) acc.sum[4].add(double(ustar[q]));
+  const long n4 = (long)(nz + 2) * plane / 4;
+  for (long q = t0; q < n4; q += ts) {
+    const long o = 4 * q;
+    const int k = udiv32(o, plane);
+    const long p2 = o - (long)k * plane;
+    T x[4], y[4], z[4];
+    if (k == 0 || k > nz) {  // p(0) with its mean, p(nz+1) undefined
+      if (k > nz) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = T(BOGUS);
+        st4(p + o, x);
+      } else if (pmean) {
+        ld4(pf + o, x);
+        const double m = pmean[0];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = T(double(x[i]) + m);
+        st4(p + o, x);
+      }
+      continue;
+    }
+    const bool lo = k == 1, hi = k == nz;
+    // dp/dz: the mean mode's difference in FP64 (mixed)
+    T dz_[4];
+    ld4(pf + o, x);
+    ld4(pf + o - plane, y);
+    const double m = pmean ? pmean[k] : 0.0;
+    const double dm = pmean ? double(rdz) * (m - pmean[k - 1]) : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dz_[i] = pmean ? T(double(rdz * (x[i] - y[i])) + dm) : rdz * (x[i] - y[i]);
+    st4(dpdz + o, dz_);
+    if (pmean) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = T(double(x[i]) + m);
+      st4(p + o, x);
+    }
+    // projection and right-hand sides, u and v with their ghost levels
+    T uv[2][4], w[4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      T* f = c ? a.v : a.u;
+      T* r = c ? ry : rx;
+      ld4((c ? dpdy : dpdx) + o, y);
+      ld4(r + o, z);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[i] = z[i] - y[i];
+      st4(r + o, z);
+      T* g = uv[c];
+      ld4(f + o, g);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = g[i] - dtt * y[i];
+      st4(f + o, g);
+      if (lo && a.lt[c]) {
+        ld4((c ? a.lv : a.lu) + p2, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = ghost_lo(a.lt[c], g[i], y[i], a.dz, T(0));
+        st4(f + o - plane, z);
+      }
+      if (hi && a.ut[c]) {
+        ld4((c ? a.tv : a.tu) + p2, y);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = ghost_hi(a.ut[c], g[i], y[i], a.dz, T(0));
+        st4(f + o + plane, z);
+      }
+    }
+    // w: the correction in FP64 (see k_projection), w(1) = w(nz+1) = 0 before
+    // the boundary conditions
+    ld4(rz + o, z);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[i] = z[i] - dz_[i];
+    st4(rz + o, z);
+    if (lo) {
+      if (a.lt[2] == 1) {
+        ld4(a.lw + p2, w);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = T(0);
+      }
+    } else {
+      ld4(a.w + o, w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = T(double(w[i]) - dtt_d * double(dz_[i]));
+    }
+    st4(a.w + o, w);
+    double ww = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ww += double(w[i]);
+    if (lo) ww *= 0.5;
+    if (hi) {
+      if (a.ut[2] == 1) {
+        ld4(a.tw + p2, z);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = T(0);
+      }
+      st4(a.w + o + plane, z);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ww += 0.5 * double(z[i]);
+    }
+    if constexpr (DIAG) {
+      ld4(dudx + o, x);
+      ld4(dvdy + o, y);
+      ld4(dwdz + o, z);
+      diag_add4(acc, nan, uv[0], uv[1], w, ww, x, y, z);
+    }
+  }
+  if constexpr (DIAG) {
+    acc.nan = nan;
+    diag_finish(acc, dg);
   }
 }
 

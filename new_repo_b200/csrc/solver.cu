@@ -302,6 +302,18 @@ class Solver final : public SolverBase {
     dim3 grid(unsigned(std::min<long>(ceil_div(n, 256L), 148)), unsigned(nops));
     KL("k_plane_ops", bytes, k_plane_ops<T><<<grid, 256, 0, st>>>(o, n));
   }
+  // the first nlev levels of up to eight fields in one launch
+  void fill_planes(int nf, T* const* dst, int nlev, T v) {
+    PlaneOps<T> o;
+    std::memset(&o, 0, sizeof(o));
+    for (int i = 0; i < nf; ++i) {
+      o.dst[i] = dst[i];
+      o.val[i] = v;
+    }
+    const long n = (long)nlev * g.plane();
+    KL("k_plane_ops", double(nf) * n * sizeof(T),
+       k_plane_ops<T><<<dim3(unsigned(std::min<long>(ceil_div(n, 256L), 148 * 8)), unsigned(nf)), 256, 0, st>>>(o, n));
+  }
   void copy(T* dst, const T* src, long n) {
     KL("k_copy", 2.0 * n * sizeof(T), k_copy<T><<<grid_for(n), 256, 0, st>>>(dst, src, n));
   }
@@ -1128,6 +1140,26 @@ class Solver final : public SolverBase {
     LES_CUDA(cudaStreamSynchronize(st));
   }
 
+  BcArgs<T> bc_args() const {
+    BcArgs<T> a;
+    a.u = F[LES_U];
+    a.v = F[LES_V];
+    a.w = F[LES_W];
+    a.lu = PL[LES_LBC_U];
+    a.lv = PL[LES_LBC_V];
+    a.lw = PL[LES_LBC_W];
+    a.tu = PL[LES_UBC_U];
+    a.tv = PL[LES_UBC_V];
+    a.tw = PL[LES_UBC_W];
+    for (int c = 0; c < 3; ++c) {
+      a.lt[c] = lbc_t[c];
+      a.ut[c] = ubc_t[c];
+    }
+    a.plane = g.plane();
+    a.nz = g.nz;
+    a.dz = T(dz());
+    return a;
+  }
   void launch_bc(int4 lt, int4 ut) {
     KL("k_set_bc", 8.0 * g.plane() * sizeof(T), k_set_bc<T><<<grid_for(g.plane()), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], PL[LES_LBC_U], PL[LES_LBC_V],
                                                     PL[LES_LBC_W], PL[LES_UBC_U], PL[LES_UBC_V], PL[LES_UBC_W],
@@ -1163,7 +1195,7 @@ class Solver final : public SolverBase {
   // sp, rf: where the filtered x spectra and the references stay (scratch
   // unless the caller keeps them)
   void grad_ptrs(T* const* f, T* const* dx, T* const* dy, int nfld, const char* tag = "grad",
-                 cplx<T>* const* sp = nullptr, T* const* rf = nullptr) {
+                 cplx<T>* const* sp = nullptr, T* const* rf = nullptr, bool wall = false) {
     if (!sp) sp = spec;
     if (!rf) rf = refbuf;
     Tag tag_(this, tag);
@@ -1183,7 +1215,20 @@ class Solver final : public SolverBase {
       b.out[2 * q + 0] = sp[q];
       b.out[2 * q + 1] = spec[3 + q];
     }
+    if (wall) {  // the wall law's filtered first level of u, v on the way
+      b.wall[0] = spec[6];
+      b.wall[1] = spec[7];
+      b.G0 = gt;
+      b.gs = T(double(g.nx * g.ny));  // the spectrum carries the factor already
+      b.ncols1 = nk2;
+      b.opitch1 = pitch(nk2);
+    }
     launch_ypass<T>(g.ny, g.ny, b, L, nfld, st);
+    if (wall) {
+      T* const r1[2] = {rf[0] + 1, rf[1] + 1};
+      Tag wtag_(this, "wall");
+      wall_store(spec[6], spec[7], r1);
+    }
     auto c = xi(XI_STORE, 3 * nfld, 0, L, g.nx, g.ny, g.lhx);
     c.nstage = 2 * nfld;
     c.kxr = kkx;  // row ky = 0 of the wavenumber table (Nyquist column zero)
@@ -1215,15 +1260,23 @@ class Solver final : public SolverBase {
     KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T), k_ddz<T><<<grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st>>>(F[dfdz], F[f], g.plane(), g.nz, T(1.0 / dz()), 1));
   }
 
-  void compute_vel_grad() override {
+  void compute_vel_grad() override { vel_grad(-1, false); }
+  // nacc >= 0: the velocity is also added to the Lagrangian accumulators on
+  // levels 0..nacc (a time step whose dynamic procedure would do so next).
+  // wall: the filtered wall law runs from the same transforms (the first
+  // level's third column output of the y pass) instead of its own three
+  // launches.
+  void vel_grad(int nacc, bool wall) {
     T* const f[3] = {F[LES_U], F[LES_V], F[LES_W]};
     T* const dx[3] = {F[LES_DUDX], F[LES_DVDX], F[LES_DWDX]};
     T* const dy[3] = {F[LES_DUDY], F[LES_DVDY], F[LES_DWDY]};
-    grad_ptrs(f, dx, dy, 3, "grad", vsp, vref);
-    set_bc();
+    grad_ptrs(f, dx, dy, 3, "grad", vsp, vref, wall);
     Tag tag_(this, "grad");
-    KL("k_ddz_vel", 6.0 * (g.nz + 1) * g.plane() * sizeof(T), k_ddz_vel<T><<<grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st>>>(
-        F[LES_U], F[LES_V], F[LES_W], F[LES_DUDZ], F[LES_DVDZ], F[LES_DWDZ], g.plane(), g.nz, T(1.0 / dz())));
+    const long n = (long)(g.nz + 1) * g.plane();
+    KL("k_bc_ddz", (6.0 * n + (nacc >= 0 ? 6.0 * (nacc + 1) * g.plane() : 0.0)) * sizeof(T),
+       k_bc_ddz<T><<<grid_for(n / 4), 256, 0, st>>>(bc_args(), F[LES_DUDZ], F[LES_DVDZ], F[LES_DWDZ], T(1.0 / dz()),
+                                                    nacc >= 0 ? F[LES_U_LAG] : nullptr, F[LES_V_LAG], F[LES_W_LAG],
+                                                    nacc));
     if (scalar_on) scalar_grad();
   }
 
@@ -1465,7 +1518,7 @@ class Solver final : public SolverBase {
       div_products(e, 3, true);
     }
     Tag tag_(this, "convec");
-    convec_ghosts(rhs);
+    if (!padd()) convec_ghosts(rhs);  // padded: written with the buffer exchange (rhs_adv)
   }
   // rhs of neq equations = products (spectra spec[q], references refbuf[6 + q])
   // + stress divergence + forcing
@@ -1590,9 +1643,21 @@ class Solver final : public SolverBase {
     }
   }
   void press_stag_array(double tadv1) override {
+    press_solve(tadv1, F[LES_P]);
     Tag tag_(this, "press");
-    if constexpr (std::is_same<T, float>::value) press_impl(tadv1, pspec[0], pspec[1]);
-    else press_impl(tadv1, spec[0], spec[1]);
+    press_finish();
+  }
+  // p (without its mean in mixed precision) -> pout, dp/dx, dp/dy
+  void press_solve(double tadv1, T* pout) {
+    Tag tag_(this, "press");
+    if constexpr (std::is_same<T, float>::value) press_impl(tadv1, pspec[0], pspec[1], pout);
+    else press_impl(tadv1, spec[0], spec[1], pout);
+  }
+  // dpdz (compute_pressure.f90:359-369), then p(nz+1) = BOGUS (:353-357)
+  void press_finish() {
+    dpdz_only();
+    KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
+       k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], mixed() ? pmean : nullptr, g.plane(), g.nz));
   }
 
   // Right-hand side in two FP64 spectra instead of three, and one after the y
@@ -1604,7 +1669,7 @@ class Solver final : public SolverBase {
   // 0.311 + 0.202 ms per step with five launches fewer, and the solve, reading
   // one spectrum instead of three, from 0.181 to 0.110 (FP64: 0.455 + 0.431 to
   // 0.325 + 0.278, and 0.190 to 0.119).
-  void press_impl(double tadv1, cplx<double>* s0, cplx<double>* s1) {
+  void press_impl(double tadv1, cplx<double>* s0, cplx<double>* s1, T* pout) {
     using S = double;
     const int nz = g.nz;
     const double c = 1.0 / double(g.nx * g.ny);
@@ -1639,16 +1704,12 @@ class Solver final : public SolverBase {
          k_tridiag<T><<<ceil_div(2L * g.ny * g.lhx, 128), 128, 0, st>>>(reinterpret_cast<double*>(s0), piv,
                                                                          reinterpret_cast<T*>(ph), pm, dstatus, g.lhx,
                                                                          g.ny, nz, dz(), drop, pp));
-    press_grad(ph);
-    // dpdz (compute_pressure.f90:359-369), then p(nz+1) = BOGUS (:353-357)
-    dpdz_only();
-    KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
-       k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], pm, g.plane(), nz));
+    press_grad(ph, pout);
   }
   // compute_press_grad: p^ (rows pitch(lhx) apart) -> dpdx, dpdy (1..nz), p
   // (0..nz+1); the y pass forms p and i ky p, the x inverse i kx p from the
   // staged p row (compute_pressure.f90:320-358)
-  void press_grad(cplx<T>* ph) {
+  void press_grad(cplx<T>* ph, T* pout) {
     auto e = yp(YP_PGRAD, 1, 2, g.lhx, g.lhx, g.ny, g.lhx, g.ny, 0);
     e.in[0] = ph;
     e.out[0] = ph;
@@ -1660,7 +1721,7 @@ class Solver final : public SolverBase {
     h.in[0] = ph;
     h.in[1] = spec[3];
     const int src[3] = {0, 1, 0};
-    T* const out[3] = {F[LES_DPDX], F[LES_DPDY], F[LES_P]};
+    T* const out[3] = {F[LES_DPDX], F[LES_DPDY], pout};
     for (int q = 0; q < 3; ++q) {
       h.src[q] = src[q];
       h.dx[q] = q == 0;
@@ -1775,10 +1836,8 @@ class Solver final : public SolverBase {
                                           mixed() ? pmean : nullptr, dstatus, g.lhx, g.ny, nz, dz(), mixed() ? 1 : 0,
                                           pitch(g.lhx), pitch(g.lhx), means, tadv2 / tadv1, 1.0 / (P.dt * tadv1),
                                           g.L));
-    press_grad(spec[0]);
-    dpdz_only();
-    KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
-       k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], mixed() ? pmean : nullptr, g.plane(), nz));
+    press_grad(spec[0], F[LES_P]);
+    press_finish();
   }
 
 
@@ -1804,27 +1863,32 @@ class Solver final : public SolverBase {
       b.in[1] = s1;
       b.out[1] = s1;
       launch_ypass<T>(g.ny, g.ny, b, 1, 2, st);
-      auto c = xi(XI_WALL, 2, 0, 1, g.nx, g.ny, nk2);
-      c.in[0] = s0;
-      c.in[1] = s1;
-      if (mixed()) {
-        c.refin[0] = refbuf[0];
-        c.refin[1] = refbuf[1];
-      }
-      c.c0 = dz();
-      c.out_pstride = g.plane();
-      c.aux[0] = PL[LES_LBC_Z0];
-      c.out[0] = PL[LES_U_STAR_AVG];
-      c.out[1] = PL[LES_LBC_U];
-      c.out[2] = PL[LES_LBC_V];
-      c.out[3] = F[LES_TXZ];
-      c.out[4] = F[LES_TYZ];
-      c.out[5] = F[LES_DUDZ];
-      c.out[6] = F[LES_DVDZ];
-      launch_xinv<T>(g.nx, c, st);
+      wall_store(s0, s1, refbuf);
     } else {
       wall_plain();
     }
+  }
+  // u*, the Neumann boundary values and the wall stress from the filtered
+  // first level of u, v (one plane of spectra, references rf[q][0])
+  void wall_store(const cplx<T>* s0, const cplx<T>* s1, T* const* rf) {
+    auto c = xi(XI_WALL, 2, 0, 1, g.nx, g.ny, nk2);
+    c.in[0] = s0;
+    c.in[1] = s1;
+    if (mixed()) {
+      c.refin[0] = rf[0];
+      c.refin[1] = rf[1];
+    }
+    c.c0 = dz();
+    c.out_pstride = g.plane();
+    c.aux[0] = PL[LES_LBC_Z0];
+    c.out[0] = PL[LES_U_STAR_AVG];
+    c.out[1] = PL[LES_LBC_U];
+    c.out[2] = PL[LES_LBC_V];
+    c.out[3] = F[LES_TXZ];
+    c.out[4] = F[LES_TYZ];
+    c.out[5] = F[LES_DUDZ];
+    c.out[6] = F[LES_DVDZ];
+    launch_xinv<T>(g.nx, c, st);
   }
   void wall_plain();
   void obukhov() override { wall_layer(); }
@@ -1940,7 +2004,7 @@ class Solver final : public SolverBase {
     const int nz = g.nz;
     if (nlev < 0) nlev = nz + 1;
     const long nacc = std::min<long>(g.field(), (long)(nlev + 1) * g.plane());  // levels 0..nlev
-    if (jtt >= P.dyn_init) {
+    if (jtt >= P.dyn_init && !lag_added) {
       KL("k_lag_accum", 9.0 * nacc * sizeof(T), k_lag_accum<T><<<grid_for(nacc), 256, 0, st>>>(F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG], F[LES_U],
                                                          F[LES_V], F[LES_W], nacc));
     }
@@ -1973,7 +2037,16 @@ class Solver final : public SolverBase {
                                                   P.dt * double(P.cs_count), beta_pow, nullptr, nlev, cs2_max));
     f_coeff_init = true;
     lagran_init = true;
-    for (int q : {LES_U_LAG, LES_V_LAG, LES_W_LAG}) fill(F[q], 0, std::min(nlev, nz + 1), T(0));
+    T* const lag[3] = {F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG]};
+    fill_planes(3, lag, std::min(nlev, nz + 1) + 1, T(0));
+  }
+  bool lag_added = false;  // this step's velocity is in the accumulators already
+  // the levels 0..n of step_body's dynamic procedure accumulates (-1: none)
+  int lag_levels(int jtt) const {
+    if (jtt < P.dyn_init) return -1;
+    if (P.sgs_model == LES_SGS_LASD) return g.nz + 1;
+    if (P.sgs_model == LES_SGS_MLP && mlp_wall_levels > 0) return std::min(mlp_wall_levels, g.nz + 1);
+    return -1;
   }
 
   void dynsmag(SgsArgs<T>& a, int jt, int jtt);
@@ -2228,15 +2301,29 @@ class Solver final : public SolverBase {
     {
       Tag tag_(this, "convec");
       const int r[3] = {LES_RHSX, LES_RHSY, LES_RHSZ}, rf[3] = {LES_RHSX_F, LES_RHSY_F, LES_RHSZ_F};
-      T* dst[6];
-      const T* src[6];
-      for (int q = 0; q < 3; ++q) {
-        dst[2 * q] = lev(F[r[q]], 0);
-        src[2 * q] = lev(F[rf[q]], 0);
-        dst[2 * q + 1] = lev(F[r[q]], g.nz + 1);
-        src[2 * q + 1] = lev(F[rf[q]], g.nz + 1);
+      if (from_spectra && padd()) {
+        // with the convective routine's own ghost values (convec_ghosts)
+        RhsGhosts<T> o;
+        for (int q = 0; q < 3; ++q) {
+          o.oldr[q] = F[r[q]];
+          o.newr[q] = F[rf[q]];
+        }
+        o.top = (long)(g.nz + 1) * g.plane();
+        o.val = T(BOGUS);
+        KL("k_rhs_ghosts", 18.0 * g.plane() * sizeof(T),
+           k_rhs_ghosts<T><<<dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256L), 148)), 6u), 256, 0, st>>>(
+               o, g.plane()));
+      } else {
+        T* dst[6];
+        const T* src[6];
+        for (int q = 0; q < 3; ++q) {
+          dst[2 * q] = lev(F[r[q]], 0);
+          src[2 * q] = lev(F[rf[q]], 0);
+          dst[2 * q + 1] = lev(F[r[q]], g.nz + 1);
+          src[2 * q + 1] = lev(F[rf[q]], g.nz + 1);
+        }
+        plane_ops(6, dst, src, nullptr);
       }
-      plane_ops(6, dst, src, nullptr);
       for (int q = 0; q < 3; ++q) std::swap(F[r[q]], F[rf[q]]);
     }
     if (from_spectra) {
@@ -2282,10 +2369,20 @@ class Solver final : public SolverBase {
   // after the copies back have started)
   void step_body(int jt, int jtt, bool with_diag) {
     LES_CUDA(cudaEventRecord(ev[0], st));
-    if (P.wall_law) wall_layer();  // obukhov + wallstress (same filtered layer)
-    compute_vel_grad();
+    // obukhov + wallstress (the same filtered layer)
+    const bool wall = P.wall_law && P.wall_model == LES_WALL_FILTER;
+    if (P.wall_law && !wall) wall_layer();
+    const int nacc = lag_levels(jtt);
+    vel_grad(nacc, wall);
     LES_CUDA(cudaEventRecord(ev[1], st));
-    sgs_stress(jt, jtt);
+    lag_added = nacc >= 0;
+    try {
+      sgs_stress(jt, jtt);
+    } catch (...) {
+      lag_added = false;
+      throw;
+    }
+    lag_added = false;
     LES_CUDA(cudaEventRecord(ev[2], st));
     rhs_adv(true);
     LES_CUDA(cudaEventRecord(ev[3], st));
@@ -2302,24 +2399,49 @@ class Solver final : public SolverBase {
     // press_from_increment forms the same pressure in FP32 without the
     // cancellation, but its FP32 four-field y pass measured slower than the
     // FP64 three-field one at 256^3 (0.47 against 0.36 ms per step)
-    press_stag_array(t1);
+    T* praw = mixed() ? sc[0] : F[LES_P];  // scratch of the dynamic procedure, free here
+    press_solve(t1, praw);
     LES_CUDA(cudaEventRecord(ev[4], st));
-    projection(t1);
-    set_bc();
-    if (with_diag) diagnostics_launch();
+    {
+      Tag tag_(this, "finish");
+      // the diagnostics ride along in FP64 and on small grids (one launch
+      // less); in FP32 their FP64 sums cost more registers (106 against 32)
+      // than the three field reads they save: apart 0.29, together 0.38 ms at
+      // 256^3
+      const bool ride = with_diag && (!mixed() || g.field() <= (4L << 20));
+      const double fields = (mixed() ? 11.0 + 6.0 : 9.0 + 7.0) + (ride ? 3.0 : 0.0);
+      auto run = [&](auto diag_c) {
+        constexpr bool DIAG = decltype(diag_c)::value;
+        const int nb = DIAG ? diag_blocks() : grid_for(g.field() / 4);
+        KL("k_step_finish", fields * g.nz * g.plane() * sizeof(T),
+           k_step_finish<T, DIAG><<<nb, 256, 0, st>>>(
+               bc_args(), praw, F[LES_P], mixed() ? pmean : nullptr, F[LES_DPDX], F[LES_DPDY], F[LES_DPDZ],
+               F[LES_RHSX], F[LES_RHSY], F[LES_RHSZ], T(1.0 / dz()), P.dt * t1, F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ],
+               PL[LES_U_STAR_AVG], diag_out()));
+      };
+      if (ride) run(std::true_type{});
+      else run(std::false_type{});
+      if (with_diag && !ride) diagnostics_launch();
+    }
     LES_CUDA(cudaEventRecord(ev[5], st));
     timed = true;
   }
   bool timed = false;
 
+  // blocks of the diagnostics' reductions: at least eight points per thread
+  // (a 32^3 grid ran its 1184 blocks' reductions for 17 us)
+  int diag_blocks() const {
+    return int(std::min<long>(DIAG_BLOCKS, std::max<long>(1, (long)g.nz * g.plane() / (256 * 8))));
+  }
+  DiagOut diag_out() const {
+    return DiagOut{part, dstatus + 1, dout, dstatus, g.plane(), P.dt, P.lx / double(g.nx), P.ly / double(g.ny), dz(),
+                   double(g.nx) * double(g.ny) * double(g.nz)};
+  }
   void diagnostics_launch() {
     Tag tag_(this, "diag");
-    KL("k_diag_partial", 6.0 * g.nz * g.plane() * sizeof(T),
-       k_diag_partial<T><<<DIAG_BLOCKS, 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], F[LES_DUDX], F[LES_DVDY],
-                                                     F[LES_DWDZ], PL[LES_U_STAR_AVG], g.plane(), g.nz, part));
-    KL("k_diag_final", double(DIAG_BLOCKS) * DIAG_NV * 8.0,
-       k_diag_final<<<1, 256, 0, st>>>(part, DIAG_BLOCKS, g.plane(), P.dt, P.lx / double(g.nx), P.ly / double(g.ny),
-                                      dz(), double(g.nx) * double(g.ny) * double(g.nz), dout, dstatus));
+    KL("k_diag", 6.0 * g.nz * g.plane() * sizeof(T),
+       k_diag<T><<<diag_blocks(), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ],
+                                                PL[LES_U_STAR_AVG], g.nz, diag_out()));
   }
   void diagnostics(double out[4]) override {
     diagnostics_launch();

@@ -834,6 +834,10 @@ struct YPArgs {
   cplx<T>* out[MAXOUT];
   const T* kkx;        // [ny][lhx]
   const T* kky;
+  // YP_GRADY, group < 2: a third output on level 1, the column times G0 gs
+  // (nullptr: none), one plane of rows opitch1 apart, columns below ncols1
+  cplx<T>* wall[2];
+  T gs;
   const T* G0;         // [ny][lhx] filter kernels (include 1/(nx ny))
   const T* G1;
   const cplx<T>* tw_in;   // length NY table
@@ -1058,9 +1062,11 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   __syncwarp();  // the column's forward reads are done before its slot is rewritten
   cplx<T>* sout = bin + c * SI;
   const bool layers = FWD && a.op == YP_PRESS && l == a.plane0 + a.nplanes - 1;
-  const int nout = layers ? 2 : a.nout;
+  const bool wall = !FWD && SAME && a.op == YP_GRADY && l == 1 && grp < 2 && a.wall[grp] && col0 < a.ncols1;
+  const int nout = layers ? 2 : a.nout + (wall ? 1 : 0);
   for (int q = 0; q < nout; ++q) {
-    if (!layers && !a.out[grp * a.nout + q]) continue;  // an optional output left out (the same for the whole CTA)
+    const bool third = wall && q == a.nout;
+    if (!layers && !third && !a.out[grp * a.nout + q]) continue;  // an optional output left out (the whole CTA)
     if (a.op == YP_FILTER2 && q == 1 && col0 >= a.ncols1) continue;  // all columns beyond the narrower filter
     if constexpr (SAME) {
       // forward output layout (groups FO) == inverse input layout; the
@@ -1100,7 +1106,16 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
                                              : cplx<T>{T(0), T(0)};
             }
         };
-        if (a.op == YP_GRADY) {
+        if (third) {
+#pragma unroll
+          for (int g = 0; g < EI / FO; ++g)
+#pragma unroll
+            for (int r = 0; r < FO; ++r) {
+              const int ky = lt + TL * g + r * (NY / FO);
+              const T gv = (kx < a.ncols1) ? a.G0[ky * a.lhx + kx] * a.gs : T(0);
+              w[g * FO + r] = c_scl(f0[g * FO + r], gv);
+            }
+        } else if (a.op == YP_GRADY) {
           fill(std::integral_constant<int, YP_GRADY>{});
         } else if (a.op == YP_GRAD) {
           fill(std::integral_constant<int, YP_GRAD>{});
@@ -1166,7 +1181,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
     }
     __syncthreads();
     // coalesced store of output q
-    const bool second = (a.op == YP_FILTER2 && q == 1);
+    const bool second = (a.op == YP_FILTER2 && q == 1) || third;
     const int lim = second ? a.ncols1 : a.ncols;
     {
       // thread -> fixed column cc, rows ky0 + TL i (as in yp_issue)
@@ -1176,8 +1191,10 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
         const int ky0 = threadIdx.x >> a.lc;
         const long opitch = second ? a.opitch1 : a.opitch;
         const int lo = (layers && q == 0) ? 0 : l;
-        cplx<T>* dst = a.out[layers ? 0 : grp * a.nout + q] + (long)lo * (second ? a.out_pstride1 : a.out_pstride) + kxx +
-                       (long)ky0 * opitch;
+        cplx<T>* plane = third ? a.wall[grp]
+                               : a.out[layers ? 0 : grp * a.nout + q] +
+                                     (long)lo * (second ? a.out_pstride1 : a.out_pstride);
+        cplx<T>* dst = plane + kxx + (long)ky0 * opitch;
         const cplx<T>* srow = bin + cc * SI + ky0;
         const long step = (long)TL * opitch;
 #pragma unroll
