@@ -1946,12 +1946,12 @@ class Solver final : public SolverBase {
       a.qs = SP.surface_flux;
       sbytes += 6.0;
     }
-    if (g.plane() % 4 == 0)
-      KL("k_sgs_tau", sbytes * (g.nz + 1) * g.plane() * sizeof(T),
-         k_sgs_tau4<T><<<dim3(unsigned((g.plane() / 4 + 255) / 256), unsigned(g.nz + 1)), 256, 0, st>>>(a));
-    else
-      KL("k_sgs_tau", 17.0 * (g.nz + 1) * g.plane() * sizeof(T),
-         k_sgs_tau<T><<<dim3(unsigned((g.plane() + 255) / 256), unsigned(g.nz + 1)), 256, 0, st>>>(a));
+    // levels per thread: enough chunks for ~6 blocks per SM, at most 16 levels
+    constexpr int V = 16 / int(sizeof(T));
+    const int bx = ceil_div(g.plane() / V, 256);
+    const int zc = int(std::min(16L, std::max(1L, (long)(g.nz + 1) * bx / (148 * 6))));
+    KL("k_sgs_tau", sbytes * n1 * sizeof(T),
+       k_sgs_tau<T, V><<<dim3(unsigned(bx), unsigned(ceil_div(g.nz + 1, zc))), 256, 0, st>>>(a, zc));
   }
 
   // dynamic-procedure contractions at both test scales (compute_dynamic_mum x2)
