@@ -1417,6 +1417,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
 enum XIOp : int {
   XI_STORE = 0,  // out[f](l) = x_f for lo[f] <= l <= hi[f]
   XI_CONV = 1,   // -u, -v, -w and the vorticity from the spectra of u, v, w and their y derivatives
+  XI_CONVS = 6,  // the gradient of theta from the spectra of theta and i ky theta
   XI_DIV = 2,    // rhs += x + dz(tz) + pf ; pressure-BC layers of the w equation
   XI_LASD = 3,   // 21 filtered fields -> L:M and M:M
   XI_WALL = 4,   // filtered u1, v1 -> u*, Neumann ghost value, wall stress
@@ -1457,6 +1458,7 @@ struct XIArgs {
   int src[MAXIN];
   int dx[MAXIN];
   const T* kxr;
+  // XI_CONVS: staged rows theta, i ky theta at level l, theta at l - 1;
   // XI_CONV: staged rows u, v, w, i ky u, i ky w at level l, then u, v at
   // l - 1; refin[0..2] the per-plane references of u, v, w; c0 = 1/dz,
   // c1 the scale of the spectra
@@ -1476,6 +1478,7 @@ struct XIArgs {
 // whose derivatives the gradients hold.
 template <typename T>
 __device__ __forceinline__ int xi_plane(const XIArgs<T>& a, int f, int l) {
+  if (a.op == XI_CONVS) return f == 2 ? l - 1 : l;
   if (a.op != XI_CONV) return l;
   if (f >= 5) return l - 1;
   if (f == 2) return l == 1 ? 0 : (l == a.nz + 1 ? l + 1 : l);
@@ -1638,9 +1641,26 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   }
   // a plain store writes straight from registers; the other ops combine
   // fields per point through shared memory
-  const bool conv = (a.op == XI_CONV);
+  const bool conv = (a.op == XI_CONV) || (a.op == XI_CONVS);
   const bool direct = (a.op == XI_STORE) || conv;
-  if (conv) {
+  if (a.op == XI_CONVS) {
+    // i kx theta over theta, d theta / dz over theta(l - 1); plane 0 holds the
+    // wall's d theta / dz(1) itself
+    cplx<T>* rows = const_cast<cplx<T>*>(stage);
+    const T rdz = T(a.c0);
+    for (int idx = threadIdx.x; idx < a.R * a.nk; idx += blockDim.x) {
+      const int r = udiv32(idx, a.nk);
+      const int m = idx - r * a.nk;
+      const int l = rowl[r];
+      if (l < 0) continue;
+      cplx<T>* q = rows + (long)r * 3 * a.nks + m;
+      const cplx<T> t = q[0];
+      if (l > 1) q[2 * a.nks] = c_scl(c_sub(t, q[2 * a.nks]), rdz);
+      q[0] = ik_mul(kxs[m], t);
+    }
+    __syncthreads();
+  }
+  if (a.op == XI_CONV) {
     // the vorticity in the staged rows: o1 over i ky w, o2 over u(l - 1), o3
     // over i ky u (compute_convective_padd.f90:145-165; the wall rows' means
     // of w derivatives over levels 1 and 2).  Boundary levels take the w of
@@ -1685,7 +1705,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     }
     // merged: the staged row of sequence s is its slot (slots past the last
     // sequence follow the staged rows)
-    const int srow = conv ? (s < nseq ? r * 7 + a.src[f] : a.R * 7 + (s - nseq)) : s;
+    const int srow = conv ? (s < nseq ? r * ns + a.src[f] : a.R * ns + (s - nseq)) : s;
     cplx<T>* seq = a.merged ? const_cast<cplx<T>*>(stage) + (long)srow * a.nks : buf + (long)s * SL;
     // c2r split: Z_m = (X_m + conj X_{M-m}) + i W^{-m} (X_m - conj X_{M-m}),
     // imaginary parts of the DC and Nyquist bins ignored
@@ -1768,7 +1788,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     if (direct) {
       if (valid && l >= a.lo[f] && l <= a.hi[f]) {
         T ref = T(0);
-        if (conv) {
+        if (a.op == XI_CONVS) {
+          if (f == 2 && l > 1 && a.refin[0]) ref = T((double(a.refin[0][l]) - double(a.refin[0][l - 1])) * a.c0);
+        } else if (conv) {
           // -u, -v, -w and their levels' references; the vertical differences'
           if (f < 3) ref = a.refin[f] ? -a.refin[f][xi_plane(a, f, l)] : T(0);
           else if (f < 5 && a.refin[0]) {
@@ -1780,7 +1802,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
           ref = a.refin[f][l];
         }
         const cplx<T> ref2 = {ref, ref};
-        const T sg = conv ? T(f < 3 ? -a.c1 : a.c1) : T(1);
+        const T sg = conv ? T(a.op == XI_CONV && f < 3 ? -a.c1 : a.c1) : T(1);
         const cplx<T> sg2 = {sg, sg};
         const long off = (long)l * a.out_pstride + (long)j * NX;
         // the store form is chosen once per sequence (outside the unrolled loop)

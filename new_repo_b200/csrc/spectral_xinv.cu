@@ -30,7 +30,7 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   // in its own staged row (the exchange slot is the row), which leaves room
   // for more rows per work item
   // (XI_CONV: six of its seven staged rows become sequences)
-  a.merged = ((a.op == XI_STORE && a.nstage == 0) || a.op == XI_CONV) ? 1 : 0;
+  a.merged = ((a.op == XI_STORE && a.nstage == 0) || a.op == XI_CONV || a.op == XI_CONVS) ? 1 : 0;
   if (a.merged) a.nks = std::max(a.nks, SL);
   auto stage_rows = [&](int R) {
     return a.merged ? R * (ns - a.nin) + pad_seqs(R * a.nin, M) : R * ns;
