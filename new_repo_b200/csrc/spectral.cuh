@@ -1554,7 +1554,25 @@ __device__ __forceinline__ void xi_issue_bulk(const XIArgs<T>& a, long item, cpl
   }
 }
 
-template <typename T, int NX>
+// The ops of the x inverse in classes, each compiled on its own.  With every op
+// in one kernel the register limit that its occupancy needs (64 in FP32, 128
+// in FP64, at 256 threads) spilled 30-190 bytes per thread into each of them;
+// apart, at 256^3 FP64: convective inputs 954 -> 870 us, the
+// contractions of the LASD model 1485 -> 1273, stress divergence 346 -> 324; at 512 x 512
+// x 96 FP32 convective inputs 807 -> 763, gradients 487 -> 457, scalar 268 ->
+// 245, stress divergence 299 -> 270.
+enum XIClass : int { XC_STORE = 0, XC_CONV = 1, XC_DIV = 2, XC_DYN = 3, XC_WALL = 4 };
+inline int xi_class(int op) {
+  switch (op) {
+    case XI_CONV: case XI_CONVS: return XC_CONV;
+    case XI_DIV: return XC_DIV;
+    case XI_LASD: case XI_SCDYN: return XC_DYN;
+    case XI_WALL: return XC_WALL;
+    default: return XC_STORE;
+  }
+}
+
+template <typename T, int NX, int CLS>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2) k_xinv(const XIArgs<T> a) {
   constexpr int M = NX / 2;
   constexpr int TL = Geo<M>::T;
@@ -1641,9 +1659,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   }
   // a plain store writes straight from registers; the other ops combine
   // fields per point through shared memory
-  const bool conv = (a.op == XI_CONV) || (a.op == XI_CONVS);
-  const bool direct = (a.op == XI_STORE) || conv;
-  if (a.op == XI_CONVS) {
+  constexpr bool conv = CLS == XC_CONV;
+  constexpr bool direct = CLS == XC_STORE || conv;
+  if (conv && a.op == XI_CONVS) {
     // i kx theta over theta, d theta / dz over theta(l - 1); plane 0 holds the
     // wall's d theta / dz(1) itself
     cplx<T>* rows = const_cast<cplx<T>*>(stage);
@@ -1660,7 +1678,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     }
     __syncthreads();
   }
-  if (a.op == XI_CONV) {
+  if (conv && a.op == XI_CONV) {
     // the vorticity in the staged rows: o1 over i ky w, o2 over u(l - 1), o3
     // over i ky u (compute_convective_padd.f90:145-165; the wall rows' means
     // of w derivatives over levels 1 and 2).  Boundary levels take the w of
@@ -1785,10 +1803,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       else split(std::false_type{}, std::false_type{});
     }
     reg_fft<T, M, true>(v, seq, lane_t, twm);
-    if (direct) {
+    if constexpr (direct) {
       if (valid && l >= a.lo[f] && l <= a.hi[f]) {
         T ref = T(0);
-        if (a.op == XI_CONVS) {
+        if (conv && a.op == XI_CONVS) {
           if (f == 2 && l > 1 && a.refin[0]) ref = T((double(a.refin[0][l]) - double(a.refin[0][l - 1])) * a.c0);
         } else if (conv) {
           // -u, -v, -w and their levels' references; the vertical differences'
@@ -1837,63 +1855,65 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         for (int rr = 0; rr < RO; ++rr) seq[lane_t + TL * gg + rr * (M / RO)] = v[gg * RO + rr];
     }
   }
-  if (!direct) {
+  if constexpr (!direct) {
   __syncthreads();
   const T* xs = reinterpret_cast<const T*>(buf);  // x_i of sequence s at xs[s*XS + i]
-  // four consecutive points per thread
-  for (int idx = threadIdx.x; idx < a.R * (NX / 4); idx += blockDim.x) {
-    const int r = idx / (NX / 4);
-    const int i0 = 4 * (idx - r * (NX / 4));
-    const int l = rowl[r];
-    if (l < 0) continue;
-    const int j = rowj[r];
-    T* xw0 = const_cast<T*>(xs) + (long)(r * a.nin) * XS + i0;
-    for (int f = 0; f < a.nin; ++f)  // this thread alone touches (r, i0..i0+3)
-      if (a.refin[f] && l >= a.lo_ref && l <= a.hi_ref) {
-        const T rf = a.refin[f][l];
+  if constexpr (CLS == XC_DIV) {
+    // compute_derivatives.f90:544-574 + LES_engine.f90:546-551, one equation
+    // per input (up to three): out[q] = rhs, aux[q] = tz, lo[q] = stag, pf[q]
+    // = forcing; out[8]/out[9] = bottom/top pressure-BC layers of the
+    // non-staggered (w) equation.  c0 = 1/dz.  Four consecutive points per
+    // thread; the tz values of every equation are loaded before the first
+    // right-hand side is stored (read-only path: nothing here writes them).
+    using V = V4<T>;
+    const T rdz = T(a.c0);
+    const long pl = a.out_pstride;
+    for (int idx = threadIdx.x; idx < a.R * (NX / 4); idx += blockDim.x) {
+      const int r = idx / (NX / 4);
+      const int i0 = 4 * (idx - r * (NX / 4));
+      const int l = rowl[r];
+      if (l < 0) continue;
+      const long p2 = (long)rowj[r] * NX + i0;
+      const long off = (long)l * pl + p2;
+      const T* x = xs + (long)(r * a.nin) * XS + i0;
+      const bool in = l >= 1 && l <= a.nz;
+      V dzq[3];
+      if (in) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) xw0[f * XS + q] += rf;
+        for (int q = 0; q < 3; ++q)
+          if (q < a.nin) {
+            const T* tz = a.aux[q];
+            dzq[q] = a.lo[q] ? rdz * (vldg<V>(tz, off + pl) - vldg<V>(tz, off))   // ddz_w
+                             : rdz * (vldg<V>(tz, off) - vldg<V>(tz, off - pl));  // ddz_uv
+          }
       }
-    if (a.op == XI_DIV) {
-      // compute_derivatives.f90:544-574 + LES_engine.f90:546-551, one
-      // equation per input: out[q] = rhs, aux[q] = tz, lo[q] = stag,
-      // pf[q] = forcing; out[8]/out[9] = bottom/top pressure-BC layers of
-      // the non-staggered (w) equation.  c0 = 1/dz.
-      using V = V4<T>;
-      const T rdz = T(a.c0);
-      const long pl = a.out_pstride;
-      const long off = (long)l * pl + (long)j * NX + i0;
-      const long p2 = (long)j * NX + i0;
-      for (int q = 0; q < a.nin; ++q) {
-        const T* tz = a.aux[q];
-        const V xq = vld<V>(static_cast<const T*>(xw0), (long)q * XS);
-        if (l >= 1 && l <= a.nz) {
-          const V dzq = a.lo[q] ? rdz * (vld<V>(tz, off + pl) - vld<V>(tz, off))   // ddz_w
-                                : rdz * (vld<V>(tz, off) - vld<V>(tz, off - pl));  // ddz_uv
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (q >= a.nin) break;
+        V xq = vld<V>(x, (long)q * XS);
+        if (a.refin[q] && l >= a.lo_ref && l <= a.hi_ref) xq = xq + vsplat<V>(a.refin[q][l]);
+        if (in) {
           const V base = a.fresh ? xq : vld<V>(a.out[q], off) + xq;
-          vst(a.out[q] + off, (base + dzq) + vsplat<V>(T(a.pf[q])));
-          if (!a.lo[q] && l == 1 && a.out[8]) vst(a.out[8] + p2, xq + dzq);
+          vst(a.out[q] + off, (base + dzq[q]) + vsplat<V>(T(a.pf[q])));
+          if (!a.lo[q] && l == 1 && a.out[8]) vst(a.out[8] + p2, xq + dzq[q]);
         }
         if (!a.lo[q] && l == a.nz + 1 && a.out[9]) vst(a.out[9] + p2, xq);
       }
-      continue;
     }
-    if (a.op == XI_WALL) continue;  // below, one point per thread
-#pragma unroll 1
-    for (int q4 = 0; q4 < 4; ++q4) {
-    const int i = i0 + q4;
-    const long off = (long)l * a.out_pstride + (long)j * NX + i;
-    const T* x = xw0 + q4;  // field f at x[f*XS]
-    switch (a.op) {
-      case XI_STORE: {
-        for (int f = 0; f < a.nin; ++f)
-          if (l >= a.lo[f] && l <= a.hi[f]) {
-            if (a.out_f32) a.outf[f][off] = float(x[f * XS]);
-            else a.out[f][off] = x[f * XS];
-          }
-        break;
-      }
-      case XI_LASD: {
+  }
+  if constexpr (CLS == XC_DYN) {
+    // one point per thread: consecutive lanes read consecutive values of
+    // every field's slot (four points per thread read them at a stride of
+    // four, four lanes to a bank, and left most threads of a one-row item
+    // idle: the 21-field contraction at 256^3 FP64 went from 1836 to 1485 us)
+    for (int idx = threadIdx.x; idx < a.R * NX; idx += blockDim.x) {
+      const int r = idx / NX;
+      const int i = idx - r * NX;
+      const int l = rowl[r];
+      if (l < 0) continue;
+      const long off = (long)l * a.out_pstride + (long)rowj[r] * NX + i;
+      const T* x = xs + (long)(r * a.nin) * XS + i;  // field f at x[f*XS]
+      if (a.op == XI_LASD) {
         // compute_LagScaleDep.f90:541-594; c0 = 2 delta^2, c1 = alpha^2
         const T uf = x[0], vf = x[XS], wf = x[2 * XS];
         const T a11 = x[3 * XS] - uf * uf;
@@ -1915,9 +1935,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         const T b33 = cst * (x[20 * XS] - tf2 * sft * s33);
         a.out[0][off] = a11 * b11 + a22 * b22 + a33 * b33 + T(2) * (a12 * b12 + a13 * b13 + a23 * b23);
         a.out[1][off] = b11 * b11 + b22 * b22 + b33 * b33 + T(2) * (b12 * b12 + b13 * b13 + b23 * b23);
-        break;
-      }
-      case XI_SCDYN: {
+      } else {
         // K_j = filt(u_j theta) - filt(u_j) filt(theta),
         // X_j = Delta^2 (filt(|S| d_j theta) - alpha^2 |S~| filt(d_j theta));
         // c0 = Delta^2, c1 = alpha^2
@@ -1935,24 +1953,22 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         const T x3 = d2 * (x[18 * XS] - tf2 * sft * x[15 * XS]);
         a.out[0][off] = k1 * x1 + k2 * x2 + k3 * x3;
         a.out[1][off] = x1 * x1 + x2 * x2 + x3 * x3;
-        break;
       }
     }
-    }
   }
-  if (a.op == XI_WALL) {
+  if constexpr (CLS == XC_WALL) {
     // compute_wall_law.f90:143-183, 247-251 on the filtered first level, one
     // point per thread (a plane is few rows, and the FP64 logarithm and
     // divisions of a point are a long dependent chain): c0 = dz, aux[0] = z0
     // plane; out: u_star_avg, lbc_u, lbc_v, txz(1), tyz(1), dudz(1), dvdz(1)
-    __syncthreads();
     for (int idx = threadIdx.x; idx < a.R * NX; idx += blockDim.x) {
       const int r = idx / NX;
       const int i = idx - r * NX;
       if (rowl[r] < 0) continue;
       const long p2 = (long)rowj[r] * NX + i;
       const T* x = xs + (long)(r * a.nin) * XS + i;
-      const double u1 = double(x[0]), v1 = double(x[XS]);
+      const T ru = a.refin[0] ? a.refin[0][rowl[r]] : T(0), rv = a.refin[1] ? a.refin[1][rowl[r]] : T(0);
+      const double u1 = double(x[0] + ru), v1 = double(x[XS] + rv);
       const double uavg = sqrt(u1 * u1 + v1 * v1);
       const double dz = a.c0;
       const double ustar = KVONK * uavg / log((0.5 * dz) / double(a.aux[0][p2]));

@@ -6,6 +6,31 @@
 
 namespace les {
 
+// the kernel of a length and class (nullptr: none): the products' lengths for
+// plain stores and the convective inputs, the grids' own for the rest
+template <typename T>
+static auto xinv_kernel(int NX, int cls) -> void (*)(XIArgs<T>) {
+  switch (NX) {
+#define XI_CASE(N) \
+  case N: if (cls == XC_STORE) return k_xinv<T, N, XC_STORE>; if (cls == XC_CONV) return k_xinv<T, N, XC_CONV>; break;
+    LES_LENGTHS(XI_CASE)
+#undef XI_CASE
+    default: return nullptr;
+  }
+  switch (NX) {
+#define XI_CASE(N)                                           \
+  case N:                                                    \
+    if (cls == XC_DIV) return k_xinv<T, N, XC_DIV>;          \
+    if (cls == XC_DYN) return k_xinv<T, N, XC_DYN>;          \
+    if (cls == XC_WALL) return k_xinv<T, N, XC_WALL>;        \
+    break;
+    XI_CASE(16) XI_CASE(32) XI_CASE(64) XI_CASE(128) XI_CASE(256) XI_CASE(512)
+#undef XI_CASE
+    default: break;
+  }
+  return nullptr;
+}
+
 template <typename T>
 void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   const int M = NX / 2;
@@ -51,15 +76,8 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
                               (a.merged ? 0 : (size_t)pad_seqs(R * a.nin, M) * SL)) +
            2 * sizeof(int) * R + (a.nstage ? sizeof(T) * (a.nk + 2) : 0) + (a.bulk ? 2 * sizeof(uint64_t) + 8 : 0);
   };
-  void (*kern)(XIArgs<T>) = nullptr;
-  switch (NX) {
-#define XI_CASE(N) \
-  case N: kern = k_xinv<T, N>; break;
-    LES_LENGTHS(XI_CASE)
-#undef XI_CASE
-    default:
-      throw CudaError(1, "xinv: unsupported transform length " + std::to_string(NX));
-  }
+  void (*const kern)(XIArgs<T>) = xinv_kernel<T>(NX, xi_class(a.op));
+  if (!kern) throw CudaError(1, "xinv: unsupported transform length " + std::to_string(NX));
   // two stages unless one stage keeps strictly more sequence slots busy
   // (more resident CTAs where shared memory limits them)
   {
@@ -97,14 +115,21 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
 
 template <typename T>
 void set_attrs_xinv() {
-#define XA(N) LES_CUDA(cudaFuncSetAttribute(k_xinv<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
+#define XA(N)                                                                                             \
+  for (int c : {XC_STORE, XC_CONV, XC_DIV, XC_DYN, XC_WALL})                                              \
+    if (auto k = xinv_kernel<T>(N, c))                                                                     \
+      LES_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
   LES_LENGTHS(XA)
 #undef XA
 }
 
-template void launch_xinv<float>(int, XIArgs<float>, cudaStream_t);
+// one translation unit per type (they compile side by side)
+#ifdef LES_XINV_DOUBLE
 template void launch_xinv<double>(int, XIArgs<double>, cudaStream_t);
-template void set_attrs_xinv<float>();
 template void set_attrs_xinv<double>();
+#else
+template void launch_xinv<float>(int, XIArgs<float>, cudaStream_t);
+template void set_attrs_xinv<float>();
+#endif
 
 }  // namespace les
