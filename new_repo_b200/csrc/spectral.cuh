@@ -118,6 +118,7 @@ enum XFOp : int {
 template <typename T>
 struct XFArgs {
   int op, nf, R;
+  int lfast;       // k_xfwd: a CTA's rows are one row of R consecutive levels
   long nrows;      // rows to process = nplanes * rows_pp
   int rows_pp;     // rows per plane of the input grid
   int plane0;      // first level
@@ -469,23 +470,31 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   int* rowj = rowl + a.R;
   for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = c_scl(a.tw[i], T(0.5));  // W^k / 2 for the split
   twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
-  const long g0 = (long)blockIdx.x * a.R;
+  // rows of this CTA: consecutive rows of the grid, or (lfast) one row of R
+  // consecutive levels
+  const int nlev = udiv32(a.nrows, a.rows_pp);
   for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
-    const long g = g0 + r;
-    rowl[r] = (g < a.nrows) ? a.plane0 + udiv32(g, a.rows_pp) : -1;
-    rowj[r] = (g < a.nrows) ? umod32(g, a.rows_pp) : 0;
+    int q, j;  // level index and row
+    if (a.lfast) {
+      q = udiv32(blockIdx.x, a.rows_pp) * a.R + r;
+      j = umod32(blockIdx.x, a.rows_pp);
+    } else {
+      const long g = (long)blockIdx.x * a.R + r;
+      q = udiv32(g, a.rows_pp);
+      j = umod32(g, a.rows_pp);
+    }
+    rowl[r] = q < nlev ? a.plane0 + q : -1;
+    rowj[r] = q < nlev ? j : 0;
   }
   __syncthreads();
   if (a.use_ref) {
     for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
-      const long g = g0 + r;
-      if (g >= a.nrows) continue;
-      const int l = a.plane0 + udiv32(g, a.rows_pp);
-      const int j = umod32(g, a.rows_pp);
+      const int l = rowl[r];
+      if (l < 0) continue;
       xf_load<T, T>(a, l, 0, 0, refs + r * a.nf, 1);
       for (int f = 0; f < a.nf; ++f) {
         if (!a.refout[f]) refs[r * a.nf + f] = T(0);
-        else if (j == 0) a.refout[f][l] = T(double(refs[r * a.nf + f]) * a.ref_mul);
+        else if (rowj[r] == 0) a.refout[f][l] = T(double(refs[r * a.nf + f]) * a.ref_mul);
       }
     }
     __syncthreads();
