@@ -446,12 +446,12 @@ int les_mlp_check_profile(les_state* s, double* out, int n);
  * launches are not counted by les_profile / les_launch_count of a state used
  * on the calling thread (the launch observer is per host thread and is
  * suspended for the duration of the call only).  It allocates
- * nothing: the tables and spectra live in one static device buffer of
+ * nothing: what it keeps in device memory lives in one static device buffer of
  * LES_NOALLOC_SCRATCH_BYTES, for callers that must not change the device
  * memory footprint (an in-situ hook in a coupled run whose memory is fully
  * committed, a process whose free memory a caching allocator holds).
- * Sizes needing more scratch than the buffer are rejected (LES_ERR_INVALID,
- * message in les_noalloc_last_error).  The first call on a device looks up
+ * Sizes whose tables and three spectra need more than the buffer are rejected
+ * (LES_ERR_INVALID, message in les_noalloc_last_error).  The first call on a device looks up
  * the buffer's address and sets kernel attributes; make it before any stream
  * capture.  All calls share the buffer of their device: calls in flight at
  * the same time on one device race.  Asynchronous on `stream` (a

@@ -335,6 +335,28 @@ constexpr int exch_shift(int N, int ES, int R, int NS, int R2) {
   if (N == 768 && ES == 16 && R == 24 && NS == 1 && R2 == 8) return 3;
   return -1;
 }
+// A sequence's exchange slot: contiguous values of its own (a pointer, laid
+// out by exch_pos), or the column of a row-major array that holds the sequence
+// itself: element i at row i, or (SH >= 0) at row i ^ ((i >> SH) & 1), which
+// for a radix-2^SH pass puts the stores of neighbouring lanes on rows of
+// different parity.
+template <typename T, int SH>
+struct ColSlot {
+  cplx<T>* p;
+  int rs;
+  __device__ __forceinline__ cplx<T>& operator[](int i) const {
+    if constexpr (SH >= 0) return p[(i ^ ((i >> SH) & 1)) * rs];
+    else return p[i * rs];
+  }
+};
+template <typename Slot>
+struct SlotPadded {
+  static constexpr bool value = true;
+};
+template <typename T, int SH>
+struct SlotPadded<ColSlot<T, SH>> {
+  static constexpr bool value = false;
+};
 template <int S>
 __device__ __forceinline__ int exch_pos(int i) {
   if constexpr (S < 0) return i + (i >> 4);
@@ -345,8 +367,8 @@ __device__ __forceinline__ int exch_pos(int i) {
 // one pass of radix R with Ns = product of the previous radices, its
 // twiddle factors at twm[OFF + (r-1) Ns + k]; then the exchange into the next
 // pass's input layout (if any)
-template <typename T, int N, int E, bool INV, int Ns, int OFF, int R, int... Rest>
-__device__ __forceinline__ void reg_passes(cplx<T>* v, cplx<T>* seq, int t, const cplx<T>* __restrict__ twm) {
+template <typename T, int N, int E, bool INV, int Ns, int OFF, int R, int... Rest, typename Slot>
+__device__ __forceinline__ void reg_passes(cplx<T>* v, Slot seq, int t, const cplx<T>* __restrict__ twm) {
   constexpr int TL = N / E;
   constexpr int G = E / R;
 #pragma unroll
@@ -365,7 +387,7 @@ __device__ __forceinline__ void reg_passes(cplx<T>* v, cplx<T>* seq, int t, cons
   if constexpr (sizeof...(Rest) > 0) {
     constexpr int R2 = FirstOf<Rest...>::value;
     constexpr int G2 = E / R2;
-    constexpr int SW = exch_shift(N, int(sizeof(cplx<T>)), R, Ns, R2);
+    constexpr int SW = SlotPadded<Slot>::value ? exch_shift(N, int(sizeof(cplx<T>)), R, Ns, R2) : 0;
     __syncwarp();
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -383,8 +405,8 @@ __device__ __forceinline__ void reg_passes(cplx<T>* v, cplx<T>* seq, int t, cons
   }
 }
 
-template <typename T, int N, bool INV, int... Rs>
-__device__ __forceinline__ void reg_fft_impl(cplx<T>* v, cplx<T>* seq, int t, const cplx<T>* twm,
+template <typename T, int N, bool INV, typename Slot, int... Rs>
+__device__ __forceinline__ void reg_fft_impl(cplx<T>* v, Slot seq, int t, const cplx<T>* twm,
                                              std::integer_sequence<int, Rs...>) {
   reg_passes<T, N, Geo<N>::E, INV, 1, 0, Rs...>(v, seq, t, twm);
 }
@@ -514,8 +536,8 @@ __device__ __forceinline__ void twm_build(const cplx<T>* tw, cplx<T>* twm, int t
 // lanes); twm holds the twiddle matrices built by twm_build<T, N, INV>.
 // Forward transforms run the plan's radices in order, inverse transforms in
 // reverse order.
-template <typename T, int N, bool INV>
-__device__ __forceinline__ void reg_fft(cplx<T>* v, cplx<T>* seq, int t, const cplx<T>* twm) {
+template <typename T, int N, bool INV, typename Slot>
+__device__ __forceinline__ void reg_fft(cplx<T>* v, Slot seq, int t, const cplx<T>* twm) {
   reg_fft_impl<T, N, INV>(v, seq, t, twm, typename PassOrder<N, INV>::seq{});
 }
 

@@ -1,9 +1,10 @@
 // les_grad_xy_noalloc: horizontal spectral derivatives of a device field
 // with every intermediate in one fixed, file-scope device buffer.
 //
-// The same three spectral passes as les_grad_velocity_filt (x r2c FFT with
-// the 1/(nx*ny) scaling, y pass with the ik multiplications and the Nyquist
-// kill, inverse x transforms of the filtered field and both derivatives),
+// The arithmetic of les_grad_velocity_filt (x r2c FFT with the 1/(nx*ny)
+// scaling, y pass with the ik multiplications and the Nyquist kill, inverse x
+// transforms of the filtered field and both derivatives): in one launch, a CTA
+// per level, where a plane fits into shared memory, else in three passes,
 // launched on caller-owned device pointers.  It exists for callers that must
 // not change the device memory footprint and so cannot allocate: an in-situ
 // analysis hook called from a coupled model whose device memory is fully
@@ -12,13 +13,15 @@
 // cache to be released.  Nothing here allocates: no cudaMalloc/cudaFree, no
 // CUDA events, no host containers, no library that allocates.
 //
-// Scratch: g_noalloc_scratch (LES_NOALLOC_SCRATCH_BYTES) holds, 256-byte
-// aligned, the wavenumber tables kkx, kky [ny][nx/2+1], the twiddle tables
-// of nx and ny, and three spectra [nlev][ny][nx/2+1] (complex FP64).  Every
-// call writes all of these before reading them, so nothing has to start at
-// zero.  All calls in the process share the buffer of their device: two calls
-// in flight at the same time on one device (different streams or host
-// threads) race on it.
+// Scratch: g_noalloc_scratch (LES_NOALLOC_SCRATCH_BYTES) has room for, 256-byte
+// aligned, the wavenumber tables kkx, kky [ny][nx/2+1], the twiddle tables of
+// nx and ny, and three spectra [nlev][ny][nx/2+1] (complex FP64): what a call
+// may need, and what decides whether its size is accepted; the three-pass form
+// uses two of the spectra, the plane form at most one and no tables.  Every
+// call writes what it reads there first, so nothing has to start at zero.  All
+// calls in the process share the buffer of their device: two calls in flight
+// at the same time on one device (different streams or host threads) race on
+// it.
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -92,6 +95,276 @@ __global__ void k_noalloc_tables(double* kkx, double* kky, cplx<double>* twx, cp
   }
 }
 
+// ---- whole planes in shared memory ----
+// A level whose spectrum fits into shared memory is differentiated by one CTA
+// in one launch: rows in by bulk copies, x transforms in place, the columns'
+// y transforms there and (F and i ky F) back without leaving registers, the x
+// inverses out; i kx F is formed as the rows are read.  The spectrum of d/dy
+// waits in a second array (two) or, where that does not fit, in the scratch
+// buffer, which L2 holds.  The twiddles and wavenumbers are computed by the
+// CTA, so the call needs no table launch.  Small planes are bound by launches
+// and latency, which the four launches of the three-pass form pay four times,
+// larger ones by shared memory, ~25 accesses per value.  Three passes against
+// this, us: 16 x 16 x 100 26.6 / 6.2, 64 x 64 x 148 41 / 12.3, 96 x 64 x 100 41
+// / 16.4, 128 x 64 x 159 (two waves) 61 / 34, 128 x 128 x 79 54 / 37.
+template <int NX, int NY>
+struct PlaneGrad {
+  static constexpr int M = NX / 2;
+  static constexpr int SLX = slot_stride(M, 16);
+  static constexpr int need = SLX > M + 1 ? SLX : M + 1;
+  // row stride in complex values: the row's slot and the M + 1 modes, 4 modulo
+  // 8, so that four columns of two neighbouring rows, and four values of two
+  // neighbouring rows, fall on eight different 16-byte banks
+  static constexpr int RS = (need + 3) / 8 * 8 + 4;
+  static constexpr int lanes_x = NY * Geo<M>::T, lanes_y = M * Geo<NY>::T;
+  static constexpr int want = ((lanes_x > lanes_y ? lanes_x : lanes_y) + 31) / 32 * 32;
+  // a thread holds two transforms of up to 24 values: all 255 registers
+  static constexpr int threads = want < 64 ? 64 : (want > 256 ? 256 : want);
+  static constexpr size_t array = sizeof(cplx<double>) * (size_t)NY * RS;
+  static constexpr size_t tables = sizeof(cplx<double>) * (NX + NY + twm_len(M, false) + twm_len(M, true) +
+                                                           twm_len(NY, false) + twm_len(NY, true)) + 16;
+  static constexpr size_t cap = 227 * 1024;
+  static constexpr bool two = 2 * array + tables <= cap;
+  static constexpr size_t smem = (two ? 2 : 1) * array + tables;
+  static_assert(smem <= cap, "plane beyond shared memory");
+};
+
+template <int NX, int NY>
+__global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
+    k_grad_plane(double* f, double* dfdx, double* dfdy, cplx<double>* scratch, double lx, double ly) {
+  using G = PlaneGrad<NX, NY>;
+  constexpr bool TWO = G::two;
+  using C = cplx<double>;
+  constexpr int M = G::M, RS = G::RS, TH = G::threads;
+  constexpr int TX = Geo<M>::T, EX = Geo<M>::E, TY = Geo<NY>::T, EY = Geo<NY>::E;
+  constexpr int XI_ = Layout<M, false>::in, XO = Layout<M, false>::out;
+  constexpr int VI = Layout<M, true>::in, VO = Layout<M, true>::out;
+  constexpr int YI = Layout<NY, false>::in, YO = Layout<NY, false>::out;
+  constexpr int ZI = Layout<NY, true>::in, ZO = Layout<NY, true>::out;
+  static_assert(ZI == YO, "the inverse y transform takes the forward one's registers");
+  // exchanges of a column: lanes of a quarter warp lie on two rows only where
+  // a column has eight lanes (NY = 128: radices 16, 8 and 8, 16)
+  using SlotF = ColSlot<double, TY == 8 ? 4 : -1>;
+  using SlotI = ColSlot<double, TY == 8 ? 3 : -1>;
+  static_assert(TY <= 4 || NY == 128, "exchange swizzle of a column");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* A = reinterpret_cast<C*>(smem_raw);
+  C* B = A + (TWO ? (long)NY * RS : 0);
+  C* twx = B + (long)NY * RS;  // exp(-2 pi i m / NX)
+  C* twy = twx + NX;
+  C* mxf = twy + NY;  // twiddle matrices: x forward, x inverse, y forward, y inverse
+  C* mxi = mxf + Twm<M, false>::len;
+  C* myf = mxi + Twm<M, true>::len;
+  C* myi = myf + Twm<NY, false>::len;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(myi + Twm<NY, true>::len);
+  const int tid = threadIdx.x;
+  const long plane = (long)blockIdx.x * NY * NX;
+  if (tid < 32) {
+    if (tid == 0) {
+      tc::mbar_init(bar, 1);
+      tc::fence_mbar_init();
+      mbar_expect_tx(bar, unsigned(NY * NX * sizeof(double)));
+    }
+    __syncwarp();
+    for (int r = tid; r < NY; r += 32) bulk_g2s(A + r * RS, f + plane + (long)r * NX, unsigned(NX * sizeof(double)), bar);
+  }
+  for (int m = tid; m < NX + NY; m += TH) {
+    const bool isx = m < NX;
+    double s, c;
+    if (isx) sincospi(-2.0 * double(m) / double(NX), &s, &c);
+    else sincospi(-2.0 * double(m - NX) / double(NY), &s, &c);
+    twx[m] = C{c, s};  // twy follows twx
+  }
+  __syncthreads();
+  twm_build<double, M, false, 2>(twx, mxf, tid, TH);
+  twm_build<double, M, true, 2>(twx, mxi, tid, TH);
+  twm_build<double, NY, false>(twy, myf, tid, TH);
+  twm_build<double, NY, true>(twy, myi, tid, TH);
+  const bool late = !tc::mbar_wait(bar, 0);
+  if (__syncthreads_or(late)) {  // as in the spectral passes: a last bounded wait, leave
+    tc::mbar_wait(bar, 0);
+    return;
+  }
+  const double pi = 3.14159265358979323846;
+  const double kx1 = 2.0 * pi / lx, ky1 = 2.0 * pi / ly;
+  // rows: body(row, lane of it, whether it is one).  (A warp reaches past the
+  // last row only where a row is one lane, whose transform exchanges nothing.)
+  static_assert(TX == 1 || NY % (32 / TX) == 0, "lanes past the last row must not exchange");
+  auto rows = [&](auto body) {
+    for (int r0 = 0; r0 < NY; r0 += TH / TX) {
+      const int r = r0 + tid / TX;
+      if (r0 + (tid & ~31) / TX >= NY) break;  // whole warp beyond the rows
+      body(r < NY ? r : 0, tid % TX, r < NY);
+    }
+  };
+  // x: r2c in place; mode M, the Nyquist bin, is killed
+  rows([&](int r, int t, bool live) {
+    const double c0 = 1.0 / (double(NX) * double(NY));
+    C* row = A + r * RS;
+    C v[EX];
+#pragma unroll
+    for (int g = 0; g < EX / XI_; ++g)
+#pragma unroll
+      for (int q = 0; q < XI_; ++q) v[g * XI_ + q] = c_scl(row[t + TX * g + q * (M / XI_)], c0);
+    reg_fft<double, M, false>(v, row, t, mxf);
+    __syncwarp();
+    if (live) {
+#pragma unroll
+      for (int g = 0; g < EX / XO; ++g)
+#pragma unroll
+        for (int q = 0; q < XO; ++q) row[t + TX * g + q * (M / XO)] = v[g * XO + q];
+    }
+    __syncwarp();
+    if (live)
+      for (int k = t; k <= M / 2; k += TX) {  // modes k and M - k need the same two values
+        const int k2 = k == 0 ? 0 : M - k;
+        const C zk = row[k], zm = row[k2];
+        row[k] = r2c_split(zk, zm, c_scl(twx[k], 0.5));
+        if (k2 > k) row[k2] = r2c_split(zm, zk, c_scl(twx[k2], 0.5));
+      }
+    __syncwarp();  // before the next row's exchange of this warp
+  });
+  __syncthreads();
+  // y: the columns of a warp vary fastest, so that the lanes of a
+  // shared-memory wavefront walk along a row.  The Nyquist row is killed; F
+  // comes back in place, i ky F in B or the scratch buffer.
+  constexpr int CW = 32 / TY;  // columns per warp
+  C* const ys = TWO ? nullptr : scratch + (long)blockIdx.x * NY * M;
+  for (int c0 = 0; c0 < M; c0 += TH / TY) {
+    const int cw = c0 + (tid >> 5) * CW;
+    if (cw >= M) break;  // whole warp
+    const int t = (tid & 31) / CW, cc = cw + (tid & 31) % CW;
+    const bool live = cc < M;
+    // lanes past the last column read it and exchange in column M, which
+    // nothing else uses
+    const int c = live ? cc : M - 1, cx = live ? cc : M;
+    C v[EY], w[EY];
+#pragma unroll
+    for (int g = 0; g < EY / YI; ++g)
+#pragma unroll
+      for (int q = 0; q < YI; ++q) v[g * YI + q] = A[(t + TY * g + q * (NY / YI)) * RS + c];
+    reg_fft<double, NY, false>(v, SlotF{A + cx, RS}, t, myf);
+#pragma unroll
+    for (int g = 0; g < EY / YO; ++g)
+#pragma unroll
+      for (int q = 0; q < YO; ++q) {
+        const int ky = t + TY * g + q * (NY / YO);
+        C& F = v[g * YO + q];
+        if (ky == NY / 2) F = C{0.0, 0.0};
+        w[g * YO + q] = ik_mul(ky1 * double(ky < NY / 2 ? ky : ky - NY), F);
+      }
+    reg_fft<double, NY, true>(w, SlotI{B + cx, RS}, t, myi);
+    if constexpr (!TWO) {
+      if (live) {
+#pragma unroll
+        for (int g = 0; g < EY / ZO; ++g)
+#pragma unroll
+          for (int q = 0; q < ZO; ++q) ys[(t + TY * g + q * (NY / ZO)) * M + c] = w[g * ZO + q];
+      }
+    } else {
+      __syncwarp();
+      if (live) {
+#pragma unroll
+        for (int g = 0; g < EY / ZO; ++g)
+#pragma unroll
+          for (int q = 0; q < ZO; ++q) B[(t + TY * g + q * (NY / ZO)) * RS + c] = w[g * ZO + q];
+      }
+    }
+    reg_fft<double, NY, true>(v, SlotI{A + cx, RS}, t, myi);
+    __syncwarp();
+    if (live) {
+#pragma unroll
+      for (int g = 0; g < EY / ZO; ++g)
+#pragma unroll
+        for (int q = 0; q < ZO; ++q) A[(t + TY * g + q * (NY / ZO)) * RS + c] = v[g * ZO + q];
+    }
+  }
+  __syncthreads();
+  // x: c2r of a row out of A (f, df/dx) and of i ky F (df/dy)
+  auto store = [&](const C* v, double* o, int r, int t) {
+#pragma unroll
+    for (int g = 0; g < EX / VO; ++g)
+#pragma unroll
+      for (int q = 0; q < VO; ++q)
+        *reinterpret_cast<C*>(o + plane + (long)r * NX + 2 * (t + TX * g + q * (M / VO))) = v[g * VO + q];
+  };
+  rows([&](int r, int t, bool live) {
+    C* row = A + r * RS;
+    C v[EX], w[EX];
+#pragma unroll
+    for (int g = 0; g < EX / VI; ++g)
+#pragma unroll
+      for (int q = 0; q < VI; ++q) {
+        const int m = t + TX * g + q * (M / VI);
+        C xk = row[m], xm = m == 0 ? C{0.0, 0.0} : row[M - m];
+        w[g * VI + q] = c2r_split(ik_mul(kx1 * double(m), xk), ik_mul(kx1 * double(M - m), xm), twx[m]);
+        if (m == 0) xk.y = 0.0;
+        v[g * VI + q] = c2r_split(xk, xm, twx[m]);
+      }
+    reg_fft<double, M, true>(v, row, t, mxi);
+    if (live) store(v, f, r, t);
+    reg_fft<double, M, true>(w, row, t, mxi);
+    if (live) store(w, dfdx, r, t);
+    const C* yr = TWO ? B + r * RS : ys + (long)r * M;
+#pragma unroll
+    for (int g = 0; g < EX / VI; ++g)
+#pragma unroll
+      for (int q = 0; q < VI; ++q) {
+        const int m = t + TX * g + q * (M / VI);
+        C xk = yr[m], xm = m == 0 ? C{0.0, 0.0} : yr[M - m];
+        if (m == 0) xk.y = 0.0;
+        v[g * VI + q] = c2r_split(xk, xm, twx[m]);
+      }
+    reg_fft<double, M, true>(v, row, t, mxi);
+    if (live) store(v, dfdy, r, t);
+    __syncwarp();
+  });
+}
+
+// the plane kernel of a grid (nullptr: none)
+struct PlaneKernel {
+  void (*run)(double*, double*, double*, cplx<double>*, double, double) = nullptr;
+  int threads = 0;
+  size_t smem = 0;
+  bool two = false;
+};
+template <int NX, int NY>
+PlaneKernel plane_kernel_of() {
+  using G = PlaneGrad<NX, NY>;
+  return {k_grad_plane<NX, NY>, G::threads, G::smem, G::two};
+}
+template <int NX>
+PlaneKernel plane_kernel_ny(int ny) {
+  switch (ny) {
+    case 16: return plane_kernel_of<NX, 16>();
+    case 32: return plane_kernel_of<NX, 32>();
+    case 64: return plane_kernel_of<NX, 64>();
+    case 128:
+      if constexpr (NX < 192) return plane_kernel_of<NX, 128>();  // beyond: more than one array
+      else return {};
+    default: return {};
+  }
+}
+PlaneKernel plane_kernel(int nx, int ny) {
+  switch (nx) {
+    case 16: return plane_kernel_ny<16>(ny);
+    case 24: return plane_kernel_ny<24>(ny);
+    case 32: return plane_kernel_ny<32>(ny);
+    case 48: return plane_kernel_ny<48>(ny);
+    case 64: return plane_kernel_ny<64>(ny);
+    case 96: return plane_kernel_ny<96>(ny);
+    case 128: return plane_kernel_ny<128>(ny);
+    case 192: return plane_kernel_ny<192>(ny);
+    case 256: return plane_kernel_ny<256>(ny);
+    default: return {};
+  }
+}
+
+// Whether a call of nlev levels takes the plane form: always where two arrays
+// fit.  The largest planes take one CTA as long as few levels take the whole
+// chip in three passes: 128 x 128 x 4 35.9 / 31.9 us, x 32 36.9 / 38.1.
+bool plane_form(const PlaneKernel& k, int nlev) { return k.run && (k.two || nlev >= 24); }
+
 // address of this device's scratch buffer; the first call on a device does
 // the setup (symbol address, kernel shared-memory attributes)
 int scratch_for_device(unsigned char** out) {
@@ -106,6 +379,11 @@ int scratch_for_device(unsigned char** out) {
     if (e != cudaSuccess)
       throw CudaError(LES_ERR_INVALID, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
     init_spectral_attributes();
+    for (int nx : {16, 24, 32, 48, 64, 96, 128, 192, 256})
+      for (int ny : {16, 32, 64, 128}) {
+        if (const PlaneKernel k = plane_kernel(nx, ny); k.run)
+          LES_CUDA(cudaFuncSetAttribute((const void*)k.run, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem)));
+      }
     addr = static_cast<unsigned char*>(p);
     g_scratch_addr[dev].store(addr);
   }
@@ -160,12 +438,19 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     unsigned char* base = nullptr;
     scratch_for_device(&base);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (const PlaneKernel pk = plane_kernel(nx, ny); plane_form(pk, nlev)) {
+      auto* ys = reinterpret_cast<cplx<double>*>(base + L.spec[0]);
+      pk.run<<<nlev, pk.threads, pk.smem, st>>>(f, dfdx, dfdy, ys, lx, ly);
+      LES_CHECK_LAUNCH();
+      g_hook = saved;
+      return rc;
+    }
     double* kkx = reinterpret_cast<double*>(base + L.kkx);
     double* kky = reinterpret_cast<double*>(base + L.kky);
     auto* twx = reinterpret_cast<cplx<double>*>(base + L.twx);
     auto* twy = reinterpret_cast<cplx<double>*>(base + L.twy);
-    cplx<double>* sp[3];
-    for (int i = 0; i < 3; ++i) sp[i] = reinterpret_cast<cplx<double>*>(base + L.spec[i]);
+    cplx<double>* sp[2];
+    for (int i = 0; i < 2; ++i) sp[i] = reinterpret_cast<cplx<double>*>(base + L.spec[i]);
     const int lhx = nx / 2 + 1;
     k_noalloc_tables<<<64, 256, 0, st>>>(kkx, kky, twx, twy, nx, ny, lx, ly);
     LES_CHECK_LAUNCH();
@@ -188,9 +473,9 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
 
     YPArgs<double> b;
     std::memset(&b, 0, sizeof(b));
-    b.op = YP_GRAD;
+    b.op = YP_GRADY;  // F and i ky F; the x inverse forms i kx F from the staged F row
     b.nin = 1;
-    b.nout = 3;
+    b.nout = 2;
     b.ncols = lhx;
     b.nk_in = lhx;
     b.nk_out = lhx;
@@ -205,7 +490,6 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     b.in[0] = sp[0];
     b.out[0] = sp[0];
     b.out[1] = sp[1];
-    b.out[2] = sp[2];
     launch_ypass<double>(ny, ny, b, nlev, 1, st);
 
     XIArgs<double> c;
@@ -219,14 +503,18 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     c.in_pstride = (long)ny * lhx;
     c.out_pstride = (long)ny * nx;
     c.tw = twx;
+    c.nstage = 2;
+    c.kxr = kkx;
+    c.in[0] = sp[0];
+    c.in[1] = sp[1];
+    double* const outs[3] = {f, dfdx, dfdy};
     for (int q = 0; q < 3; ++q) {
-      c.in[q] = sp[q];
+      c.src[q] = q == 2 ? 1 : 0;
+      c.dx[q] = q == 1;
+      c.out[q] = outs[q];
       c.lo[q] = 0;
       c.hi[q] = nlev - 1;
     }
-    c.out[0] = f;
-    c.out[1] = dfdx;
-    c.out[2] = dfdy;
     launch_xinv<double>(nx, c, st);
   } catch (const CudaError& e) {
     std::snprintf(g_noalloc_error, sizeof(g_noalloc_error), "%s", e.what());

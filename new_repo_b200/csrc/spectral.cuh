@@ -809,7 +809,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
 
 // --------------------------------------------------------------- ypass ----
 enum YPOp : int {
-  YP_GRAD = 0,     // f -> f, i kx f, i ky f           (Nyquist killed)
   YP_DIV2 = 1,     // (fx, fy) -> i kx fx + i ky fy     (Nyquist killed)
   YP_FWDKILL = 2,  // f -> f, no inverse y transform    (Nyquist killed)
   YP_PGRAD = 3,    // p^ (already y-spectral) -> p, i ky p   (i kx p in the x inverse)
@@ -859,12 +858,6 @@ template <typename T, int NY>
 __device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int ky, cplx<T> F0, cplx<T> F1) {
   const cplx<T> zero = {T(0), T(0)};
   switch (a.op) {
-    case YP_GRAD: {
-      if (ky == NY / 2 || kx == a.nxh) return zero;
-      if (q == 0) return F0;
-      if (q == 1) return ik_mul(a.kkx[ky * a.lhx + kx], F0);
-      return ik_mul(a.kky[ky * a.lhx + kx], F0);
-    }
     case YP_GRADY: {
       if (ky == NY / 2 || kx == a.nxh) return zero;
       if (q == 0) return F0;
@@ -899,12 +892,7 @@ __device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int 
 template <typename T, int NY, int OP>
 __device__ __forceinline__ cplx<T> yp_op_c(const YPArgs<T>& a, int q, int kx, int ky, cplx<T> F0, T kxv, T kyv) {
   const cplx<T> zero = {T(0), T(0)};
-  if constexpr (OP == YP_GRAD) {
-    if (ky == NY / 2 || kx == a.nxh) return zero;
-    if (q == 0) return F0;
-    if (q == 1) return ik_mul(kxv, F0);
-    return ik_mul(kyv, F0);
-  } else if constexpr (OP == YP_GRADY) {
+  if constexpr (OP == YP_GRADY) {
     if (ky == NY / 2 || kx == a.nxh) return zero;
     if (q == 0) return F0;
     return ik_mul(kyv, F0);
@@ -1126,8 +1114,6 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
             }
         } else if (a.op == YP_GRADY) {
           fill(std::integral_constant<int, YP_GRADY>{});
-        } else if (a.op == YP_GRAD) {
-          fill(std::integral_constant<int, YP_GRAD>{});
         } else if (a.op == YP_PGRAD) {
           fill(std::integral_constant<int, YP_PGRAD>{});
         } else {
