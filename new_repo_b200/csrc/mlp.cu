@@ -46,15 +46,8 @@ __device__ __forceinline__ float tanh_fast(float x) {
 constexpr float GELU_C0 = 0.7978845608028654f;  // sqrt(2 / pi)
 constexpr float GELU_C1 = 0.044715f;
 // x/2 (1 + t) = fma(x/2, t, x/2) with u = x (c0 + c0 c1 x^2): five FP32
-// operations and one MUFU per evaluation (the epilogues are issue bound)
-__device__ __forceinline__ float gelu(float x) {
-  const float u = x * fmaf(GELU_C0 * GELU_C1, x * x, GELU_C0);
-  const float t = tanh_fast(u);
-  const float hx = 0.5f * x;
-  return fmaf(hx, t, hx);
-}
-// the same on a pair of values with the packed FP32x2 instructions of sm_100
-// (per component the rounding of the scalar form: results are bit-identical)
+// operations and one MUFU per evaluation (the epilogues are issue bound), on
+// a pair of values with the packed FP32x2 instructions of sm_100
 __device__ __forceinline__ float2 gelu2(float2 x) {
   const float2 x2 = __fmul2_rn(x, x);
   const float2 p = __ffma2_rn(make_float2(GELU_C0 * GELU_C1, GELU_C0 * GELU_C1), x2, make_float2(GELU_C0, GELU_C0));
@@ -63,9 +56,18 @@ __device__ __forceinline__ float2 gelu2(float2 x) {
   const float2 hx = __fmul2_rn(make_float2(0.5f, 0.5f), x);
   return __ffma2_rn(hx, t, hx);
 }
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float t = tanh_fast(GELU_C0 * fmaf(GELU_C1 * x, x * x, x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_C0 * fmaf(3.0f * GELU_C1, x * x, 1.0f);
+// gelu of a pair (the same operations) and its derivative
+//   (1 + t) / 2 + x / 2 (1 - t^2) du/dx, from the one tanh
+__device__ __forceinline__ float2 gelu2_grad(float2 x, float2& d) {
+  auto all = [](float v) { return make_float2(v, v); };
+  const float2 x2 = __fmul2_rn(x, x);
+  const float2 u = __fmul2_rn(x, __ffma2_rn(all(GELU_C0 * GELU_C1), x2, all(GELU_C0)));
+  const float2 t = make_float2(tanh_fast(u.x), tanh_fast(u.y));
+  const float2 hx = __fmul2_rn(all(0.5f), x);
+  const float2 s = __ffma2_rn(make_float2(-t.x, -t.y), t, all(1.0f));
+  const float2 du = __ffma2_rn(all(3.0f * GELU_C0 * GELU_C1), x2, all(GELU_C0));
+  d = __ffma2_rn(__fmul2_rn(hx, s), du, __ffma2_rn(all(0.5f), t, all(0.5f)));
+  return __ffma2_rn(hx, t, hx);
 }
 
 __device__ __forceinline__ uint16_t bf16_bits(float x) {
@@ -420,18 +422,6 @@ __device__ __forceinline__ void put_features(S_t& S, int row, const float* x) {
   *reinterpret_cast<uint4*>(S.A1 + kmaj_off(row, 8, 256)) = c1;
 }
 
-// write 64 values as row `row` of a K-major (sbo 1024) BF16 tile
-__device__ __forceinline__ void put_row64(unsigned char* tile, int row, const float* v) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 q;
-    q.x = pack_bf16x2(v[8 * c + 0], v[8 * c + 1]);
-    q.y = pack_bf16x2(v[8 * c + 2], v[8 * c + 3]);
-    q.z = pack_bf16x2(v[8 * c + 4], v[8 * c + 5]);
-    q.w = pack_bf16x2(v[8 * c + 6], v[8 * c + 7]);
-    *reinterpret_cast<uint4*>(tile + kmaj_off(row, 8 * c, 1024)) = q;
-  }
-}
 // write 16 values as columns 16 c .. 16 c + 15 of row `row` of a K-major (sbo 1024) BF16 tile
 __device__ __forceinline__ void put16(unsigned char* tile, int row, int c, const float* v) {
 #pragma unroll
@@ -444,19 +434,6 @@ __device__ __forceinline__ void put16(unsigned char* tile, int row, int c, const
     *reinterpret_cast<uint4*>(tile + kmaj_off(row, 16 * c + 8 * h, 1024)) = q;
   }
 }
-__device__ __forceinline__ float tile_val(const unsigned char* tile, int row, int k, int sbo) {
-  const uint16_t b = *reinterpret_cast<const uint16_t*>(tile + kmaj_off(row, k, sbo));
-  return __uint_as_float(uint32_t(b) << 16);
-}
-
-// 64 TMEM columns of this thread's lane starting at column col
-__device__ __forceinline__ void tmem_row64(uint32_t tbase, int col, float* v) {
-  const uint32_t lane = uint32_t((threadIdx.x / 32) * 32) << 16;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) tc::tmem_ld16(tbase + lane + uint32_t(col + 16 * j), v + 16 * j);
-  tc::tmem_wait_ld();
-}
-
 // issue one tensor-core stage (thread 0) and wait for it (bounded);
 // returns false (and flags the status) when the wait ran out
 // stage 0: D = X . W1, 1: D = H1 . W2, 2: D = G2 . W2^T, D at TMEM column dcol
@@ -616,6 +593,14 @@ __global__ void __launch_bounds__(TILE, 6) k_mlp_infer(const MlpFeatIn<T> a, T* 
 // One launch: each CTA loops over tiles of samples [tile*128, +128) < n,
 // forward + backward.  Gradient of L = mean_i (y_i - t_i)^2 with inv_n = 1/n.
 //
+// Bound by the chain of a tile (four GEMMs and the epilogues between them; the
+// TMEM columns leave room for one CTA per SM), so two threads share a sample,
+// 32 hidden units each, one tanh serves a unit's GELU and its derivative,
+// which waits in registers for the backward pass, a tile's samples are loaded
+// during the tile before, and the weight GEMM runs into the next tile's first
+// stage: 100003 samples 79 us with one thread per sample and four tanh per
+// unit, 38 us so (200000 samples 134 and 58).
+//
 // The weight gradients are one more tensor-core GEMM per tile, accumulated
 // in TMEM over all of a CTA's tiles and added to m.grad once per CTA:
 // D[128 x 192] += AW[128 x 128] . BW[192 x 128]^T (K = the 128 samples),
@@ -624,60 +609,54 @@ __global__ void __launch_bounds__(TILE, 6) k_mlp_infer(const MlpFeatIn<T> a, T* 
 // D[k][n] = dW2, D[64 + f][64 + k] = dW1, D[72][n] = db2, D[72][64 + k] =
 // db1, D[73][128 + i] = dw3 (db3 = sum dy on the CUDA cores).  Operands are
 // BF16 (the oracle rounds the same values), accumulation FP32.  The
-// transposed tiles are built from the K-major sample-row tiles by 8 x 8
-// transposes of core matrices (16-byte loads and stores, byte permutes).
+// transposed tiles are built from the K-major sample-row tiles by transposes
+// of 8 x 8 core matrices.
 constexpr int AW_ROWS = 128, BW_ROWS = 192, W_SBO = 2048;  // K = 128 samples: 16 chunks of 128 B per row group
 constexpr uint32_t IDESC_W = tc::idesc_bf16_f32(128, 192);
 constexpr uint32_t TM_Z1 = 0, TM_Z2 = 64, TM_D1 = 128, TM_W = 256;  // TMEM columns
+constexpr int TRAIN_THREADS = 2 * TILE;
 
 struct TrainSmem {
   MlpSmem s;
   alignas(1024) unsigned char AW[AW_ROWS / 8 * W_SBO];   // 32 KB
   alignas(1024) unsigned char BW[BW_ROWS / 8 * W_SBO];   // 48 KB
   alignas(1024) unsigned char T64[TILE * 64 * 2];        // 16 KB sample-row staging (h2, delta1)
+  float ys[2][TILE];                                     // the output layer's halves
   float dsum[TILE / 32];
   uint64_t wbar;
 };
 
-// 8 x 8 transpose of 16-bit elements: in[r] = row r (8 values in a uint4),
-// out[c] = column c
-__device__ __forceinline__ void transpose8x8(const uint4* in, uint4* out) {
-  uint32_t w[8][4];
+// Core matrices (sample group sg, feature chunk fc) of a sample-row K-major
+// tile (sbo_src, NC chunks) -> core matrices (feature group row0 / 8 + fc,
+// sample chunk sg) of a transposed tile (sbo W_SBO), by warp w of NW: four 8 x
+// 8 matrices at a time by ldmatrix.trans and stmatrix, a core matrix being the
+// 128 contiguous bytes that these read and write without conflicts (16-byte
+// accesses of a matrix per thread put eight lanes on one bank).
+template <int NC, int NW>
+__device__ __forceinline__ void transpose_tile(const unsigned char* src, int sbo_src, unsigned char* dst, int row0,
+                                               int w) {
+  const int l = threadIdx.x & 31;
+  constexpr int N = TILE / 8 * NC / 4 / NW;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    w[r][0] = in[r].x;
-    w[r][1] = in[r].y;
-    w[r][2] = in[r].z;
-    w[r][3] = in[r].w;
+  for (int it = 0; it < N; ++it) {
+    const int mi = (w * N + it) * 4 + (l >> 3);
+    const int sg = mi / NC, fc = mi % NC;
+    uint32_t r0, r1, r2, r3;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(tc::smem_u32(src + sg * sbo_src + fc * 128 + 16 * (l & 7)))
+                 : "memory");
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(
+                     tc::smem_u32(dst + (row0 / 8 + fc) * W_SBO + sg * 128 + 16 * (l & 7))),
+                 "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+                 : "memory");
   }
-  uint32_t o[8][4];  // o[c][p]: column c, rows 2p and 2p + 1
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-      o[c][p] = __byte_perm(w[2 * p][c >> 1], w[2 * p + 1][c >> 1], (c & 1) ? 0x7632 : 0x5410);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) out[c] = make_uint4(o[c][0], o[c][1], o[c][2], o[c][3]);
 }
 
-// core matrix (sample group sg, feature chunk fc) of a sample-row K-major tile
-// (sbo_src) -> core matrix (feature group row0 / 8 + fc, sample chunk sg) of a
-// transposed tile (sbo W_SBO)
-__device__ __forceinline__ void transpose_block(const unsigned char* src, int sbo_src, unsigned char* dst, int row0,
-                                                int sg, int fc) {
-  uint4 in[8], out[8];
-  const unsigned char* sp = src + sg * sbo_src + fc * 128;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) in[r] = *reinterpret_cast<const uint4*>(sp + 16 * r);
-  transpose8x8(in, out);
-  unsigned char* dp = dst + (row0 / 8 + fc) * W_SBO + sg * 128;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dp + 16 * c) = out[c];
-}
-
-// the weight-gradient GEMM of one tile into TMEM columns TM_W.. (thread 0);
-// waits (bounded) so the next tile may overwrite AW / BW
-__device__ __forceinline__ bool tc_weights(TrainSmem& TS, uint32_t& wphase, unsigned* status, bool first) {
+// issue the weight-gradient GEMM of one tile into TMEM columns TM_W.. (thread
+// 0).  A wait for a later GEMM of this thread covers it: commits complete with
+// everything that the thread issued before.
+__device__ __forceinline__ void tc_weights(TrainSmem& TS, bool first) {
   MlpSmem& S = TS.s;
   if (threadIdx.x == 0) {
     tc::fence_after_sync();
@@ -687,18 +666,12 @@ __device__ __forceinline__ bool tc_weights(TrainSmem& TS, uint32_t& wphase, unsi
       tc::mma_bf16(S.tmem + TM_W, tc::smem_desc(aw + 256 * ks, 128, W_SBO), tc::smem_desc(bw + 256 * ks, 128, W_SBO),
                    IDESC_W, (!first || ks > 0) ? 1u : 0u);
     tc::mma_commit(&TS.wbar);
-    S.ok = tc::mbar_wait(&TS.wbar, wphase) ? 1 : 0;
-    if (!S.ok) atomicOr(status, 16u);
   }
-  wphase ^= 1u;
-  __syncthreads();
-  tc::fence_after_sync();
-  return S.ok != 0;
 }
 
-__global__ void __launch_bounds__(TILE) k_mlp_train(MlpDevice m, const float* X, const float* Tg, long n,
-                                                    float inv_n, float* y_out, float* loss, unsigned* status,
-                                                    MlpPerm pm) {
+__global__ void __launch_bounds__(TRAIN_THREADS) k_mlp_train(MlpDevice m, const float* X, const float* Tg, long n,
+                                                             float inv_n, float* y_out, float* loss,
+                                                             unsigned* status, MlpPerm pm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   TrainSmem& TS = *reinterpret_cast<TrainSmem*>(smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023));
   MlpSmem& S = TS.s;
@@ -708,77 +681,110 @@ __global__ void __launch_bounds__(TILE) k_mlp_train(MlpDevice m, const float* X,
     tc::mbar_init(&TS.wbar, 1);
   }
   const int tid = threadIdx.x;
+  const int row = tid & (TILE - 1), half = tid / TILE;  // sample of the tile, half of the hidden units
   // AW rows 72..127: row 72 ones, the rest zero (row 73 is rewritten per tile)
-  for (int i = tid; i < (AW_ROWS - 72) * TILE; i += TILE) {
+  for (int i = tid; i < (AW_ROWS - 72) * TILE; i += TRAIN_THREADS) {
     const int r = 72 + i / TILE, c = i % TILE;
     *reinterpret_cast<uint16_t*>(TS.AW + kmaj_off(r, c, W_SBO)) = bf16_bits(r == 72 ? 1.0f : 0.0f);
   }
   tc_setup(S, 512);  // z1, z2, delta1 (64 columns each) and the 192 weight-gradient columns
   float ab3 = 0.0f, aloss = 0.0f;
   uint32_t phase = 0, wphase = 0;
-  bool first = true, wfail = false;
+  bool first = true;
   const long ntiles = (n + TILE - 1) / TILE;
-  const int sg = tid >> 3, fc = tid & 7;  // this thread's core matrix of the 64-wide tiles
-  for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long q = tile * TILE + tid;
+  const int warp = tid >> 5;
+  const uint32_t lane = uint32_t(row / 32 * 32) << 16;  // TMEM lanes of this warp
+  // sample q: target, and in the first half the features (rows of 32 bytes)
+  float x[8], tg;
+  auto load = [&](long q) {
     const bool valid = q < n;
-    const long src = pm.n ? long((pm.a * (unsigned long long)(pm.off + q) + pm.b) % (unsigned long long)pm.n) : q;
-    float x[8];
-    for (int i = 0; i < 8; ++i) x[i] = valid ? X[src * 8 + i] : 0.0f;
-    const float tg = valid ? Tg[src] : 0.0f;
-    put_features(S, tid, x);
+    const long src = !valid ? 0 : pm.n ? long((pm.a * (unsigned long long)(pm.off + q) + pm.b) % (unsigned long long)pm.n) : q;
+    tg = valid ? Tg[src] : 0.0f;
+    if (half == 0) {
+      const float4* p = reinterpret_cast<const float4*>(X + src * 8);
+      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float4 a = valid ? p[0] : z, b = valid ? p[1] : z;
+      x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+      x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    }
+  };
+  load((long)blockIdx.x * TILE + row);
+  for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const long q = tile * TILE + row;
+    const bool valid = q < n;
+    const float t0 = tg;
+    if (half == 0) put_features(S, row, x);
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
-    if (tid < 16) transpose_block(S.A1, 256, TS.AW, 64, tid, 0);  // x^T -> AW rows 64..71
+    if (tile + gridDim.x < ntiles) load(q + (long)gridDim.x * TILE);
+    // (its wait covers the last tile's weight GEMM: AW, BW and T64 are free after it)
     if (!tc_stage(S, phase, status, 0, TM_Z1)) break;
-    // the layer outputs stay in TMEM (z1 at TM_Z1, z2 at TM_Z2) and are read
-    // back 16 columns at a time where they are needed, so that no 64-value
-    // row is live across a stage
-    const uint32_t lane = uint32_t((tid / 32) * 32) << 16;
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c) {  // h1 = gelu(z1 + b1)
+    if (warp == 0) transpose_tile<1, 1>(S.A1, 256, TS.AW, 64, 0);  // x^T -> AW rows 64..71
+    // 16 columns of a layer's output at a time; gelu' of this thread's 32
+    // units stays in registers for the backward pass
+    float2 g1[16], g2[16];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {  // h1 = gelu(z1 + b1)
+      const int c = 2 * half + k;
       float v[16];
       tc::tmem_ld16(S.tmem + lane + TM_Z1 + 16 * c, v);
       tc::tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu(v[i] + S.b1[16 * c + i]);
-      put16(S.A2, tid, c, v);
+      for (int i = 0; i < 16; i += 2) {
+        const float2 h = gelu2_grad(
+            __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(S.b1[16 * c + i], S.b1[16 * c + i + 1])),
+            g1[8 * k + i / 2]);
+        v[i] = h.x;
+        v[i + 1] = h.y;
+      }
+      put16(S.A2, row, c, v);
     }
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
-    transpose_block(S.A2, 1024, TS.AW, 0, sg, fc);  // h1^T -> AW rows 0..63 (the BF16 values layer 2 uses)
+    transpose_tile<8, 8>(S.A2, 1024, TS.AW, 0, warp);  // h1^T -> AW rows 0..63 (the BF16 values layer 2 uses)
     if (!tc_stage(S, phase, status, 1, TM_Z2)) break;
-    float y = S.b3;
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    float2 y2 = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {  // h2 = gelu(z2 + b2) and the output layer
+      const int c = 2 * half + k;
       float v[16];
       tc::tmem_ld16(S.tmem + lane + TM_Z2 + 16 * c, v);
       tc::tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) y += S.w3[16 * c + i] * gelu(v[i] + S.b2[16 * c + i]);
-    }
-    if (y_out && valid) y_out[q] = y;
-    const float dy = valid ? 2.0f * (y - tg) * inv_n : 0.0f;
-    if (valid) aloss += (y - tg) * (y - tg) * inv_n;
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c) {  // h2 and g2 = dy w3 gelu'(z2)
-      float v[16], h2[16], g2[16];
-      tc::tmem_ld16(S.tmem + lane + TM_Z2 + 16 * c, v);
-      tc::tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float z2 = v[i] + S.b2[16 * c + i];
-        h2[i] = gelu(z2);
-        g2[i] = dy * S.w3[16 * c + i] * gelu_grad(z2);
+      for (int i = 0; i < 16; i += 2) {
+        const int u = 16 * c + i;
+        const float2 h =
+            gelu2_grad(__fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(S.b2[u], S.b2[u + 1])), g2[8 * k + i / 2]);
+        y2 = __ffma2_rn(make_float2(S.w3[u], S.w3[u + 1]), h, y2);
+        v[i] = h.x;
+        v[i + 1] = h.y;
       }
-      put16(S.G2, tid, c, g2);
-      put16(TS.T64, tid, c, h2);
+      put16(TS.T64, row, c, v);
     }
-    *reinterpret_cast<uint16_t*>(TS.AW + kmaj_off(73, tid, W_SBO)) = bf16_bits(dy);
-    {  // db3: sum of dy over the tile
-      float d = dy;
+    TS.ys[half][row] = y2.x + y2.y;
+    __syncthreads();
+    const float y = S.b3 + (TS.ys[0][row] + TS.ys[1][row]);
+    const float dy = valid ? 2.0f * (y - t0) * inv_n : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {  // g2 = dy w3 gelu'(z2)
+      const int c = 2 * half + k;
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) {
+        const int u = 16 * c + i;
+        const float2 d = __fmul2_rn(__fmul2_rn(make_float2(dy, dy), make_float2(S.w3[u], S.w3[u + 1])), g2[8 * k + i / 2]);
+        v[i] = d.x;
+        v[i + 1] = d.y;
+      }
+      put16(S.G2, row, c, v);
+    }
+    if (half == 0) {
+      if (y_out && valid) y_out[q] = y;
+      if (valid) aloss += (y - t0) * (y - t0) * inv_n;
+      *reinterpret_cast<uint16_t*>(TS.AW + kmaj_off(73, row, W_SBO)) = bf16_bits(dy);
+      float d = dy;  // db3: sum of dy over the tile
       for (int off = 16; off > 0; off >>= 1) d += __shfl_down_sync(0xffffffffu, d, off);
       if ((tid & 31) == 0) TS.dsum[tid >> 5] = d;
     }
@@ -786,63 +792,74 @@ __global__ void __launch_bounds__(TILE) k_mlp_train(MlpDevice m, const float* X,
     tc::fence_before_sync();
     __syncthreads();
     if (tid == 0) ab3 += (TS.dsum[0] + TS.dsum[1]) + (TS.dsum[2] + TS.dsum[3]);
-    transpose_block(S.G2, 1024, TS.BW, 0, sg, fc);     // g2^T -> BW rows 0..63
-    transpose_block(TS.T64, 1024, TS.BW, 128, sg, fc); // h2^T -> BW rows 128..191
+    transpose_tile<8, 8>(S.G2, 1024, TS.BW, 0, warp);      // g2^T -> BW rows 0..63
+    transpose_tile<8, 8>(TS.T64, 1024, TS.BW, 128, warp);  // h2^T -> BW rows 128..191
     if (!tc_stage(S, phase, status, 2, TM_D1)) break;
     // delta1 = (g2 . W2^T) * gelu'(z1); h2's transpose finished before the
     // stage's barrier, so T64 is free
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      float d1[16], z1[16];
-      tc::tmem_ld16(S.tmem + lane + TM_D1 + 16 * c, d1);
-      tc::tmem_ld16(S.tmem + lane + TM_Z1 + 16 * c, z1);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = 2 * half + k;
+      float v[16];
+      tc::tmem_ld16(S.tmem + lane + TM_D1 + 16 * c, v);
       tc::tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) d1[i] *= gelu_grad(z1[i] + S.b1[16 * c + i]);
-      put16(TS.T64, tid, c, d1);
+      for (int i = 0; i < 16; i += 2) {
+        const float2 d = __fmul2_rn(make_float2(v[i], v[i + 1]), g1[8 * k + i / 2]);
+        v[i] = d.x;
+        v[i + 1] = d.y;
+      }
+      put16(TS.T64, row, c, v);
     }
     __syncthreads();
-    transpose_block(TS.T64, 1024, TS.BW, 64, sg, fc);  // delta1^T -> BW rows 64..127
+    transpose_tile<8, 8>(TS.T64, 1024, TS.BW, 64, warp);  // delta1^T -> BW rows 64..127
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
-    if (!tc_weights(TS, wphase, status, first)) {
-      wfail = true;
-      break;
-    }
+    tc_weights(TS, first);
     first = false;
+    wphase ^= 1u;
   }
+  // the last weight GEMM (also before the TMEM is freed after a failed stage)
+  if (tid == 0 && !first && !tc::mbar_wait(&TS.wbar, wphase ^ 1u)) {
+    S.ok = 0;
+    atomicOr(status, 16u);
+  }
+  __syncthreads();
+  tc::fence_after_sync();
   // the weight gradients: thread r reads TMEM lane r (D row r); every warp
-  // runs the same loads (tcgen05.ld is warp-collective)
+  // of a half runs the same loads (tcgen05.ld is warp-collective)
   // This CTA's gradient goes to its own row of m.gpart (every entry written
   // by one thread; zeros when the CTA had no tile), summed over the CTAs in
   // a fixed order by k_mlp_grad_reduce.
   float* gp = m.gpart + (size_t)blockIdx.x * MLP_NP;
   const bool have = !first && S.ok;
-  {
-    float v[64];
-    if (have) tmem_row64(S.tmem, TM_W, v);
-    if (tid < 64)
-      for (int i = 0; i < 64; ++i) gp[MLP_O_W2 + tid * MLP_H + i] = have ? v[i] : 0.0f;  // dW2[tid][.]
-    else if (tid == 72)
-      for (int i = 0; i < 64; ++i) gp[MLP_O_B2 + i] = have ? v[i] : 0.0f;
-    if (have) tmem_row64(S.tmem, TM_W + 64, v);
-    if (tid >= 64 && tid < 72)
-      for (int i = 0; i < 64; ++i) gp[MLP_O_W1 + (tid - 64) * MLP_H + i] = have ? v[i] : 0.0f;  // dW1
-    else if (tid == 72)
-      for (int i = 0; i < 64; ++i) gp[MLP_O_B1 + i] = have ? v[i] : 0.0f;
-    if (have) tmem_row64(S.tmem, TM_W + 128, v);
-    if (tid == 73)
-      for (int i = 0; i < 64; ++i) gp[MLP_O_W3 + i] = have ? v[i] : 0.0f;
+  float v[64];
+  auto row64 = [&](uint32_t col) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tc::tmem_ld16(S.tmem + lane + col + 16 * j, v + 16 * j);
+    tc::tmem_wait_ld();
+  };
+  auto put = [&](int at) {
+#pragma unroll
+    for (int i = 0; i < 64; ++i) gp[at + i] = have ? v[i] : 0.0f;
+  };
+  if (half == 0) {
+    if (have) row64(TM_W);
+    if (row < 64) put(MLP_O_W2 + row * MLP_H);  // dW2[row][.]
+    else if (row == 72) put(MLP_O_B2);
+  } else {
+    if (have) row64(TM_W + 64);
+    if (row >= 64 && row < 72) put(MLP_O_W1 + (row - 64) * MLP_H);  // dW1
+    else if (row == 72) put(MLP_O_B1);
+    if (have) row64(TM_W + 128);
+    if (row == 73) put(MLP_O_W3);
   }
-  // a weight GEMM whose wait ran out may still be in flight: wait (bounded)
-  // for it before the TMEM is freed
-  if (tid == 0 && !S.ok && wfail) tc::mbar_wait(&TS.wbar, wphase ^ 1u);
   tc_teardown(S, 512, phase);
   if (tid == 0) gp[MLP_O_B3] = ab3;
   for (int off = 16; off > 0; off >>= 1) aloss += __shfl_down_sync(0xffffffffu, aloss, off);
   __syncthreads();  // the last tile's reads of dsum (ab3) are done: reuse it for the warps' losses
-  if ((tid & 31) == 0) TS.dsum[tid >> 5] = aloss;
+  if (half == 0 && (tid & 31) == 0) TS.dsum[tid >> 5] = aloss;
   __syncthreads();
   if (tid == 0) {
     float l = 0.0f;
@@ -851,18 +868,32 @@ __global__ void __launch_bounds__(TILE) k_mlp_train(MlpDevice m, const float* X,
   }
 }
 
-// m.grad = the sum of the CTAs' gradient rows, CTA by CTA in index order;
-// *loss (when given) the same sum of their losses
-__global__ void k_mlp_grad_reduce(MlpDevice m, int nctas, float* loss) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < MLP_NP; i += gridDim.x * blockDim.x) {
-    float g = 0.0f;
-    for (int b = 0; b < nctas; ++b) g += m.gpart[(size_t)b * MLP_NP + i];
+// m.grad = the sum of the CTAs' gradient rows in a fixed order: eight threads
+// per entry, each the rows of a run of CTAs, then the runs in order (one thread
+// per entry left the 148 rows' loads in a chain on 19 blocks: 15 us, so 8.5);
+// *loss (when given) the sum of their losses by one warp
+__global__ void __launch_bounds__(256) k_mlp_grad_reduce(MlpDevice m, int nctas, float* loss) {
+  __shared__ float part[8][32];
+  const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + c, per = (nctas + 7) / 8;
+  float g = 0.0f;
+  if (i < MLP_NP) {
+    const int end = min(nctas, (r + 1) * per);
+#pragma unroll 8
+    for (int b = r * per; b < end; ++b) g += m.gpart[(size_t)b * MLP_NP + i];
+  }
+  part[r][c] = g;
+  __syncthreads();
+  if (r == 0 && i < MLP_NP) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) g += part[q][c];
     m.grad[i] = g;
   }
-  if (loss && blockIdx.x == 0 && threadIdx.x == 0) {
+  if (loss && blockIdx.x == 0 && r == 1) {
     float l = 0.0f;
-    for (int b = 0; b < nctas; ++b) l += m.lpart[b];
-    *loss = l;
+    for (int b = c; b < nctas; b += 32) l += m.lpart[b];
+    for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
+    if (c == 0) *loss = l;
   }
 }
 
@@ -987,11 +1018,11 @@ void mlp_grad(MlpDevice& m, const float* x, const float* t, long n, float* y_out
   const long ntiles = (n + TILE - 1) / TILE;
   const int grid = int(std::max<long>(1, std::min<long>(ntiles, (long)MLP_TRAIN_CTAS)));
   hook_before("k_mlp_train", double(n) * 36.0);
-  k_mlp_train<<<grid, TILE, train_smem(), st>>>(m, x, t, n, 1.0f / float(n), y_out, loss_dev, status, perm);
+  k_mlp_train<<<grid, TRAIN_THREADS, train_smem(), st>>>(m, x, t, n, 1.0f / float(n), y_out, loss_dev, status, perm);
   LES_CHECK_LAUNCH();
   hook_after();
   hook_before("k_mlp_grad_reduce", double(grid + 1) * MLP_NP * 4.0);
-  k_mlp_grad_reduce<<<19, 256, 0, st>>>(m, grid, loss_dev);
+  k_mlp_grad_reduce<<<(MLP_NP + 31) / 32, 256, 0, st>>>(m, grid, loss_dev);
   LES_CHECK_LAUNCH();
   hook_after();
 }
