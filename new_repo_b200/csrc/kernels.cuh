@@ -10,6 +10,7 @@ namespace les {
 template <typename T>
 __global__ void k_set_bc(T* u, T* v, T* w, const T* lu, const T* lv, const T* lw, const T* tu, const T* tv,
                          const T* tw, int4 lt, int4 ut, long plane, int nz, T dz) {
+  dep_wait();
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
     const long b0 = p, b1 = plane + p, t0 = (long)nz * plane + p, t1 = (long)(nz + 1) * plane + p;
     if (lt.x == 1) u[b0] = T(2) * lu[p] - u[b1];
@@ -80,6 +81,7 @@ __device__ __forceinline__ T ghost_hi(int t, T x, T b, T dz, T old) {
 template <typename T>
 __global__ void __launch_bounds__(256) k_bc_ddz(const BcArgs<T> a, T* dudz, T* dvdz, T* dwdz, T rdz, T* ul, T* vl,
                                                 T* wl, int nacc) {
+  dep_wait();
   const long plane = a.plane, n4 = (long)(a.nz + 1) * plane / 4;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
     const long o = plane + 4 * q;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(256) k_bc_ddz(const BcArgs<T> a, T* dudz, T* d
 
 template <typename T>
 __global__ void k_ddz(T* out, const T* f, long plane, int nz, T rdz, int w_to_uvp) {
+  dep_wait();
   const long n = (long)(nz + 1) * plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = plane + q;
@@ -176,6 +179,7 @@ __global__ void k_ddz(T* out, const T* f, long plane, int nz, T rdz, int w_to_uv
 
 template <typename T>
 __global__ void k_fill(T* f, long n, T val) {
+  dep_wait();
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) f[q] = val;
 }
 
@@ -189,6 +193,7 @@ struct PlaneOps {
 };
 template <typename T>
 __global__ void k_plane_ops(const PlaneOps<T> ops, long n) {
+  dep_wait();
   const int op = blockIdx.y;
   T* d = ops.dst[op];
   const T* s = ops.src[op];
@@ -208,6 +213,7 @@ struct RhsGhosts {
 };
 template <typename T>
 __global__ void k_rhs_ghosts(const RhsGhosts<T> a, long plane) {
+  dep_wait();
   const int q = blockIdx.y >> 1;
   const long o = (blockIdx.y & 1) ? a.top : 0;
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
@@ -218,11 +224,13 @@ __global__ void k_rhs_ghosts(const RhsGhosts<T> a, long plane) {
 
 template <typename T>
 __global__ void k_scale(T* f, long n, T c) {
+  dep_wait();
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) f[q] = c * f[q];
 }
 
 template <typename D, typename S>
 __global__ void k_convert(D* dst, const S* src, long n) {
+  dep_wait();
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x)
     dst[q] = D(src[q]);
 }
@@ -235,6 +243,7 @@ struct Convert3 {
 };
 template <typename D, typename S>
 __global__ void k_convert3(const Convert3<D, S> a, long n) {
+  dep_wait();
   D* __restrict__ d = a.dst[blockIdx.y];
   const S* __restrict__ s = a.src[blockIdx.y];
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) d[q] = D(s[q]);
@@ -242,6 +251,7 @@ __global__ void k_convert3(const Convert3<D, S> a, long n) {
 
 template <typename T>
 __global__ void k_copy(T* dst, const T* src, long n) {
+  dep_wait();
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) dst[q] = src[q];
 }
 
@@ -340,6 +350,7 @@ __device__ __forceinline__ void stv(T* p, const T* v) {
 // FP64.
 template <typename T, int V>
 __global__ void __launch_bounds__(256) k_sgs_tau(const SgsArgs<T> a, int zc) {
+  dep_wait();
   const long pl = a.plane;
   const long p = V * (blockIdx.x * (long)blockDim.x + threadIdx.x);
   if (p >= pl) return;
@@ -488,6 +499,7 @@ __global__ void __launch_bounds__(256) k_sgs_tau(const SgsArgs<T> a, int zc) {
 // S_ij and |S| on levels 1..nz+1 (written for the dynamic procedure).
 template <typename T>
 __global__ void k_sij(const SgsArgs<T> a) {
+  dep_wait();
   const long n = (long)(a.nz + 1) * a.plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = a.plane + q;
@@ -504,6 +516,7 @@ __global__ void k_sij(const SgsArgs<T> a) {
 // Lagrangian scale-dependent dynamic model (compute_LagScaleDep.f90)
 template <typename T>
 __global__ void k_lag_accum(T* ul, T* vl, T* wl, const T* u, const T* v, const T* w, long n) {
+  dep_wait();
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     ul[q] = ul[q] + u[q];
     vl[q] = vl[q] + v[q];
@@ -546,6 +559,7 @@ __device__ __forceinline__ long ff_off(int i, int j, int k, const LagGeom& g) {
 template <typename T>
 __global__ void k_lag_interp(const T* ul, const T* vl, const T* wl, const T* F0, const T* F1, const T* F2,
                              const T* F3, T* N0, T* N1, T* N2, T* N3, LagGeom g) {
+  dep_wait();
   // grid: (plane / blockDim.x, nlev); one point per thread, level
   // blockIdx.y + 1, and one 32-bit division for the (i, j) of the point
   const long pl = g.plane;
@@ -622,6 +636,7 @@ template <typename T>
 __global__ void k_lasd_update(T* FLM, T* FMM, T* FQN, T* FNN, const T* LM, const T* MM, const T* QN, const T* NN,
                               T* cs, T* beta, int init, long plane, int nz, double opftdelta, double lagran_dt,
                               double beta_pow, const T* cs_init = nullptr, int nlev = -1, double cs_max = 0.0) {
+  dep_wait();
   const long n = (long)(nlev < 0 ? nz + 1 : nlev) * plane;  // levels 1..nlev
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = plane + q;
@@ -685,6 +700,7 @@ __global__ void k_lasd_update(T* FLM, T* FMM, T* FQN, T* FNN, const T* LM, const
 template <typename T>
 __global__ void k_ab2(T* u, T* v, T* w, const T* rx, const T* ry, const T* rz, const T* fx, const T* fy,
                       const T* fz, long plane, int nz, T dt, T t1, T t2) {
+  dep_wait();
   const long n = (long)(nz + 2) * plane;
   if (plane % 4 == 0) {  // four consecutive points (one level) per thread
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n / 4; q += (long)gridDim.x * blockDim.x) {
@@ -733,6 +749,7 @@ __global__ void k_ab2(T* u, T* v, T* w, const T* rx, const T* ry, const T* rz, c
 template <typename T>
 __global__ void k_projection(T* u, T* v, T* w, T* rx, T* ry, T* rz, const T* dpdx, const T* dpdy, const T* dpdz,
                              long plane, int nz, double dtt_d) {
+  dep_wait();
   const long n = (long)(nz + 2) * plane;
   const T dtt = T(dtt_d);
   if (plane % 4 == 0) {  // four consecutive points (one level) per thread
@@ -792,6 +809,7 @@ __global__ void k_projection(T* u, T* v, T* w, T* rx, T* ry, T* rz, const T* dpd
 // p = fluctuation + FP64 mean profile (mixed precision only), p(nz+1) = BOGUS
 template <typename T>
 __global__ void k_p_finish(T* p, const double* pmean, long plane, int nz) {
+  dep_wait();
   const long top = (long)(nz + 1) * plane;
   const long t0 = blockIdx.x * (long)blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
   for (long q = t0; q < plane; q += ts) p[top + q] = T(BOGUS);
@@ -856,6 +874,7 @@ template <typename O>
 __global__ void __launch_bounds__(128) k_tridiag(double* r, const double* __restrict__ piv, O* __restrict__ phat,
                                                  double* pmean, unsigned* status, int lhx, int ny, int nz, double dz,
                                                  int drop_mean, int opitch) {
+  dep_wait();
   const long sp = (long)ny * lhx;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= 2 * sp) return;
@@ -1250,6 +1269,7 @@ __device__ __forceinline__ void diag_add4(DiagAcc& a, int& nan, const T* U, cons
 template <typename T>
 __global__ void __launch_bounds__(256) k_diag(const T* u, const T* v, const T* w, const T* dudx, const T* dvdy,
                                               const T* dwdz, const T* ustar, int nz, const DiagOut d) {
+  dep_wait();
   DiagAcc a;
   const long plane = d.plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < plane; q += (long)gridDim.x * blockDim.x)
@@ -1294,6 +1314,7 @@ __global__ void __launch_bounds__(256) k_step_finish(const BcArgs<T> a, const T*
                                                      const T* dpdx, const T* dpdy, T* dpdz, T* rx, T* ry, T* rz,
                                                      T rdz, double dtt_d, const T* dudx, const T* dvdy,
                                                      const T* dwdz, const T* ustar, const DiagOut dg) {
+  dep_wait();
   const long plane = a.plane;
   const int nz = a.nz;
   const T dtt = T(dtt_d);
@@ -1435,6 +1456,7 @@ struct PlaneSumIn {
 template <typename T>
 __global__ void __launch_bounds__(256) k_plane_sums(const PlaneSumIn<T> in, double* part, long plane, int k0,
                                                     long chunk) {
+  dep_wait();
   const int k = k0 + blockIdx.y;
   const T* x = in.f[blockIdx.z] + (long)k * plane;
   const long q0 = blockIdx.x * chunk, q1 = min(plane, q0 + chunk);
@@ -1488,6 +1510,7 @@ __device__ __forceinline__ double plane_sum_of(const double* part, int f, int i,
 }
 // plane means out[f L + k], k = k0 .. k0 + nlev - 1
 __global__ void k_sums_mean(const double* part, double* out, int nf, int nlev, int nch, long plane, int k0, int L) {
+  dep_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < nf * nlev) out[(q / nlev) * L + k0 + q % nlev] = plane_sum_of(part, q / nlev, q % nlev, nlev, nch) / double(plane);
 }
@@ -1501,6 +1524,7 @@ __device__ __forceinline__ double level_ratio(const double* part, int i, int nle
 // max(0, <KX> / <XX>) * scale, the reduction of compute_DynSmag.f90:61-245
 // written to a per-level array.
 __global__ void k_sums_ratio(const double* part, double* kapd, int nlev, int nch, long plane, double scale) {
+  dep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nlev) kapd[1 + i] = level_ratio(part, i, nlev, nch, plane) * scale;
 }
@@ -1508,6 +1532,7 @@ __global__ void k_sums_ratio(const double* part, double* kapd, int nlev, int nch
 // Smagorinsky): grid (blocks per level, nlev)
 template <typename T>
 __global__ void k_sums_spread(const double* part, T* cs, int nlev, int nch, long plane, double cs_max) {
+  dep_wait();
   __shared__ double res;
   if (threadIdx.x == 0) {
     res = level_ratio(part, blockIdx.y, nlev, nch, plane);
@@ -1523,6 +1548,7 @@ __global__ void k_sums_spread(const double* part, T* cs, int nlev, int nch, long
 // flux, -qs / (kappa u* dz/2), zero where u* = 0.
 template <typename T>
 __global__ void k_scalar_wall(T* dtdz1, const T* ustar, long plane, double qs, double half_dz) {
+  dep_wait();
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
     const double us = double(ustar[p]);
     dtdz1[p] = (us != 0.0) ? T(-qs / (KVONK * us * half_dz)) : T(0);
@@ -1533,6 +1559,7 @@ __global__ void k_scalar_wall(T* dtdz1, const T* ustar, long plane, double qs, d
 // on levels 1..nz (the ghost values follow with k_scalar_bc)
 template <typename T>
 __global__ void k_ab2_scalar(T* th, const T* r, const T* rf, long plane, int nz, T dt, T t1, T t2) {
+  dep_wait();
   const long n = (long)nz * plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = plane + q;
@@ -1544,6 +1571,7 @@ __global__ void k_ab2_scalar(T* th, const T* r, const T* rf, long plane, int nz,
 // theta(0) = 0, theta(nz+1) = theta(nz) + g_top dz.
 template <typename T>
 __global__ void k_scalar_bc(T* th, long plane, int nz, T gdz) {
+  dep_wait();
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
     th[p] = T(0);
     th[(long)(nz + 1) * plane + p] = th[(long)nz * plane + p] + gdz;
@@ -1556,6 +1584,7 @@ __global__ void k_scalar_bc(T* th, long plane, int nz, T gdz) {
 template <typename T>
 __global__ void k_forcing(T* rx, T* ry, T* rz, const T* u, const T* v, const T* w, const double* mean,
                           const double* sp, long plane, int nz, int L, T f, T ug, T vg) {
+  dep_wait();
   const long n = (long)nz * plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = plane + q;
@@ -1581,6 +1610,7 @@ __global__ void k_forcing(T* rx, T* ry, T* rz, const T* u, const T* v, const T* 
 // theta_w(k) = (theta(k) + theta(k-1)) / 2; tmean = plane means of theta.
 template <typename T>
 __global__ void k_buoyancy(T* rz, const T* th, const double* tmean, long plane, int nz, T beta) {
+  dep_wait();
   const long n = (long)(nz - 1) * plane;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const long o = 2 * plane + q;

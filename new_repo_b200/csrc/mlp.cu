@@ -347,6 +347,7 @@ __global__ void k_mlp_normalize(float* x, float* t, long n, const float* stats) 
 
 // ---------------------------------------------------------- packing ----
 __global__ void k_mlp_pack(const float* p, uint16_t* img) {
+  dep_wait();
   unsigned char* base = reinterpret_cast<unsigned char*>(img);
   for (int i = threadIdx.x; i < 64 * 16; i += blockDim.x) {  // B1[n][k] = W1[k][n], k < 8
     const int n = i / 16, k = i % 16;
@@ -498,6 +499,7 @@ __device__ __forceinline__ void tc_teardown(S_t& S, uint32_t ncols, uint32_t pha
 // neutral variant is compiled without it (fewer registers, one more CTA per SM)
 template <typename T, bool RI>
 __global__ void __launch_bounds__(TILE, 6) k_mlp_infer(const MlpFeatIn<T> a, T* cs, MlpDevice m, unsigned* status) {
+  dep_wait();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   InferSmem& S = *reinterpret_cast<InferSmem*>(smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023));
   load_images(S, m.img, m.params, m.stats);
@@ -675,7 +677,6 @@ __global__ void __launch_bounds__(TRAIN_THREADS) k_mlp_train(MlpDevice m, const 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   TrainSmem& TS = *reinterpret_cast<TrainSmem*>(smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023));
   MlpSmem& S = TS.s;
-  load_images(S, m.img, m.params, m.stats);
   if (threadIdx.x == 0) {
     S.ok = 1;
     tc::mbar_init(&TS.wbar, 1);
@@ -687,6 +688,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS) k_mlp_train(MlpDevice m, const 
     const int r = 72 + i / TILE, c = i % TILE;
     *reinterpret_cast<uint16_t*>(TS.AW + kmaj_off(r, c, W_SBO)) = bf16_bits(r == 72 ? 1.0f : 0.0f);
   }
+  dep_wait();
+  load_images(S, m.img, m.params, m.stats);
   tc_setup(S, 512);  // z1, z2, delta1 (64 columns each) and the 192 weight-gradient columns
   float ab3 = 0.0f, aloss = 0.0f;
   uint32_t phase = 0, wphase = 0;
@@ -873,6 +876,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS) k_mlp_train(MlpDevice m, const 
 // per entry left the 148 rows' loads in a chain on 19 blocks: 15 us, so 8.5);
 // *loss (when given) the sum of their losses by one warp
 __global__ void __launch_bounds__(256) k_mlp_grad_reduce(MlpDevice m, int nctas, float* loss) {
+  dep_wait();
   __shared__ float part[8][32];
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + c, per = (nctas + 7) / 8;
@@ -898,6 +902,7 @@ __global__ void __launch_bounds__(256) k_mlp_grad_reduce(MlpDevice m, int nctas,
 }
 
 __global__ void k_mlp_adam(float* p, const float* g, float* mm, float* vv, int step, float lr) {
+  dep_wait();
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.0f - powf(b1, float(step)), c2 = 1.0f - powf(b2, float(step));
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < MLP_NP; i += gridDim.x * blockDim.x) {
@@ -910,6 +915,7 @@ __global__ void k_mlp_adam(float* p, const float* g, float* mm, float* vv, int s
 
 // out[0]: flagged columns; out[1 + i]: columns where feature i left the range
 __global__ void k_mlp_count_flags(const int* flag, long plane, int* out) {
+  dep_wait();
   int c[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < plane; q += (long)gridDim.x * blockDim.x) {
     const int f = flag[q];
@@ -928,6 +934,7 @@ __global__ void k_mlp_count_flags(const int* flag, long plane, int* out) {
 // blockIdx.y = level - 1; err2[k] accumulates the squared log differences of level k
 template <typename T>
 __global__ void k_mlp_blend(T* cs, const T* cs_dyn, const int* flag, long plane, double* err2, int check) {
+  dep_wait();
   const int k = 1 + blockIdx.y;
   double e = 0.0;
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
@@ -982,8 +989,8 @@ void mlp_infer(const MlpFeatIn<T>& in, T* cs, MlpDevice& m, unsigned* status, cu
   const long ntiles = (n + TILE - 1) / TILE;
   const int grid = int(std::min<long>(ntiles, 148L * 6));  // 6 CTAs per SM fit (79 registers, 32 KB, 64 TMEM columns each)
   hook_before("k_mlp_infer", double(n) * 11 * sizeof(T));
-  if (in.dtdz) k_mlp_infer<T, true><<<grid, TILE, infer_smem(), st>>>(in, cs, m, status);
-  else k_mlp_infer<T, false><<<grid, TILE, infer_smem(), st>>>(in, cs, m, status);
+  if (in.dtdz) launch_dep(k_mlp_infer<T, true>, grid, TILE, infer_smem(), st, in, cs, m, status);
+  else launch_dep(k_mlp_infer<T, false>, grid, TILE, infer_smem(), st, in, cs, m, status);
   LES_CHECK_LAUNCH();
   hook_after();
 }
@@ -1008,7 +1015,7 @@ void mlp_reset_range(MlpDevice& m, cudaStream_t st) {
 
 void mlp_pack(MlpDevice& m, cudaStream_t st) {
   hook_before("k_mlp_pack", double(MLP_NP) * 4 + IMG_BYTES);
-  k_mlp_pack<<<1, 256, 0, st>>>(m.params, m.img);
+  launch_dep(k_mlp_pack, 1, 256, 0, st, m.params, m.img);
   LES_CHECK_LAUNCH();
   hook_after();
 }
@@ -1018,18 +1025,18 @@ void mlp_grad(MlpDevice& m, const float* x, const float* t, long n, float* y_out
   const long ntiles = (n + TILE - 1) / TILE;
   const int grid = int(std::max<long>(1, std::min<long>(ntiles, (long)MLP_TRAIN_CTAS)));
   hook_before("k_mlp_train", double(n) * 36.0);
-  k_mlp_train<<<grid, TRAIN_THREADS, train_smem(), st>>>(m, x, t, n, 1.0f / float(n), y_out, loss_dev, status, perm);
+  launch_dep(k_mlp_train, grid, TRAIN_THREADS, train_smem(), st, m, x, t, n, 1.0f / float(n), y_out, loss_dev, status, perm);
   LES_CHECK_LAUNCH();
   hook_after();
   hook_before("k_mlp_grad_reduce", double(grid + 1) * MLP_NP * 4.0);
-  k_mlp_grad_reduce<<<(MLP_NP + 31) / 32, 256, 0, st>>>(m, grid, loss_dev);
+  launch_dep(k_mlp_grad_reduce, (MLP_NP + 31) / 32, 256, 0, st, m, grid, loss_dev);
   LES_CHECK_LAUNCH();
   hook_after();
 }
 
 void mlp_adam(MlpDevice& m, int step, float lr, cudaStream_t st) {
   hook_before("k_mlp_adam", double(MLP_NP) * 20);
-  k_mlp_adam<<<19, 256, 0, st>>>(m.params, m.grad, m.adam_m, m.adam_v, step, lr);
+  launch_dep(k_mlp_adam, 19, 256, 0, st, m.params, m.grad, m.adam_m, m.adam_v, step, lr);
   LES_CHECK_LAUNCH();
   hook_after();
   mlp_pack(m, st);
@@ -1106,7 +1113,7 @@ void mlp_fit_stats(MlpDevice& m, cudaStream_t st) {
 int mlp_count_flags(MlpDevice& m, int* dcount, int* per_feature, cudaStream_t st) {
   LES_CUDA(cudaMemsetAsync(dcount, 0, 9 * sizeof(int), st));
   hook_before("k_mlp_count_flags", double(m.plane) * 4);
-  k_mlp_count_flags<<<148, 256, 0, st>>>(m.colflag, m.plane, dcount);
+  launch_dep(k_mlp_count_flags, 148, 256, 0, st, m.colflag, m.plane, dcount);
   LES_CHECK_LAUNCH();
   hook_after();
   int h[9];
@@ -1124,7 +1131,7 @@ void mlp_blend(T* cs, const T* cs_dyn, MlpDevice& m, int nz, bool check, double*
   LES_CUDA(cudaMemsetAsync(derr, 0, sizeof(double) * NB * (nz + 2), st));
   const long n = (long)(nz + 1) * m.plane;
   hook_before("k_mlp_blend", double(n) * 3 * sizeof(T));
-  k_mlp_blend<T><<<dim3(NB, nz + 1), 256, 0, st>>>(cs, cs_dyn, m.colflag, m.plane, derr, check ? 1 : 0);
+  launch_dep(k_mlp_blend<T>, dim3(NB, nz + 1), 256, 0, st, cs, cs_dyn, m.colflag, m.plane, derr, check ? 1 : 0);
   LES_CHECK_LAUNCH();
   hook_after();
   if (check) {

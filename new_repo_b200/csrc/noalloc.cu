@@ -71,6 +71,7 @@ ScratchLayout scratch_layout(int nx, int ny, int nlev) {
 // and the exp(-2 pi i m / n) twiddle tables, computed on the device
 __global__ void k_noalloc_tables(double* kkx, double* kky, cplx<double>* twx, cplx<double>* twy, int nx, int ny,
                                  double lx, double ly) {
+  dep_wait();
   const int lhx = nx / 2 + 1, lhy = ny / 2 + 1;
   const double pi = 3.14159265358979323846;
   const long n = (long)ny * lhx;
@@ -106,7 +107,8 @@ __global__ void k_noalloc_tables(double* kkx, double* kky, cplx<double>* twx, cp
 // and latency, which the four launches of the three-pass form pay four times,
 // larger ones by shared memory, ~25 accesses per value.  Three passes against
 // this, us: 16 x 16 x 100 26.6 / 6.2, 64 x 64 x 148 41 / 12.3, 96 x 64 x 100 41
-// / 16.4, 128 x 64 x 159 (two waves) 61 / 34, 128 x 128 x 79 54 / 37.
+// / 16.4, 128 x 64 x 159 (two waves) 61 / 34, 128 x 128 x 79 54 / 37; with
+// dependent launches 4.2, 10.3, 13.8, 31.8 and 49 / 34.4.
 template <int NX, int NY>
 struct PlaneGrad {
   static constexpr int M = NX / 2;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
       tc::fence_mbar_init();
       mbar_expect_tx(bar, unsigned(NY * NX * sizeof(double)));
     }
+    dep_wait();
     __syncwarp();
     for (int r = tid; r < NY; r += 32) bulk_g2s(A + r * RS, f + plane + (long)r * NX, unsigned(NX * sizeof(double)), bar);
   }
@@ -180,6 +183,7 @@ __global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
   twm_build<double, M, true, 2>(twx, mxi, tid, TH);
   twm_build<double, NY, false>(twy, myf, tid, TH);
   twm_build<double, NY, true>(twy, myi, tid, TH);
+  dep_wait();
   const bool late = !tc::mbar_wait(bar, 0);
   if (__syncthreads_or(late)) {  // as in the spectral passes: a last bounded wait, leave
     tc::mbar_wait(bar, 0);
@@ -362,8 +366,9 @@ PlaneKernel plane_kernel(int nx, int ny) {
 
 // Whether a call of nlev levels takes the plane form: always where two arrays
 // fit.  The largest planes take one CTA as long as few levels take the whole
-// chip in three passes: 128 x 128 x 4 35.9 / 31.9 us, x 32 36.9 / 38.1.
-bool plane_form(const PlaneKernel& k, int nlev) { return k.run && (k.two || nlev >= 24); }
+// chip in three passes, us: 128 x 128 x 24 34.2 / 28.7, x 40 34.3 / 32.8, x 50
+// 34.3 / 36.9; 256 x 64 x 24 28.8 / 28.7, x 40 28.9 / 32.8.
+bool plane_form(const PlaneKernel& k, int nlev) { return k.run && (k.two || nlev >= 40); }
 
 // address of this device's scratch buffer; the first call on a device does
 // the setup (symbol address, kernel shared-memory attributes)
@@ -440,7 +445,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (const PlaneKernel pk = plane_kernel(nx, ny); plane_form(pk, nlev)) {
       auto* ys = reinterpret_cast<cplx<double>*>(base + L.spec[0]);
-      pk.run<<<nlev, pk.threads, pk.smem, st>>>(f, dfdx, dfdy, ys, lx, ly);
+      launch_dep(pk.run, nlev, pk.threads, pk.smem, st, f, dfdx, dfdy, ys, lx, ly);
       LES_CHECK_LAUNCH();
       g_hook = saved;
       return rc;
@@ -452,7 +457,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     cplx<double>* sp[2];
     for (int i = 0; i < 2; ++i) sp[i] = reinterpret_cast<cplx<double>*>(base + L.spec[i]);
     const int lhx = nx / 2 + 1;
-    k_noalloc_tables<<<64, 256, 0, st>>>(kkx, kky, twx, twy, nx, ny, lx, ly);
+    launch_dep(k_noalloc_tables, 64, 256, 0, st, kkx, kky, twx, twy, nx, ny, lx, ly);
     LES_CHECK_LAUNCH();
 
     XFArgs<double> a;
@@ -473,6 +478,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
 
     YPArgs<double> b;
     std::memset(&b, 0, sizeof(b));
+    b.dep = 1;  // (the x pass above has waited for the tables)
     b.op = YP_GRADY;  // F and i ky F; the x inverse forms i kx F from the staged F row
     b.nin = 1;
     b.nout = 2;
@@ -494,6 +500,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
 
     XIArgs<double> c;
     std::memset(&c, 0, sizeof(c));
+    c.dep = 1;
     c.op = XI_STORE;
     c.nin = 3;
     c.rows_pp = ny;

@@ -287,7 +287,7 @@ class Solver final : public SolverBase {
   T* lev(T* f, int k) const { return f + (long)k * g.plane(); }
   void fill(T* f, int k0, int k1, T v) {
     const long n = (long)(k1 - k0 + 1) * g.plane();
-    KL("k_fill", double(n) * sizeof(T), k_fill<T><<<grid_for(n), 256, 0, st>>>(lev(f, k0), n, v));
+    KL("k_fill", double(n) * sizeof(T), launch_dep(k_fill<T>, grid_for(n), 256, 0, st, lev(f, k0), n, v));
   }
   // plane-sized copies / fills batched into one launch (src null: fill)
   void plane_ops(int nops, T* const* dst, const T* const* src, const T* val) {
@@ -302,7 +302,7 @@ class Solver final : public SolverBase {
     double bytes = 0.0;
     for (int i = 0; i < nops; ++i) bytes += (o.src[i] ? 2.0 : 1.0) * n * sizeof(T);
     dim3 grid(unsigned(std::min<long>(ceil_div(n, 256L), 148)), unsigned(nops));
-    KL("k_plane_ops", bytes, k_plane_ops<T><<<grid, 256, 0, st>>>(o, n));
+    KL("k_plane_ops", bytes, launch_dep(k_plane_ops<T>, grid, 256, 0, st, o, n));
   }
   // the first nlev levels of up to eight fields in one launch
   void fill_planes(int nf, T* const* dst, int nlev, T v) {
@@ -314,13 +314,13 @@ class Solver final : public SolverBase {
     }
     const long n = (long)nlev * g.plane();
     KL("k_plane_ops", double(nf) * n * sizeof(T),
-       k_plane_ops<T><<<dim3(unsigned(std::min<long>(ceil_div(n, 256L), 148 * 8)), unsigned(nf)), 256, 0, st>>>(o, n));
+       launch_dep(k_plane_ops<T>, dim3(unsigned(std::min<long>(ceil_div(n, 256L), 148 * 8)), unsigned(nf)), 256, 0, st, o, n));
   }
   void copy(T* dst, const T* src, long n) {
-    KL("k_copy", 2.0 * n * sizeof(T), k_copy<T><<<grid_for(n), 256, 0, st>>>(dst, src, n));
+    KL("k_copy", 2.0 * n * sizeof(T), launch_dep(k_copy<T>, grid_for(n), 256, 0, st, dst, src, n));
   }
   void fill_plane(T* f, T v) {
-    KL("k_fill", double(g.plane()) * sizeof(T), k_fill<T><<<grid_for(g.plane()), 256, 0, st>>>(f, g.plane(), v));
+    KL("k_fill", double(g.plane()) * sizeof(T), launch_dep(k_fill<T>, grid_for(g.plane()), 256, 0, st, f, g.plane(), v));
   }
 
   // Compensated FP64 sums of each of levels k0 .. k0 + nlev - 1 of up to six
@@ -338,13 +338,13 @@ class Solver final : public SolverBase {
     const int nch = int(std::max(1L, std::min({want, g.plane() / 2048, (long)PSUM_CHUNKS})));
     const long chunk = (long)ceil_div(ceil_div(g.plane(), nch), 4) * 4;
     KL("k_plane_sums", double(nf) * nlev * g.plane() * sizeof(T),
-       k_plane_sums<T><<<dim3(unsigned(nch), unsigned(nlev), unsigned(nf)), 256, 0, st>>>(in, psum, g.plane(), k0, chunk));
+       launch_dep(k_plane_sums<T>, dim3(unsigned(nch), unsigned(nlev), unsigned(nf)), 256, 0, st, in, psum, g.plane(), k0, chunk));
     return nch;
   }
   void plane_means(std::initializer_list<const T*> f, int k0, int nlev, double* out) {
     const int nch = plane_sums(f, k0, nlev), nf = int(f.size());
     KL("k_sums_mean", 16.0 * nf * nlev * nch,
-       k_sums_mean<<<ceil_div((long)nf * nlev, 64), 64, 0, st>>>(psum, out, nf, nlev, nch, g.plane(), k0, g.L));
+       launch_dep(k_sums_mean, ceil_div((long)nf * nlev, 64), 64, 0, st, psum, out, nf, nlev, nch, g.plane(), k0, g.L));
   }
 
   // row pitch of the spectral buffers: whole 8-value groups (64 B in FP32),
@@ -355,6 +355,7 @@ class Solver final : public SolverBase {
     XFArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.op = op;
+    a.dep = 1;
     a.nf = nf;
     a.plane0 = plane0;
     a.rows_pp = rows_pp;
@@ -373,6 +374,7 @@ class Solver final : public SolverBase {
     YPArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.op = op;
+    a.dep = 1;
     a.nin = nin;
     a.nout = nout;
     a.ncols = ncols;
@@ -395,6 +397,7 @@ class Solver final : public SolverBase {
     XIArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.op = op;
+    a.dep = 1;
     a.nin = nin;
     a.plane0 = plane0;
     a.rows_pp = rows_pp;
@@ -756,7 +759,7 @@ class Solver final : public SolverBase {
       dynamic_mum(a, true);
       const long n1 = (long)(g.nz + 1) * g.plane();
       KL("k_lasd_update", 14.0 * n1 * sizeof(T),
-         k_lasd_update<T><<<grid_for(n1), 256, 0, st>>>(sc[0], sc[12], sc[13], sc[14], sc[7], sc[8], sc[9], sc[10],
+         launch_dep(k_lasd_update<T>, grid_for(n1), 256, 0, st, sc[0], sc[12], sc[13], sc[14], sc[7], sc[8], sc[9], sc[10],
                                                        sc[11], sc[1], 1, g.plane(), g.nz, 1.5 * delta,
                                                        P.dt * double(P.cs_count), beta_pow, cs_prev, -1, cs2_max));
       std::vector<double> prof(g.L, 0.0);
@@ -897,7 +900,7 @@ class Solver final : public SolverBase {
       stat_iterations = 0;
     }
     KL("k_plane_accum", 20.0 * plane,
-       k_plane_accum<T><<<grid_for(plane), 256, 0, st>>>(PL[LES_U_STAR_AVG], stat_ustar, plane));
+       launch_dep(k_plane_accum<T>, grid_for(plane), 256, 0, st, PL[LES_U_STAR_AVG], stat_ustar, plane));
     if (write) {
       const auto h = to_host(stat_ustar, plane);
       write_host(base + "_2D.dat", {h.data()}, plane);
@@ -906,7 +909,7 @@ class Solver final : public SolverBase {
     StatFields<T> sf{F[LES_U],   F[LES_V],   F[LES_W],   F[LES_P],    F[LES_TXX],  F[LES_TYY], F[LES_TZZ],
                      F[LES_TXY], F[LES_TXZ], F[LES_TYZ], F[LES_DUDZ], F[LES_DVDZ], F[LES_NU_T], F[LES_CS_OPT2]};
     KL("k_stat_accum", double(n) * (16.0 * STAT_NQ + 16.0 * sizeof(T)),
-       k_stat_accum<T><<<grid_for(n), 256, 0, st>>>(sf, stat_acc, plane, g.nz));
+       launch_dep(k_stat_accum<T>, grid_for(n), 256, 0, st, sf, stat_acc, plane, g.nz));
     if (write) {
       const auto h = to_host(stat_acc, STAT_NQ * n);
       std::vector<const double*> parts;
@@ -961,7 +964,7 @@ class Solver final : public SolverBase {
     Tag tag_(this, "tke");
     const long plane = g.plane();
     KL("k_tke_cpress", 6.0 * g.field() * sizeof(T),
-       k_tke_cpress<T><<<grid_for(g.field()), 256, 0, st>>>(F[LES_P], F[LES_U], F[LES_V], F[LES_W], F[LES_CS_OPT2],
+       launch_dep(k_tke_cpress<T>, grid_for(g.field()), 256, 0, st, F[LES_P], F[LES_U], F[LES_V], F[LES_W], F[LES_CS_OPT2],
                                                              tke_f[0], plane, g.nz));
     grad_ptrs(&tke_f[0], &tke_f[1], &tke_f[2], 1);
     TkeFields<T> tf{F[LES_U],    F[LES_V],    F[LES_W],    F[LES_DUDX], F[LES_DUDY], F[LES_DUDZ],
@@ -970,12 +973,12 @@ class Solver final : public SolverBase {
                     F[LES_CS_OPT2], tke_f[0], tke_f[1], tke_f[2]};
     const dim3 grid(tke_nch, g.nz);
     const double idz = 1.0 / dz(), bytes = 26.0 * g.nz * plane * sizeof(T);
-    KL("k_tke_partial", bytes, k_tke_partial<T, 0, 16><<<grid, 256, 0, st>>>(tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, k_tke_partial<T, 16, 16><<<grid, 256, 0, st>>>(tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, k_tke_partial<T, 32, 16><<<grid, 256, 0, st>>>(tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, k_tke_partial<T, 48, 13><<<grid, 256, 0, st>>>(tf, tke_part, plane, P.wall_law, idz));
+    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 0, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
+    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 16, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
+    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 32, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
+    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 48, 13>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
     KL("k_tke_final", 8.0 * g.nz * tke_nch * TKE_NQ,
-       k_tke_final<<<grid_for((long)g.nz * TKE_NQ), 256, 0, st>>>(tke_part, tke_nch, g.nz,
+       launch_dep(k_tke_final, grid_for((long)g.nz * TKE_NQ), 256, 0, st, tke_part, tke_nch, g.nz,
                                                                  double(g.nx) * double(g.ny), tke_avar));
     if (jt % tke_period == 0) {
       // avg_var :408-418: record ii (nz FP64 values, the 4-byte record units
@@ -1014,7 +1017,7 @@ class Solver final : public SolverBase {
     } else {
       if (!staging) staging = track(dalloc<double>(g.field()));
       LES_CUDA(cudaMemcpyAsync(staging, h, n * sizeof(double), cudaMemcpyHostToDevice, st));
-      KL("k_convert", 12.0 * n, k_convert<T, double><<<grid_for(n), 256, 0, st>>>(lev(F[field], k0), staging, n));
+      KL("k_convert", 12.0 * n, launch_dep(k_convert<T, double>, grid_for(n), 256, 0, st, lev(F[field], k0), staging, n));
     }
   }
   void download_async(int field, double* h, int k0, int k1) override {
@@ -1024,7 +1027,7 @@ class Solver final : public SolverBase {
       LES_CUDA(cudaMemcpyAsync(h, lev(F[field], k0), n * sizeof(double), cudaMemcpyDeviceToHost, st));
     } else {
       if (!staging) staging = track(dalloc<double>(g.field()));
-      KL("k_convert", 12.0 * n, k_convert<double, T><<<grid_for(n), 256, 0, st>>>(staging, lev(F[field], k0), n));
+      KL("k_convert", 12.0 * n, launch_dep(k_convert<double, T>, grid_for(n), 256, 0, st, staging, lev(F[field], k0), n));
       LES_CUDA(cudaMemcpyAsync(h, staging, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
   }
@@ -1113,7 +1116,7 @@ class Solver final : public SolverBase {
           long n;
           chunk(c, k0, n);
           LES_CUDA(cudaStreamWaitEvent(st, ev_inc[q * nchunk + c], 0));
-          KL("k_convert", 12.0 * n, k_convert<T, double><<<grid_for(n), 256, 0, st>>>(
+          KL("k_convert", 12.0 * n, launch_dep(k_convert<T, double>, grid_for(n), 256, 0, st,
                                         lev(F[fid[q]], k0), stage_in[q] + k0 * g.plane(), n));
         }
     }
@@ -1129,7 +1132,7 @@ class Solver final : public SolverBase {
         chunk(c, k0, n);
         if constexpr (!f64) {  // the copy back of a chunk starts once that chunk is converted
           Tag tag_(this, "io");
-          KL("k_convert", 12.0 * n, k_convert<double, T><<<grid_for(n), 256, 0, st>>>(
+          KL("k_convert", 12.0 * n, launch_dep(k_convert<double, T>, grid_for(n), 256, 0, st,
                                         stage_out[q] + k0 * g.plane(), lev(F[fid[q]], k0), n));
           LES_CUDA(cudaEventRecord(ev_cvt[q * nchunk + c], st));
           LES_CUDA(cudaStreamWaitEvent(sd2h, ev_cvt[q * nchunk + c], 0));
@@ -1189,7 +1192,7 @@ class Solver final : public SolverBase {
     return a;
   }
   void launch_bc(int4 lt, int4 ut) {
-    KL("k_set_bc", 8.0 * g.plane() * sizeof(T), k_set_bc<T><<<grid_for(g.plane()), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], PL[LES_LBC_U], PL[LES_LBC_V],
+    KL("k_set_bc", 8.0 * g.plane() * sizeof(T), launch_dep(k_set_bc<T>, grid_for(g.plane()), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], PL[LES_LBC_U], PL[LES_LBC_V],
                                                     PL[LES_LBC_W], PL[LES_UBC_U], PL[LES_UBC_V], PL[LES_UBC_W],
                                                     lt, ut, g.plane(), g.nz, T(P.lz / double(g.nz))));
   }
@@ -1282,10 +1285,10 @@ class Solver final : public SolverBase {
   void grad_velocity_filt(int f, int dfdx, int dfdy) override { grad_fields(&f, &dfdx, &dfdy, 1); }
 
   void ddz_uv(int dfdz, int f) override {
-    KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T), k_ddz<T><<<grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st>>>(F[dfdz], F[f], g.plane(), g.nz, T(1.0 / dz()), 0));
+    KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T), launch_dep(k_ddz<T>, grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st, F[dfdz], F[f], g.plane(), g.nz, T(1.0 / dz()), 0));
   }
   void ddz_w(int dfdz, int f) override {
-    KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T), k_ddz<T><<<grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st>>>(F[dfdz], F[f], g.plane(), g.nz, T(1.0 / dz()), 1));
+    KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T), launch_dep(k_ddz<T>, grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st, F[dfdz], F[f], g.plane(), g.nz, T(1.0 / dz()), 1));
   }
 
   void compute_vel_grad() override { vel_grad(-1, false); }
@@ -1302,7 +1305,7 @@ class Solver final : public SolverBase {
     Tag tag_(this, "grad");
     const long n = (long)(g.nz + 1) * g.plane();
     KL("k_bc_ddz", (6.0 * n + (nacc >= 0 ? 6.0 * (nacc + 1) * g.plane() : 0.0)) * sizeof(T),
-       k_bc_ddz<T><<<grid_for(n / 4), 256, 0, st>>>(bc_args(), F[LES_DUDZ], F[LES_DVDZ], F[LES_DWDZ], T(1.0 / dz()),
+       launch_dep(k_bc_ddz<T>, grid_for(n / 4), 256, 0, st, bc_args(), F[LES_DUDZ], F[LES_DVDZ], F[LES_DWDZ], T(1.0 / dz()),
                                                     nacc >= 0 ? F[LES_U_LAG] : nullptr, F[LES_V_LAG], F[LES_W_LAG],
                                                     nacc));
     if (scalar_on) scalar_grad();
@@ -1562,6 +1565,7 @@ class Solver final : public SolverBase {
     };
     YRArgs<T> b;
     std::memset(&b, 0, sizeof(b));
+    b.dep = 1;
     for (int q = 0; q < neq; ++q) {
       b.p[q] = spec[q];
       b.sx[q] = spec[11 + slot(e[q].tx)];
@@ -1629,6 +1633,7 @@ class Solver final : public SolverBase {
     XFArgs<S> a;
     std::memset(&a, 0, sizeof(a));
     a.op = op;
+    a.dep = 1;
     a.nf = nf;
     a.plane0 = plane0;
     a.rows_pp = g.ny;
@@ -1646,6 +1651,7 @@ class Solver final : public SolverBase {
     YPArgs<S> a;
     std::memset(&a, 0, sizeof(a));
     a.op = op;
+    a.dep = 1;
     a.nin = nin;
     a.nout = nout;
     a.ncols = g.lhx;
@@ -1686,7 +1692,7 @@ class Solver final : public SolverBase {
   void press_finish() {
     dpdz_only();
     KL("k_p_finish", (mixed() ? 2.0 * g.field() : double(g.plane())) * sizeof(T),
-       k_p_finish<T><<<grid_for(g.field() / 4), 256, 0, st>>>(F[LES_P], mixed() ? pmean : nullptr, g.plane(), g.nz));
+       launch_dep(k_p_finish<T>, grid_for(g.field() / 4), 256, 0, st, F[LES_P], mixed() ? pmean : nullptr, g.plane(), g.nz));
   }
 
   // Right-hand side in two FP64 spectra instead of three, and one after the y
@@ -1730,7 +1736,7 @@ class Solver final : public SolverBase {
       slab_solve<S, T>(s0, ph, pm, drop, pp, g.lhx);
     else
       KL("k_tridiag", (56.0 + 8.0 + 2.0 * sizeof(T)) * double(g.L) * g.ny * g.lhx,
-         k_tridiag<T><<<ceil_div(2L * g.ny * g.lhx, 128), 128, 0, st>>>(reinterpret_cast<double*>(s0), piv,
+         launch_dep(k_tridiag<T>, ceil_div(2L * g.ny * g.lhx, 128), 128, 0, st, reinterpret_cast<double*>(s0), piv,
                                                                          reinterpret_cast<T*>(ph), pm, dstatus, g.lhx,
                                                                          g.ny, nz, dz(), drop, pp));
     press_grad(ph, pout);
@@ -1820,7 +1826,7 @@ class Solver final : public SolverBase {
     sweep_scratch();
     const int nz = g.nz;
     const double c = 1.0 / double(g.nx * g.ny);
-    KL("k_scale", 2.0 * g.plane() * sizeof(T), k_scale<T><<<grid_for(g.plane()), 256, 0, st>>>(PL[LES_BOTTOM_WK_PRESS], g.plane(), T(c)));
+    KL("k_scale", 2.0 * g.plane() * sizeof(T), launch_dep(k_scale<T>, grid_for(g.plane()), 256, 0, st, PL[LES_BOTTOM_WK_PRESS], g.plane(), T(c)));
     cplx<T>* bot = spec[8];
     cplx<T>* top = spec[9];
     {
@@ -1980,7 +1986,7 @@ class Solver final : public SolverBase {
     const int bx = ceil_div(g.plane() / V, 256);
     const int zc = int(std::min(16L, std::max(1L, (long)(g.nz + 1) * bx / (148 * 6))));
     KL("k_sgs_tau", sbytes * n1 * sizeof(T),
-       k_sgs_tau<T, V><<<dim3(unsigned(bx), unsigned(ceil_div(g.nz + 1, zc))), 256, 0, st>>>(a, zc));
+       launch_dep(k_sgs_tau<T, V>, dim3(unsigned(bx), unsigned(ceil_div(g.nz + 1, zc))), 256, 0, st, a, zc));
   }
 
   // dynamic-procedure contractions at both test scales (compute_dynamic_mum x2)
@@ -1990,7 +1996,7 @@ class Solver final : public SolverBase {
     const long n1 = (long)nlev * g.plane();
     SgsArgs<T> ab = a;
     ab.nz = nlev - 1;  // k_sij covers levels 1..nz+1 of its arguments
-    KL("k_sij", 16.0 * n1 * sizeof(T), k_sij<T><<<grid_for(n1), 256, 0, st>>>(ab));
+    KL("k_sij", 16.0 * n1 * sizeof(T), launch_dep(k_sij<T>, grid_for(n1), 256, 0, st, ab));
     auto x = xf(XF_LASD, 21, 1, nlev, g.nx, g.ny, nk2);
     x.in[0] = F[LES_U];
     x.in[1] = F[LES_V];
@@ -2034,7 +2040,7 @@ class Solver final : public SolverBase {
     if (nlev < 0) nlev = nz + 1;
     const long nacc = std::min<long>(g.field(), (long)(nlev + 1) * g.plane());  // levels 0..nlev
     if (jtt >= P.dyn_init && !lag_added) {
-      KL("k_lag_accum", 9.0 * nacc * sizeof(T), k_lag_accum<T><<<grid_for(nacc), 256, 0, st>>>(F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG], F[LES_U],
+      KL("k_lag_accum", 9.0 * nacc * sizeof(T), launch_dep(k_lag_accum<T>, grid_for(nacc), 256, 0, st, F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG], F[LES_U],
                                                          F[LES_V], F[LES_W], nacc));
     }
     if (jtt < P.dyn_init) {
@@ -2047,7 +2053,7 @@ class Solver final : public SolverBase {
     if (f_coeff_init) {
       LagGeom geo{g.nx, g.ny, nz, g.plane(), P.lag_halo, P.dt, P.lx / double(g.nx), P.ly / double(g.ny), dz(),
                   double(P.cs_count), nlev};
-      KL("k_lag_interp", 11.0 * n1 * sizeof(T), k_lag_interp<T><<<dim3(unsigned((g.plane() + 255) / 256), unsigned(nlev)), 256, 0, st>>>(F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG], F[LES_F_LM],
+      KL("k_lag_interp", 11.0 * n1 * sizeof(T), launch_dep(k_lag_interp<T>, dim3(unsigned((g.plane() + 255) / 256), unsigned(nlev)), 256, 0, st, F[LES_U_LAG], F[LES_V_LAG], F[LES_W_LAG], F[LES_F_LM],
                                                    F[LES_F_MM], F[LES_F_QN], F[LES_F_NN], sc[11], sc[12], sc[13],
                                                    sc[14], geo));
       if (nlev == nz + 1) {
@@ -2060,7 +2066,7 @@ class Solver final : public SolverBase {
         for (int t = 0; t < 4; ++t) copy(lev(F[fl[t]], 1), lev(sc[11 + t], 1), n1);
       }
     }
-    KL("k_lasd_update", 14.0 * n1 * sizeof(T), k_lasd_update<T><<<grid_for(n1), 256, 0, st>>>(F[LES_F_LM], F[LES_F_MM], F[LES_F_QN], F[LES_F_NN], sc[7],
+    KL("k_lasd_update", 14.0 * n1 * sizeof(T), launch_dep(k_lasd_update<T>, grid_for(n1), 256, 0, st, F[LES_F_LM], F[LES_F_MM], F[LES_F_QN], F[LES_F_NN], sc[7],
                                                   sc[8], sc[9], sc[10], F[LES_CS_OPT2], F[LES_BETA],
                                                   f_coeff_init ? 0 : 1, g.plane(), nz, 1.5 * delta,
                                                   P.dt * double(P.cs_count), beta_pow, nullptr, nlev, cs2_max));
@@ -2134,7 +2140,7 @@ class Solver final : public SolverBase {
   }
   void scalar_bc() {
     KL("k_scalar_bc", 3.0 * g.plane() * sizeof(T),
-       k_scalar_bc<T><<<grid_for(g.plane()), 256, 0, st>>>(F[LES_THETA], g.plane(), g.nz, T(SP.top_gradient * dz())));
+       launch_dep(k_scalar_bc<T>, grid_for(g.plane()), 256, 0, st, F[LES_THETA], g.plane(), g.nz, T(SP.top_gradient * dz())));
   }
   void scalar_set_initial(const double* theta) override {
     if (!scalar_on) throw CudaError(1, "scalar not initialised (les_scalar_init)");
@@ -2174,10 +2180,10 @@ class Solver final : public SolverBase {
     Tag tag_(this, "scalar");
     grad_ptrs(&F[LES_THETA], &F[LES_DTDX], &F[LES_DTDY], 1, "scalar", &tsp, &tref);
     KL("k_ddz", 2.0 * (g.nz + 1) * g.plane() * sizeof(T),
-       k_ddz<T><<<grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st>>>(F[LES_DTDZ], F[LES_THETA], g.plane(), g.nz,
+       launch_dep(k_ddz<T>, grid_for((long)(g.nz + 1) * g.plane()), 256, 0, st, F[LES_DTDZ], F[LES_THETA], g.plane(), g.nz,
                                                                        T(1.0 / dz()), 0));
     KL("k_scalar_wall", 2.0 * g.plane() * sizeof(T),
-       k_scalar_wall<T><<<grid_for(g.plane()), 256, 0, st>>>(lev(F[LES_DTDZ], 1), PL[LES_U_STAR_AVG], g.plane(),
+       launch_dep(k_scalar_wall<T>, grid_for(g.plane()), 256, 0, st, lev(F[LES_DTDZ], 1), PL[LES_U_STAR_AVG], g.plane(),
                                                              SP.surface_flux, 0.5 * dz()));
   }
 
@@ -2187,7 +2193,7 @@ class Solver final : public SolverBase {
     const int nlev = g.nz + 1;
     const long n1 = (long)nlev * g.plane();
     SgsArgs<T> ab = a;
-    KL("k_sij", 16.0 * n1 * sizeof(T), k_sij<T><<<grid_for(n1), 256, 0, st>>>(ab));
+    KL("k_sij", 16.0 * n1 * sizeof(T), launch_dep(k_sij<T>, grid_for(n1), 256, 0, st, ab));
     auto x = xf(XF_SCDYN, 19, 1, nlev, g.nx, g.ny, nk2);
     x.in[0] = F[LES_U];
     x.in[1] = F[LES_V];
@@ -2216,7 +2222,7 @@ class Solver final : public SolverBase {
     z.out[1] = sc[8];
     launch_xinv<T>(g.nx, z, st);
     const int nch = plane_sums({sc[7], sc[8]}, 1, nlev);
-    KL("k_sums_ratio", 32.0 * nlev * nch, k_sums_ratio<<<ceil_div(nlev, 64), 64, 0, st>>>(psum, kapd, nlev, nch, g.plane(),
+    KL("k_sums_ratio", 32.0 * nlev * nch, launch_dep(k_sums_ratio, ceil_div(nlev, 64), 64, 0, st, psum, kapd, nlev, nch, g.plane(),
                                                                                    delta * delta));
   }
 
@@ -2320,7 +2326,7 @@ class Solver final : public SolverBase {
       if (sponge_frac > 0.0)
         plane_means({F[LES_U], F[LES_V], F[LES_W]}, 1, g.nz, means);
       KL("k_forcing", 7.0 * g.nz * g.plane() * sizeof(T),
-         k_forcing<T><<<grid_for((long)g.nz * g.plane()), 256, 0, st>>>(
+         launch_dep(k_forcing<T>, grid_for((long)g.nz * g.plane()), 256, 0, st,
              F[LES_RHSX], F[LES_RHSY], F[LES_RHSZ], F[LES_U], F[LES_V], F[LES_W], means,
              sponge_frac > 0.0 ? spong : nullptr, g.plane(), g.nz, L, T(coriol), T(ug), T(vg)));
     }
@@ -2344,7 +2350,7 @@ class Solver final : public SolverBase {
       Tag tag_(this, "scalar");
       plane_means({F[LES_THETA]}, 0, L, means + 3 * L);
       KL("k_buoyancy", 3.0 * (g.nz - 1) * g.plane() * sizeof(T),
-         k_buoyancy<T><<<grid_for((long)(g.nz - 1) * g.plane()), 256, 0, st>>>(F[LES_RHSZ], F[LES_THETA], means + 3 * L,
+         launch_dep(k_buoyancy<T>, grid_for((long)(g.nz - 1) * g.plane()), 256, 0, st, F[LES_RHSZ], F[LES_THETA], means + 3 * L,
                                                                                g.plane(), g.nz, T(SP.buoyancy)));
     }
   }
@@ -2372,7 +2378,7 @@ class Solver final : public SolverBase {
         o.top = (long)(g.nz + 1) * g.plane();
         o.val = T(BOGUS);
         KL("k_rhs_ghosts", 18.0 * g.plane() * sizeof(T),
-           k_rhs_ghosts<T><<<dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256L), 148)), 6u), 256, 0, st>>>(
+           launch_dep(k_rhs_ghosts<T>, dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256L), 148)), 6u), 256, 0, st,
                o, g.plane()));
       } else {
         T* dst[6];
@@ -2405,13 +2411,13 @@ class Solver final : public SolverBase {
 
   void ab2(double tadv1, double tadv2) override {
     Tag tag_(this, "ab2");
-    KL("k_ab2", 12.0 * g.nz * g.plane() * sizeof(T), k_ab2<T><<<grid_for(g.field()), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
+    KL("k_ab2", 12.0 * g.nz * g.plane() * sizeof(T), launch_dep(k_ab2<T>, grid_for(g.field()), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
                                                  F[LES_RHSZ], F[LES_RHSX_F], F[LES_RHSY_F], F[LES_RHSZ_F],
                                                  g.plane(), g.nz, T(P.dt), T(tadv1), T(tadv2)));
     if (scalar_on)
     {
       KL("k_ab2_scalar", 4.0 * g.nz * g.plane() * sizeof(T),
-         k_ab2_scalar<T><<<grid_for((long)g.nz * g.plane()), 256, 0, st>>>(
+         launch_dep(k_ab2_scalar<T>, grid_for((long)g.nz * g.plane()), 256, 0, st,
              F[LES_THETA], F[LES_RHS_T], F[LES_RHS_T_F], g.plane(), g.nz, T(P.dt), T(tadv1), T(tadv2)));
       scalar_bc();
     }
@@ -2420,7 +2426,7 @@ class Solver final : public SolverBase {
   void projection(double tadv1) override {
     Tag tag_(this, "projection");
     // dpdz was formed by press_stag_array; this applies LES_engine.f90:303-331
-    KL("k_projection", 15.0 * g.nz * g.plane() * sizeof(T), k_projection<T><<<grid_for(g.field()), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
+    KL("k_projection", 15.0 * g.nz * g.plane() * sizeof(T), launch_dep(k_projection<T>, grid_for(g.field()), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
                                                         F[LES_RHSZ], F[LES_DPDX], F[LES_DPDY], F[LES_DPDZ],
                                                         g.plane(), g.nz, P.dt * tadv1));
   }
@@ -2475,7 +2481,7 @@ class Solver final : public SolverBase {
         constexpr bool DIAG = decltype(diag_c)::value;
         const int nb = DIAG ? diag_blocks() : grid_for(g.field() / 4);
         KL("k_step_finish", fields * g.nz * g.plane() * sizeof(T),
-           k_step_finish<T, DIAG><<<nb, 256, 0, st>>>(
+           launch_dep(k_step_finish<T, DIAG>, nb, 256, 0, st,
                bc_args(), praw, F[LES_P], mixed() ? pmean : nullptr, F[LES_DPDX], F[LES_DPDY], F[LES_DPDZ],
                F[LES_RHSX], F[LES_RHSY], F[LES_RHSZ], T(1.0 / dz()), P.dt * t1, F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ],
                PL[LES_U_STAR_AVG], diag_out()));
@@ -2501,7 +2507,7 @@ class Solver final : public SolverBase {
   void diagnostics_launch() {
     Tag tag_(this, "diag");
     KL("k_diag", 6.0 * g.nz * g.plane() * sizeof(T),
-       k_diag<T><<<diag_blocks(), 256, 0, st>>>(F[LES_U], F[LES_V], F[LES_W], F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ],
+       launch_dep(k_diag<T>, diag_blocks(), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], F[LES_DUDX], F[LES_DVDY], F[LES_DWDZ],
                                                 PL[LES_U_STAR_AVG], g.nz, diag_out()));
   }
   void diagnostics(double out[4]) override {
@@ -2646,7 +2652,7 @@ void Solver<T>::dynsmag(SgsArgs<T>& a, int jt, int jtt) {
   dynamic_mum(a, false);
   const int nlev = g.nz + 1, nch = plane_sums({sc[7], sc[8]}, 1, nlev);
   KL("k_sums_spread", double(nlev) * g.plane() * sizeof(T),
-     k_sums_spread<T><<<dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256), 32)), unsigned(nlev)), 256, 0, st>>>(
+     launch_dep(k_sums_spread<T>, dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256), 32)), unsigned(nlev)), 256, 0, st,
          psum, F[LES_CS_OPT2], nlev, nch, g.plane(), cs2_max));
 }
 

@@ -117,6 +117,7 @@ enum XFOp : int {
 
 template <typename T>
 struct XFArgs {
+  int dep;         // launched by launch_dep: the tables are constant
   int op, nf, R;
   int lfast;       // k_xfwd: a CTA's rows are one row of R consecutive levels
   long nrows;      // rows to process = nplanes * rows_pp
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     rowl[r] = q < nlev ? a.plane0 + q : -1;
     rowj[r] = q < nlev ? j : 0;
   }
+  dep_wait();
   __syncthreads();
   if (a.use_ref) {
     for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
@@ -652,8 +654,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
   int* rowl = reinterpret_cast<int*>(refs + ((nseq + 1) & ~1));
   int* rowj = rowl + a.R;
   const long nitems = (a.nrows + a.R - 1) / a.R;
-  // the first copies start before the tables are built (warp 0 sets up the
-  // barriers and issues them)
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = c_scl(a.tw[i], T(0.5));  // W^k / 2 for the split
+  twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
+  dep_wait();
+  // warp 0 sets up the barriers and issues the first copies
   if (threadIdx.x < 32) {
     if (threadIdx.x == 0) {
       tc::mbar_init(&bars[0], 1);
@@ -672,8 +676,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
     return T(a.c0) * a.in[f][(long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride];
   };
   T ref_next = ref_of(blockIdx.x);
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = c_scl(a.tw[i], T(0.5));  // W^k / 2 for the split
-  twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
   __syncthreads();
   unsigned phase = 0;  // bit b: parity of the next completion of bars[b]
   int stg = 0;
@@ -826,6 +828,7 @@ enum YPOp : int {
 
 template <typename T>
 struct YPArgs {
+  int dep;         // launched by launch_dep: the tables are constant
   int op, nin, nout, C, lc;  // C = 1 << lc columns per CTA
   int SI;                    // column stride of the shared stages (>= both lengths' slots)
   int ncols;           // columns processed
@@ -964,6 +967,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   if constexpr (!FWD) twm_build<T, NYO, true>(a.tw_out, two, threadIdx.x, blockDim.x);
   if (a.kky)
     for (int i = threadIdx.x; i < NY; i += blockDim.x) kyrow[i] = a.kky[(long)i * a.lhx];
+  dep_wait();
   // persistent CTAs: work item = (column block, plane, group); with two
   // stages the columns of the next item are copied into the other input
   // stage asynchronously while this one is transformed, with one stage they
@@ -1214,6 +1218,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
 // stresses (i kx t_x + i ky t_y), their sum, and one inverse transform.
 template <typename T>
 struct YRArgs {
+  int dep;         // launched by launch_dep: the tables are constant
   int C, lc, SI;       // C = 1 << lc columns per CTA, column stride of a shared slot
   int nslot;           // shared slots (set by the launcher): 2 = a copy runs under every transform
   int ncols;           // output columns
@@ -1280,6 +1285,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   twm_build<T, N, false>(a.tw_s, tws, threadIdx.x, blockDim.x);
   twm_build<T, N, true>(a.tw_s, twi, threadIdx.x, blockDim.x);
   for (int i = threadIdx.x; i < N; i += blockDim.x) kyrow[i] = a.kky[(long)i * a.lhx];
+  dep_wait();
   const int ncb = (a.ncols + C - 1) / C;
   const long nitems = (long)ncb * a.nplanes * a.ngroups;
   // input `in` (0 products, 1 t_x, 2 t_y) of item `item` into ring slot `sl`
@@ -1421,6 +1427,7 @@ enum XIOp : int {
 
 template <typename T>
 struct XIArgs {
+  int dep;         // launched by launch_dep: the tables are constant
   int op, nin, R;
   long nrows;
   int rows_pp;
@@ -1597,10 +1604,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       (reinterpret_cast<uintptr_t>(kxs + (a.nstage ? a.nk + 2 : 0)) + 7) & ~uintptr_t(7));
   // persistent CTAs over batches of R rows; with two stages the spectral
   // rows of the next batch are copied into the other stage while this one
-  // is transformed, with one stage after this batch's last read of it.  The
-  // first copies start before the tables are built (warp 0 sets up the
-  // barriers and issues them).
+  // is transformed, with one stage after this batch's last read of it (warp 0
+  // sets up the barriers and issues the bulk copies).
   const long nitems = (a.nrows + a.R - 1) / a.R;
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = a.tw[i];
+  twm_build<T, M, true, 2>(a.tw, twm, threadIdx.x, blockDim.x);
+  if (a.nstage)
+    for (int i = threadIdx.x; i < a.nk; i += blockDim.x) kxs[i] = a.kxr[i];
+  dep_wait();
   if (a.bulk) {
     if (threadIdx.x < 32) {
       if (threadIdx.x == 0) {
@@ -1615,10 +1626,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     xi_issue<T>(a, blockIdx.x, stage0);
     cp_async_commit();
   }
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) tw[i] = a.tw[i];
-  twm_build<T, M, true, 2>(a.tw, twm, threadIdx.x, blockDim.x);
-  if (a.nstage)
-    for (int i = threadIdx.x; i < a.nk; i += blockDim.x) kxs[i] = a.kxr[i];
   __syncthreads();
   unsigned phase = 0;  // bit b: parity of the next completion of bars[b]
   int stg = 0;

@@ -39,7 +39,8 @@ static void launch_xfwd_row(int NX, XFArgs<T>& a, cudaStream_t st) {
   const long nitems = ceil_div(a.nrows, a.R);
   if (nitems == 0) return;
   const int grid = int(std::min<long>(nitems, (long)resident_ctas((const void*)kern, 256, smem)));
-  kern<<<grid, 256, smem, st>>>(a);
+  if (a.dep) launch_dep(kern, grid, 256, smem, st, a);
+  else kern<<<grid, 256, smem, st>>>(a);
   LES_CHECK_LAUNCH();
 }
 
@@ -106,7 +107,8 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
             8L * ngrp * a.R <= 9L * nlev;
   const int grid = a.lfast ? a.rows_pp * ngrp : ceil_div(a.nrows, a.R);
   if (grid == 0) return;
-  kern<<<grid, XF_THREADS, smem, st>>>(a);
+  if (a.dep) launch_dep(kern, grid, XF_THREADS, smem, st, a);
+  else kern<<<grid, XF_THREADS, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
 }

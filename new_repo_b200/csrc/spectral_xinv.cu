@@ -107,7 +107,8 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
     else if (a.op == XI_WALL) nout = 7;
     hook_before("xinv", double(a.nrows) * ns * a.nk * sizeof(cplx<T>) + double(a.nrows) * NX * (nout + rmw) * osz);
   }
-  kern<<<grid, 256, smem, st>>>(a);
+  if (a.dep) launch_dep(kern, grid, 256, smem, st, a);
+  else kern<<<grid, 256, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
 }

@@ -105,7 +105,8 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
   const int grid = int(std::min<long>(nitems, (long)resident_ctas((const void*)kern, threads, smem)));
   hook_before("ypass", double(nplanes) * ngroups * a.ncols * sizeof(cplx<T>) *
                            (double(a.op == YP_PGRAD ? 1 : a.nin) * NY + double(a.nout) * NYO));
-  kern<<<grid, threads, smem, st>>>(a);
+  if (a.dep) launch_dep(kern, grid, threads, smem, st, a);
+  else kern<<<grid, threads, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
 }
@@ -172,7 +173,8 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
   const int grid = int(std::min<long>(items(lc), (long)resident_ctas((const void*)kern, threads, smem)));
   hook_before("yrhs", double(a.nplanes) * a.ngroups * sizeof(cplx<T>) *
                           (double(a.nkp) * NF + 2.0 * a.ncols * N + double(a.ncols) * N));
-  kern<<<grid, threads, smem, st>>>(a);
+  if (a.dep) launch_dep(kern, grid, threads, smem, st, a);
+  else kern<<<grid, threads, smem, st>>>(a);
   LES_CHECK_LAUNCH();
   hook_after();
 }

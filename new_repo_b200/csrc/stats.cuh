@@ -25,6 +25,7 @@ struct StatFields {
 // first level is reset to zero on every call (:378-384).
 template <typename T>
 __global__ void __launch_bounds__(256) k_stat_accum(StatFields<T> f, double* __restrict__ acc, long plane, int nz) {
+  dep_wait();
   const long n = (long)nz * plane;
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n; o += (long)gridDim.x * blockDim.x) {
     const long c = o + plane;  // level 1 + o / plane of the (0..nz+1) storage
@@ -70,7 +71,8 @@ __global__ void __launch_bounds__(256) k_stat_accum(StatFields<T> f, double* __r
 
 // io_2D_stat_averages (:316-320): running sum of the friction-velocity plane
 template <typename T>
-__global__ void k_plane_accum(const T* __restrict__ x, double* __restrict__ acc, long plane) {
+__global__ void k_plane_accum(const T* x, double* acc, long plane) {
+  dep_wait();
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < plane; o += (long)gridDim.x * blockDim.x)
     acc[o] = __dadd_rn(acc[o], double(x[o]));
 }
@@ -185,6 +187,7 @@ __device__ __forceinline__ void tke_point(const TkeFields<T>& f, long o, long pl
 template <typename T, int Q0, int NQ>
 __global__ void __launch_bounds__(256) k_tke_partial(TkeFields<T> f, double* __restrict__ part, long plane, int wall,
                                                      double idz) {
+  dep_wait();
   const int k = 1 + blockIdx.y;
   const long base = (long)k * plane;
   double acc[NQ];
@@ -213,7 +216,8 @@ __global__ void __launch_bounds__(256) k_tke_partial(TkeFields<T> f, double* __r
 
 // avar(q, k) += (sum of the shares) / (nx ny)  (avg_var :400-406 with
 // compute_planar_average utility_tools.f90:59-92)
-__global__ void k_tke_final(const double* __restrict__ part, int nch, int nz, double npts, double* __restrict__ avar) {
+__global__ void k_tke_final(const double* part, int nch, int nz, double npts, double* avar) {
+  dep_wait();
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nz * TKE_NQ; idx += gridDim.x * blockDim.x) {
     const int k0 = idx / TKE_NQ, q = idx % TKE_NQ;
     double s = 0.0;
@@ -228,8 +232,8 @@ __global__ void k_tke_final(const double* __restrict__ part, int nch, int nz, do
 // is unset memory, taken here as zero.  Both reach only the dpdz profile at
 // levels 1 and nz.
 template <typename T>
-__global__ void k_tke_cpress(const T* __restrict__ p, const T* __restrict__ u, const T* __restrict__ v,
-                             const T* __restrict__ w, const T* __restrict__ cs, T* __restrict__ c, long plane, int nz) {
+__global__ void k_tke_cpress(const T* p, const T* u, const T* v, const T* w, const T* cs, T* c, long plane, int nz) {
+  dep_wait();
   const long n = (long)(nz + 2) * plane;
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n; o += (long)gridDim.x * blockDim.x) {
     const long k = udiv32(o, plane);

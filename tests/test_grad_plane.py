@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 SIZES = [(16, 16, 1), (16, 128, 3), (24, 16, 2), (24, 32, 5), (32, 64, 150), (48, 32, 3), (48, 128, 2), (64, 128, 4),
          (96, 64, 3), (96, 128, 2), (128, 16, 2), (128, 64, 3), (192, 16, 2), (192, 64, 2), (256, 16, 2), (256, 32, 149),
-         (256, 64, 24), (128, 128, 23), (128, 128, 24)]
+         (256, 64, 24), (256, 64, 40), (128, 128, 23), (128, 128, 24), (128, 128, 39), (128, 128, 40)]
 
 
 @pytest.mark.parametrize("nx,ny,nlev", SIZES)
