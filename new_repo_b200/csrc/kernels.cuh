@@ -202,26 +202,6 @@ __global__ void k_plane_ops(const PlaneOps<T> ops, long n) {
     d[q] = s ? s[q] : v;
 }
 
-// Ghost levels of the three right-hand sides as their buffers change roles:
-// the old buffer (next rhs_f) takes rhs_f's ghost levels, the new one val.
-// grid (.., 6): blockIdx.y = equation and level.
-template <typename T>
-struct RhsGhosts {
-  T *oldr[3], *newr[3];  // the two buffers of each equation
-  long top;              // offset of level nz + 1
-  T val;
-};
-template <typename T>
-__global__ void k_rhs_ghosts(const RhsGhosts<T> a, long plane) {
-  dep_wait();
-  const int q = blockIdx.y >> 1;
-  const long o = (blockIdx.y & 1) ? a.top : 0;
-  for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < plane; p += (long)gridDim.x * blockDim.x) {
-    a.oldr[q][o + p] = a.newr[q][o + p];
-    a.newr[q][o + p] = a.val;
-  }
-}
-
 template <typename T>
 __global__ void k_scale(T* f, long n, T c) {
   dep_wait();
@@ -1608,16 +1588,44 @@ __global__ void k_forcing(T* rx, T* ry, T* rz, const T* u, const T* v, const T* 
 
 // Buoyancy on w nodes k = 2..nz: rz += beta (theta_w - <theta_w>),
 // theta_w(k) = (theta(k) + theta(k-1)) / 2; tmean = plane means of theta.
+// With w given the whole right-hand side of w is there now, and w advances as
+// in k_ab2 (four points per thread; a plane is at least 16 x 16).
 template <typename T>
-__global__ void k_buoyancy(T* rz, const T* th, const double* tmean, long plane, int nz, T beta) {
+__global__ void k_buoyancy(T* rz, const T* th, const double* tmean, long plane, int nz, T beta, T* w, const T* fz, T dt,
+                           T t1, T t2) {
   dep_wait();
-  const long n = (long)(nz - 1) * plane;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-    const long o = 2 * plane + q;
+  const long n = (long)(nz + 2) * plane;
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n / 4; q += (long)gridDim.x * blockDim.x) {
+    const long o = 4 * q;
     const int k = udiv32(o, plane);
-    const T tw = T(0.5) * (th[o] + th[o - plane]);
-    const T twm = T(0.5 * (tmean[k] + tmean[k - 1]));
-    rz[o] = rz[o] + beta * (tw - twm);
+    T x[4], r[4], f[4], a[4], b[4];
+    if (k < 1 || k > nz) {
+      if (w) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = T(0);
+        st4(w + o, x);
+      }
+      continue;
+    }
+    if (k == 1 && !w) continue;
+    ld4(rz + o, r);
+    if (w) {
+      ld4(w + o, x);
+      ld4(fz + o, f);
+    }
+    if (k > 1) {
+      ld4(th + o, a);
+      ld4(th + o - plane, b);
+      const T twm = T(0.5 * (tmean[k] + tmean[k - 1]));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = r[i] + beta * (T(0.5) * (a[i] + b[i]) - twm);
+      st4(rz + o, r);
+    }
+    if (w) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = x[i] + dt * (t1 * r[i] + t2 * f[i]);
+      st4(w + o, x);
+    }
   }
 }
 

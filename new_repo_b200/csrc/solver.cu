@@ -1546,15 +1546,33 @@ class Solver final : public SolverBase {
       const DivEq e[3] = {{LES_RHSX, LES_TXX, LES_TXY, LES_TXZ, 1, P.pfx},
                           {LES_RHSY, LES_TXY, LES_TYY, LES_TYZ, 1, P.pfy},
                           {LES_RHSZ, LES_TXZ, LES_TYZ, LES_TZZ, 0, 0.0}};
-      div_products(e, 3, true, mixed());
+      div_products(e, 3, true, mixed(), padd() ? 2 : 0);
     }
     Tag tag_(this, "convec");
-    if (!padd()) convec_ghosts(rhs);  // padded: written with the buffer exchange (rhs_adv)
+    if (!padd()) convec_ghosts(rhs);  // padded: the convective routine's own, BOGUS, come with the divergence
+  }
+  // The time advance at the end of the right-hand sides of a step: an equation
+  // whose divergence is the last thing added to it advances there (the x
+  // inverse has rhs in registers: one read of it and two launches less per
+  // step, 32 x 32 x 16 152.5 -> 148.5 us, 256^3 mixed 3934 -> 3885, FP64 8018 ->
+  // 7939, 512 x 512 x 96 with a buoyant scalar 10280 -> 10200); with Coriolis or sponge terms the momentum advances
+  // after those (k_ab2), with buoyancy w does with that (k_buoyancy).
+  struct {
+    bool on = false;
+    double t1 = 0.0, t2 = 0.0;
+  } adv;
+  bool momentum_advances() const { return adv.on && coriol == 0.0 && !(sponge_frac > 0.0); }
+  bool buoyant() const { return scalar_on && SP.buoyancy != 0.0; }
+  bool advances(int rhs) const {
+    if (rhs == LES_RHS_T) return adv.on;
+    return momentum_advances() && !(rhs == LES_RHSZ && buoyant());
   }
   // rhs of neq equations = products (spectra spec[q], references refbuf[6 + q])
   // + stress divergence + forcing
   // (refs: the products' references are to be added, mixed precision)
-  void div_products(const DivEq* e, int neq, bool layers, bool refs) {
+  // (adv.on: they end with the time advance of what they drive, see XIArgs;
+  // ghosts: with the ghost levels of their buffers)
+  void div_products(const DivEq* e, int neq, bool layers, bool refs, int ghosts) {
     const int nz = g.nz, FNY = padd() ? g.ny2 : g.ny, nc = g.nx / 2;
     int ids[6], nid = 0;
     auto slot = [&](int fid) {
@@ -1613,6 +1631,22 @@ class Solver final : public SolverBase {
     c.hi_ref = nz;
     c.out[8] = layers ? PL[LES_BOTTOM_WK_PRESS] : nullptr;
     c.out[9] = layers ? PL[LES_TOP_WK_PRESS] : nullptr;
+    c.adv_ghosts = ghosts;
+    for (int q = 0; q < neq; ++q) {
+      int var = -1, f = -1;
+      switch (e[q].rhs) {
+        case LES_RHSX: var = LES_U; f = LES_RHSX_F; break;
+        case LES_RHSY: var = LES_V; f = LES_RHSY_F; break;
+        case LES_RHSZ: var = LES_W; f = LES_RHSZ_F; c.adv_lid[q] = ADV_ZERO; break;
+        case LES_RHS_T: var = LES_THETA; f = LES_RHS_T_F; c.adv_lid[q] = ADV_LID; break;
+      }
+      c.adv_f[q] = F[f];
+      c.adv_v[q] = advances(e[q].rhs) ? F[var] : nullptr;
+    }
+    c.adv_dt = P.dt;
+    c.adv_t1 = adv.t1;
+    c.adv_t2 = adv.t2;
+    c.adv_top = SP.top_gradient * dz();
     launch_xinv<T>(g.nx, c, st);
   }
 
@@ -2315,7 +2349,7 @@ class Solver final : public SolverBase {
     launch_xinv<T>(FNX, c, st);
     scalar_products();
     const DivEq e{LES_RHS_T, LES_QX, LES_QY, LES_QZ, 1, 0.0};
-    div_products(&e, 1, false, false);
+    div_products(&e, 1, false, false, 1);
   }
 
   // after the momentum right-hand side: forcing, scalar rhs, buoyancy
@@ -2331,12 +2365,24 @@ class Solver final : public SolverBase {
              sponge_frac > 0.0 ? spong : nullptr, g.plane(), g.nz, L, T(coriol), T(ug), T(vg)));
     }
     if (!scalar_on) return;
+    // the buoyancy first: the scalar may advance with its right-hand side
+    if (buoyant()) {
+      Tag tag_(this, "scalar");
+      plane_means({F[LES_THETA]}, 0, L, means + 3 * L);
+      const bool w = momentum_advances();
+      KL("k_buoyancy", (w ? 6.0 : 3.0) * g.nz * g.plane() * sizeof(T),
+         launch_dep(k_buoyancy<T>, grid_for(g.field() / 4), 256, 0, st, F[LES_RHSZ], F[LES_THETA], means + 3 * L,
+                    g.plane(), g.nz, T(SP.buoyancy), w ? F[LES_W] : nullptr, F[LES_RHSZ_F], T(P.dt), T(adv.t1),
+                    T(adv.t2)));
+    }
     {
       Tag tag_(this, "scalar");
       // rhs_t_f = rhs_t (buffer exchange, as the momentum's)
-      T* const dst[2] = {lev(F[LES_RHS_T], 0), lev(F[LES_RHS_T], g.nz + 1)};
-      const T* const src[2] = {lev(F[LES_RHS_T_F], 0), lev(F[LES_RHS_T_F], g.nz + 1)};
-      plane_ops(2, dst, src, nullptr);
+      if (!from_spectra) {
+        T* const dst[2] = {lev(F[LES_RHS_T], 0), lev(F[LES_RHS_T], g.nz + 1)};
+        const T* const src[2] = {lev(F[LES_RHS_T_F], 0), lev(F[LES_RHS_T_F], g.nz + 1)};
+        plane_ops(2, dst, src, nullptr);
+      }
       std::swap(F[LES_RHS_T], F[LES_RHS_T_F]);
     }
     if (from_spectra) {
@@ -2345,13 +2391,6 @@ class Solver final : public SolverBase {
       scalar_convec();
       DivEq e{LES_RHS_T, LES_QX, LES_QY, LES_QZ, 1, 0.0};
       div_eqs(&e, 1, false, "scalar");
-    }
-    if (SP.buoyancy != 0.0) {
-      Tag tag_(this, "scalar");
-      plane_means({F[LES_THETA]}, 0, L, means + 3 * L);
-      KL("k_buoyancy", 3.0 * (g.nz - 1) * g.plane() * sizeof(T),
-         launch_dep(k_buoyancy<T>, grid_for((long)(g.nz - 1) * g.plane()), 256, 0, st, F[LES_RHSZ], F[LES_THETA], means + 3 * L,
-                                                                               g.plane(), g.nz, T(SP.buoyancy)));
     }
   }
 
@@ -2368,19 +2407,7 @@ class Solver final : public SolverBase {
     {
       Tag tag_(this, "convec");
       const int r[3] = {LES_RHSX, LES_RHSY, LES_RHSZ}, rf[3] = {LES_RHSX_F, LES_RHSY_F, LES_RHSZ_F};
-      if (from_spectra && padd()) {
-        // with the convective routine's own ghost values (convec_ghosts)
-        RhsGhosts<T> o;
-        for (int q = 0; q < 3; ++q) {
-          o.oldr[q] = F[r[q]];
-          o.newr[q] = F[rf[q]];
-        }
-        o.top = (long)(g.nz + 1) * g.plane();
-        o.val = T(BOGUS);
-        KL("k_rhs_ghosts", 18.0 * g.plane() * sizeof(T),
-           launch_dep(k_rhs_ghosts<T>, dim3(unsigned(std::min<long>(ceil_div(g.plane(), 256L), 148)), 6u), 256, 0, st,
-               o, g.plane()));
-      } else {
+      if (!(from_spectra && padd())) {  // (there the divergence writes them: div_products)
         T* dst[6];
         const T* src[6];
         for (int q = 0; q < 3; ++q) {
@@ -2409,13 +2436,15 @@ class Solver final : public SolverBase {
     rhs_extras(from_spectra);
   }
 
-  void ab2(double tadv1, double tadv2) override {
+  void ab2(double tadv1, double tadv2) override { advance(tadv1, tadv2, true, scalar_on); }
+  void advance(double tadv1, double tadv2, bool momentum, bool scalar) {
     Tag tag_(this, "ab2");
-    KL("k_ab2", 12.0 * g.nz * g.plane() * sizeof(T), launch_dep(k_ab2<T>, grid_for(g.field()), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
-                                                 F[LES_RHSZ], F[LES_RHSX_F], F[LES_RHSY_F], F[LES_RHSZ_F],
-                                                 g.plane(), g.nz, T(P.dt), T(tadv1), T(tadv2)));
-    if (scalar_on)
-    {
+    if (momentum)
+      KL("k_ab2", 12.0 * g.nz * g.plane() * sizeof(T),
+         launch_dep(k_ab2<T>, grid_for(g.field()), 256, 0, st, F[LES_U], F[LES_V], F[LES_W], F[LES_RHSX], F[LES_RHSY],
+                    F[LES_RHSZ], F[LES_RHSX_F], F[LES_RHSY_F], F[LES_RHSZ_F], g.plane(), g.nz, T(P.dt), T(tadv1),
+                    T(tadv2)));
+    if (scalar) {
       KL("k_ab2_scalar", 4.0 * g.nz * g.plane() * sizeof(T),
          launch_dep(k_ab2_scalar<T>, grid_for((long)g.nz * g.plane()), 256, 0, st,
              F[LES_THETA], F[LES_RHS_T], F[LES_RHS_T_F], g.plane(), g.nz, T(P.dt), T(tadv1), T(tadv2)));
@@ -2451,8 +2480,6 @@ class Solver final : public SolverBase {
     }
     lag_added = false;
     LES_CUDA(cudaEventRecord(ev[2], st));
-    rhs_adv(true);
-    LES_CUDA(cudaEventRecord(ev[3], st));
     double t1, t2;
     if (jtt == 1) {
       t1 = 1.0;
@@ -2461,7 +2488,20 @@ class Solver final : public SolverBase {
       t1 = 1.5;
       t2 = 1.0 - t1;
     }
-    ab2(t1, t2);
+    adv.on = true;
+    adv.t1 = t1;
+    adv.t2 = t2;
+    bool momentum;
+    try {
+      momentum = momentum_advances();
+      rhs_adv(true);
+    } catch (...) {
+      adv.on = false;
+      throw;
+    }
+    adv.on = false;
+    LES_CUDA(cudaEventRecord(ev[3], st));
+    if (!momentum) advance(t1, t2, true, false);
     // the reference's formulation (FP64 transforms of u* in mixed precision);
     // press_from_increment forms the same pressure in FP32 without the
     // cancellation, but its FP32 four-field y pass measured slower than the

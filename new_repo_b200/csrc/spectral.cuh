@@ -1425,6 +1425,7 @@ enum XIOp : int {
   XI_SCDYN = 5,  // 19 filtered fields of the dynamic Prandtl model -> K.X and X.X
 };
 
+enum : int { ADV_KEEP = 0, ADV_ZERO = 1, ADV_LID = 2 };
 template <typename T>
 struct XIArgs {
   int dep;         // launched by launch_dep: the tables are constant
@@ -1448,6 +1449,17 @@ struct XIArgs {
   const T* refin[MAXIN];  // per-level values added back to input field f
   int lo_ref, hi_ref;     // combining ops: on these levels
   int fresh;              // XI_DIV: the input is the whole horizontal part, out is not read
+  // XI_DIV inside a time step: equation q's variable adv_v[q] (nullptr: not
+  // here) advances by dt (t1 rhs + t2 adv_f[q]); its levels 0 and nz + 1 stay
+  // (ADV_KEEP), become zero (ADV_ZERO) or zero and level nz plus adv_top
+  // (ADV_LID).  adv_ghosts: the ghost levels of the right-hand sides as their
+  // buffers change roles: adv_f takes out's, and out takes BOGUS (2) or keeps
+  // its own (1).
+  T* adv_v[3];
+  T* adv_f[3];
+  int adv_lid[3];
+  int adv_ghosts;
+  double adv_dt, adv_t1, adv_t2, adv_top;
   T* out[16];
   float* outf[16];  // FP32 outputs of an FP64 transform (out_f32 = 1, XI_STORE)
   int out_f32;
@@ -1864,42 +1876,52 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     // compute_derivatives.f90:544-574 + LES_engine.f90:546-551, one equation
     // per input (up to three): out[q] = rhs, aux[q] = tz, lo[q] = stag, pf[q]
     // = forcing; out[8]/out[9] = bottom/top pressure-BC layers of the
-    // non-staggered (w) equation.  c0 = 1/dz.  Four consecutive points per
-    // thread; the tz values of every equation are loaded before the first
-    // right-hand side is stored (read-only path: nothing here writes them).
+    // non-staggered (w) equation.  c0 = 1/dz.  Four consecutive points of one
+    // equation per thread, everything it reads requested before its first
+    // store (all equations of a point per thread spilled 70-240 bytes).
     using V = V4<T>;
     const T rdz = T(a.c0);
     const long pl = a.out_pstride;
-    for (int idx = threadIdx.x; idx < a.R * (NX / 4); idx += blockDim.x) {
-      const int r = idx / (NX / 4);
-      const int i0 = 4 * (idx - r * (NX / 4));
+    for (int idx = threadIdx.x; idx < nseq * (NX / 4); idx += blockDim.x) {
+      const int s = idx / (NX / 4);
+      const int i0 = 4 * (idx - s * (NX / 4));
+      const int r = udiv32(s, a.nin), q = s - r * a.nin;
       const int l = rowl[r];
       if (l < 0) continue;
       const long p2 = (long)rowj[r] * NX + i0;
       const long off = (long)l * pl + p2;
-      const T* x = xs + (long)(r * a.nin) * XS + i0;
-      const bool in = l >= 1 && l <= a.nz;
-      V dzq[3];
-      if (in) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-          if (q < a.nin) {
-            const T* tz = a.aux[q];
-            dzq[q] = a.lo[q] ? rdz * (vldg<V>(tz, off + pl) - vldg<V>(tz, off))   // ddz_w
-                             : rdz * (vldg<V>(tz, off) - vldg<V>(tz, off - pl));  // ddz_uv
-          }
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        if (q >= a.nin) break;
-        V xq = vld<V>(x, (long)q * XS);
-        if (a.refin[q] && l >= a.lo_ref && l <= a.hi_ref) xq = xq + vsplat<V>(a.refin[q][l]);
-        if (in) {
-          const V base = a.fresh ? xq : vld<V>(a.out[q], off) + xq;
-          vst(a.out[q] + off, (base + dzq[q]) + vsplat<V>(T(a.pf[q])));
-          if (!a.lo[q] && l == 1 && a.out[8]) vst(a.out[8] + p2, xq + dzq[q]);
+      T* out = a.out[q];
+      T* u = a.adv_v[q];
+      V xq = vld<V>(xs, (long)s * XS + i0);
+      if (l >= 1 && l <= a.nz) {
+        const T* tz = a.aux[q];
+        const V t0 = vldg<V>(tz, off), t1 = vldg<V>(tz, a.lo[q] ? off + pl : off - pl);
+        V uo = vsplat<V>(T(0)), fo = uo;
+        if (u) {
+          uo = vld<V>(u, off);
+          fo = vld<V>(a.adv_f[q], off);
         }
+        if (a.refin[q] && l >= a.lo_ref && l <= a.hi_ref) xq = xq + vsplat<V>(a.refin[q][l]);
+        const V dzq = rdz * (a.lo[q] ? t1 - t0 : t0 - t1);  // ddz_w, ddz_uv
+        const V base = a.fresh ? xq : vld<V>(out, off) + xq;
+        const V rhs = (base + dzq) + vsplat<V>(T(a.pf[q]));
+        vst(out + off, rhs);
+        if (u) {
+          const V un = uo + T(a.adv_dt) * (T(a.adv_t1) * rhs + T(a.adv_t2) * fo);
+          vst(u + off, un);
+          if (a.adv_lid[q] == ADV_LID && l == a.nz) vst(u + off + pl, un + vsplat<V>(T(a.adv_top)));
+          if (a.adv_lid[q] != ADV_KEEP && l == 1) vst(u + p2, vsplat<V>(T(0)));
+        }
+        if (!a.lo[q] && l == 1 && a.out[8]) vst(a.out[8] + p2, xq + dzq);
+      } else {
+        if (a.refin[q] && l >= a.lo_ref && l <= a.hi_ref) xq = xq + vsplat<V>(a.refin[q][l]);
         if (!a.lo[q] && l == a.nz + 1 && a.out[9]) vst(a.out[9] + p2, xq);
+        if (u && a.adv_lid[q] == ADV_ZERO && l == a.nz + 1) vst(u + off, vsplat<V>(T(0)));
+      }
+      if (a.adv_ghosts && (l == 1 || l == a.nz + 1)) {
+        const long gh = l == 1 ? p2 : off;
+        vst(a.adv_f[q] + gh, vld<V>(out, gh));
+        if (a.adv_ghosts == 2) vst(out + gh, vsplat<V>(T(BOGUS)));
       }
     }
   }
