@@ -602,11 +602,14 @@ __device__ __forceinline__ void xr_issue(const XFArgs<T>& a, long item, cplx<T>*
     const long g = item * a.R + r;
     return xr_source<T, S>(a, f, a.plane0 + udiv32(g, a.rows_pp), umod32(g, a.rows_pp));
   };
-  unsigned mine = 0;
-  for (int s = lane; s < nrow; s += 32)
-    if (source(s)) mine += RB;
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if (lane == 0) mbar_expect_tx(mbar, mine);
+  unsigned bytes = nrow * RB;
+  if (a.op == XF_PRESS) {  // some have no source
+    bytes = 0;
+    for (int s = lane; s < nrow; s += 32)
+      if (source(s)) bytes += RB;
+    for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
+  }
+  if (lane == 0) mbar_expect_tx(mbar, bytes);
   __syncwarp();
   tc::fence_async_smem();  // earlier generic accesses of this stage come first
   for (int s = lane; s < nrow; s += 32) {
@@ -1435,6 +1438,7 @@ struct XIArgs {
   int plane0;
   int nk;          // modes present in the input rows (rest zero)
   int ipitch;      // complex values between input rows (>= nk; 0: nk)
+  int nkc;         // values of a row that are copied: nk, in FP32 rounded up to whole 16 bytes where the pitch allows (set by the launcher)
   int nks;         // complex values between staged rows in shared memory (set by the launcher)
   int stage_rows;  // staged rows per stage (set by the launcher)
   int nbuf;        // input stages (set by the launcher): 2 = the next item's rows load during this one
@@ -1525,46 +1529,32 @@ __device__ __forceinline__ void xi_issue(const XIArgs<T>& a, long item, cplx<T>*
   }
 }
 
-// the same with bulk copies, issued by warp 0: lane 0 announces the bytes
-// of every valid row's aligned part, then each lane copies whole rows; a
-// row whose addresses are not 16-byte aligned (none when the launcher set
-// a.bulk) and the last value of an odd FP32 row go by plain loads and stores
-// (visible after the barrier that follows the wait)
+// the same with bulk copies, issued by warp 0 (the other warps wait for what it
+// issues, so nothing is looked at twice): lane 0 announces the bytes of every
+// valid row's whole 16-byte parts, then each lane copies whole rows (their
+// addresses are 16-byte aligned: a.bulk); the last value of an odd FP32 row
+// without one to spare goes by a plain load and store (visible after the
+// barrier that follows the wait)
 template <typename T>
 __device__ __forceinline__ void xi_issue_bulk(const XIArgs<T>& a, long item, cplx<T>* stage, uint64_t* mbar) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   const int ns = a.nstage ? a.nstage : a.nin;
   const long rows_left = a.nrows - item * a.R;
-  const int nvalid = int(rows_left < a.R ? rows_left : a.R);
-  const unsigned rb = unsigned(a.nk * sizeof(cplx<T>));
+  const int nrow = int(rows_left < a.R ? rows_left : a.R) * ns;
+  const unsigned rb = unsigned(a.nkc * sizeof(cplx<T>));
   const unsigned rbulk = rb & ~15u;
-  auto aligned = [&](int s) {
-    const int r = udiv32(s, ns), f = s - r * ns;
-    const cplx<T>* row = xi_row(a, f, item * a.R + r);
-    const cplx<T>* dst = stage + (long)s * a.nks;
-    return ((reinterpret_cast<uintptr_t>(row) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-  };
-  const int nrow = nvalid * ns;
-  unsigned mine = 0;
-  for (int s = lane; s < nrow; s += 32)
-    if (rbulk && aligned(s)) mine += rbulk;
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
   // the barrier's one arrival carries every byte the copies below bring (an
   // item always has a valid row, so the phase completes)
-  if (lane == 0) mbar_expect_tx(mbar, mine);
+  if (lane == 0) mbar_expect_tx(mbar, nrow * rbulk);
   __syncwarp();
   tc::fence_async_smem();  // earlier generic reads of this stage come first
   for (int s = lane; s < nrow; s += 32) {
     const int r = udiv32(s, ns), f = s - r * ns;
     const cplx<T>* row = xi_row(a, f, item * a.R + r);
     cplx<T>* dst = stage + (long)s * a.nks;
-    int m0 = 0;
-    if (rbulk && aligned(s)) {
-      bulk_g2s(dst, row, rbulk, mbar);
-      m0 = int(rbulk / sizeof(cplx<T>));
-    }
-    for (int m = m0; m < a.nk; ++m) dst[m] = row[m];
+    bulk_g2s(dst, row, rbulk, mbar);
+    if (rb != rbulk) dst[a.nkc - 1] = row[a.nkc - 1];
   }
 }
 

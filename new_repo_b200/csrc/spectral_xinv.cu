@@ -47,8 +47,12 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
     // lanes, the TL lanes of 32 / TL sequences per warp in different rows;
     // a stride of TL (mod the values per wavefront) puts those rows on
     // disjoint banks, as slot_stride does for the sequence slots
+    // (an odd FP32 row is copied with one value more, whole 16 bytes: its
+    // last value alone went by a load in front of every batch, and where the
+    // stride then was odd the rows went without bulk copies)
     const int W = 128 / int(sizeof(cplx<T>)), TL = lanes(M);
-    a.nks = a.nk;
+    a.nkc = (a.nk * sizeof(cplx<T>)) % 16 != 0 && a.ipitch > a.nk ? a.nk + 1 : a.nk;
+    a.nks = TL < W ? a.nk : a.nkc;
     if (TL < W) a.nks += ((TL % W - a.nk % W) % W + W) % W;
   }
   // a plain store with one staged row per sequence transforms each sequence
@@ -61,15 +65,16 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
     return a.merged ? R * (ns - a.nin) + pad_seqs(R * a.nin, M) : R * ns;
   };
   // bulk staging: one cp.async.bulk per staged row needs 16-byte aligned
-  // rows in global memory (pitch and plane stride) and in the stages (stage
-  // base and row stride); the kernel checks every row's addresses again and
-  // copies a row that fails with plain loads
+  // rows in global memory (base, pitch and plane stride) and in the stages
+  // (stage base and row stride)
   {
     const size_t cs = sizeof(cplx<T>);
     a.bulk = ((cs * a.ipitch) % 16 == 0 && (cs * a.in_pstride) % 16 == 0 && (cs * a.nks) % 16 == 0 &&
               (cs * (NX + twm_len(M, true))) % 16 == 0 && a.nk * cs >= 16)
                  ? 1
                  : 0;
+    for (int f = 0; f < ns; ++f)
+      if (reinterpret_cast<uintptr_t>(a.in[f]) % 16 != 0) a.bulk = 0;
   }
   auto smem_nb = [&](int R, int nb) {
     return sizeof(cplx<T>) * (NX + twm_len(M, true) + nb * (((size_t)stage_rows(R) * a.nks + 1) & ~size_t(1)) +
