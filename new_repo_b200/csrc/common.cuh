@@ -46,6 +46,22 @@ __device__ __forceinline__ cplx<T> ik_mul(T k, cplx<T> a) {
 __device__ __forceinline__ int udiv32(long n, long d) { return int(unsigned(n) / unsigned(d)); }
 __device__ __forceinline__ int umod32(long n, long d) { return int(unsigned(n) % unsigned(d)); }
 
+// n / d for 0 <= n < 2^31 and a divisor that the host knows, by the multiply,
+// add and shift of Granlund and Montgomery (PLDI 1994): a division by a
+// run-time divisor is some twenty dependent instructions, and the spectral
+// passes do several in a row where a block's other warps wait for the result.
+struct FastDiv {
+  unsigned m, s;
+  __device__ __forceinline__ int operator()(long n) const { return int((__umulhi(unsigned(n), m) + unsigned(n)) >> s); }
+};
+inline FastDiv fast_div(long d) {
+  FastDiv f;
+  f.s = 0;
+  while ((1l << f.s) < d) ++f.s;
+  f.m = unsigned(((1ull << 32) * ((1ull << f.s) - (unsigned long long)d)) / (unsigned long long)d + 1);
+  return f;
+}
+
 // Device status bits (read back by les_get_status).
 enum StatusBits : unsigned {
   ST_NAN = 1u << 0,          // NaN in the velocity (LES_engine.f90:583-616)

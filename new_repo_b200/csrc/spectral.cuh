@@ -117,6 +117,7 @@ enum XFOp : int {
 
 template <typename T>
 struct XFArgs {
+  FastDiv d_rows, d_nf, d_ns;  // division by rows_pp, nf, nsrc (set by the launcher)
   int dep;         // launched by launch_dep: the tables are constant
   int op, nf, R;
   int lfast;       // k_xfwd: a CTA's rows are one row of R consecutive levels
@@ -473,16 +474,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   twm_build<T, M, false, 2>(a.tw, twm, threadIdx.x, blockDim.x);
   // rows of this CTA: consecutive rows of the grid, or (lfast) one row of R
   // consecutive levels
-  const int nlev = udiv32(a.nrows, a.rows_pp);
+  const int nlev = a.d_rows(a.nrows);
   for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
     int q, j;  // level index and row
     if (a.lfast) {
-      q = udiv32(blockIdx.x, a.rows_pp) * a.R + r;
-      j = umod32(blockIdx.x, a.rows_pp);
+      q = a.d_rows(blockIdx.x);
+      j = blockIdx.x - q * a.rows_pp;
+      q = q * a.R + r;
     } else {
       const long g = (long)blockIdx.x * a.R + r;
-      q = udiv32(g, a.rows_pp);
-      j = umod32(g, a.rows_pp);
+      q = a.d_rows(g);
+      j = int(g) - q * a.rows_pp;
     }
     rowl[r] = q < nlev ? a.plane0 + q : -1;
     rowj[r] = q < nlev ? j : 0;
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
       for (int r = 0; r < RO; ++r) seq[lane_t + TL * g + r * (M / RO)] = v[g * RO + r];
     __syncwarp();
     if (s < nseq) {
-      const int r = udiv32(s, a.nf);
+      const int r = a.d_nf(s);
       const int f = s - r * a.nf;
       const int l = rowl[r];
       if (l >= 0) {
@@ -598,9 +600,9 @@ __device__ __forceinline__ void xr_issue(const XFArgs<T>& a, long item, cplx<T>*
   const int nrow = int(left < a.R ? left : a.R) * ns;
   constexpr unsigned RB = NX * sizeof(S);
   auto source = [&](int s) {
-    const int r = udiv32(s, ns), f = s - r * ns;
-    const long g = item * a.R + r;
-    return xr_source<T, S>(a, f, a.plane0 + udiv32(g, a.rows_pp), umod32(g, a.rows_pp));
+    const int r = a.d_ns(s), f = s - r * ns;
+    const int g = int(item) * a.R + r, q = a.d_rows(g);
+    return xr_source<T, S>(a, f, a.plane0 + q, g - q * a.rows_pp);
   };
   unsigned bytes = nrow * RB;
   if (a.op == XF_PRESS) {  // some have no source
@@ -673,10 +675,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
   // the reference of row r, field f of a batch (one per thread; R nf <= 256)
   auto ref_of = [&](long item) -> T {
     if (!a.use_ref || item >= nitems || threadIdx.x >= nseq) return T(0);
-    const int r = udiv32(threadIdx.x, a.nf), f = threadIdx.x - r * a.nf;
+    const int r = a.d_nf(threadIdx.x), f = threadIdx.x - r * a.nf;
     const long g = item * a.R + r;
     if (g >= a.nrows || !a.refout[f]) return T(0);
-    return T(a.c0) * a.in[f][(long)(a.plane0 + udiv32(g, a.rows_pp)) * a.in_pstride];
+    return T(a.c0) * a.in[f][(long)(a.plane0 + a.d_rows(g)) * a.in_pstride];
   };
   T ref_next = ref_of(blockIdx.x);
   __syncthreads();
@@ -687,17 +689,19 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
     cplx<T>* stage = stg ? stage1 : stage0;
     if (a.nbuf > 1 && next < nitems) xr_issue<T, S, NX, SL>(a, next, stg ? stage0 : stage1, &bars[stg ^ 1]);
     const long g0 = item * a.R;
-    for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
+    for (int r = blockDim.x - 1 - threadIdx.x; r < a.R; r += blockDim.x) {  // (not warp 0, which issues)
       const long g = g0 + r;
-      rowl[r] = (g < a.nrows) ? a.plane0 + udiv32(g, a.rows_pp) : -1;
-      rowj[r] = (g < a.nrows) ? umod32(g, a.rows_pp) : 0;
+      const int q = a.d_rows(g);
+      rowl[r] = (g < a.nrows) ? a.plane0 + q : -1;
+      rowj[r] = (g < a.nrows) ? int(g) - q * a.rows_pp : 0;
     }
     if (a.use_ref && threadIdx.x < nseq) {
-      const int r = udiv32(threadIdx.x, a.nf), f = threadIdx.x - r * a.nf;
+      const int r = a.d_nf(threadIdx.x), f = threadIdx.x - r * a.nf;
       const long g = g0 + r;
+      const int q = a.d_rows(g);
       refs[threadIdx.x] = ref_next;
-      if (g < a.nrows && a.refout[f] && umod32(g, a.rows_pp) == 0)
-        a.refout[f][a.plane0 + udiv32(g, a.rows_pp)] = T(double(ref_next) * a.ref_mul);
+      if (g < a.nrows && a.refout[f] && int(g) == q * a.rows_pp)
+        a.refout[f][a.plane0 + q] = T(double(ref_next) * a.ref_mul);
     }
     ref_next = ref_of(next);
     const bool late = !tc::mbar_wait(&bars[stg], (phase >> stg) & 1u);
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfwd_row(const 
       const int s = base + threadIdx.x / TL;
       if (base + (threadIdx.x / 32) * (32 / TL) >= npad) break;  // whole warp beyond the slots
       const bool valid = s < nseq;
-      const int r = valid ? udiv32(s, a.nf) : 0;
+      const int r = valid ? a.d_nf(s) : 0;
       const int f = valid ? s - r * a.nf : 0;
       const int l = valid ? rowl[r] : -1;
       // slots past the last sequence follow the staged rows
@@ -831,6 +835,7 @@ enum YPOp : int {
 
 template <typename T>
 struct YPArgs {
+  FastDiv d_ncb, d_np;  // division by the column blocks, nplanes (set by the launcher)
   int dep;         // launched by launch_dep: the tables are constant
   int op, nin, nout, C, lc;  // C = 1 << lc columns per CTA
   int SI;                    // column stride of the shared stages (>= both lengths' slots)
@@ -913,9 +918,9 @@ __device__ __forceinline__ cplx<T> yp_op_c(const YPArgs<T>& a, int q, int kx, in
 template <typename T, int NY>
 __device__ __forceinline__ void yp_issue(const YPArgs<T>& a, long item, int ncb, cplx<T>* bin) {
   const int C = a.C, SI = a.SI;
-  const int col0 = umod32(item, ncb) * C;
-  const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
-  const int grp = udiv32(item, (long)ncb * a.nplanes);
+  const int pq = a.d_ncb(item), grp = a.d_np(pq);
+  const int col0 = (int(item) - pq * ncb) * C;
+  const int l = a.plane0 + pq - grp * a.nplanes;
   // thread -> fixed column c, rows ky0 + TL i: the CTA has C x TL threads,
   // so every thread copies NY / TL rows at a compile-time count and the
   // addresses advance by constant strides (an unrolled loop)
@@ -994,9 +999,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
     cp_async_wait<0>();
   }
   __syncthreads();
-  const int col0 = umod32(item, ncb) * C;
-  const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
-  const int grp = udiv32(item, (long)ncb * a.nplanes);
+  const int pq = a.d_ncb(item), grp = a.d_np(pq);
+  const int col0 = (int(item) - pq * ncb) * C;
+  const int l = a.plane0 + pq - grp * a.nplanes;
   const int c = threadIdx.x / TL;
   const int lt = threadIdx.x % TL;
   const int kx = col0 + c;
@@ -1221,6 +1226,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
 // stresses (i kx t_x + i ky t_y), their sum, and one inverse transform.
 template <typename T>
 struct YRArgs {
+  FastDiv d_ncb, d_np;  // division by the column blocks, nplanes (set by the launcher)
   int dep;         // launched by launch_dep: the tables are constant
   int C, lc, SI;       // C = 1 << lc columns per CTA, column stride of a shared slot
   int nslot;           // shared slots (set by the launcher): 2 = a copy runs under every transform
@@ -1294,9 +1300,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   // input `in` (0 products, 1 t_x, 2 t_y) of item `item` into ring slot `sl`
   auto issue = [&](long item, int in, int sl) {
     if (item < nitems) {
-      const int col0 = umod32(item, ncb) * C;
-      const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
-      const int grp = udiv32(item, (long)ncb * a.nplanes);
+      const int pq = a.d_ncb(item), grp = a.d_np(pq);
+      const int col0 = (int(item) - pq * ncb) * C;
+      const int l = a.plane0 + pq - grp * a.nplanes;
       cplx<T>* slot = ring + sl * C * SI;
       if (in == 0)
         yr_copy<T, NF, TL>(a, a.p[grp], (long)l * a.pstride, a.ppitch, col0, l <= a.lp ? a.nkp : 0, slot);
@@ -1328,7 +1334,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   const int lt = threadIdx.x % TL;
   int sl = 0;  // slot of the current input
   for (long item = blockIdx.x; item < nitems; item += gridDim.x, sl ^= flip) {
-    const int col0 = umod32(item, ncb) * C;
+    const int pq = a.d_ncb(item), grp = a.d_np(pq);
+    const int col0 = (int(item) - pq * ncb) * C;
     const int kx = col0 + c;
     const bool live = kx < a.ncols && kx != a.nxh;
     cplx<T> w[E];  // the sum, forward output layout of N (groups FO)
@@ -1399,8 +1406,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
 #pragma unroll
         for (int r = 0; r < IO; ++r) seq[lt + TL * g + r * (N / IO)] = w[g * IO + r];
       __syncthreads();
-      const int l = a.plane0 + umod32(udiv32(item, ncb), a.nplanes);
-      const int grp = udiv32(item, (long)ncb * a.nplanes);
+      const int l = a.plane0 + pq - grp * a.nplanes;
       const int cc = threadIdx.x & (C - 1);
       const int kxx = col0 + cc;
       if (kxx < a.ncols) {
@@ -1431,6 +1437,7 @@ enum XIOp : int {
 enum : int { ADV_KEEP = 0, ADV_ZERO = 1, ADV_LID = 2 };
 template <typename T>
 struct XIArgs {
+  FastDiv d_rows, d_ns, d_nin, d_nk;  // division by rows_pp, the staged rows per grid row, nin, nk (set by the launcher)
   int dep;         // launched by launch_dep: the tables are constant
   int op, nin, R;
   long nrows;
@@ -1504,8 +1511,8 @@ __device__ __forceinline__ int xi_plane(const XIArgs<T>& a, int f, int l) {
 }
 template <typename T>
 __device__ __forceinline__ const cplx<T>* xi_row(const XIArgs<T>& a, int f, long g) {
-  const int l = a.plane0 + udiv32(g, a.rows_pp);
-  return a.in[f] + (long)xi_plane(a, f, l) * a.in_pstride + long(umod32(g, a.rows_pp)) * a.ipitch;
+  const int q = a.d_rows(g), j = int(g) - q * a.rows_pp;
+  return a.in[f] + (long)xi_plane(a, f, a.plane0 + q) * a.in_pstride + (long)j * a.ipitch;
 }
 
 // x inverse pass: start the copies of the spectral rows of batch `item`
@@ -1518,7 +1525,7 @@ __device__ __forceinline__ void xi_issue(const XIArgs<T>& a, long item, cplx<T>*
   const int ns = a.nstage ? a.nstage : a.nin;
   const int nrow = a.R * ns;
   for (int s = warp; s < nrow; s += nwarps) {
-    const int r = s / ns;
+    const int r = a.d_ns(s);
     const int f = s - r * ns;
     const long g = item * a.R + r;
     const bool valid = g < a.nrows;
@@ -1550,7 +1557,7 @@ __device__ __forceinline__ void xi_issue_bulk(const XIArgs<T>& a, long item, cpl
   __syncwarp();
   tc::fence_async_smem();  // earlier generic reads of this stage come first
   for (int s = lane; s < nrow; s += 32) {
-    const int r = udiv32(s, ns), f = s - r * ns;
+    const int r = a.d_ns(s), f = s - r * ns;
     const cplx<T>* row = xi_row(a, f, item * a.R + r);
     cplx<T>* dst = stage + (long)s * a.nks;
     bulk_g2s(dst, row, rbulk, mbar);
@@ -1647,10 +1654,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     cp_async_wait<0>();
   }
   const long g0 = item * a.R;
-  for (int r = threadIdx.x; r < a.R; r += blockDim.x) {
+  for (int r = blockDim.x - 1 - threadIdx.x; r < a.R; r += blockDim.x) {  // (not warp 0, which issues)
     const long g = g0 + r;
-    rowl[r] = (g < a.nrows) ? a.plane0 + udiv32(g, a.rows_pp) : -1;
-    rowj[r] = (g < a.nrows) ? umod32(g, a.rows_pp) : 0;
+    const int q = a.d_rows(g);
+    rowl[r] = (g < a.nrows) ? a.plane0 + q : -1;
+    rowj[r] = (g < a.nrows) ? int(g) - q * a.rows_pp : 0;
   }
   if (__syncthreads_or(late)) {
     // the copies did not complete within the limit: record it, give the
@@ -1671,7 +1679,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     cplx<T>* rows = const_cast<cplx<T>*>(stage);
     const T rdz = T(a.c0);
     for (int idx = threadIdx.x; idx < a.R * a.nk; idx += blockDim.x) {
-      const int r = udiv32(idx, a.nk);
+      const int r = a.d_nk(idx);
       const int m = idx - r * a.nk;
       const int l = rowl[r];
       if (l < 0) continue;
@@ -1690,7 +1698,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     cplx<T>* rows = const_cast<cplx<T>*>(stage);
     const T rdz = T(a.c0);
     for (int idx = threadIdx.x; idx < a.R * a.nk; idx += blockDim.x) {
-      const int r = udiv32(idx, a.nk);
+      const int r = a.d_nk(idx);
       const int m = idx - r * a.nk;
       const int l = rowl[r];
       if (l < 0) continue;
@@ -1717,7 +1725,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
   for (int base = 0; base < npad; base += blockDim.x / TL) {
     const int s = base + threadIdx.x / TL;
     if (base + (threadIdx.x / 32) * (32 / TL) >= npad) break;  // whole warp beyond the slots
-    const int r = udiv32(s, a.nin);
+    const int r = a.d_nin(s);
     const int f = s - r * a.nin;
     const bool valid = (s < nseq) && (rowl[r < a.R ? r : 0] >= 0);
     int l = 0, j = 0;
@@ -1875,7 +1883,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     for (int idx = threadIdx.x; idx < nseq * (NX / 4); idx += blockDim.x) {
       const int s = idx / (NX / 4);
       const int i0 = 4 * (idx - s * (NX / 4));
-      const int r = udiv32(s, a.nin), q = s - r * a.nin;
+      const int r = a.d_nin(s), q = s - r * a.nin;
       const int l = rowl[r];
       if (l < 0) continue;
       const long p2 = (long)rowj[r] * NX + i0;

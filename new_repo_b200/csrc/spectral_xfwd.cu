@@ -1,4 +1,4 @@
-// Instantiation and launch of the x forward passes (k_xfwd, k_xfwd_st) for
+// Instantiation and launch of the x forward passes (k_xfwd, k_xfwd_row) for
 // every supported transform length.
 #include "spectral_launch.cuh"
 
@@ -12,6 +12,7 @@ static void launch_xfwd_row(int NX, XFArgs<T>& a, cudaStream_t st) {
   const int M = NX / 2;
   const int SL = slot_stride(M, int(sizeof(cplx<T>)));
   a.nsrc = a.op == XF_PRESS ? 4 : a.nf;
+  a.d_ns = fast_div(a.nsrc);
   auto stage_rows = [&](int R) { return R * (a.nsrc - a.nf) + pad_seqs(R * a.nf, M); };
   auto smem_nb = [&](int R, int nb) {
     return sizeof(cplx<T>) * (NX + twm_len(M, false) + (size_t)nb * stage_rows(R) * SL) + 2 * sizeof(uint64_t) +
@@ -48,6 +49,8 @@ template <typename T>
 void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   const int M = NX / 2;
   if (a.opitch == 0) a.opitch = a.nk;
+  a.d_rows = fast_div(a.rows_pp);
+  a.d_nf = fast_div(a.nf);
   a.in_rstride = NX;
   const bool press = a.op == XF_PRESS;
   static const int nin_of_op[] = {0, 9, 6, 10, 3, 6, 14, 9};

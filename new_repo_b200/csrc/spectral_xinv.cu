@@ -42,6 +42,10 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   // and stages from best_rows below
   const int SL = slot_stride(M, int(sizeof(cplx<T>)));
   const int ns = a.nstage ? a.nstage : a.nin;  // staged rows per grid row
+  a.d_rows = fast_div(a.rows_pp);
+  a.d_ns = fast_div(ns);
+  a.d_nin = fast_div(a.nin);
+  a.d_nk = fast_div(a.nk);
   {
     // staged row stride: the split reads a row's modes at consecutive
     // lanes, the TL lanes of 32 / TL sequences per warp in different rows;

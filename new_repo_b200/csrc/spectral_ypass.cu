@@ -99,6 +99,8 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
   const int threads = a.C * TL;
   a.nplanes = nplanes;
   a.ngroups = ngroups;
+  a.d_ncb = fast_div(ceil_div(a.ncols, a.C));
+  a.d_np = fast_div(nplanes);
   const long nitems = (long)ceil_div(a.ncols, a.C) * nplanes * ngroups;
   if (nitems == 0) return;
   // persistent grid: the CTAs that fit on the device at once
@@ -171,6 +173,8 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
   if (items(lc) == 0) return;
   const int threads = a.C * TL;
   const int grid = int(std::min<long>(items(lc), (long)resident_ctas((const void*)kern, threads, smem)));
+  a.d_ncb = fast_div(ceil_div(a.ncols, a.C));
+  a.d_np = fast_div(a.nplanes);
   hook_before("yrhs", double(a.nplanes) * a.ngroups * sizeof(cplx<T>) *
                           (double(a.nkp) * NF + 2.0 * a.ncols * N + double(a.ncols) * N));
   if (a.dep) launch_dep(kern, grid, threads, smem, st, a);
