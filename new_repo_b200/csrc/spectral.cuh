@@ -1741,7 +1741,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     // imaginary parts of the DC and Nyquist bins ignored
     cplx<T> v[E];
     const int fs = a.nstage ? a.src[f] : f;
-    const bool dxf = a.nstage && a.dx[f];
+    const bool dxf = CLS == XC_STORE && a.nstage && a.dx[f];
     const cplx<T>* row = valid ? stage + (long)(r * ns + fs) * a.nks : nullptr;  // the staged spectral row
     // The per-sequence choices (d/dx, whether every mode below M is present)
     // are made once here, not inside the unrolled element loop: with nk >= M
@@ -1781,8 +1781,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         }
     };
     if constexpr (sizeof(T) == 8) {
-      // FP64: one generic loop (the specialised copies cost the double
-      // precision kernels register spills at their 128-register budget)
+      // FP64: one generic loop (the specialised copies spill at the
+      // 128-register budget: 256^3 gradients 511 -> 603 us)
 #pragma unroll
       for (int gg = 0; gg < E / RI; ++gg)
 #pragma unroll
