@@ -899,25 +899,21 @@ class Solver final : public SolverBase {
       if (std::fclose(f) != 0) throw CudaError(22, "cannot write statistics file " + base + "_info.txt");
       stat_iterations = 0;
     }
-    KL("k_plane_accum", 20.0 * plane,
-       launch_dep(k_plane_accum<T>, grid_for(plane), 256, 0, st, PL[LES_U_STAR_AVG], stat_ustar, plane));
-    if (write) {
-      const auto h = to_host(stat_ustar, plane);
-      write_host(base + "_2D.dat", {h.data()}, plane);
-      LES_CUDA(cudaMemsetAsync(stat_ustar, 0, plane * sizeof(double), st));
-    }
     StatFields<T> sf{F[LES_U],   F[LES_V],   F[LES_W],   F[LES_P],    F[LES_TXX],  F[LES_TYY], F[LES_TZZ],
                      F[LES_TXY], F[LES_TXZ], F[LES_TYZ], F[LES_DUDZ], F[LES_DVDZ], F[LES_NU_T], F[LES_CS_OPT2]};
     KL("k_stat_accum", double(n) * (16.0 * STAT_NQ + 16.0 * sizeof(T)),
-       launch_dep(k_stat_accum<T>, grid_for(n), 256, 0, st, sf, stat_acc, plane, g.nz));
+       launch_dep(k_stat_accum<T>, grid_for(n), 256, 0, st, sf, stat_acc, plane, g.nz, PL[LES_U_STAR_AVG],
+                  stat_ustar));
     if (write) {
+      const auto h2 = to_host(stat_ustar, plane);
+      write_host(base + "_2D.dat", {h2.data()}, plane);
+      LES_CUDA(cudaMemsetAsync(stat_ustar, 0, plane * sizeof(double), st));
       const auto h = to_host(stat_acc, STAT_NQ * n);
       std::vector<const double*> parts;
       for (int q = 0; q < STAT_NQ; ++q) parts.push_back(h.data() + q * n);
       write_host(base + "_3D.dat", parts, n);
       LES_CUDA(cudaMemsetAsync(stat_acc, 0, STAT_NQ * n * sizeof(double), st));
     }
-    LES_CUDA(cudaStreamSynchronize(st));
   }
   void stat_sums(int index, double* out) override {
     if (!stat_acc) throw CudaError(1, "running statistics are not initialised (les_stat_init)");
@@ -973,10 +969,7 @@ class Solver final : public SolverBase {
                     F[LES_CS_OPT2], tke_f[0], tke_f[1], tke_f[2]};
     const dim3 grid(tke_nch, g.nz);
     const double idz = 1.0 / dz(), bytes = 26.0 * g.nz * plane * sizeof(T);
-    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 0, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 16, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 32, 16>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
-    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T, 48, 13>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
+    KL("k_tke_partial", bytes, launch_dep(k_tke_partial<T>, grid, 256, 0, st, tf, tke_part, plane, P.wall_law, idz));
     KL("k_tke_final", 8.0 * g.nz * tke_nch * TKE_NQ,
        launch_dep(k_tke_final, grid_for((long)g.nz * TKE_NQ), 256, 0, st, tke_part, tke_nch, g.nz,
                                                                  double(g.nx) * double(g.ny), tke_avar));
@@ -999,7 +992,6 @@ class Solver final : public SolverBase {
       LES_CUDA(cudaMemsetAsync(tke_avar, 0, (long)TKE_NQ * g.nz * sizeof(double), st));
       ++tke_ii;
     }
-    LES_CUDA(cudaStreamSynchronize(st));
   }
   void tke_sums(double* out, int* record) override {
     if (!tke_avar) throw CudaError(1, "TKE budget is not initialised (les_tke_init)");

@@ -22,16 +22,28 @@ struct StatFields {
 // Each product is rounded on its own (no fused multiply-add), so that the FP64
 // sums equal those of the reference's expression order: x**3 = (x*x)*x,
 // x**4 = (x*x)*(x*x).  uw and vw interpolate u, v to the w node; their
-// first level is reset to zero on every call (:378-384).
+// first level is reset to zero on every call (:378-384).  A point's 26 sums
+// are all requested before the first is stored (added one by one, each load
+// waited behind the store in front of it: 128 x 64 x 41 FP64 82 us, so
+// 31); the running sum of the friction-velocity plane
+// (io_2D_stat_averages :316-320) goes with the first level.
 template <typename T>
-__global__ void __launch_bounds__(256) k_stat_accum(StatFields<T> f, double* __restrict__ acc, long plane, int nz) {
+__global__ void __launch_bounds__(256, 2) k_stat_accum(StatFields<T> f, double* acc, long plane, int nz,
+                                                       const T* ustar, double* ustar_acc) {
   dep_wait();
   const long n = (long)nz * plane;
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n; o += (long)gridDim.x * blockDim.x) {
     const long c = o + plane;  // level 1 + o / plane of the (0..nz+1) storage
+    const bool first = o < plane;
+    double* const a = acc + o;
+    double s[STAT_NQ];
+#pragma unroll
+    for (int q = 0; q < STAT_NQ; ++q) s[q] = a[q * n];
     const double u = f.u[c], v = f.v[c], w = f.w[c], p = f.p[c];
-    double* a = acc + o;
-    auto add = [&](int q, double x) { a[q * n] = __dadd_rn(a[q * n], x); };
+    const double txx = f.txx[c], tyy = f.tyy[c], tzz = f.tzz[c], txy = f.txy[c], txz = f.txz[c], tyz = f.tyz[c];
+    const double dudz = f.dudz[c], dvdz = f.dvdz[c], nut = f.nut[c], cs = f.cs[c];
+    const double ud = first ? 0.0 : double(f.u[c - plane]), vd = first ? 0.0 : double(f.v[c - plane]);
+    auto add = [&](int q, double x) { s[q] = __dadd_rn(s[q], x); };
     add(0, u);
     add(1, v);
     add(2, w);
@@ -47,34 +59,27 @@ __global__ void __launch_bounds__(256) k_stat_accum(StatFields<T> f, double* __r
     add(11, __dmul_rn(v2, v2));
     add(12, __dmul_rn(w2, w2));
     add(13, __dmul_rn(u, v));
-    if (o < plane) {
-      a[14 * n] = 0.0;
-      a[15 * n] = 0.0;
+    if (first) {
+      s[14] = 0.0;
+      s[15] = 0.0;
+      ustar_acc[o] = __dadd_rn(ustar_acc[o], double(ustar[o]));
     } else {
-      const double um = __dmul_rn(0.5, __dadd_rn(double(f.u[c - plane]), u));
-      const double vm = __dmul_rn(0.5, __dadd_rn(double(f.v[c - plane]), v));
-      add(14, __dmul_rn(w, um));
-      add(15, __dmul_rn(w, vm));
+      add(14, __dmul_rn(w, __dmul_rn(0.5, __dadd_rn(ud, u))));
+      add(15, __dmul_rn(w, __dmul_rn(0.5, __dadd_rn(vd, v))));
     }
-    add(16, f.txx[c]);
-    add(17, f.tyy[c]);
-    add(18, f.tzz[c]);
-    add(19, f.txy[c]);
-    add(20, f.txz[c]);
-    add(21, f.tyz[c]);
-    add(22, f.dudz[c]);
-    add(23, f.dvdz[c]);
-    add(24, f.nut[c]);
-    add(25, __dsqrt_rn(double(f.cs[c])));
+    add(16, txx);
+    add(17, tyy);
+    add(18, tzz);
+    add(19, txy);
+    add(20, txz);
+    add(21, tyz);
+    add(22, dudz);
+    add(23, dvdz);
+    add(24, nut);
+    add(25, __dsqrt_rn(cs));
+#pragma unroll
+    for (int q = 0; q < STAT_NQ; ++q) a[q * n] = s[q];
   }
-}
-
-// io_2D_stat_averages (:316-320): running sum of the friction-velocity plane
-template <typename T>
-__global__ void k_plane_accum(const T* x, double* acc, long plane) {
-  dep_wait();
-  for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < plane; o += (long)gridDim.x * blockDim.x)
-    acc[o] = __dadd_rn(acc[o], double(x[o]));
 }
 
 // ---------------------------------------------------------------------------
@@ -181,36 +186,43 @@ __device__ __forceinline__ void tke_point(const TkeFields<T>& f, long o, long pl
   put(60, C * uz);
 }
 
-// Quantities [Q0, Q0 + NQ) of every point of level 1 + blockIdx.y, summed
-// over the blockIdx.x-th share of the plane in a fixed order (per thread,
-// then a shuffle tree per warp, then warps in order) -> part.
-template <typename T, int Q0, int NQ>
-__global__ void __launch_bounds__(256) k_tke_partial(TkeFields<T> f, double* __restrict__ part, long plane, int wall,
-                                                     double idz) {
+// The quantities of every point of level 1 + blockIdx.y, summed over the
+// blockIdx.x-th share of the plane in a fixed order (per thread, then a tree
+// over the lanes, then warps in order) -> part.  All 61 sums in registers: one
+// read of the fields (in four launches of 16 sums each: 128 x 64 x 41 FP64 56
+// us, so 30).  The tree halves the values as it halves the lanes: each
+// lane hands its partner the half of the sums that the partner keeps, 62
+// exchanges instead of five per sum and the same additions.
+template <typename T>
+__global__ void __launch_bounds__(256) k_tke_partial(TkeFields<T> f, double* part, long plane, int wall, double idz) {
   dep_wait();
   const int k = 1 + blockIdx.y;
   const long base = (long)k * plane;
-  double acc[NQ];
+  double acc[64];
 #pragma unroll
-  for (int i = 0; i < NQ; ++i) acc[i] = 0.0;
+  for (int i = 0; i < 64; ++i) acc[i] = 0.0;
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < plane; o += (long)gridDim.x * blockDim.x)
-    tke_point(f, base + o, plane, k == 1, wall != 0, idz, [&](int q, double x) {
-      if (q >= Q0 && q < Q0 + NQ) acc[q - Q0] += x;
-    });
-  __shared__ double red[8][NQ];
+    tke_point(f, base + o, plane, k == 1, wall != 0, idz, [&](int q, double x) { acc[q] += x; });
+  __shared__ double red[8][64];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int q0 = 0;  // first of the sums that this lane keeps
 #pragma unroll
-  for (int i = 0; i < NQ; ++i) {
-    double v = acc[i];
+  for (int s = 16, half = 32; s > 0; s >>= 1, half >>= 1) {
+    const bool up = lane & s;
+    if (up) q0 += half;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    if (lane == 0) red[wid][i] = v;
+    for (int i = 0; i < half; ++i) {
+      const double give = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+      acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+    }
   }
+  red[wid][q0] = acc[0];
+  red[wid][q0 + 1] = acc[1];
   __syncthreads();
-  for (int i = threadIdx.x; i < NQ; i += blockDim.x) {
+  for (int i = threadIdx.x; i < TKE_NQ; i += blockDim.x) {
     double s = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][i];
-    part[((long)blockIdx.y * gridDim.x + blockIdx.x) * TKE_NQ + Q0 + i] = s;
+    part[((long)blockIdx.y * gridDim.x + blockIdx.x) * TKE_NQ + i] = s;
   }
 }
 
