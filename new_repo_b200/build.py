@@ -16,7 +16,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 BUILD = HERE.parent / "_build"
 LIB = HERE / "liblesgpu.so"
-SOURCES = ["spectral_inst.cu", "spectral_xfwd.cu", "spectral_xinv.cu", "spectral_xinv_f64.cu", "spectral_ypass.cu", "solver.cu", "capi.cu", "mlp.cu", "noalloc.cu"]
+SOURCES = ["spectral_inst.cu", "spectral_xfwd.cu", "spectral_xinv.cu", "spectral_xinv_f64.cu", "spectral_ypass.cu", "spectral_ypass_f64.cu", "solver.cu", "capi.cu", "mlp.cu", "noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-strict-aliasing",
          "--expt-relaxed-constexpr", "-I", str(HERE.parent / "include")]
@@ -32,7 +32,7 @@ def nvcc() -> str:
 def _stale(obj: Path, src: Path) -> bool:
     if not obj.exists():
         return True
-    deps = [src] + list(CSRC.glob("*.cuh")) + ([CSRC / "spectral_xinv.cu"] if src.stem == "spectral_xinv_f64" else []) + [HERE.parent / "include" / "lesgpu.h"]
+    deps = [src] + list(CSRC.glob("*.cuh")) + ([src.with_name(src.name.replace("_f64", ""))] if "_f64" in src.name else []) + [HERE.parent / "include" / "lesgpu.h"]
     t = obj.stat().st_mtime
     return any(d.stat().st_mtime > t for d in deps if d.exists())
 

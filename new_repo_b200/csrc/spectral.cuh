@@ -863,53 +863,43 @@ struct YPArgs {
   const cplx<T>* tw_out;  // length NYO table
 };
 
-// Elementwise spectral op at (kx, ky) for output q; F0/F1 are the forward
-// transforms of the (up to two) input fields at that point.
-template <typename T, int NY>
-__device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int ky, cplx<T> F0, cplx<T> F1) {
-  const cplx<T> zero = {T(0), T(0)};
-  switch (a.op) {
-    case YP_GRADY: {
-      if (ky == NY / 2 || kx == a.nxh) return zero;
-      if (q == 0) return F0;
-      return ik_mul(a.kky[ky * a.lhx + kx], F0);
-    }
-    case YP_DIV2: {
-      if (ky == NY / 2 || kx == a.nxh) return zero;
-      return c_add(ik_mul(a.kkx[ky * a.lhx + kx], F0), ik_mul(a.kky[ky * a.lhx + kx], F1));
-    }
-    case YP_FWDKILL:
-      return (ky == NY / 2 || kx == a.nxh) ? zero : F0;
-    case YP_FILTER1:
-    case YP_FILTER2: {
-      const T g = (q == 0 ? a.G0 : a.G1)[ky * a.lhx + kx];
-      return cplx<T>{F0.x * g, F0.y * g};
-    }
-    case YP_MASK:
-    case YP_MASKY: {
-      if (!(ky <= a.tt || ky >= NY - a.tt)) return zero;
-      return q == 0 ? F0 : ik_mul(a.kky[ky * a.lhx + kx], F0);
-    }
-    default:
-      return F0;  // YP_PAD / YP_TRUNC: position remap only
+// The ops of the y passes in classes, each compiled on its own (FP64: with every
+// op in one kernel 200-350 bytes per thread spilled at the register limit that
+// three blocks per SM need; the test-filtered fields at 128^3 took 312 us so,
+// 183 apart, at 256^3 1978 and 1850, FP32 at 512 x 512 x 96 1835 and 1490).
+// Length-changing passes are YC_OTHER.
+enum YPClass : int { YC_FWD = 0, YC_GRADY = 1, YC_PGRAD = 2, YC_FILTER = 3, YC_DIV2 = 4, YC_OTHER = 5 };
+inline int yp_class(int op) {
+  switch (op) {
+    case YP_FWDKILL: case YP_PRESS: return YC_FWD;
+    case YP_GRADY: return YC_GRADY;
+    case YP_PGRAD: return YC_PGRAD;
+    case YP_FILTER1: case YP_FILTER2: return YC_FILTER;
+    case YP_DIV2: return YC_DIV2;
+    default: return YC_OTHER;
   }
 }
 
-// yp_op for an op fixed at compile time, with the wavenumbers of the point
-// given: kxv = kkx(kx) of the thread's column (row 0 of the table) and kyv =
-// kky(ky) of the row (column 0).  The tables hold 2 pi / l times the wrapped
+// Output q at (kx, ky) of a column's forward transform F0, kyv = kky(ky) of the
+// row (column 0 of the table).  The tables hold 2 pi / l times the wrapped
 // index, zeroed on the Nyquist row / column only, so away from those the
 // values are the table's; the kills below reproduce the zeros.
-template <typename T, int NY, int OP>
-__device__ __forceinline__ cplx<T> yp_op_c(const YPArgs<T>& a, int q, int kx, int ky, cplx<T> F0, T kxv, T kyv) {
+template <typename T, int NY, int CLS>
+__device__ __forceinline__ cplx<T> yp_op(const YPArgs<T>& a, int q, int kx, int ky, cplx<T> F0, T kyv) {
   const cplx<T> zero = {T(0), T(0)};
-  if constexpr (OP == YP_GRADY) {
+  if constexpr (CLS == YC_GRADY) {
     if (ky == NY / 2 || kx == a.nxh) return zero;
     if (q == 0) return F0;
     return ik_mul(kyv, F0);
-  } else {  // YP_PGRAD: no kill, the Nyquist row / column of the tables are zero
+  } else if constexpr (CLS == YC_PGRAD) {  // no kill, the Nyquist row / column of the tables are zero
     if (q == 0) return F0;
     return ik_mul(kx == a.nxh ? T(0) : kyv, F0);
+  } else if constexpr (CLS == YC_FILTER) {
+    const T g = (q == 0 ? a.G0 : a.G1)[ky * a.lhx + kx];
+    return cplx<T>{F0.x * g, F0.y * g};
+  } else {  // YP_MASK, YP_MASKY: columns and kept rows below the Nyquist ones
+    if (!(ky <= a.tt || ky >= NY - a.tt)) return zero;
+    return q == 0 ? F0 : ik_mul(kyv, F0);
   }
 }
 
@@ -940,13 +930,12 @@ __device__ __forceinline__ void yp_issue(const YPArgs<T>& a, long item, int ncb,
   }
 }
 
-// FWD: forward transforms only (YP_FWDKILL, YP_PRESS), compiled without the
-// inverse so that it keeps fewer registers.  FP64: 168 registers (three CTAs
-// of 128 threads) where the compiler would take 255 (two); the passes with
-// several outputs spill ~200 bytes for it and still gain (the 21 test-filtered
-// fields at 256^3: 2965 -> 2286 us, then 1993 without the columns past the
-// narrower filter).
-template <typename T, int NY, int NYO, bool FWD = false>
+// YC_FWD: forward transforms only, compiled without the inverse so that it
+// keeps fewer registers.  FP64: 168 registers (three CTAs of 128 threads) where
+// the compiler would take 255 (two); the 21 test-filtered fields at 256^3: 2965
+// -> 2286 us, 1993 without the columns past the narrower filter, 1850 in a
+// class of their own.
+template <typename T, int NY, int NYO, int CLS>
 __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3 : 2)
     k_ypass(const YPArgs<T> a) {
   constexpr int TL = Geo<NY>::T;
@@ -957,7 +946,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   constexpr int FO = Layout<NY, false>::out;   // forward output groups
   constexpr int II = Layout<NYO, true>::in;    // inverse input groups
   constexpr int IO = Layout<NYO, true>::out;   // inverse output groups
-  constexpr bool SAME = (NY == NYO);
+  constexpr bool SAME = (NY == NYO), FWD = CLS == YC_FWD;
+  static_assert(SAME || CLS == YC_OTHER, "a class keeps the length");
   static_assert(!SAME || FO == II, "forward output layout must feed the inverse");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* twi = reinterpret_cast<cplx<T>*>(smem_raw);  // twiddle matrices, forward NY
@@ -970,7 +960,6 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   // the inverse transform, its output layout and the coalesced copy-out use
   // the first input row of each column of the current stage, free once the
   // forward transforms hold their values in registers
-  static_assert(!FWD || NY == NYO, "forward-only y passes keep the length");
   twm_build<T, NY, false>(a.tw_in, twi, threadIdx.x, blockDim.x);
   if constexpr (!FWD) twm_build<T, NYO, true>(a.tw_out, two, threadIdx.x, blockDim.x);
   if (a.kky)
@@ -1011,7 +1000,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
   cplx<T> w[EO];
   {
     cplx<T>* seq = bin + c * SI;
-    if (a.op == YP_PGRAD) {
+    if constexpr (CLS == YC_PGRAD) {
       // input is already y-spectral: load it in the inverse input layout
 #pragma unroll
       for (int g = 0; g < EI / II; ++g)
@@ -1039,44 +1028,42 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
             for (int r = 0; r < FI; ++r) f0[g * FI + r] = seq1[lt + TL * g + r * (NY / FI)];
           reg_fft<T, NY, false>(f0, seq1, lt, twi);
         }
-      } else if constexpr (SAME) {
-        if (a.op == YP_DIV2) {
-          const cplx<T> zero = {T(0), T(0)};
+      } else if constexpr (CLS == YC_DIV2) {
+        const cplx<T> zero = {T(0), T(0)};
 #pragma unroll
-          for (int g = 0; g < EI / FO; ++g)
+        for (int g = 0; g < EI / FO; ++g)
 #pragma unroll
-            for (int r = 0; r < FO; ++r) {
-              const int ky = lt + TL * g + r * (NY / FO);
-              const bool kill = (ky == NY / 2) || (kx == a.nxh) || (kx >= a.ncols);
-              w[g * FO + r] = kill ? zero : ik_mul(a.kkx[kx], f0[g * FO + r]);
-            }
-          cplx<T>* seq1 = bin + (C + c) * SI;
+          for (int r = 0; r < FO; ++r) {
+            const int ky = lt + TL * g + r * (NY / FO);
+            const bool kill = (ky == NY / 2) || (kx == a.nxh) || (kx >= a.ncols);
+            w[g * FO + r] = kill ? zero : ik_mul(a.kkx[kx], f0[g * FO + r]);
+          }
+        cplx<T>* seq1 = bin + (C + c) * SI;
 #pragma unroll
-          for (int g = 0; g < EI / FI; ++g)
+        for (int g = 0; g < EI / FI; ++g)
 #pragma unroll
-            for (int r = 0; r < FI; ++r) f0[g * FI + r] = seq1[lt + TL * g + r * (NY / FI)];
-          reg_fft<T, NY, false>(f0, seq1, lt, twi);
+          for (int r = 0; r < FI; ++r) f0[g * FI + r] = seq1[lt + TL * g + r * (NY / FI)];
+        reg_fft<T, NY, false>(f0, seq1, lt, twi);
 #pragma unroll
-          for (int g = 0; g < EI / FO; ++g)
+        for (int g = 0; g < EI / FO; ++g)
 #pragma unroll
-            for (int r = 0; r < FO; ++r) {
-              const int ky = lt + TL * g + r * (NY / FO);
-              const bool kill = (ky == NY / 2) || (kx == a.nxh) || (kx >= a.ncols);
-              if (!kill) w[g * FO + r] = c_add(w[g * FO + r], ik_mul(kyrow[ky], f0[g * FO + r]));
-            }
-        }
+          for (int r = 0; r < FO; ++r) {
+            const int ky = lt + TL * g + r * (NY / FO);
+            const bool kill = (ky == NY / 2) || (kx == a.nxh) || (kx >= a.ncols);
+            if (!kill) w[g * FO + r] = c_add(w[g * FO + r], ik_mul(kyrow[ky], f0[g * FO + r]));
+          }
       }
     }
   }
   __syncwarp();  // the column's forward reads are done before its slot is rewritten
   cplx<T>* sout = bin + c * SI;
   const bool layers = FWD && a.op == YP_PRESS && l == a.plane0 + a.nplanes - 1;
-  const bool wall = !FWD && SAME && a.op == YP_GRADY && l == 1 && grp < 2 && a.wall[grp] && col0 < a.ncols1;
+  const bool wall = CLS == YC_GRADY && l == 1 && grp < 2 && a.wall[grp] && col0 < a.ncols1;
   const int nout = layers ? 2 : a.nout + (wall ? 1 : 0);
   for (int q = 0; q < nout; ++q) {
     const bool third = wall && q == a.nout;
     if (!layers && !third && !a.out[grp * a.nout + q]) continue;  // an optional output left out (the whole CTA)
-    if (a.op == YP_FILTER2 && q == 1 && col0 >= a.ncols1) continue;  // all columns beyond the narrower filter
+    if (CLS == YC_FILTER && a.op == YP_FILTER2 && q == 1 && col0 >= a.ncols1) continue;  // all columns beyond the narrower filter
     if constexpr (SAME) {
       // forward output layout (groups FO) == inverse input layout; the
       // stress divergence already holds its result in w
@@ -1100,21 +1087,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
             }
             slot = kill ? cplx<T>{T(0), T(0)} : x;
           }
-      } else if (a.op != YP_DIV2) {
-        // the derivative ops with the op fixed per loop (no per-element
-        // dispatch) and the wavenumbers from registers / shared memory
-        const T kxv = (kx < a.ncols && a.kkx) ? a.kkx[kx] : T(0);
-        auto fill = [&](auto opc) {
-          constexpr int OP = decltype(opc)::value;
-#pragma unroll
-          for (int g = 0; g < EI / FO; ++g)
-#pragma unroll
-            for (int r = 0; r < FO; ++r) {
-              const int ky = lt + TL * g + r * (NY / FO);
-              w[g * FO + r] = (kx < a.ncols) ? yp_op_c<T, NY, OP>(a, q, kx, ky, f0[g * FO + r], kxv, kyrow[ky])
-                                             : cplx<T>{T(0), T(0)};
-            }
-        };
+      } else if constexpr (CLS != YC_DIV2) {
         if (third) {
 #pragma unroll
           for (int g = 0; g < EI / FO; ++g)
@@ -1124,17 +1097,14 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
               const T gv = (kx < a.ncols1) ? a.G0[ky * a.lhx + kx] * a.gs : T(0);
               w[g * FO + r] = c_scl(f0[g * FO + r], gv);
             }
-        } else if (a.op == YP_GRADY) {
-          fill(std::integral_constant<int, YP_GRADY>{});
-        } else if (a.op == YP_PGRAD) {
-          fill(std::integral_constant<int, YP_PGRAD>{});
         } else {
 #pragma unroll
           for (int g = 0; g < EI / FO; ++g)
 #pragma unroll
             for (int r = 0; r < FO; ++r) {
               const int ky = lt + TL * g + r * (NY / FO);
-              w[g * FO + r] = (kx < a.ncols) ? yp_op<T, NY>(a, q, kx, ky, f0[g * FO + r], f0[g * FO + r])
+              const T kyv = CLS == YC_FILTER ? T(0) : kyrow[ky];
+              w[g * FO + r] = (kx < a.ncols) ? yp_op<T, NY, CLS>(a, q, kx, ky, f0[g * FO + r], kyv)
                                              : cplx<T>{T(0), T(0)};
             }
         }
@@ -1188,7 +1158,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
     }
     __syncthreads();
     // coalesced store of output q
-    const bool second = (a.op == YP_FILTER2 && q == 1) || third;
+    const bool second = (CLS == YC_FILTER && a.op == YP_FILTER2 && q == 1) || third;
     const int lim = second ? a.ncols1 : a.ncols;
     {
       // thread -> fixed column cc, rows ky0 + TL i (as in yp_issue)

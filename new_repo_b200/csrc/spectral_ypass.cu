@@ -6,12 +6,22 @@
 
 namespace les {
 
-// the y-pass kernel of a length pair; the forward-only variant exists for
-// equal lengths (nullptr otherwise)
+// the y-pass kernel of a length pair and class (nullptr: none)
 template <typename T, int A, int B>
-static void (*ypass_kernel(bool fwd))(YPArgs<T>) {
-  if constexpr (A == B) return fwd ? k_ypass<T, A, A, true> : k_ypass<T, A, B>;
-  else return fwd ? nullptr : k_ypass<T, A, B>;
+static void (*ypass_kernel(int cls))(YPArgs<T>) {
+  if constexpr (A == B) {
+    switch (cls) {
+      case YC_FWD: return k_ypass<T, A, A, YC_FWD>;
+      case YC_GRADY: return k_ypass<T, A, A, YC_GRADY>;
+      case YC_PGRAD: return k_ypass<T, A, A, YC_PGRAD>;
+      case YC_FILTER: return k_ypass<T, A, A, YC_FILTER>;
+      case YC_DIV2: return k_ypass<T, A, A, YC_DIV2>;
+      default: break;
+    }
+  } else if (cls != YC_OTHER) {
+    return nullptr;
+  }
+  return k_ypass<T, A, B, YC_OTHER>;
 }
 
 template <typename T>
@@ -38,11 +48,11 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
            sizeof(T) * ((NY + 3) & ~3);
   };
   const int key = NY * 10000 + NYO;
-  const bool fwd = (a.op == YP_FWDKILL || a.op == YP_PRESS);
+  const int cls = yp_class(a.op);
   void (*kern)(YPArgs<T>) = nullptr;
   switch (key) {
 #define YP_CASE(A, B) \
-  case A * 10000 + B: kern = ypass_kernel<T, A, B>(fwd); break;
+  case A * 10000 + B: kern = ypass_kernel<T, A, B>(cls); break;
     YP_CASE(16, 16) YP_CASE(32, 32) YP_CASE(64, 64) YP_CASE(128, 128) YP_CASE(256, 256) YP_CASE(512, 512)
     YP_CASE(16, 24) YP_CASE(32, 48) YP_CASE(64, 96) YP_CASE(128, 192) YP_CASE(256, 384) YP_CASE(512, 768)
     YP_CASE(24, 16) YP_CASE(48, 32) YP_CASE(96, 64) YP_CASE(192, 128) YP_CASE(384, 256) YP_CASE(768, 512)
@@ -50,7 +60,7 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
     default:
       throw CudaError(1, "ypass: unsupported length pair " + std::to_string(NY) + "->" + std::to_string(NYO));
   }
-  if (!kern) throw CudaError(1, "ypass: a forward-only pass keeps the length");
+  if (!kern) throw CudaError(1, "ypass: this op keeps the length");
   // columns per CTA (C * TL threads, at least a warp) and input stages: the
   // most busy warps per SM -- resident CTAs (shared memory, registers,
   // threads) times the warps whose columns exist; on a tie two stages (the
@@ -68,7 +78,9 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
     for (int ns = 2; ns >= 1; --ns)
       for (int lc = 0; (1 << lc) * TL <= std::min(256, lim.max_threads); ++lc) {
         const int C = 1 << lc, threads = C * TL;
-        if (threads < 32) continue;
+        // whole sectors per row piece (FP32 256-point columns two at a time for a
+        // seventeenth warp took 364 us where eight at a time take 195)
+        if (threads < 32 || C * sizeof(cplx<T>) < 32) continue;
         const size_t sm = smem_for(C, ns);
         if (sm > SMEM_CAP) break;
         const int warp_regs = ((regs * 32 + 255) / 256) * 256;
@@ -151,7 +163,7 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
     for (int q = 0; (1 << q) * TL <= std::min(256, lim.max_threads); ++q) {
       const int threads = (1 << q) * TL;
       const size_t sm = smem_for(1 << q, ns);
-      if (threads < 32) continue;
+      if (threads < 32 || (sizeof(cplx<T>) << q) < 32) continue;  // whole sectors per row piece
       if (sm > SMEM_CAP) break;
       const int ctas = std::min({int(SM_SMEM / (sm + 1024)), 65536 / (warp_regs * (threads / 32)), 2048 / threads, 32});
       if (ctas < 1) break;
@@ -190,23 +202,25 @@ void set_attrs_ypass() {
   LES_CUDA(cudaFuncSetAttribute(k_yrhs<T, 3 * B / 2, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
   YR(16) YR(32) YR(64) YR(128) YR(256) YR(512)
 #undef YR
-#define YA(A, B) \
-  LES_CUDA(cudaFuncSetAttribute(k_ypass<T, A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-#define YF(A) \
-  LES_CUDA(cudaFuncSetAttribute(k_ypass<T, A, A, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-  YF(16) YF(32) YF(64) YF(128) YF(256) YF(512)
-#undef YF
+#define YA(A, B)                                                                                          \
+  for (int c : {YC_FWD, YC_GRADY, YC_PGRAD, YC_FILTER, YC_DIV2, YC_OTHER})                                        \
+    if (auto k = ypass_kernel<T, A, B>(c))                                                               \
+      LES_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
   YA(16, 16) YA(32, 32) YA(64, 64) YA(128, 128) YA(256, 256) YA(512, 512)
   YA(16, 24) YA(32, 48) YA(64, 96) YA(128, 192) YA(256, 384) YA(512, 768)
   YA(24, 16) YA(48, 32) YA(96, 64) YA(192, 128) YA(384, 256) YA(768, 512)
 #undef YA
 }
 
-template void launch_ypass<float>(int, int, YPArgs<float>, int, int, cudaStream_t);
+// one translation unit per type (they compile side by side)
+#ifdef LES_YPASS_DOUBLE
 template void launch_ypass<double>(int, int, YPArgs<double>, int, int, cudaStream_t);
-template void launch_yrhs<float>(int, int, YRArgs<float>, cudaStream_t);
 template void launch_yrhs<double>(int, int, YRArgs<double>, cudaStream_t);
-template void set_attrs_ypass<float>();
 template void set_attrs_ypass<double>();
+#else
+template void launch_ypass<float>(int, int, YPArgs<float>, int, int, cudaStream_t);
+template void launch_yrhs<float>(int, int, YRArgs<float>, cudaStream_t);
+template void set_attrs_ypass<float>();
+#endif
 
 }  // namespace les
