@@ -2108,7 +2108,9 @@ class Solver final : public SolverBase {
   int lag_levels(int jtt) const {
     if (jtt < P.dyn_init) return -1;
     if (P.sgs_model == LES_SGS_LASD) return g.nz + 1;
-    if (P.sgs_model == LES_SGS_MLP && mlp_wall_levels > 0) return std::min(mlp_wall_levels, g.nz + 1);
+    // (an update without weights is refused by mlp_sgs: nothing is added then)
+    if (P.sgs_model == LES_SGS_MLP && mlp_wall_levels > 0 && (mlp_ready || jtt % P.cs_count != 0))
+      return std::min(mlp_wall_levels, g.nz + 1);
     return -1;
   }
 
