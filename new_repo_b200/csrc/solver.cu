@@ -129,6 +129,7 @@ class Solver final : public SolverBase {
     k_tridiag_factor<<<ceil_div((long)g.ny * g.lhx, 64), 64, 0, st>>>(piv, kkxd, kkyd, g.lhx, g.ny, g.nz, dz());
     LES_CHECK_LAUNCH();
     pmean = track(dalloc<double>(g.L));
+    psum = track(dalloc<double>(2 * (PSUM_BLOCKS + 6L * g.L)));
     part = track(dalloc<double>(DIAG_BLOCKS * DIAG_NV));
     dout = track(dalloc<double>(8));
     dstatus = track(dalloc<unsigned>(4));
@@ -326,16 +327,17 @@ class Solver final : public SolverBase {
   // Compensated FP64 sums of each of levels k0 .. k0 + nlev - 1 of up to six
   // fields, in nch chunks per level (returned) into psum.  Chunks: ~8 blocks
   // per SM over the whole launch, none below 2048 points (eight points per
-  // thread, under which a block is all reduction).
+  // thread, under which a block is all reduction).  nf nlev nch stays below
+  // PSUM_BLOCKS + nf nlev, so psum is small and comes with the state: a time
+  // step allocates nothing.
   double* psum = nullptr;
-  static constexpr int PSUM_CHUNKS = 128;
+  static constexpr long PSUM_BLOCKS = 148 * 8;
   int plane_sums(std::initializer_list<const T*> f, int k0, int nlev) {
-    if (!psum) psum = track(dalloc<double>((long)6 * g.L * PSUM_CHUNKS * 2));
     PlaneSumIn<T> in{};
     int nf = 0;
     for (const T* x : f) in.f[nf++] = x;
-    const long want = ceil_div(148L * 8, (long)nf * nlev);
-    const int nch = int(std::max(1L, std::min({want, g.plane() / 2048, (long)PSUM_CHUNKS})));
+    const long want = ceil_div(PSUM_BLOCKS, (long)nf * nlev);
+    const int nch = int(std::max(1L, std::min(want, g.plane() / 2048)));
     const long chunk = (long)ceil_div(ceil_div(g.plane(), nch), 4) * 4;
     KL("k_plane_sums", double(nf) * nlev * g.plane() * sizeof(T),
        launch_dep(k_plane_sums<T>, dim3(unsigned(nch), unsigned(nlev), unsigned(nf)), 256, 0, st, in, psum, g.plane(), k0, chunk));
