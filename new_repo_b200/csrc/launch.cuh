@@ -25,7 +25,13 @@ inline void hook_after() {
 }
 
 bool supported_length(int n);
-void init_spectral_attributes();
+
+// What a grid's spectral kernels are for: everything a state of type T
+// launches, the FP64 pressure spectra of a mixed-precision state, or the
+// gradients of a caller's field.
+enum SpectralUse : int { SU_STATE = 0, SU_PRESSURE = 1, SU_GRAD = 2 };
+template <typename T>
+void init_spectral_attributes(SpectralUse use, int nx, int ny);
 
 template <typename T>
 void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st);

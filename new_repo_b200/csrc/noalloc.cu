@@ -383,7 +383,8 @@ int scratch_for_device(unsigned char** out) {
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess)
       throw CudaError(LES_ERR_INVALID, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-    init_spectral_attributes();
+    for (int nx : {16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 768})
+      for (int ny : {16, 32, 64, 128, 256, 512}) init_spectral_attributes<double>(SU_GRAD, nx, ny);
     for (int nx : {16, 24, 32, 48, 64, 96, 128, 192, 256})
       for (int ny : {16, 32, 64, 128}) {
         if (const PlaneKernel k = plane_kernel(nx, ny); k.run)

@@ -109,7 +109,8 @@ class Solver final : public SolverBase {
     LES_CUDA(cudaSetDevice(p.device));
     LES_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     for (auto& e : ev) LES_CUDA(cudaEventCreate(&e));
-    init_spectral_attributes();  // once per device (this one is current)
+    init_spectral_attributes<T>(SU_STATE, p.nx, p.ny);
+    if (std::is_same<T, float>::value) init_spectral_attributes<double>(SU_PRESSURE, p.nx, p.ny);
     const long nf = g.field();
     for (int i = 0; i < LES_THETA; ++i) F[i] = track(dalloc<T>(nf));  // scalar fields: les_scalar_init
     for (int i = 0; i < LES_NPLANES; ++i) PL[i] = track(dalloc<T>(g.plane()));

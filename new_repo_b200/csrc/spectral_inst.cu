@@ -113,25 +113,48 @@ bool supported_length(int n) {
   }
 }
 
-// cudaFuncSetAttribute applies to the current device only: done once per
-// device ordinal (fixed table and a mutex, no heap allocation), so states on
-// several devices of one process, and threads creating them at once, all
-// launch with the shared-memory limit raised
-void init_spectral_attributes() {
+namespace {
+int length_index(int n) {  // of a supported length
+  int i = 0;
+#define LI(N) if (n == N) return i; ++i;
+  LES_LENGTHS(LI)
+#undef LI
+  throw CudaError(1, "no FFT plan for length " + std::to_string(n));
+}
+}  // namespace
+
+// cudaFuncSetAttribute applies to the current device only, and loads the
+// kernel: done for the kernels of a grid, once per device ordinal (fixed table
+// and a mutex, no heap allocation), so states on several devices of one
+// process, and threads creating them at once, all launch with the
+// shared-memory limit raised.  (Loading all 264 kernels of every length, type
+// and class took a process's first state 74 ms; its own twenty or thirty 43 to
+// 58 ms, 23 to 30 ms with uncompressed device code, see build.py.)
+template <typename T>
+void init_spectral_attributes(SpectralUse use, int nx, int ny) {
   static std::mutex mu;
-  static bool done[256] = {};
+  static bool done[256][3][2][12];  // device, use, direction, length
   int dev = 0;
   LES_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 256) throw CudaError(1, "device ordinal out of range");
+  bool& dx = done[dev][use][0][length_index(nx)];
+  bool& dy = done[dev][use][1][length_index(ny)];
   std::lock_guard<std::mutex> lock(mu);
-  if (done[dev]) return;
-  set_attrs_xfwd<float>();
-  set_attrs_xfwd<double>();
-  set_attrs_xinv<float>();
-  set_attrs_xinv<double>();
-  set_attrs_ypass<float>();
-  set_attrs_ypass<double>();
-  done[dev] = true;
+  if (!dx) {
+    set_attrs_xfwd<T>(use, nx);
+    if (use != SU_PRESSURE) set_attrs_xinv<T>(use, nx);
+    if (use == SU_STATE) {  // the padded products' length
+      set_attrs_xfwd<T>(use, 3 * nx / 2);
+      set_attrs_xinv<T>(use, 3 * nx / 2);
+    }
+    dx = true;
+  }
+  if (!dy) {
+    set_attrs_ypass<T>(use, ny);
+    dy = true;
+  }
 }
+template void init_spectral_attributes<float>(SpectralUse, int, int);
+template void init_spectral_attributes<double>(SpectralUse, int, int);
 
 }  // namespace les

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <string>
 
+#include "launch.cuh"
 #include "spectral.cuh"
 
 namespace les {
@@ -77,9 +78,14 @@ inline int best_rows(const void* kern, int seq_per_row, int TL, SmemFn smem_for,
 }
 
 
-// shared-memory limits of each family's kernels on the current device
-template <typename T> void set_attrs_xfwd();
-template <typename T> void set_attrs_xinv();
-template <typename T> void set_attrs_ypass();
+// shared-memory limit of a kernel on the current device
+template <typename... P>
+inline void raise_smem(void (*kern)(P...)) {
+  if (kern) LES_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
+}
+// of each family's kernels of a length (y: of a grid) for a use
+template <typename T> void set_attrs_xfwd(SpectralUse use, int NX);
+template <typename T> void set_attrs_xinv(SpectralUse use, int NX);
+template <typename T> void set_attrs_ypass(SpectralUse use, int NY);
 
 }  // namespace les

@@ -118,19 +118,23 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
 
 
 template <typename T>
-void set_attrs_xfwd() {
-#define XA(N)                                                                                       \
-  LES_CUDA(cudaFuncSetAttribute(k_xfwd<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  LES_CUDA(cudaFuncSetAttribute(k_xfwd_row<T, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  if constexpr (std::is_same<T, double>::value)                                                       \
-    LES_CUDA(cudaFuncSetAttribute(k_xfwd_row<T, N, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-  LES_LENGTHS(XA)
+void set_attrs_xfwd(SpectralUse use, int NX) {
+  switch (NX) {
+#define XA(N)                                                                                             \
+  case N:                                                                                                 \
+    if (use == SU_STATE) raise_smem(k_xfwd<T, N>);                                                         \
+    if (use != SU_PRESSURE) raise_smem(k_xfwd_row<T, N, T>);                                               \
+    if constexpr (std::is_same<T, double>::value) if (use == SU_PRESSURE) raise_smem(k_xfwd_row<T, N, float>); \
+    break;
+    LES_LENGTHS(XA)
 #undef XA
+    default: break;
+  }
 }
 
 template void launch_xfwd<float>(int, XFArgs<float>, cudaStream_t);
 template void launch_xfwd<double>(int, XFArgs<double>, cudaStream_t);
-template void set_attrs_xfwd<float>();
-template void set_attrs_xfwd<double>();
+template void set_attrs_xfwd<float>(SpectralUse, int);
+template void set_attrs_xfwd<double>(SpectralUse, int);
 
 }  // namespace les

@@ -124,22 +124,18 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
 
 
 template <typename T>
-void set_attrs_xinv() {
-#define XA(N)                                                                                             \
-  for (int c : {XC_STORE, XC_CONV, XC_DIV, XC_DYN, XC_WALL})                                              \
-    if (auto k = xinv_kernel<T>(N, c))                                                                     \
-      LES_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-  LES_LENGTHS(XA)
-#undef XA
+void set_attrs_xinv(SpectralUse use, int NX) {
+  for (int c : {XC_STORE, XC_CONV, XC_DIV, XC_DYN, XC_WALL})
+    if (c == XC_STORE || use == SU_STATE) raise_smem(xinv_kernel<T>(NX, c));
 }
 
 // one translation unit per type (they compile side by side)
 #ifdef LES_XINV_DOUBLE
 template void launch_xinv<double>(int, XIArgs<double>, cudaStream_t);
-template void set_attrs_xinv<double>();
+template void set_attrs_xinv<double>(SpectralUse, int);
 #else
 template void launch_xinv<float>(int, XIArgs<float>, cudaStream_t);
-template void set_attrs_xinv<float>();
+template void set_attrs_xinv<float>(SpectralUse, int);
 #endif
 
 }  // namespace les

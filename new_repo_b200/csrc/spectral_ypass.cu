@@ -196,31 +196,35 @@ void launch_yrhs(int NF, int N, YRArgs<T> a, cudaStream_t st) {
 }
 
 template <typename T>
-void set_attrs_ypass() {
-#define YR(B)                                                                                                  \
-  LES_CUDA(cudaFuncSetAttribute(k_yrhs<T, B, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP)); \
-  LES_CUDA(cudaFuncSetAttribute(k_yrhs<T, 3 * B / 2, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-  YR(16) YR(32) YR(64) YR(128) YR(256) YR(512)
-#undef YR
-#define YA(A, B)                                                                                          \
-  for (int c : {YC_FWD, YC_GRADY, YC_PGRAD, YC_FILTER, YC_DIV2, YC_OTHER})                                        \
-    if (auto k = ypass_kernel<T, A, B>(c))                                                               \
-      LES_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP));
-  YA(16, 16) YA(32, 32) YA(64, 64) YA(128, 128) YA(256, 256) YA(512, 512)
-  YA(16, 24) YA(32, 48) YA(64, 96) YA(128, 192) YA(256, 384) YA(512, 768)
-  YA(24, 16) YA(48, 32) YA(96, 64) YA(192, 128) YA(384, 256) YA(768, 512)
+void set_attrs_ypass(SpectralUse use, int NY) {
+  switch (NY) {
+#define YA(N)                                                             \
+  case N:                                                                 \
+    if (use == SU_STATE) {                                                \
+      for (int c : {YC_FWD, YC_GRADY, YC_PGRAD, YC_FILTER, YC_DIV2, YC_OTHER}) raise_smem(ypass_kernel<T, N, N>(c)); \
+      raise_smem(ypass_kernel<T, N, 3 * N / 2>(YC_OTHER));                \
+      raise_smem(ypass_kernel<T, 3 * N / 2, N>(YC_OTHER));                \
+      raise_smem(k_yrhs<T, N, N>);                                        \
+      raise_smem(k_yrhs<T, 3 * N / 2, N>);                                \
+    } else {                                                              \
+      raise_smem(ypass_kernel<T, N, N>(use == SU_PRESSURE ? YC_FWD : YC_GRADY)); \
+    }                                                                     \
+    break;
+    YA(16) YA(32) YA(64) YA(128) YA(256) YA(512)
 #undef YA
+    default: break;
+  }
 }
 
 // one translation unit per type (they compile side by side)
 #ifdef LES_YPASS_DOUBLE
 template void launch_ypass<double>(int, int, YPArgs<double>, int, int, cudaStream_t);
 template void launch_yrhs<double>(int, int, YRArgs<double>, cudaStream_t);
-template void set_attrs_ypass<double>();
+template void set_attrs_ypass<double>(SpectralUse, int);
 #else
 template void launch_ypass<float>(int, int, YPArgs<float>, int, int, cudaStream_t);
 template void launch_yrhs<float>(int, int, YRArgs<float>, cudaStream_t);
-template void set_attrs_ypass<float>();
+template void set_attrs_ypass<float>(SpectralUse, int);
 #endif
 
 }  // namespace les
