@@ -36,7 +36,7 @@ def nvcc() -> str:
 def _stale(obj: Path, src: Path) -> bool:
     if not obj.exists():
         return True
-    deps = [src, Path(__file__)] + list(CSRC.glob("*.cuh")) + ([src.with_name(src.name.replace("_f64", ""))] if "_f64" in src.name else []) + [HERE.parent / "include" / "lesgpu.h"]
+    deps = [src, Path(__file__)] + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) + ([src.with_name(src.name.replace("_f64", ""))] if "_f64" in src.name else []) + [HERE.parent / "include" / "lesgpu.h"]
     t = obj.stat().st_mtime
     return any(d.stat().st_mtime > t for d in deps if d.exists())
 

@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "launch.cuh"
+#include "launch_cache.hpp"
 
 namespace les {
 
@@ -27,54 +28,33 @@ int sm_count() {
   return n;
 }
 
-// CTAs of `kern` resident on the current device at once; cached in a fixed
-// table (no heap allocation: the allocation-free entry point launches these
-// kernels too)
-struct ResidentEntry {
-  int dev;
-  const void* kern;
-  int threads;
-  size_t smem;
-  int n;
-};
+// CTAs of `kern` resident on the current device at once
 int resident_ctas(const void* kern, int threads, size_t smem) {
   static std::mutex mu;
-  static ResidentEntry table[256];
-  static int used = 0;
+  static LaunchCache<int, RESIDENT_CACHE> cache;
   int dev = 0;
   LES_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < used; ++i) {
-    const ResidentEntry& e = table[i];
-    if (e.dev == dev && e.kern == kern && e.threads == threads && e.smem == smem) return e.n;
-  }
+  if (const int* n = cache.find(dev, kern, threads, smem)) return *n;
   int per_sm = 0;
   LES_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
   const int n = std::max(1, per_sm) * sm_count();
-  if (used < 256) table[used++] = ResidentEntry{dev, kern, threads, smem, n};
+  cache.put(dev, kern, threads, smem, n);
   return n;
 }
 
-
 // registers per thread and the largest CTA of `kern` on the current device
-// (fixed table, as above)
 KernelLimits kernel_limits(const void* kern) {
   static std::mutex mu;
-  static struct {
-    int dev;
-    const void* kern;
-    KernelLimits lim;
-  } table[128];
-  static int used = 0;
+  static LaunchCache<KernelLimits, LIMITS_CACHE> cache;
   int dev = 0;
   LES_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < used; ++i)
-    if (table[i].dev == dev && table[i].kern == kern) return table[i].lim;
+  if (const KernelLimits* l = cache.find(dev, kern, 0, 0)) return *l;
   cudaFuncAttributes fa;
   LES_CUDA(cudaFuncGetAttributes(&fa, kern));
   const KernelLimits lim{fa.numRegs, fa.maxThreadsPerBlock};
-  if (used < 128) table[used++] = {dev, kern, lim};
+  cache.put(dev, kern, 0, 0, lim);
   return lim;
 }
 
