@@ -455,11 +455,16 @@ int les_mlp_check_profile(les_state* s, double* out, int n);
  * the buffer's address and sets kernel attributes; make it before any stream
  * capture.  All calls share the buffer of their device: calls in flight at
  * the same time on one device race.  Asynchronous on `stream` (a
- * cudaStream_t; NULL is the default stream). */
+ * cudaStream_t; NULL is the default stream): what goes wrong on the device
+ * after that is told by les_noalloc_status. */
 #define LES_NOALLOC_SCRATCH_BYTES (32u << 20)
 int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx, int ny, int nlev, double lx, double ly,
                         void* stream);
 const char* les_noalloc_last_error(void);
+/* The current device's sticky status bits of les_grad_xy_noalloc, cleared on
+ * read (synchronises `stream`): 32 a bulk-copy wait ran out and a part of the
+ * outputs of a call was not written; 0 otherwise. */
+int les_noalloc_status(unsigned* bits, void* stream);
 
 #ifdef __cplusplus
 }

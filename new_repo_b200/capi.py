@@ -138,6 +138,7 @@ PROTOTYPES = {
     "les_mlp_set_wall_levels": [_P, _I],
     "les_mlp_check_profile": [_P, _D, _I],
     "les_grad_xy_noalloc": [_P, _P, _P, _I, _I, _I, C.c_double, C.c_double, _P],
+    "les_noalloc_status": [C.POINTER(C.c_uint), _P],
 }
 
 _lib = None

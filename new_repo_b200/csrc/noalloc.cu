@@ -36,9 +36,12 @@ namespace {
 
 constexpr size_t kScratchBytes = LES_NOALLOC_SCRATCH_BYTES;
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
+__device__ unsigned g_noalloc_status;  // sticky status bits (les_noalloc_status)
 
 constexpr int kMaxDevices = 64;
-std::atomic<unsigned char*> g_scratch_addr[kMaxDevices] = {};  // per device, set by the first call on it
+// per device, set by the first call on it (the scratch last)
+std::atomic<unsigned char*> g_scratch_addr[kMaxDevices] = {};
+std::atomic<unsigned*> g_status_addr[kMaxDevices] = {};
 
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
@@ -133,7 +136,7 @@ struct PlaneGrad {
 
 template <int NX, int NY>
 __global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
-    k_grad_plane(double* f, double* dfdx, double* dfdy, cplx<double>* scratch, double lx, double ly) {
+    k_grad_plane(double* f, double* dfdx, double* dfdy, cplx<double>* scratch, unsigned* status, double lx, double ly) {
   using G = PlaneGrad<NX, NY>;
   constexpr bool TWO = G::two;
   using C = cplx<double>;
@@ -185,7 +188,8 @@ __global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
   twm_build<double, NY, true>(twy, myi, tid, TH);
   dep_wait();
   const bool late = !tc::mbar_wait(bar, 0);
-  if (__syncthreads_or(late)) {  // as in the spectral passes: a last bounded wait, leave
+  if (__syncthreads_or(late)) {  // as in the spectral passes: record it, a last bounded wait, leave
+    if (tid == 0) atomicOr(status, unsigned(ST_COPY_WAIT));
     tc::mbar_wait(bar, 0);
     return;
   }
@@ -327,7 +331,7 @@ __global__ void __launch_bounds__(PlaneGrad<NX, NY>::threads)
 
 // the plane kernel of a grid (nullptr: none)
 struct PlaneKernel {
-  void (*run)(double*, double*, double*, cplx<double>*, double, double) = nullptr;
+  void (*run)(double*, double*, double*, cplx<double>*, unsigned*, double, double) = nullptr;
   int threads = 0;
   size_t smem = 0;
   bool two = false;
@@ -391,6 +395,10 @@ int scratch_for_device(unsigned char** out) {
           LES_CUDA(cudaFuncSetAttribute((const void*)k.run, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem)));
       }
     addr = static_cast<unsigned char*>(p);
+    e = cudaGetSymbolAddress(&p, g_noalloc_status);
+    if (e != cudaSuccess)
+      throw CudaError(LES_ERR_INVALID, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
+    g_status_addr[dev].store(static_cast<unsigned*>(p));
     g_scratch_addr[dev].store(addr);
   }
   *out = addr;
@@ -405,6 +413,33 @@ thread_local char g_noalloc_error[256];
 }
 
 extern "C" const char* les_noalloc_last_error(void) { return g_noalloc_error; }
+
+extern "C" int les_noalloc_status(unsigned* bits, void* stream) {
+  using namespace les;
+  g_noalloc_error[0] = '\0';
+  auto fail = [](const char* msg) {
+    std::snprintf(g_noalloc_error, sizeof(g_noalloc_error), "%s", msg);
+    return LES_ERR_INVALID;
+  };
+  if (!bits) return fail("les_noalloc_status: null argument");
+  *bits = 0;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev < 0 || dev >= kMaxDevices)) return fail("device ordinal out of range");
+  if (e == cudaSuccess) {
+    unsigned* const word = g_status_addr[dev].load();
+    if (!word) return LES_OK;  // no call on this device yet
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    e = cudaMemcpyAsync(bits, word, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(word, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  if (e != cudaSuccess) {
+    std::snprintf(g_noalloc_error, sizeof(g_noalloc_error), "%s", cuda_error_text("les_noalloc_status", e).c_str());
+    return cuda_status_code(e);
+  }
+  return LES_OK;
+}
 
 extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx, int ny, int nlev, double lx,
                                    double ly, void* stream) {
@@ -442,11 +477,11 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
   int rc = LES_OK;
   try {
     unsigned char* base = nullptr;
-    scratch_for_device(&base);
+    unsigned* const status = g_status_addr[scratch_for_device(&base)].load();
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (const PlaneKernel pk = plane_kernel(nx, ny); plane_form(pk, nlev)) {
       auto* ys = reinterpret_cast<cplx<double>*>(base + L.spec[0]);
-      launch_dep(pk.run, nlev, pk.threads, pk.smem, st, f, dfdx, dfdy, ys, lx, ly);
+      launch_dep(pk.run, nlev, pk.threads, pk.smem, st, f, dfdx, dfdy, ys, status, lx, ly);
       LES_CHECK_LAUNCH();
       g_hook = saved;
       return rc;
@@ -464,6 +499,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     XFArgs<double> a;
     std::memset(&a, 0, sizeof(a));
     a.op = XF_SCALE;
+    a.status = status;
     a.nf = 1;
     a.rows_pp = ny;
     a.nrows = (long)nlev * ny;
@@ -503,6 +539,7 @@ extern "C" int les_grad_xy_noalloc(double* f, double* dfdx, double* dfdy, int nx
     std::memset(&c, 0, sizeof(c));
     c.dep = 1;
     c.op = XI_STORE;
+    c.status = status;
     c.nin = 3;
     c.rows_pp = ny;
     c.nrows = (long)nlev * ny;
