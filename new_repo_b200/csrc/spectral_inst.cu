@@ -101,6 +101,10 @@ int length_index(int n) {  // of a supported length
 #undef LI
   throw CudaError(1, "no FFT plan for length " + std::to_string(n));
 }
+// done already: type, device, use, direction, length (not inside the template,
+// whose statics two copies of the library in one process would share)
+std::mutex g_init_mutex;
+bool g_init_done[2][256][3][2][12];
 }  // namespace
 
 // cudaFuncSetAttribute applies to the current device only, and loads the
@@ -112,14 +116,13 @@ int length_index(int n) {  // of a supported length
 // 58 ms, 23 to 30 ms with uncompressed device code, see build.py.)
 template <typename T>
 void init_spectral_attributes(SpectralUse use, int nx, int ny) {
-  static std::mutex mu;
-  static bool done[256][3][2][12];  // device, use, direction, length
   int dev = 0;
   LES_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 256) throw CudaError(1, "device ordinal out of range");
-  bool& dx = done[dev][use][0][length_index(nx)];
-  bool& dy = done[dev][use][1][length_index(ny)];
-  std::lock_guard<std::mutex> lock(mu);
+  auto& done = g_init_done[std::is_same<T, double>::value][dev][use];
+  bool& dx = done[0][length_index(nx)];
+  bool& dy = done[1][length_index(ny)];
+  std::lock_guard<std::mutex> lock(g_init_mutex);
   if (!dx) {
     set_attrs_xfwd<T>(use, nx);
     if (use != SU_PRESSURE) set_attrs_xinv<T>(use, nx);
