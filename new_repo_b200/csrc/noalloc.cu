@@ -108,10 +108,10 @@ __global__ void k_noalloc_tables(double* kkx, double* kky, cplx<double>* twx, cp
 // buffer, which L2 holds.  The twiddles and wavenumbers are computed by the
 // CTA, so the call needs no table launch.  Small planes are bound by launches
 // and latency, which the four launches of the three-pass form pay four times,
-// larger ones by shared memory, ~25 accesses per value.  Three passes against
-// this, us: 16 x 16 x 100 26.6 / 6.2, 64 x 64 x 148 41 / 12.3, 96 x 64 x 100 41
-// / 16.4, 128 x 64 x 159 (two waves) 61 / 34, 128 x 128 x 79 54 / 37; with
-// dependent launches 4.2, 10.3, 13.8, 31.8 and 49 / 34.4.
+// larger ones by shared memory, ~25 accesses per value.  us, three passes / this:
+// 16 x 16 x 100 26.6 / 6.2, 64 x 64 x 148 41 / 12.3, 96 x 64 x 100 41 / 16.4, 128
+// x 64 x 159 (two waves) 61 / 34, 128 x 128 x 79 54 / 37; with dependent launches
+// 16.4 / 4.0, 39 / 10.3, 33 / 13.8, 51 / 31.8 and 45 / 34.4.
 template <int NX, int NY>
 struct PlaneGrad {
   static constexpr int M = NX / 2;
@@ -132,6 +132,14 @@ struct PlaneGrad {
   static constexpr bool two = 2 * array + tables <= cap;
   static constexpr size_t smem = (two ? 2 : 1) * array + tables;
   static_assert(smem <= cap, "plane beyond shared memory");
+  // Levels from which the plane form is the faster one.  One wave of CTAs takes
+  // the same time at any number of levels, three passes of few levels a launch's
+  // time each: planes of up to 8192 points and 192 x 64 win at any number (us,
+  // plane / three passes: 128 x 64 x 1 16.0 / 20.5, 64 x 128 x 1 17.4 / 18.5, 192
+  // x 64 x 2 25.7 / 25.7), the larger ones where three passes grow past them: 128
+  // x 128 x 42 34.3 / 30.8, x 44 34.3 / 34.8; 256 x 64 x 29 29.0 / 26.7, x 30 29.0
+  // / 30.2; 96 x 128 x 28 25.4 / 24.6, x 30 25.4 / 25.5.
+  static constexpr int from = NX * NY <= 8192 || NX == 192 ? 1 : NX == 128 ? 44 : 30;
 };
 
 template <int NX, int NY>
@@ -334,12 +342,12 @@ struct PlaneKernel {
   void (*run)(double*, double*, double*, cplx<double>*, unsigned*, double, double) = nullptr;
   int threads = 0;
   size_t smem = 0;
-  bool two = false;
+  int from = 0;
 };
 template <int NX, int NY>
 PlaneKernel plane_kernel_of() {
   using G = PlaneGrad<NX, NY>;
-  return {k_grad_plane<NX, NY>, G::threads, G::smem, G::two};
+  return {k_grad_plane<NX, NY>, G::threads, G::smem, G::from};
 }
 template <int NX>
 PlaneKernel plane_kernel_ny(int ny) {
@@ -368,11 +376,8 @@ PlaneKernel plane_kernel(int nx, int ny) {
   }
 }
 
-// Whether a call of nlev levels takes the plane form: always where two arrays
-// fit.  The largest planes take one CTA as long as few levels take the whole
-// chip in three passes, us: 128 x 128 x 24 34.2 / 28.7, x 40 34.3 / 32.8, x 50
-// 34.3 / 36.9; 256 x 64 x 24 28.8 / 28.7, x 40 28.9 / 32.8.
-bool plane_form(const PlaneKernel& k, int nlev) { return k.run && (k.two || nlev >= 40); }
+// whether a call of nlev levels takes the plane form
+bool plane_form(const PlaneKernel& k, int nlev) { return k.run && nlev >= k.from; }
 
 // address of this device's scratch buffer; the first call on a device does
 // the setup (symbol address, kernel shared-memory attributes)
