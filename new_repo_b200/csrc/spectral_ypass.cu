@@ -117,8 +117,16 @@ void launch_ypass(int NY, int NYO, YPArgs<T> a, int nplanes, int ngroups, cudaSt
   if (nitems == 0) return;
   // persistent grid: the CTAs that fit on the device at once
   const int grid = int(std::min<long>(nitems, (long)resident_ctas((const void*)kern, threads, smem)));
-  hook_before("ypass", double(nplanes) * ngroups * a.ncols * sizeof(cplx<T>) *
-                           (double(a.op == YP_PGRAD ? 1 : a.nin) * NY + double(a.nout) * NYO));
+  // columns written: an output may be left out, the narrower filter has fewer,
+  // the wall law's is one plane, the boundary layers add one
+  double ocols = 0.0;
+  for (int q = 0; q < ngroups * a.nout; ++q)
+    if (a.out[q]) ocols += double(nplanes) * (a.op == YP_FILTER2 && q % a.nout == 1 ? a.ncols1 : a.ncols);
+  if (a.op == YP_GRADY)
+    for (int q = 0; q < std::min(ngroups, 2); ++q) ocols += a.wall[q] ? a.ncols1 : 0;
+  if (a.op == YP_PRESS) ocols += a.ncols;
+  hook_before("ypass", sizeof(cplx<T>) * (double(nplanes) * ngroups * a.ncols * (a.op == YP_PGRAD ? 1 : a.nin) * NY +
+                                          ocols * NYO));
   if (a.dep) launch_dep(kern, grid, threads, smem, st, a);
   else kern<<<grid, threads, smem, st>>>(a);
   LES_CHECK_LAUNCH();
