@@ -672,8 +672,8 @@ __device__ __forceinline__ void tc_weights(TrainSmem& TS, bool first) {
 }
 
 __global__ void __launch_bounds__(TRAIN_THREADS) k_mlp_train(MlpDevice m, const float* X, const float* Tg, long n,
-                                                             float inv_n, float* y_out, float* loss,
-                                                             unsigned* status, MlpPerm pm) {
+                                                             float inv_n, float* y_out, unsigned* status,
+                                                             MlpPerm pm) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   TrainSmem& TS = *reinterpret_cast<TrainSmem*>(smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023));
   MlpSmem& S = TS.s;
@@ -1025,7 +1025,7 @@ void mlp_grad(MlpDevice& m, const float* x, const float* t, long n, float* y_out
   const long ntiles = (n + TILE - 1) / TILE;
   const int grid = int(std::max<long>(1, std::min<long>(ntiles, (long)MLP_TRAIN_CTAS)));
   hook_before("k_mlp_train", double(n) * 36.0);
-  launch_dep(k_mlp_train, grid, TRAIN_THREADS, train_smem(), st, m, x, t, n, 1.0f / float(n), y_out, loss_dev, status, perm);
+  launch_dep(k_mlp_train, grid, TRAIN_THREADS, train_smem(), st, m, x, t, n, 1.0f / float(n), y_out, status, perm);
   LES_CHECK_LAUNCH();
   hook_after();
   hook_before("k_mlp_grad_reduce", double(grid + 1) * MLP_NP * 4.0);

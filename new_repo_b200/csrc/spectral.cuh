@@ -137,7 +137,7 @@ struct XFArgs {
   double c0, c1, c2, c3;
   double rc1;      // XF_PRESS: 1 / c1
   const T* in[16];
-  const float* inf[16];  // FP32 inputs of an FP64 transform (in_f32 = 1)
+  const float* inf[16];  // FP32 inputs of an FP64 transform (in_f32 = 1; whole rows only)
   int in_f32;
   cplx<T>* out[MAXIN];
   long out_pstride;  // rows_pp * nk
@@ -263,10 +263,7 @@ __device__ __forceinline__ void xf_load_op(const XFArgs<T>& a, int l, int j, int
     else vst(v + f * vs, x);
   };
   {
-    if constexpr (OP == XF_SCALE) {
-      for (int f = 0; f < a.nf; ++f)
-        put(f, T(a.c0) * (a.in_f32 ? vldg<V>(a.inf[f], off) : vldg<V>(a.in[f], off)));
-    } else if constexpr (OP == XF_CONV_IN) {
+    if constexpr (OP == XF_CONV_IN) {
       // compute_convective_padd.f90:133-165
       const T c = T(a.c0);
       put(0, -c * vldg<V>(a.in[0], off));
@@ -434,7 +431,6 @@ __device__ __forceinline__ void xf_load_op(const XFArgs<T>& a, int l, int j, int
 template <typename T, typename V>
 __device__ __forceinline__ void xf_load(const XFArgs<T>& a, int l, int j, int i, T* v, int vs) {
   switch (a.op) {
-    case XF_SCALE: xf_load_op<T, V, XF_SCALE, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_CONV_IN: xf_load_op<T, V, XF_CONV_IN, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_PROD: xf_load_op<T, V, XF_PROD, false>(a, l, j, i, v, vs, nullptr); break;
     case XF_LASD: xf_load_op<T, V, XF_LASD, false>(a, l, j, i, v, vs, nullptr); break;
@@ -527,7 +523,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
     else load_rows(op_c, std::false_type{});
   };
   switch (a.op) {
-    case XF_SCALE: load_op(std::integral_constant<int, XF_SCALE>{}); break;
     case XF_CONV_IN: load_op(std::integral_constant<int, XF_CONV_IN>{}); break;
     case XF_PROD: load_op(std::integral_constant<int, XF_PROD>{}); break;
     case XF_LASD: load_op(std::integral_constant<int, XF_LASD>{}); break;
@@ -1442,8 +1437,6 @@ struct XIArgs {
   int adv_ghosts;
   double adv_dt, adv_t1, adv_t2, adv_top;
   T* out[16];
-  float* outf[16];  // FP32 outputs of an FP64 transform (out_f32 = 1, XI_STORE)
-  int out_f32;
   const T* aux[8];
   const cplx<T>* tw;  // exp(-2 pi i m / NX), m < NX
   // several transforms of one staged row: nstage rows per grid row are
@@ -1806,17 +1799,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
         const cplx<T> sg2 = {sg, sg};
         const long off = (long)l * a.out_pstride + (long)j * NX;
         // the store form is chosen once per sequence (outside the unrolled loop)
-        auto store = [&](auto form_c) {
-          constexpr int FORM = decltype(form_c)::value;
+        auto store = [&](auto pair_c) {
 #pragma unroll
           for (int gg = 0; gg < E / RO; ++gg)
 #pragma unroll
             for (int rr = 0; rr < RO; ++rr) {
               const int m = lane_t + TL * gg + rr * (M / RO);
               const cplx<T> z = c_fma(v[gg * RO + rr], sg2, ref2);
-              if constexpr (FORM == 0) {
-                *reinterpret_cast<float2*>(a.outf[f] + off + 2 * m) = make_float2(float(z.x), float(z.y));
-              } else if constexpr (FORM == 1) {
+              if constexpr (decltype(pair_c)::value) {
                 // one 8-byte (FP32) / 16-byte (FP64) store per output pair
                 *reinterpret_cast<cplx<T>*>(a.out[f] + off + 2 * m) = z;
               } else {
@@ -1825,9 +1815,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (NX <= 256 ? 4 : 3) : 2)
               }
             }
         };
-        if (a.out_f32) store(std::integral_constant<int, 0>{});
-        else if (a.pair_store) store(std::integral_constant<int, 1>{});
-        else store(std::integral_constant<int, 2>{});
+        if (a.pair_store) store(std::true_type{});
+        else store(std::false_type{});
       }
     } else {
       __syncwarp();

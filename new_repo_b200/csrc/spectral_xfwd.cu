@@ -57,16 +57,13 @@ void launch_xfwd(int NX, XFArgs<T> a, cudaStream_t st) {
   const int nin = a.op == XF_SCALE ? a.nf : nin_of_op[a.op];
   const size_t isz = (a.in_f32 ? sizeof(float) : sizeof(T));
   hook_before("xfwd", double(a.nrows) * NX * nin * isz + double(a.nrows) * (press ? 2 : a.nf) * a.nk * sizeof(cplx<T>));
-  // whole rows go by bulk copies, which want 16-byte aligned rows; XF_PRESS
-  // runs on the solver's own (aligned) fields only
-  bool rows = press || a.op == XF_SCALE;
-  for (int f = 0; f < (press ? 5 : a.nf) && rows; ++f) {
-    const void* q = a.in_f32 ? (const void*)a.inf[f] : (const void*)a.in[f];
-    rows = reinterpret_cast<uintptr_t>(q) % 16 == 0;
-  }
-  rows = rows && (isz * a.in_pstride) % 16 == 0 && (isz * NX) % 16 == 0;
-  if (press && !rows) throw CudaError(1, "xfwd: pressure inputs not 16-byte aligned");
-  if (rows) {
+  // scalings and the pressure take whole rows, which go by bulk copies: every
+  // caller's rows are 16-byte aligned
+  if (press || a.op == XF_SCALE) {
+    bool aligned = (isz * a.in_pstride) % 16 == 0 && (isz * NX) % 16 == 0;
+    for (int f = 0; f < (press ? 5 : a.nf); ++f)
+      aligned = aligned && reinterpret_cast<uintptr_t>(a.in_f32 ? (const void*)a.inf[f] : (const void*)a.in[f]) % 16 == 0;
+    if (!aligned) throw CudaError(1, "xfwd: input rows not 16-byte aligned");
     if (a.in_f32) {
       if constexpr (std::is_same<T, double>::value) launch_xfwd_row<T, float>(NX, a, st);
       else throw CudaError(1, "xfwd: FP32 inputs are for FP64 transforms");

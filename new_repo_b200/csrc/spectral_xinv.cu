@@ -109,14 +109,13 @@ void launch_xinv(int NX, XIArgs<T> a, cudaStream_t st) {
   if (nitems == 0) return;
   const int grid = int(std::min<long>(nitems, (long)resident_ctas((const void*)kern, 256, smem)));
   {
-    const size_t osz = (a.out_f32 ? sizeof(float) : sizeof(T));
     int rows = 0, vals = a.nin;  // spectral rows read (a spectrum staged at two levels once), values read and written
     for (int f = 0; f < ns; ++f) rows += std::find(a.in, a.in + f, a.in[f]) == a.in + f;
     if (a.op == XI_DIV)  // tz and rhs, the old rhs unless fresh; with the advance the variable twice and the last rhs
       for (int q = 0; q < a.nin; ++q) vals += 1 + (a.fresh ? 0 : 1) + (a.adv_v[q] ? 3 : 0);
     else if (a.op == XI_LASD || a.op == XI_SCDYN) vals = 2;
     else if (a.op == XI_WALL) vals = 7;
-    hook_before("xinv", double(a.nrows) * rows * a.nk * sizeof(cplx<T>) + double(a.nrows) * NX * vals * osz);
+    hook_before("xinv", double(a.nrows) * rows * a.nk * sizeof(cplx<T>) + double(a.nrows) * NX * vals * sizeof(T));
   }
   if (a.dep) launch_dep(kern, grid, 256, smem, st, a);
   else kern<<<grid, 256, smem, st>>>(a);
