@@ -114,9 +114,11 @@ inline std::string cuda_error_text(const char* call, cudaError_t e) {
 // whole of it and its memory to settle, and calls dep_wait() before it reads or
 // writes anything that another kernel touches.  What stays outside (constant
 // tables, shared-memory set-up, the launch itself) overlaps the end of the
-// kernel in front; a launch of any other kind waits as usual.  Kernel arguments
-// that point to changing data carry no const __restrict__ here: such loads may
-// be moved in front of the wait.  (Letting the next launch start earlier, as
+// kernel in front; a launch of any other kind waits as usual.  Pointers to
+// changing data carry no const __restrict__ in such a kernel: loads through them
+// may be moved in front of the wait.  (The x passes' read-only loads, vldg in
+// spectral.cuh, are safe: their addresses come from shared memory that is
+// filled and synchronised after the wait.)  (Letting the next launch start earlier, as
 // soon as all blocks of this one run, slowed large grids: its waiting blocks
 // take the room of running ones.)  Per step, us, plain / so / early: 32 x 32 x
 // 16 196 / 155 / 175, 64^3 mixed 249 / 206 / 232, 128^3 FP64 1256 / 1226 / 1328,

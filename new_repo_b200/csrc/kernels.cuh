@@ -575,7 +575,7 @@ __global__ void k_lag_interp(const T* ul, const T* vl, const T* wl, const T* F0,
     T v[4][8];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const T* __restrict__ F = Fs[t];
+      const T* F = Fs[t];
       v[t][0] = F[n000];
       v[t][1] = F[n00z];
       v[t][2] = F[n0y0];
