@@ -2512,9 +2512,12 @@ class Solver final : public SolverBase {
       Tag tag_(this, "finish");
       // the diagnostics ride along in FP64 and on small grids (one launch
       // less); in FP32 their FP64 sums cost more registers (106 against 32)
-      // than the three field reads they save: apart 0.29, together 0.38 ms at
-      // 256^3
-      const bool ride = with_diag && (!mixed() || g.field() <= (4L << 20));
+      // than the three field reads they save.  A step, us, together / apart:
+      // FP64 32 x 32 x 16 132 / 131, 128 x 64 x 41 270 / 275, 128^3 964 / 967,
+      // 256^3 6217 / 6234, 512 x 512 x 96 10725 / 10759; mixed 32 x 32 x 16 121 /
+      // 121, 64^3 194 / 193, 128 x 128 x 64 387 / 380, 128^3 646 / 634, 256^3
+      // 3577 / 3468
+      const bool ride = with_diag && (!mixed() || g.field() <= (1L << 19));
       const double fields = (mixed() ? 11.0 + 6.0 : 9.0 + 7.0) + (ride ? 3.0 : 0.0);
       auto run = [&](auto diag_c) {
         constexpr bool DIAG = decltype(diag_c)::value;
