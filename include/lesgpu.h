@@ -158,7 +158,8 @@ int les_press_stag_array(les_state* s, double tadv1);
  * against increments ~ dt rhs), so the transforms run in the state's
  * precision (the kx = ky = 0 column from FP64 plane means).  les_step keeps
  * the reference's formulation.  Preconditions: rhs, rhs_f and the gradients
- * unchanged since the advance, w(nz+1) = 0. */
+ * unchanged since the advance, w(nz+1) = 0.  The first call on a state
+ * allocates the scratch of its sweep (24 bytes per mode and level). */
 int les_press_from_increment(les_state* s, double tadv1, double tadv2);
 /* z-slab decomposition of the pressure solve, emulated on this GPU: with
  * nslabs > 1 the tridiagonal systems of press_stag_array (and of les_step)
@@ -288,7 +289,9 @@ int les_checkpoint_read(les_state* s, const char* path, int lagran_init);
  * sums.  out_path is prefixed as is (the reference's trim(out_path)).  The
  * caller applies the driver's condition stat_flag .and. jt_total >
  * start_stats (LES_engine.f90:368-370).  les_stat_sums copies sum index
- * 0..25 (nx*ny*nz values) or 26 (the u* plane) to the host.
+ * 0..25 (nx*ny*nz values) or 26 (the u* plane) to the host.  A call that
+ * writes no file returns when its work is queued on the state's stream, as the
+ * operators do; les_stat_sums and les_sync wait for it.
  * les_stat_spectra replaces io_stat_spectra (:566-620): inside the four
  * fixed jt_total windows and every 10th jt it writes
  * <out_path>SP_<jt_total:09>.dat with u, v, w on levels 1..nz.
@@ -311,7 +314,8 @@ int les_stat_spectra(les_state* s, int jt, int jt_total, const char* out_path);
  * pdwdz pdwdx pdudz) and, when mod(jt, tke_period) == 0, writes record ii
  * (nz FP64 values at byte offset (ii-1)*8*nz: direct access with recl = 2*nz
  * in 4-byte units) of ta1_profiles/<name>.out holding profile / tke_period,
- * then restarts the profiles and advances ii.  The caller applies
+ * then restarts the profiles and advances ii.  A call that writes no record
+ * returns when its work is queued (les_tke_sums and les_sync wait for it).  The caller applies
  * tke_flag .and. jt_total > start_tke (LES_engine.f90:377-380).
  * les_tke_sums copies the 61 x nz profiles (name-major) and the next record
  * number.  Errors: 1 not initialised / invalid period, 22 file open or write. */
@@ -418,7 +422,10 @@ int les_mlp_fit_stats(les_state* s);
  * last batch loss of each epoch, val_loss the validation loss (or -1) */
 int les_mlp_train(les_state* s, int epochs, int tiles_per_step, double lr, double* loss_epochs,
                   double* val_loss);
-/* network output (normalised units) for n host feature rows x[n][8] */
+/* network output (normalised units) for n host feature rows x[n][8].  The
+ * state keeps the device memory of this call's and the next one's rows (36 to
+ * 40 bytes each) for later calls, up to 64 MB in all, until it is destroyed; a
+ * larger call's is freed when it returns. */
 int les_mlp_forward(les_state* s, const float* x, long n, float* y);
 /* gradient of mean((y - t)^2) over n host rows into grad[LES_MLP_NPARAM] */
 int les_mlp_grad(les_state* s, const float* x, const float* t, long n, float* grad, float* loss);

@@ -121,8 +121,8 @@ inline std::string cuda_error_text(const char* call, cudaError_t e) {
 // filled and synchronised after the wait.)  (Letting the next launch start earlier, as
 // soon as all blocks of this one run, slowed large grids: its waiting blocks
 // take the room of running ones.)  Per step, us, plain / so / early: 32 x 32 x
-// 16 196 / 155 / 175, 64^3 mixed 249 / 206 / 232, 128^3 FP64 1256 / 1226 / 1328,
-// 256^3 mixed 3994 / 3935 / 4355.
+// 16 196 / 153 / 175, 64^3 mixed 249 / 207 / 232, 128^3 FP64 1256 / 1215 / 1328,
+// 256^3 mixed 3994 / 3912 / 4355.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
