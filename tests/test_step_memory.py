@@ -22,12 +22,15 @@ OPTIONS = {
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("option", OPTIONS)
 def test_steps_leave_free_memory_as_it_is(gpu, option, precision):
+    import gc
+
     import torch
 
     from new_repo_b200 import LES, RunParams, log_law_noise
 
     p = RunParams(nx=16, ny=16, nz=600, dt=1e-5, lbc_dz0=1e-4, pfx=1.0, cs_count=2, dyn_init=1,
                   sgs_model="dyn_Smag" if option == "dyn_Smag" else "cst_Smag")
+    gc.collect()  # states that earlier tests left behind
     free = []
     for _ in range(2):  # the first state loads the kernels
         les = LES(p, precision=precision)
